@@ -130,7 +130,7 @@ template <> struct Idx<float> {
     }
 };
 
-// Warp sum of a double over the lanes that share (lane mod stride).
+// Warp sum of a double over the lanes that share (lane mod stride); stride 32: v itself.
 __device__ __forceinline__ double warp_sum_strided(double v, int stride)
 {
     for (int o = 16; o >= stride; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

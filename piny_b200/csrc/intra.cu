@@ -18,20 +18,33 @@
 
 namespace pinyb200 {
 
-// Block-level reduction of per-thread energy/virial sums by bead: shared
-// FP64 atomics (S_NSLOT slots per bead), then one global atomic per (bead,
-// slot) per block.  Every thread of the block must call it.
+// Per-thread energy/virial sums v of a 256-thread block, thread t holding
+// bead t % P (P a power of two up to 64), added to acc[bead][slot]: lanes of
+// one bead by shuffles, then the block's warps through shared memory, then
+// one global atomic per (bead, slot).  Every thread of the block must call
+// it.  (Shared FP64 atomics instead of the shuffles serialise: with one bead
+// all 256 threads of a block met at 7 addresses, and each of the three
+// intramolecular kernels took 35-41 us of the 256- and 4096-molecule boxes;
+// now 3-5 us.)
 template <int NV>
-__device__ __forceinline__ void block_acc(double *acc, int P, int b, const int *slot, const double *v, double *sh)
+__device__ __forceinline__ void block_acc(double *acc, int P, const int *slot, const double *v)
 {
-    for (int i = threadIdx.x; i < P * NV; i += blockDim.x) sh[i] = 0.0;
-    __syncthreads();
+    __shared__ double sh[NV][8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int G = P < 32 ? P : 32;
 #pragma unroll
-    for (int c = 0; c < NV; c++)
-        if (v[c] != 0.0) atomicAdd(&sh[b * NV + c], v[c]);
+    for (int c = 0; c < NV; c++) {
+        const double t = warp_sum_strided(v[c], G);
+        if (lane < G) sh[c][w][lane] = t;
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < P * NV; i += blockDim.x)
-        if (sh[i] != 0.0) atomicAdd(&acc[(size_t)(i / NV) * S_NSLOT + slot[i % NV]], sh[i]);
+    const int wstep = P > 32 ? P / 32 : 1;  // warps w, w + wstep, ... hold the same beads
+    for (int i = threadIdx.x; i < P * NV; i += blockDim.x) {
+        const int c = i / P, b = i - c * P;
+        double t = 0.0;
+        for (int k = b >> 5; k < 8; k += wstep) t += sh[c][k][b & 31];
+        if (t != 0.0) atomicAdd(&acc[(size_t)b * S_NSLOT + slot[c]], t);
+    }
 }
 
 // out[c][r] = in[r][c] for an rows x cols matrix of doubles, through a
@@ -151,7 +164,6 @@ __device__ __forceinline__ void bond_body(const IntraArgs &a, int nbond, const i
                                                    const double *__restrict__ eq, const double *__restrict__ cc,
                                                    const double *__restrict__ dc, const VBlk vb)
 {
-    __shared__ double sh[64 * 7];
     const long long t0 = (long long)vb.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)vb.gx * blockDim.x;  // a multiple of P
     const int b = (int)(t0 % a.P);
@@ -177,7 +189,7 @@ __device__ __forceinline__ void bond_body(const IntraArgs &a, int nbond, const i
     if (a.energy) {
         const int slot[7] = {S_VBOND, S_PXX, S_PYY, S_PZZ, S_PXY, S_PXZ, S_PYZ};
         const double vals[7] = {v, p[0], p[1], p[2], p[3], p[4], p[5]};
-        block_acc<7>(a.acc, a.P, b, slot, vals, sh);
+        block_acc<7>(a.acc, a.P, slot, vals);
     }
 }
 
@@ -240,7 +252,6 @@ __device__ __forceinline__ void bend_body(const IntraArgs &a, int nbend, const i
                                                    const double *__restrict__ bc, const double *__restrict__ bs,
                                                    const double *__restrict__ bdc, const double *__restrict__ bds, const VBlk vb)
 {
-    __shared__ double sh[64 * 7];
     const long long t0 = (long long)vb.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)vb.gx * blockDim.x;  // a multiple of P
     const int b = (int)(t0 % a.P);
@@ -264,7 +275,7 @@ __device__ __forceinline__ void bend_body(const IntraArgs &a, int nbend, const i
     if (a.energy) {
         const int slot[7] = {S_VBEND, S_PXX, S_PYY, S_PZZ, S_PXY, S_PXZ, S_PYZ};
         const double vals[7] = {v, p[0], p[1], p[2], p[3], p[4], p[5]};
-        block_acc<7>(a.acc, a.P, b, slot, vals, sh);
+        block_acc<7>(a.acc, a.P, slot, vals);
     }
 }
 
@@ -279,7 +290,6 @@ __device__ __forceinline__ void ecor_body(const IntraArgs &a, int necor, const i
                                                    const int *__restrict__ j2s, int nsplin, double rmin, double dr,
                                                    double dri, const double4 *__restrict__ tab, const VBlk vb)
 {
-    __shared__ double sh[64 * 7];
     const long long t0 = (long long)vb.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)vb.gx * blockDim.x;  // a multiple of P
     const int b = (int)(t0 % a.P);
@@ -308,7 +318,7 @@ __device__ __forceinline__ void ecor_body(const IntraArgs &a, int necor, const i
     if (a.energy) {
         const int slot[7] = {S_VECOR, S_PXX, S_PYY, S_PZZ, S_PXY, S_PXZ, S_PYZ};
         const double vals[7] = {v, p[0], p[1], p[2], p[3], p[4], p[5]};
-        block_acc<7>(a.acc, a.P, b, slot, vals, sh);
+        block_acc<7>(a.acc, a.P, slot, vals);
     }
 }
 

@@ -948,6 +948,24 @@ __device__ __noinline__ void mol_pair_near(const double *__restrict__ posT, cons
     }
 }
 
+// A 128-thread block's energy and virial sums (sacc[k][t], thread t holding
+// bead t % G) added to acc[bead][slot], summed over the block first: an
+// atomic per bead, sum and block instead of one per warp (or lane group).
+// Every thread of the block must call it.
+template <int G>
+__device__ __forceinline__ void pair_energy_flush(const double (*sacc)[128], double *acc)
+{
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int c = threadIdx.x >> 5; c < 8; c += 4) {
+        double t = (sacc[c][lane] + sacc[c][lane + 32]) + (sacc[c][lane + 64] + sacc[c][lane + 96]);
+        if (G < 32) t = warp_sum_strided(t, G);
+        // sums 0, 1: S_VVDW, S_VCOUL; 2..7: S_PXX..S_PYZ
+        if (lane < G && t != 0.0) atomicAdd(&acc[(size_t)lane * S_NSLOT + (c < 2 ? S_VVDW + c : S_PXX + c - 2)], t);
+    }
+}
+
 template <typename R, int P, int NS, bool FAST, bool ENERGY>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : PINYB200_MOL_BLOCKS64)
     mol_pair_kernel(MolArgs a, Cell cell)
@@ -1146,15 +1164,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
             for (int c = 0; c < 6; c++) sacc[2 + c][threadIdx.x] += (double)pvs[c];
         }
     }
-    if (ENERGY) {
-        const int slot[8] = {S_VVDW, S_VCOUL, S_PXX, S_PYY, S_PZZ, S_PXY, S_PXZ, S_PYZ};
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            double t = sacc[c][threadIdx.x];
-            if (G < 32) t = warp_sum_strided(t, G);
-            if (G == 32 || sub == 0) atomicAdd(&a.acc[(size_t)b * S_NSLOT + slot[c]], t);
-        }
-    }
+    if (ENERGY) pair_energy_flush<G>(sacc, a.acc + (size_t)32 * blockIdx.y * S_NSLOT);
 }
 
 // ---------------------------------------------------------------------------
@@ -1449,15 +1459,7 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
             for (int c = 0; c < 6; c++) sacc[2 + c][threadIdx.x] += (double)pvs[c];
         }
     }
-    if (ENERGY) {
-        const int slot[8] = {S_VVDW, S_VCOUL, S_PXX, S_PYY, S_PZZ, S_PXY, S_PXZ, S_PYZ};
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            double t = sacc[c][threadIdx.x];
-            if (G < 32) t = warp_sum_strided(t, G);
-            if (G == 32 || sub == 0) atomicAdd(&a.acc[(size_t)b * S_NSLOT + slot[c]], t);
-        }
-    }
+    if (ENERGY) pair_energy_flush<G>(sacc, a.acc + (size_t)32 * vb.y * S_NSLOT);
 }
 
 
