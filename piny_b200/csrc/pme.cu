@@ -33,6 +33,7 @@
 
 #include "boxtab.cuh"
 #include "common.cuh"
+#include "fft.cuh"
 
 namespace pinyb200 {
 
@@ -1234,30 +1235,9 @@ __device__ void smem_fft(typename Cplx<R>::T *sm, int N, int nl, int ls, int es,
     }
 }
 
-// FFT of length NF known at compile time (NF > 0), else run-time N.
-template <typename R, int NF>
-__device__ __forceinline__ void line_fft(typename Cplx<R>::T *sm, int N, int nl, int ls, int es, const R *tw, int sign)
-{
-    if constexpr (NF > 0) {
-        if (sign > 0) fft_pow2_inl<R, NF, 1>(sm, nl, ls, es, tw);
-        else fft_pow2_inl<R, NF, -1>(sm, nl, ls, es, tw);
-    } else {
-        smem_fft<R>(sm, N, nl, ls, es, tw, sign);
-    }
-}
-
-// Resident blocks per SM the FP32 plane and slab kernels of compile-time
-// length are compiled for (their registers: 65536 / (256 x this)); the
-// FP64 ones and the multi-box ones (whose run-time argument table costs
-// registers) hold 2.
-#ifndef PINYB200_FFT_BLOCKS
-#define PINYB200_FFT_BLOCKS 4
-#endif
-#ifndef PINYB200_PLANE_BLOCKS
-#define PINYB200_PLANE_BLOCKS PINYB200_FFT_BLOCKS  // the plane passes alone (their shared plane allows 6)
-#endif
-#define PINYB200_FFT_LB(R, NF) (NF > 0 ? (sizeof(R) == 4 ? PINYB200_FFT_BLOCKS : 2) : 1)
-#define PINYB200_PLANE_LB(R, NF) (NF > 0 ? (sizeof(R) == 4 ? PINYB200_PLANE_BLOCKS : 2) : 1)
+// Plane and slab kernels of meshes whose lengths are known only at run time
+// (not cubic, or an edge fft.cuh does not build): one complex line per real
+// row, every length from order to 256.
 
 template <typename R>
 __device__ __forceinline__ void load_twiddles(R *dst, const R *src, int N)
@@ -1267,12 +1247,11 @@ __device__ __forceinline__ void load_twiddles(R *dst, const R *src, int N)
 
 // Forward transform of one (bead, c) plane along a then b; half spectrum
 // (a <= Na/2) out.  Shared: plane [Nb][Na+1] complex, twiddles.
-template <typename R, int NF>
+template <typename R>
 __device__ __forceinline__ void plane_fwd_body(const R *__restrict__ q, typename Cplx<R>::T *__restrict__ spec, int Na,
                                                int Nb, int Nc, const R *__restrict__ twa, const R *__restrict__ twb,
                                                const VBlk vb)
 {
-    if (NF > 0) Na = Nb = NF;  // cubic power-of-two grid known at compile time
     (void)Nc;
     typedef typename Cplx<R>::T C2;
     extern __shared__ unsigned char smem_raw[];
@@ -1292,29 +1271,28 @@ __device__ __forceinline__ void plane_fwd_body(const R *__restrict__ q, typename
         pl[(idx / Na) * ls + idx % Na] = v;
     }
     __syncthreads();
-    line_fft<R, NF>(pl, Na, Nb, ls, 1, ta, +1);   // along a, every row
-    line_fft<R, NF>(pl, Nb, Nh, 1, ls, tb, +1);   // along b, columns a <= Na/2
+    smem_fft<R>(pl, Na, Nb, ls, 1, ta, +1);   // along a, every row
+    smem_fft<R>(pl, Nb, Nh, 1, ls, tb, +1);   // along b, columns a <= Na/2
     C2 *dst = spec + plane * (size_t)Nb * Nh;
     for (int idx = threadIdx.x; idx < Nb * Nh; idx += blockDim.x) dst[idx] = pl[(idx / Nh) * ls + idx % Nh];
 }
 
-template <typename R, int NF>
-__global__ void __launch_bounds__(256, PINYB200_PLANE_LB(R, NF)) plane_fwd_kernel(const R *__restrict__ q, typename Cplx<R>::T *__restrict__ spec,
+template <typename R>
+__global__ void __launch_bounds__(256) plane_fwd_kernel(const R *__restrict__ q, typename Cplx<R>::T *__restrict__ spec,
                                                         int Na, int Nb, int Nc, const R *__restrict__ twa,
                                                         const R *__restrict__ twb)
 {
-    plane_fwd_body<R, NF>(q, spec, Na, Nb, Nc, twa, twb, hw_blk());
+    plane_fwd_body<R>(q, spec, Na, Nb, Nc, twa, twb, hw_blk());
 }
 
 // Inverse of plane_fwd: half spectrum in, along b, Hermitian completion of
 // each row (U(Na-a) = conj U(a) once b and c are back in real space), along
 // a, real part out.
-template <typename R, int NF>
+template <typename R>
 __device__ __forceinline__ void plane_inv_body(const typename Cplx<R>::T *__restrict__ spec, R *__restrict__ phi, int Na,
                                                int Nb, int Nc, const R *__restrict__ twa, const R *__restrict__ twb,
                                                const VBlk vb)
 {
-    if (NF > 0) Na = Nb = NF;  // cubic power-of-two grid known at compile time
     (void)Nc;
     typedef typename Cplx<R>::T C2;
     extern __shared__ unsigned char smem_raw[];
@@ -1329,7 +1307,7 @@ __device__ __forceinline__ void plane_inv_body(const typename Cplx<R>::T *__rest
     const C2 *src = spec + plane * (size_t)Nb * Nh;
     for (int idx = threadIdx.x; idx < Nb * Nh; idx += blockDim.x) pl[(idx / Nh) * ls + idx % Nh] = src[idx];
     __syncthreads();
-    line_fft<R, NF>(pl, Nb, Nh, 1, ls, tb, -1);
+    smem_fft<R>(pl, Nb, Nh, 1, ls, tb, -1);
     for (int idx = threadIdx.x; idx < Nb * Na; idx += blockDim.x) {
         const int b = idx / Na, a = idx % Na;
         if (a >= Nh) {
@@ -1339,29 +1317,28 @@ __device__ __forceinline__ void plane_inv_body(const typename Cplx<R>::T *__rest
         }
     }
     __syncthreads();
-    line_fft<R, NF>(pl, Na, Nb, ls, 1, ta, -1);
+    smem_fft<R>(pl, Na, Nb, ls, 1, ta, -1);
     R *dst = phi + plane * Na * Nb;
     for (int idx = threadIdx.x; idx < Na * Nb; idx += blockDim.x) dst[idx] = pl[(idx / Na) * ls + idx % Na].x;
 }
 
-template <typename R, int NF>
-__global__ void __launch_bounds__(256, PINYB200_PLANE_LB(R, NF)) plane_inv_kernel(const typename Cplx<R>::T *__restrict__ spec, R *__restrict__ phi,
+template <typename R>
+__global__ void __launch_bounds__(256) plane_inv_kernel(const typename Cplx<R>::T *__restrict__ spec, R *__restrict__ phi,
                                                         int Na, int Nb, int Nc, const R *__restrict__ twa,
                                                         const R *__restrict__ twb)
 {
-    plane_inv_body<R, NF>(spec, phi, Na, Nb, Nc, twa, twb, hw_blk());
+    plane_inv_body<R>(spec, phi, Na, Nb, Nc, twa, twb, hw_blk());
 }
 
 // One (bead, b) slab of the half spectrum: FFT along c, energy and virial
 // of the k-sphere terms (ewald3d_pme.c:366-425), multiplication by the
 // influence function, inverse FFT along c.  Half-spectrum points with
 // 0 < a < Na/2 stand for two full-grid points; E = 1/2 sum_full w |S|^2.
-template <typename R, int NF>
+template <typename R>
 __device__ __forceinline__ void conv_c_body(typename Cplx<R>::T *__restrict__ spec, const R *__restrict__ filt, int Na,
                                             int Nb, int Nc, const R *__restrict__ twc, const Cell &cell, double alp,
                                             double *__restrict__ acc, int energy, const VBlk vb)
 {
-    if (NF > 0) Na = Nb = Nc = NF;  // cubic power-of-two grid known at compile time
     typedef typename Cplx<R>::T C2;
     extern __shared__ unsigned char smem_raw[];
     C2 *sl = (C2 *)smem_raw;
@@ -1378,7 +1355,7 @@ __device__ __forceinline__ void conv_c_body(typename Cplx<R>::T *__restrict__ sp
         sl[c * ls + a] = base[c * cstride + a];
     }
     __syncthreads();
-    line_fft<R, NF>(sl, Nc, Nh, 1, ls, tc, +1);
+    smem_fft<R>(sl, Nc, Nh, 1, ls, tc, +1);
     // per-point energy and virial terms in R (FP32 for MIXED), summed in FP64
     double e = 0, pxx = 0, pyy = 0, pzz = 0, pxy = 0, pxz = 0, pyz = 0;
     const R kb = (R)(b <= Nb / 2 ? b : b - Nb);
@@ -1412,7 +1389,7 @@ __device__ __forceinline__ void conv_c_body(typename Cplx<R>::T *__restrict__ sp
         sl[c * ls + a] = s;
     }
     __syncthreads();
-    line_fft<R, NF>(sl, Nc, Nh, 1, ls, tc, -1);
+    smem_fft<R>(sl, Nc, Nh, 1, ls, tc, -1);
     for (int idx = threadIdx.x; idx < Nc * Nh; idx += blockDim.x) {
         const int c = idx / Nh, a = idx % Nh;
         base[c * cstride + a] = sl[c * ls + a];
@@ -1440,13 +1417,13 @@ __device__ __forceinline__ void conv_c_body(typename Cplx<R>::T *__restrict__ sp
     }
 }
 
-template <typename R, int NF>
-__global__ void __launch_bounds__(256, PINYB200_FFT_LB(R, NF)) conv_c_kernel(typename Cplx<R>::T *__restrict__ spec, const R *__restrict__ filt,
+template <typename R>
+__global__ void __launch_bounds__(256) conv_c_kernel(typename Cplx<R>::T *__restrict__ spec, const R *__restrict__ filt,
                                                      int Na, int Nb, int Nc, const R *__restrict__ twc,
                                                      const __grid_constant__ Cell cell, double alp,
                                                      double *__restrict__ acc, int energy)
 {
-    conv_c_body<R, NF>(spec, filt, Na, Nb, Nc, twc, cell, alp, acc, energy, hw_blk());
+    conv_c_body<R>(spec, filt, Na, Nb, Nc, twc, cell, alp, acc, energy, hw_blk());
 }
 
 // ---------------------------------------------------------------------------
@@ -1489,30 +1466,30 @@ size_t pme_slab_smem(int Na, int Nc, bool fp64)
     return cs * (size_t)Nc * (Na / 2 + 2) + rs * 2 * (size_t)Nc;
 }
 
-// The three FFT kernels for grids of compile-time edge NF (0: run time).
-template <typename R, int NF>
-static cudaError_t launch_fft_t(pinyb200_ctx *c, const PmeArgs &a, const Cell &cell, typename Cplx<R>::T *spec,
+// The three FFT kernels for meshes of run-time lengths.
+template <typename R>
+static cudaError_t launch_fft_rt(pinyb200_ctx *c, const PmeArgs &a, const Cell &cell, typename Cplx<R>::T *spec,
                                 const R *filt, const R *const *tw, size_t sp, size_t ss, bool energy)
 {
     cudaError_t err = cudaSuccess;
     // opt in to more than 48 KB of dynamic shared memory where a plane needs it
     if (sp > 48 * 1024) {
-        err = smem_optin((const void *)plane_fwd_kernel<R, NF>, (int)sp);
+        err = smem_optin((const void *)plane_fwd_kernel<R>, (int)sp);
         if (err == cudaSuccess)
-            err = smem_optin((const void *)plane_inv_kernel<R, NF>, (int)sp);
+            err = smem_optin((const void *)plane_inv_kernel<R>, (int)sp);
         if (err != cudaSuccess) return err;
     }
     if (ss > 48 * 1024) {
-        err = smem_optin((const void *)conv_c_kernel<R, NF>, (int)ss);
+        err = smem_optin((const void *)conv_c_kernel<R>, (int)ss);
         if (err != cudaSuccess) return err;
     }
-    plane_fwd_kernel<R, NF><<<a.P * a.Nc, 256, sp, c->stream>>>((const R *)a.grid, spec, a.Na, a.Nb, a.Nc, tw[0],
+    plane_fwd_kernel<R><<<a.P * a.Nc, 256, sp, c->stream>>>((const R *)a.grid, spec, a.Na, a.Nb, a.Nc, tw[0],
                                                                 tw[1]);
     if ((err = kt_mark(c, "pme_plane_fwd")) != cudaSuccess) return err;
-    conv_c_kernel<R, NF><<<a.P * a.Nb, 256, ss, c->stream>>>(spec, filt, a.Na, a.Nb, a.Nc, tw[2], cell, c->alp_ewd,
+    conv_c_kernel<R><<<a.P * a.Nb, 256, ss, c->stream>>>(spec, filt, a.Na, a.Nb, a.Nc, tw[2], cell, c->alp_ewd,
                                                              c->d_acc, energy ? 1 : 0);
     if ((err = kt_mark(c, "pme_conv_c")) != cudaSuccess) return err;
-    plane_inv_kernel<R, NF><<<a.P * a.Nc, 256, sp, c->stream>>>(spec, (R *)a.grid, a.Na, a.Nb, a.Nc, tw[0], tw[1]);
+    plane_inv_kernel<R><<<a.P * a.Nc, 256, sp, c->stream>>>(spec, (R *)a.grid, a.Na, a.Nb, a.Nc, tw[0], tw[1]);
     if ((err = kt_mark(c, "pme_plane_inv")) != cudaSuccess) return err;
     return cudaGetLastError();
 }
@@ -1537,6 +1514,33 @@ static PmeArgs pme_args_of(pinyb200_ctx *c)
     a.rhead = (int4 *)c->d_pme_head;
     a.rw = c->d_pme_w;
     return a;
+}
+
+static FftArgs fft_args(void *grid, void *spec, const void *filt, const void *tw, const Cell &cell, pinyb200_ctx *c,
+                        bool energy)
+{
+    FftArgs f;
+    f.grid = grid;
+    f.spec = spec;
+    f.filt = filt;
+    f.tw = tw;
+    f.cell = cell;
+    f.alp = c->alp_ewd;
+    f.acc = c->d_acc;
+    f.energy = energy ? 1 : 0;
+    return f;
+}
+
+// Transforms, convolution and inverse transforms of one context's mesh: the
+// kernels of compile-time edge where built (every cubic mesh PINY chooses up
+// to 128^3), else those of run-time lengths.
+template <typename R>
+static cudaError_t launch_fft(pinyb200_ctx *c, const PmeArgs &a, const Cell &cell, typename Cplx<R>::T *spec,
+                              const R *filt, const R *const *tw, size_t sp, size_t ss, bool energy)
+{
+    if (fft_fixed_edge(a.Na, a.Nb, a.Nc))
+        return launch_fft_fixed<R>(c, a.Na, a.P, fft_args(a.grid, spec, filt, tw[0], cell, c, energy));
+    return launch_fft_rt<R>(c, a, cell, spec, filt, tw, sp, ss, energy);
 }
 
 // Tile binning arguments of a context's PME mesh for spline order NI and
@@ -1609,14 +1613,7 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy)
     const size_t sp = pme_plane_smem(a.Na, a.Nb, f64), ss = pme_slab_smem(a.Na, a.Nc, f64);
     C2 *spec = (C2 *)c->d_spec;
     const R *filt = f64 ? (const R *)c->d_filter : (const R *)((const double *)c->d_filter + G);
-    const bool cube = a.Na == a.Nb && a.Na == a.Nc;
-    switch (cube ? a.Na : 0) {
-    case 16: err = launch_fft_t<R, 16>(c, a, cell, spec, filt, tw, sp, ss, energy); break;
-    case 32: err = launch_fft_t<R, 32>(c, a, cell, spec, filt, tw, sp, ss, energy); break;
-    case 64: err = launch_fft_t<R, 64>(c, a, cell, spec, filt, tw, sp, ss, energy); break;
-    case 128: err = launch_fft_t<R, 128>(c, a, cell, spec, filt, tw, sp, ss, energy); break;
-    default: err = launch_fft_t<R, 0>(c, a, cell, spec, filt, tw, sp, ss, energy); break;
-    }
+    err = launch_fft<R>(c, a, cell, spec, filt, tw, sp, ss, energy);
     if (err != cudaSuccess) return err;
     if (full) gather_tile_kernel<R, NI, TT><<<tgrid, 256, st, c->stream>>>(a, cell, t);
     else gather_tile_c_kernel<R, NI, TT><<<tgrid, 256, st, c->stream>>>(a, cell, t);
@@ -1691,13 +1688,8 @@ struct PmeBox {
     Cell cell;
 };
 
-// Resident blocks per SM of the multi-box plane FFT passes and gather (their
-// run-time argument tables cost registers over the one-box kernels'): 3 and
-// 4 (80 and 64 registers, 16-36 bytes of spills) take the 64-box C4 step
-// from 5.56 to 5.36 ms against 2 and 1.
-#ifndef PINYB200_PLANE_BATCH_BLOCKS
-#define PINYB200_PLANE_BATCH_BLOCKS 3
-#endif
+// Resident blocks per SM of the multi-box gather (its run-time argument table
+// costs registers over the one-box kernel's): 4 (64 registers).
 #ifndef PINYB200_GATHER_BATCH_BLOCKS
 #define PINYB200_GATHER_BATCH_BLOCKS 4
 #endif
@@ -1740,39 +1732,31 @@ __global__ void __launch_bounds__(256, NI <= 8 ? PINYB200_GATHER_BATCH_BLOCKS : 
     PINYB200_BOX_LOOP(t, i, vb, (gather_tile_c_body<R, NI, TT>(t.arg[i].a, t.arg[i].cell, t.arg[i].t, vb)));
 }
 
-template <typename R, int NF>
-__global__ void __launch_bounds__(256, NF > 0 ? PINYB200_PLANE_BATCH_BLOCKS : 1)
-    plane_fwd_batch_kernel(const __grid_constant__ BoxTab<FftBox> t)
+template <typename R>
+__global__ void __launch_bounds__(256) plane_fwd_batch_kernel(const __grid_constant__ BoxTab<FftBox> t)
 {
     typedef typename Cplx<R>::T C2;
     PINYB200_BOX_LOOP(t, i, vb,
-                      (plane_fwd_body<R, NF>((const R *)t.arg[i].q, (C2 *)t.arg[i].spec, t.arg[i].Na, t.arg[i].Nb,
+                      (plane_fwd_body<R>((const R *)t.arg[i].q, (C2 *)t.arg[i].spec, t.arg[i].Na, t.arg[i].Nb,
                                              t.arg[i].Nc, (const R *)t.arg[i].tw[0], (const R *)t.arg[i].tw[1], vb)));
 }
 
-// (the multi-box slab pass: at 3, 80 registers spill 236 bytes and the C4
-// step takes 5.50 against 5.37 ms)
-#ifndef PINYB200_CONV_BATCH_BLOCKS
-#define PINYB200_CONV_BATCH_BLOCKS 2
-#endif
-template <typename R, int NF>
-__global__ void __launch_bounds__(256, NF > 0 ? PINYB200_CONV_BATCH_BLOCKS : 1)
-    conv_c_batch_kernel(const __grid_constant__ BoxTab<FftBox> t)
+template <typename R>
+__global__ void __launch_bounds__(256) conv_c_batch_kernel(const __grid_constant__ BoxTab<FftBox> t)
 {
     typedef typename Cplx<R>::T C2;
     PINYB200_BOX_LOOP(t, i, vb,
-                      (conv_c_body<R, NF>((C2 *)t.arg[i].spec, (const R *)t.arg[i].filt, t.arg[i].Na, t.arg[i].Nb,
+                      (conv_c_body<R>((C2 *)t.arg[i].spec, (const R *)t.arg[i].filt, t.arg[i].Na, t.arg[i].Nb,
                                           t.arg[i].Nc, (const R *)t.arg[i].tw[2], t.arg[i].cell, t.arg[i].alp,
                                           t.arg[i].acc, t.arg[i].energy, vb)));
 }
 
-template <typename R, int NF>
-__global__ void __launch_bounds__(256, NF > 0 ? PINYB200_PLANE_BATCH_BLOCKS : 1)
-    plane_inv_batch_kernel(const __grid_constant__ BoxTab<FftBox> t)
+template <typename R>
+__global__ void __launch_bounds__(256) plane_inv_batch_kernel(const __grid_constant__ BoxTab<FftBox> t)
 {
     typedef typename Cplx<R>::T C2;
     PINYB200_BOX_LOOP(t, i, vb,
-                      (plane_inv_body<R, NF>((const C2 *)t.arg[i].spec, (R *)t.arg[i].q, t.arg[i].Na, t.arg[i].Nb,
+                      (plane_inv_body<R>((const C2 *)t.arg[i].spec, (R *)t.arg[i].q, t.arg[i].Na, t.arg[i].Nb,
                                              t.arg[i].Nc, (const R *)t.arg[i].tw[0], (const R *)t.arg[i].tw[1], vb)));
 }
 
@@ -1823,8 +1807,7 @@ static cudaError_t pme_batch_tiles_n(int NI, const std::vector<PmeBox> &bx, cons
 }
 
 // stage 0 forward plane FFT, 1 c-axis FFT with the convolution, 2 inverse
-// plane FFT for the boxes of one mesh
-template <int NF>
+// plane FFT for the boxes of one mesh of run-time lengths
 static cudaError_t pme_batch_fft(const std::vector<FftBox> &bx, const std::vector<int> &P, int sm_count,
                                  cudaStream_t st, int stage)
 {
@@ -1838,13 +1821,13 @@ static cudaError_t pme_batch_fft(const std::vector<FftBox> &bx, const std::vecto
         tb.add(bx[i], P[i] * (stage == 1 ? bx[i].Nb : bx[i].Nc), 1, work);
     }
     if (stage == 0)
-        return launch_tables(tb, (const void *)plane_fwd_batch_kernel<R, NF>, 256, sp, sm_count,
-                             [&](const BoxTab<FftBox> &t, int g) { plane_fwd_batch_kernel<R, NF><<<g, 256, sp, st>>>(t); });
+        return launch_tables(tb, (const void *)plane_fwd_batch_kernel<R>, 256, sp, sm_count,
+                             [&](const BoxTab<FftBox> &t, int g) { plane_fwd_batch_kernel<R><<<g, 256, sp, st>>>(t); });
     if (stage == 1)
-        return launch_tables(tb, (const void *)conv_c_batch_kernel<R, NF>, 256, ss, sm_count,
-                             [&](const BoxTab<FftBox> &t, int g) { conv_c_batch_kernel<R, NF><<<g, 256, ss, st>>>(t); });
-    return launch_tables(tb, (const void *)plane_inv_batch_kernel<R, NF>, 256, sp, sm_count,
-                         [&](const BoxTab<FftBox> &t, int g) { plane_inv_batch_kernel<R, NF><<<g, 256, sp, st>>>(t); });
+        return launch_tables(tb, (const void *)conv_c_batch_kernel<R>, 256, ss, sm_count,
+                             [&](const BoxTab<FftBox> &t, int g) { conv_c_batch_kernel<R><<<g, 256, ss, st>>>(t); });
+    return launch_tables(tb, (const void *)plane_inv_batch_kernel<R>, 256, sp, sm_count,
+                         [&](const BoxTab<FftBox> &t, int g) { plane_inv_batch_kernel<R><<<g, 256, sp, st>>>(t); });
 }
 
 static cudaError_t pme_batch_tiles_group(const std::pair<int, int> &key, const std::vector<PmeBox> &bx,
@@ -1918,12 +1901,23 @@ cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::
     for (int stage = 0; stage < 3 && err == cudaSuccess; stage++)
         for (auto &kv : ffts) {
             const int Na = std::get<0>(kv.first), Nb = std::get<1>(kv.first), Nc = std::get<2>(kv.first);
-            switch (Na == Nb && Na == Nc ? Na : 0) {
-            case 16: err = pme_batch_fft<16>(kv.second.first, kv.second.second, sm_count, st, stage); break;
-            case 32: err = pme_batch_fft<32>(kv.second.first, kv.second.second, sm_count, st, stage); break;
-            case 64: err = pme_batch_fft<64>(kv.second.first, kv.second.second, sm_count, st, stage); break;
-            case 128: err = pme_batch_fft<128>(kv.second.first, kv.second.second, sm_count, st, stage); break;
-            default: err = pme_batch_fft<0>(kv.second.first, kv.second.second, sm_count, st, stage); break;
+            if (fft_fixed_edge(Na, Nb, Nc)) {
+                std::vector<FftArgs> fx;
+                for (const FftBox &b : kv.second.first) {
+                    FftArgs f;
+                    f.grid = const_cast<void *>(b.q);
+                    f.spec = b.spec;
+                    f.filt = b.filt;
+                    f.tw = b.tw[0];
+                    f.cell = b.cell;
+                    f.alp = b.alp;
+                    f.acc = b.acc;
+                    f.energy = b.energy;
+                    fx.push_back(f);
+                }
+                err = launch_fft_fixed_batch(Na, fx, kv.second.second, sm_count, st, stage);
+            } else {
+                err = pme_batch_fft(kv.second.first, kv.second.second, sm_count, st, stage);
             }
             if (err != cudaSuccess) break;
         }
@@ -2209,14 +2203,7 @@ static cudaError_t launch_pme_adjoint_t(pinyb200_ctx *c, const Cell &cell, const
     const size_t sp = pme_plane_smem(a.Na, a.Nb, f64), ss = pme_slab_smem(a.Na, a.Nc, f64);
     C2 *spec = (C2 *)c->d_spec;
     const R *filt = f64 ? (const R *)c->d_filter : (const R *)((const double *)c->d_filter + G);
-    const bool cube = a.Na == a.Nb && a.Na == a.Nc;
-    switch (cube ? a.Na : 0) {
-    case 16: err = launch_fft_t<R, 16>(c, a, cell, spec, filt, tw, sp, ss, false); break;
-    case 32: err = launch_fft_t<R, 32>(c, a, cell, spec, filt, tw, sp, ss, false); break;
-    case 64: err = launch_fft_t<R, 64>(c, a, cell, spec, filt, tw, sp, ss, false); break;
-    case 128: err = launch_fft_t<R, 128>(c, a, cell, spec, filt, tw, sp, ss, false); break;
-    default: err = launch_fft_t<R, 0>(c, a, cell, spec, filt, tw, sp, ss, false); break;
-    }
+    err = launch_fft<R>(c, a, cell, spec, filt, tw, sp, ss, false);
     if (err != cudaSuccess) return err;
     long long gb = (nrec + 127) / 128;
     if (gb > (long long)c->sm_count * 8) gb = (long long)c->sm_count * 8;
