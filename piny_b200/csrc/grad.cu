@@ -15,6 +15,9 @@
 //          dF_k += sum_s u_s . (-H w)_s + sum_M (sum_c dcoef_c Fbar_c) . F_raw,M
 //          dE_k += -sum_M F_raw,M . w_M
 // H is the Hessian of the energy (pairs, excluded-pair correction, PME).
+#include <algorithm>
+#include <vector>
+
 #include "common.cuh"
 
 namespace pinyb200 {
@@ -26,14 +29,19 @@ __device__ __forceinline__ void ld3(const double *T, int P, int i, int b, double
     z = T[(3 * (size_t)i + 2) * P + b];
 }
 
-// Per-thread channel sums flushed through shared memory; every thread of the
-// block must call it.
+// Per-thread channel sums, added to the totals through warp sums and shared
+// memory; every thread of the block must call it.  (Shared FP64 atomics of
+// every thread met at the same few addresses: 20-30 us a kernel.)
 __device__ __forceinline__ void grad_flush(const GradArgs &g, const double *acc, double *sh)
 {
     for (int i = threadIdx.x; i < 2 * g.K; i += blockDim.x) sh[i] = 0.0;
     __syncthreads();
-    for (int i = 0; i < 2 * g.K; i++)
-        if (acc[i] != 0.0) atomicAdd(&sh[i], acc[i]);
+    for (int i = 0; i < 2 * g.K; i++) {
+        const double v = acc[i];
+        if (!__any_sync(0xffffffffu, v != 0.0)) continue;
+        const double t = warp_sum(v);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&sh[i], t);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * g.K; i += blockDim.x)
         if (sh[i] != 0.0) atomicAdd(&g.gacc[i], sh[i]);
@@ -121,8 +129,8 @@ __device__ __forceinline__ R spline_deriv(const V &c, R del)
 
 struct GradPairArgs {
     const int *row, *col;  // force-bearing list (CSR)
-    int natm, P, ntyp, nsplin, nuniq, use_xmod;
-    const double *posT, *xmod;
+    int natm, P, ntyp, nsplin, nuniq, use_xmod, nseg;
+    const double *posT, *xmod, *uT;
     const int *atm_typ;
     const double *charge;
     const int *inter_map;
@@ -131,39 +139,66 @@ struct GradPairArgs {
     const void *tab;
 };
 
-// Pairs: one thread per (row i, bead), beads fastest.
+// The channels one pass over the pairs serves: at most one with charge
+// tangents, one with ghost tangents and two with table tangents (the nine
+// q-TIP4P/F parameters have exactly these); number -1: none.
+struct GradPairSel {
+    int kq, kw, kt[2];
+    const double *dq, *w;
+    const void *tt[2];
+    unsigned tmask[2];  // tables with a non-zero tangent (bit u, u < 32)
+};
+
+// Pairs: a warp per row i and segment, lanes = beads x neighbours as in the
+// site kernel (pair.cu), one shared list for all beads; rows of a molecule go
+// to neighbouring warps, which find each other's j data in L1.  The channels'
+// sums stay in registers.  Bound: FP64 separations and conversions, and the
+// L2 reads of positions and u.  1024 TIP4P/F x 16 beads, FP32: 2164 us as one
+// thread per (row, bead) with a loop over all channels per pair.
 template <typename R>
-__global__ void __launch_bounds__(128) grad_pair_kernel(GradPairArgs a, GradArgs g, Cell cell)
+__global__ void __launch_bounds__(128) grad_pair_kernel(const __grid_constant__ GradPairArgs a,
+                                                        const __grid_constant__ GradPairSel c,
+                                                        const __grid_constant__ Cell cell, double *__restrict__ gacc)
 {
     typedef typename Vec4<R>::T V;
-    __shared__ double sh[2 * PINYB200_MAX_TAN];
-    double acc[2 * PINYB200_MAX_TAN];
-    for (int k = 0; k < 2 * g.K; k++) acc[k] = 0.0;
+    __shared__ double sh[7][4];
     const V *__restrict__ tab = (const V *)a.tab;
     const int P = a.P, nsm2 = a.nsplin - 2;
     const size_t tstride = (size_t)a.nuniq * a.nsplin;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < (long long)a.natm * P;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(t % P), i = (int)(t / P);
-        const int beg = a.row[i], end = a.row[i + 1];
-        if (beg == end) continue;
-        double xi, yi, zi, uix, uiy, uiz;
+    const int lane = threadIdx.x & 31;
+    const int G = P < 32 ? P : 32, jpi = 32 / G, sub = lane / G;
+    const int b = lane - sub * G + 32 * blockIdx.y;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    double eq = 0, fq = 0, fw = 0, et[2] = {0, 0}, ft[2] = {0, 0};
+    for (int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < a.natm * a.nseg; item += nwarps) {
+        const int seg = item / a.natm, i = item - seg * a.natm;
+        const int end = a.row[i + 1];
+        int k = a.row[i] + seg * jpi + sub;
+        if (k >= end) continue;
+        double xi, yi, zi, uix, uiy, uiz, wix = 0, wiy = 0, wiz = 0;
         ld3(a.posT, P, i, b, xi, yi, zi);
-        ld3(g.uT, P, i, b, uix, uiy, uiz);
+        ld3(a.uT, P, i, b, uix, uiy, uiz);
+        if (c.w) ld3(c.w, P, i, b, wix, wiy, wiz);
         const int ti = a.atm_typ[i];
-        const double qi = a.charge[i];
-        for (int jj = beg; jj < end; jj++) {
-            const int j = a.col[jj];
+        const R qi = (R)a.charge[i], dqi = c.dq ? (R)c.dq[i] : (R)0;
+        double xmi = 0, ymi = 0, zmi = 0;
+        if (a.use_xmod) {
+            xmi = a.xmod[3 * i];
+            ymi = a.xmod[3 * i + 1];
+            zmi = a.xmod[3 * i + 2];
+        }
+        for (; k < end; k += a.nseg * jpi) {
+            const int j = a.col[k];
             const int pt = pair_type(ti, a.atm_typ[j], a.ntyp);
             const int u = a.inter_map[pt];
-            double xj, yj, zj;
+            double xj, yj, zj, ujx, ujy, ujz;
             ld3(a.posT, P, j, b, xj, yj, zj);
+            ld3(a.uT, P, j, b, ujx, ujy, ujz);
             double dx = __dsub_rn(xi, xj), dy = __dsub_rn(yi, yj), dz = __dsub_rn(zi, zj);
             if (a.use_xmod) {
                 double shx = 0, shy = 0, shz = 0;
-                period_pimd_exact(shx, shy, shz, __dsub_rn(a.xmod[3 * i], a.xmod[3 * j]),
-                                  __dsub_rn(a.xmod[3 * i + 1], a.xmod[3 * j + 1]),
-                                  __dsub_rn(a.xmod[3 * i + 2], a.xmod[3 * j + 2]), cell);
+                period_pimd_exact(shx, shy, shz, __dsub_rn(xmi, a.xmod[3 * j]), __dsub_rn(ymi, a.xmod[3 * j + 1]),
+                                  __dsub_rn(zmi, a.xmod[3 * j + 2]), cell);
                 dx = __dadd_rn(dx, shx);
                 dy = __dadd_rn(dy, shy);
                 dz = __dadd_rn(dz, shz);
@@ -173,56 +208,61 @@ __global__ void __launch_bounds__(128) grad_pair_kernel(GradPairArgs a, GradArgs
             const R rx = (R)dx, ry = (R)dy, rz = (R)dz;
             const R r = Idx<R>::dist(rx, ry, rz);
             if (!(r < (R)a.cutoff[pt])) continue;
-            R del;
-            const int kk = Idx<R>::knot(r, (R)a.rmin[u], (R)a.dr[u], (R)a.dri[u], nsm2, del);
-            const size_t off = (size_t)u * a.nsplin + (kk - 1);
             const R dri = (R)a.dri[u];
-            const R qj = (R)a.charge[j];
-            const R q2 = (R)qi * qj;
-            const V cC = ldg4(tab + T_CDV0C * tstride + off), eC = ldg4(tab + T_CV0C * tstride + off);
-            const bool vdw = a.has_vdw[u] != 0;
-            const R sC = spline_eval<V, R>(cC, del), sEC = spline_eval<V, R>(eC, del);
-            R dv = q2 * sC, dvp = q2 * spline_deriv<V, R>(cC, del) * dri;
-            if (vdw) {
-                const V cV = ldg4(tab + T_CDV0 * tstride + off);
-                dv += spline_eval<V, R>(cV, del);
-                dvp += spline_deriv<V, R>(cV, del) * dri;
-            }
-            double ujx, ujy, ujz;
-            ld3(g.uT, P, j, b, ujx, ujy, ujz);
+            R del;
+            const int kk = Idx<R>::knot(r, (R)a.rmin[u], (R)a.dr[u], dri, nsm2, del);
+            const size_t off = (size_t)u * a.nsplin + (kk - 1);
             const R ux = (R)(uix - ujx), uy = (R)(uiy - ujy), uz = (R)(uiz - ujz);
             const R ur = ux * rx + uy * ry + uz * rz;
-            for (int k = 0; k < g.K; k++) {
-                const GradChan &ch = g.ch[k];
-                R eT = 0, fT = 0;
-                if (ch.dq) {
-                    const R tq = (R)(ch.dq[i] * a.charge[j] + qi * ch.dq[j]);
-                    eT += tq * sEC;
-                    fT += tq * sC;
+            const R qj = (R)a.charge[j];
+            const V cC = ldg4(tab + T_CDV0C * tstride + off);
+            const R sC = spline_eval<V, R>(cC, del);
+            if (c.dq) {
+                const R tq = dqi * qj + qi * (R)c.dq[j];
+                if (tq != (R)0) {
+                    eq += (double)(tq * spline_eval<V, R>(ldg4(tab + T_CV0C * tstride + off), del));
+                    fq += (double)(ur * (tq * sC));
                 }
-                if (ch.ttab) {
-                    const V *tt = (const V *)ch.ttab;
-                    eT += spline_eval<V, R>(ldg4(tt + off), del);
-                    fT += spline_eval<V, R>(ldg4(tt + tstride + off), del);
+            }
+#pragma unroll
+            for (int t = 0; t < 2; t++)
+                if (c.tt[t] && (u >= 32 || (c.tmask[t] >> u & 1u))) {
+                    const V *tt = (const V *)c.tt[t];
+                    et[t] += (double)spline_eval<V, R>(ldg4(tt + off), del);
+                    ft[t] += (double)(ur * spline_eval<V, R>(ldg4(tt + tstride + off), del));
                 }
-                double f = (double)(ur * fT);
-                if (ch.w) {
-                    double wix, wiy, wiz, wjx, wjy, wjz;
-                    ld3(ch.w, P, i, b, wix, wiy, wiz);
-                    ld3(ch.w, P, j, b, wjx, wjy, wjz);
-                    const R wx = (R)(wix - wjx), wy = (R)(wiy - wjy), wz = (R)(wiz - wjz);
-                    if (wx != (R)0 || wy != (R)0 || wz != (R)0) {
-                        const R uw = ux * wx + uy * wy + uz * wz, rw = rx * wx + ry * wy + rz * wz;
-                        // -(u . H w) of the pair: F_i = r dv(r)
-                        f += (double)(uw * dv + ur * rw * dvp / r);
+            if (c.w) {
+                double wjx, wjy, wjz;
+                ld3(c.w, P, j, b, wjx, wjy, wjz);
+                const R wx = (R)(wix - wjx), wy = (R)(wiy - wjy), wz = (R)(wiz - wjz);
+                if (wx != (R)0 || wy != (R)0 || wz != (R)0) {
+                    const R q2 = qi * qj;
+                    R dv = q2 * sC, dvp = q2 * spline_deriv<V, R>(cC, del) * dri;
+                    if (a.has_vdw[u]) {
+                        const V cV = ldg4(tab + T_CDV0 * tstride + off);
+                        dv += spline_eval<V, R>(cV, del);
+                        dvp += spline_deriv<V, R>(cV, del) * dri;
                     }
+                    // -(u . H w) of the pair: F_i = r dv(r)
+                    const R uw = ux * wx + uy * wy + uz * wz, rw = rx * wx + ry * wy + rz * wz;
+                    fw += (double)(uw * dv + ur * rw * dvp / r);
                 }
-                acc[2 * k] += (double)eT / (double)P;
-                acc[2 * k + 1] += f;
             }
         }
     }
-    grad_flush(g, acc, sh);
+    const double v[7] = {eq, et[0], et[1], fq, ft[0], ft[1], fw};
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+        const double t = warp_sum(v[k]);
+        if (lane == 0) sh[k][threadIdx.x >> 5] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        const int k = threadIdx.x;
+        const double t = (sh[k][0] + sh[k][1]) + (sh[k][2] + sh[k][3]);
+        const int ch = k == 6 ? c.kw : (k % 3 == 0 ? c.kq : c.kt[k % 3 - 1]);
+        if (ch >= 0 && t != 0.0) atomicAdd(&gacc[2 * ch + (k >= 3)], k < 3 ? t / (double)P : t);
+    }
 }
 
 // Excluded charged pairs (ecor): V = q_i q_j S(cv0), F_i = r q_i q_j S(cdv0).
@@ -447,12 +487,34 @@ cudaError_t launch_grad_terms(pinyb200_ctx *c, const Cell &cell, const GradArgs 
     a.dr = s.dr;
     a.dri = s.dri;
     a.has_vdw = s.has_vdw;
-    if (c->precision == PINYB200_FP64) {
-        a.tab = s.tab64;
-        grad_pair_kernel<double><<<nblk((long long)s.natm * P, 128, sm), 128, 0, st>>>(a, g, cell);
-    } else {
-        a.tab = s.tab32;
-        grad_pair_kernel<float><<<nblk((long long)s.natm * P, 128, sm), 128, 0, st>>>(a, g, cell);
+    a.uT = g.uT;
+    a.tab = c->precision == PINYB200_FP64 ? (const void *)s.tab64 : (const void *)s.tab32;
+    // segments per row so that small systems still give every SM some 32 warps
+    a.nseg = (int)std::max(1LL, std::min(8LL, (long long)sm * 32 / std::max(1, s.natm)));
+    // channels in passes of one charge, one ghost and two table tangents
+    std::vector<int> kq, kw, kt;
+    for (int k = 0; k < g.K; k++) {
+        if (g.ch[k].dq) kq.push_back(k);
+        if (g.ch[k].w) kw.push_back(k);
+        if (g.ch[k].ttab) kt.push_back(k);
+    }
+    const dim3 pgrid((unsigned)std::min<long long>(((long long)s.natm * a.nseg + 3) / 4, (long long)sm * 64),
+                     P > 32 ? P / 32 : 1);
+    for (size_t n = 0; n < kq.size() || n < kw.size() || 2 * n < kt.size(); n++) {
+        GradPairSel sel;
+        sel.kq = n < kq.size() ? kq[n] : -1;
+        sel.kw = n < kw.size() ? kw[n] : -1;
+        sel.dq = sel.kq >= 0 ? g.ch[sel.kq].dq : nullptr;
+        sel.w = sel.kw >= 0 ? g.ch[sel.kw].w : nullptr;
+        for (int t = 0; t < 2; t++) {
+            sel.kt[t] = 2 * n + t < kt.size() ? kt[2 * n + t] : -1;
+            sel.tt[t] = sel.kt[t] >= 0 ? g.ch[sel.kt[t]].ttab : nullptr;
+            sel.tmask[t] = sel.kt[t] >= 0 ? c->grad.tmask[sel.kt[t]] : 0u;
+        }
+        if (c->precision == PINYB200_FP64)
+            grad_pair_kernel<double><<<pgrid, 128, 0, st>>>(a, sel, cell, g.gacc);
+        else
+            grad_pair_kernel<float><<<pgrid, 128, 0, st>>>(a, sel, cell, g.gacc);
     }
     if (s.necor)
         grad_ecor_kernel<<<nblk((long long)s.necor * P, 256, sm), 256, 0, st>>>(
@@ -531,6 +593,10 @@ int pinyb200_grad_prepare(pinyb200_ctx *c, int ntan, const pinyb200_tangent *tan
             const size_t per = (size_t)s.nsplin;
             std::vector<double> all((size_t)2 * 4 * s.nuniq * per, 0.0), tmp, zero(per, 0.0);
             const double *src[2] = {t.dcv0, t.dcdv0};
+            gh.tmask[k] = 0u;
+            for (int kind = 0; kind < 2; kind++)
+                for (size_t e = 0; src[kind] && e < (size_t)s.nuniq * per; e++)
+                    if (src[kind][e] != 0.0 && e / per < 32) gh.tmask[k] |= 1u << (e / per);
             for (int kind = 0; kind < 2; kind++)
                 for (int u = 0; u < s.nuniq; u++) {
                     table_coefs(src[kind] ? src[kind] + (size_t)u * per : zero.data(), s.nsplin, tmp);

@@ -121,6 +121,7 @@ struct GradHost {
     double dq_dot_q[PINYB200_MAX_TAN];  // sum_i q_i dq_i
     double dq_sum[PINYB200_MAX_TAN];    // sum_i dq_i
     double dclong[PINYB200_MAX_TAN];
+    unsigned tmask[PINYB200_MAX_TAN] = {0};  // tables with a non-zero tangent (bit u, u < 32)
     double *d_u = nullptr;              // [natm][3][P]
     double *d_gacc = nullptr;           // [K][2]
     void *d_grid2 = nullptr;            // PME: dipole spread of u, then its convolution
