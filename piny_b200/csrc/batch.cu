@@ -190,7 +190,7 @@ int fused_enqueue(pinyb200_batch *bt, const double *const *d_pos, const double *
         q.kind = 1;
         q.box.push_back(c);
         q.cell.push_back(cells[i]);
-        q.work += 300.0 * c->chunk_cap * c->P;
+        q.work += 37.5 * c->chunk_cap * c->mol_iters * c->P;
     }
     std::vector<Branch> br;
     for (auto &kv : groups) br.push_back(kv.second);

@@ -235,10 +235,20 @@ static int pme_alloc(pinyb200_ctx *c, int nbeads, const int *ngrid, int n_interp
         const size_t csz = f64 ? sizeof(double2) : sizeof(float2);
         CK(cudaMalloc(&c->d_grid, rsz * G * nbeads));
         CK(cudaMalloc(&c->d_spec, csz * (size_t)Nc * Nb * (Na / 2 + 1) * nbeads));
-        // charge bins per grid tile and bead: 16^3 tiles, or 8^3 on small
-        // meshes so that spread and gather still get enough blocks
+        // Charge bins per grid tile and bead: tiles of 16 points, or of 8
+        // where those would leave fewer than two blocks per SM with at least
+        // 16 charges per small tile (or less than a block per SM in any
+        // case): the smaller tiles' halos are 2.2 times the flush and load
+        // traffic.  PME of 1024 x 16 on 32^3 104 -> 79 us, 1024 x 32 174 ->
+        // 118, 1501 x 8 on 36^3 125 -> 73, 256 x 1 FP64 71 -> 46 with 8
+        // (bins of 16: 128, 256, 216, 8); 256 x 32 on 32^3 75 against 77
+        // with 16 (256 bins of 96), 8000 x 4 on 80^3 131 against 141 (500).
         {
-            const int rc2 = pme_tiles_setup(c, std::min(Na, std::min(Nb, Nc)) >= 32 ? 16 : 8);
+            const int nmin = std::min(Na, std::min(Nb, Nc));
+            auto tiles = [&](int T) { return (long long)((Na + T - 1) / T) * ((Nb + T - 1) / T) * ((Nc + T - 1) / T); };
+            const long long bins = tiles(16) * nbeads;
+            const bool small = bins < c->sm_count || (bins < 2LL * c->sm_count && d.nchrg >= 16 * tiles(8));
+            const int rc2 = pme_tiles_setup(c, nmin < 32 || small ? 8 : 16);
             if (rc2) return rc2;
         }
         CK(cudaMalloc(&c->d_pme_ovf, (size_t)std::max(1, d.nchrg) * nbeads * sizeof(int)));
@@ -319,6 +329,70 @@ void pinyb200::pme_res_free(pinyb200_ctx *c)
     for (void *q : ptrs)
         if (q) cudaFree(q);
     p = PmeSet();
+}
+// Whether every molecule (n0 consecutive sites) is a water as the staging and
+// finishing kernels take it: sites O H H or O H H M, both O-H bonds of one
+// type and the H-O-H bend of one type, M (when there) placed from O H H, the
+// charges on every site, or on all but O, and the exclusion correction
+// between all charged sites (or none at all).  Term order and direction are
+// free.
+static void water_setup(pinyb200_ctx *c, const pinyb200_system *s, int n0)
+{
+    const int nmol = c->nmol;
+    c->water_ok = false;
+    if ((n0 != 3 && n0 != 4) || nmol < 1) return;
+    bool ch[4] = {false, false, false, false};
+    for (int k = 0; k < n0; k++) ch[k] = s->charge[k] != 0.0;
+    const bool q0 = ch[0];
+    for (int k = 1; k < n0; k++)
+        if (!ch[k]) return;
+    if (n0 == 4 && q0) return;
+    auto local = [&](int i, int &m) {
+        m = i / n0;
+        return i - m * n0;
+    };
+    std::vector<int> seen(nmol, 0);
+    if (s->nbond != 2 * nmol || s->nbend != nmol) return;
+    for (int k = 0; k < s->nbond; k++) {
+        int m1, m2, a = local(s->bond_j1[k], m1), b = local(s->bond_j2[k], m2);
+        if (m1 != m2 || s->bond_typ[k] != s->bond_typ[0] || std::min(a, b) != 0 || std::max(a, b) > 2) return;
+        seen[m1] += 1 << (2 * (std::max(a, b) - 1));
+    }
+    for (int m = 0; m < nmol; m++)
+        if (seen[m] != 5) return;
+    std::fill(seen.begin(), seen.end(), 0);
+    for (int k = 0; k < s->nbend; k++) {
+        int m1, m2, m3, a = local(s->bend_j1[k], m1), b = local(s->bend_j2[k], m2), d = local(s->bend_j3[k], m3);
+        if (m1 != m2 || m1 != m3 || s->bend_typ[k] != s->bend_typ[0] || b != 0 || std::min(a, d) != 1 ||
+            std::max(a, d) != 2 || seen[m1]++)
+            return;
+    }
+    if (n0 == 4) {
+        if (s->nghost != nmol || s->ghost_ncomp != 3) return;
+        for (int m = 0; m < nmol; m++) {
+            if (s->ghost_atom[m] != 4 * m + 3) return;
+            for (int k = 0; k < 3; k++)
+                if (s->ghost_comp[3 * m + k] != 4 * m + k) return;
+        }
+    } else if (s->nghost != 0) {
+        return;
+    }
+    const int nq = q0 ? n0 : n0 - 1, s0 = q0 ? 0 : 1, npair = nq * (nq - 1) / 2;
+    if (s->necor != 0) {
+        if (s->necor != nmol * npair) return;
+        std::fill(seen.begin(), seen.end(), 0);
+        for (int k = 0; k < s->necor; k++) {
+            int m1, m2, a = local(s->ecor_j1[k], m1), b = local(s->ecor_j2[k], m2);
+            if (m1 != m2 || a == b || std::min(a, b) < s0) return;
+            const int bit = 1 << (4 * std::min(a, b) + std::max(a, b));
+            if (seen[m1] & bit) return;
+            seen[m1] |= bit;
+        }
+    }
+    c->water_ok = true;
+    c->water_q0 = q0;
+    c->water_bond = s->bond_typ[0];
+    c->water_bend = s->bend_typ[0];
 }
 
 // Per-site-pair parameters of the MIXED molecule-pair kernel
@@ -431,7 +505,7 @@ int pinyb200_destroy(pinyb200_ctx *c)
         if (c->ev[i]) cudaEventDestroy(c->ev[i]);
     for (void *p : c->grad.dev) cudaFree(p);
     c->grad.dev.clear();
-    cudaEvent_t evx[4] = {c->ev_fork, c->ev_join, c->ev_pme[0], c->ev_pme[1]};
+    cudaEvent_t evx[5] = {c->ev_fork, c->ev_stage, c->ev_join, c->ev_pme[0], c->ev_pme[1]};
     for (cudaEvent_t ev : evx)
         if (ev) cudaEventDestroy(ev);
     if (c->pme_stream) cudaStreamDestroy(c->pme_stream);
@@ -463,6 +537,7 @@ int pinyb200_create(const pinyb200_system *s, int nbeads, int precision, pinyb20
     CK(cudaStreamCreateWithFlags(&c->pme_stream, cudaStreamNonBlocking));
     for (int i = 0; i < 8; i++) CK(cudaEventCreate(&c->ev[i]));
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
     for (int i = 0; i < 2; i++) CK(cudaEventCreate(&c->ev_pme[i]));
 
@@ -646,6 +721,7 @@ int pinyb200_create(const pinyb200_system *s, int nbeads, int precision, pinyb20
             for (size_t m = 0; m < mstart.size(); m++) strided &= mstart[m] == (int)m * n0;
             c->mol_stride = strided ? n0 : 0;
             if (strided && precision == PINYB200_MIXED) mixed_setup(c, s, n0);
+            if (strided) water_setup(c, s, n0);
         }
     }
     CK(cudaMalloc(&c->d_err, sizeof(int)));
@@ -730,7 +806,11 @@ int pinyb200_build_list(pinyb200_ctx *c, const double *pos1, const double *xmod,
             std::vector<int> mrow(c->nmol + 1);
             CK(cudaMemcpy(mrow.data(), c->d_mrow, mrow.size() * sizeof(int), cudaMemcpyDeviceToHost));
             const int jpi = c->P >= 32 ? 1 : 32 / c->P;
-            const int ch = PINYB200_MOL_CHUNK * jpi;
+            // small systems: shorter chunks, so that each of about 20 resident
+            // warps per SM gets two
+            c->mol_iters = (int)std::max(1LL, std::min<long long>(PINYB200_MOL_CHUNK,
+                                                                  tot[2] / ((long long)jpi * c->sm_count * 40)));
+            const int ch = c->mol_iters * jpi;
             std::vector<int> chunks;
             for (int m = 0; m < c->nmol; m++)
                 for (int k = mrow[m]; k < mrow[m + 1]; k += ch) {
@@ -822,6 +902,18 @@ int pinyb200_get_list(pinyb200_ctx *c, int *pi, int *pj, long cap, long *npairs)
 // Device evaluation on inputs already in d_posT (and d_xmod for PIMD).
 }  // extern "C"
 
+// The pair kernel the system, cell, flags and tuning ask for.
+static cudaError_t launch_pair_any(pinyb200_ctx *c, const Cell &cell, int flags, bool energy)
+{
+    const bool ortho = cell.h[1] == 0.0 && cell.h[2] == 0.0 && cell.h[3] == 0.0 && cell.h[5] == 0.0 &&
+                       cell.h[6] == 0.0 && cell.h[7] == 0.0;
+    if (c->use_mol && c->mol_ok && ortho && c->pair_variant == 0 && !(flags & PINYB200_SITE_PAIRS) && c->mix_ok)
+        return launch_mol_pair_mixed(c, cell, energy);
+    if (c->use_mol && c->mol_ok && ortho && c->pair_variant != 1 && !(flags & PINYB200_SITE_PAIRS))
+        return launch_mol_pair(c, cell, energy);
+    return launch_pair(c, cell, energy);
+}
+
 // Everything one evaluation does on the device, enqueued on c->stream (PME
 // forks to the context's PME stream and joins back); no host
 // synchronisation, so it can be captured in a CUDA graph.  timing: record
@@ -857,13 +949,7 @@ int pinyb200::evaluate_enqueue(pinyb200_ctx *c, const Cell &cell, int flags, boo
         c->stream = main_stream;
         CK(perr);
     }
-    const bool ortho = cell.h[1] == 0.0 && cell.h[2] == 0.0 && cell.h[3] == 0.0 && cell.h[5] == 0.0 &&
-                       cell.h[6] == 0.0 && cell.h[7] == 0.0;
-    if (c->use_mol && c->mol_ok && ortho && c->pair_variant == 0 && !(flags & PINYB200_SITE_PAIRS) && c->mix_ok)
-        CK(launch_mol_pair_mixed(c, cell, energy));
-    else if (c->use_mol && c->mol_ok && ortho && c->pair_variant != 1 && !(flags & PINYB200_SITE_PAIRS))
-        CK(launch_mol_pair(c, cell, energy));
-    else CK(launch_pair(c, cell, energy));
+    CK(launch_pair_any(c, cell, flags, energy));
     CK(kt_mark(c, "pair"));
     if (respa_w) {
         // RESPA outer level: the weighted pair forces from the plain ones
@@ -873,6 +959,7 @@ int pinyb200::evaluate_enqueue(pinyb200_ctx *c, const Cell &cell, int flags, boo
         if (c->r_int_res_ter) CK(launch_pair_respa(c, cell, 4, respa_w));
     }
     if (timing) CK(ev_rec(c->ev[2], c->stream));
+    if (timing) CK(ev_rec(c->ev[5], c->stream));
     CK(launch_intra(c, cell, energy));
     CK(kt_mark(c, "intra (bond, bend, ecor)"));
     if (respa_w) {
@@ -961,6 +1048,64 @@ __global__ void centroid_kernel(const double *__restrict__ posT, double *__restr
     xm[t] = s / (double)P;
 }
 
+// The evaluation of a box of water molecules (pinyb200_ctx::water_ok): one
+// staging kernel, the pair kernel beside the PME chain, one finishing kernel.
+// The charge grid is cleared on the PME stream from the start, and PME waits
+// only for the staging, not for a list update.
+static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, const Cell &cell, int flags,
+                         double *d_force, bool timing, double *h_acc)
+{
+    const bool energy = !(flags & PINYB200_NO_ENERGY);
+    cudaStream_t main_stream = c->stream;
+    const bool overlap = c->pme_overlap && !c->kt_on;
+    cudaStream_t pme = overlap ? c->pme_stream : c->stream;
+    auto on = [&](cudaStream_t st, cudaError_t (*f)(pinyb200_ctx *)) {
+        c->stream = st;
+        const cudaError_t e = f(c);
+        c->stream = main_stream;
+        return e;
+    };
+    if (timing) CK(ev_rec(c->ev[0], c->stream));
+    CK(cudaEventRecord(c->ev_fork, c->stream));
+    if (overlap) CK(cudaStreamWaitEvent(pme, c->ev_fork, 0));
+    CK(on(pme, launch_pme_clear));
+    CK(kt_mark(c, "pme_grid_clear (memset)"));
+    CK(launch_water_stage(c, cell, d_pos, d_xmod));
+    CK(kt_mark(c, "stage"));
+    CK(cudaEventRecord(c->ev_stage, c->stream));
+    if (overlap) CK(cudaStreamWaitEvent(pme, c->ev_stage, 0));
+    {
+        c->stream = pme;
+        cudaError_t perr = timing ? ev_rec(c->ev_pme[0], c->stream) : cudaSuccess;
+        if (perr == cudaSuccess) perr = launch_pme(c, cell, energy, true);
+        if (perr == cudaSuccess && timing) perr = ev_rec(c->ev_pme[1], c->stream);
+        if (perr == cudaSuccess) perr = cudaEventRecord(c->ev_join, c->stream);
+        c->stream = main_stream;
+        CK(perr);
+    }
+    if (flags & PINYB200_UPDATE_LIST) {
+        // PINY's list test (and rebuild) from these positions, on the device
+        int rc = list_update_enqueue(c, d_pos, c->P > 1 ? c->d_xmod : nullptr, cell, c->stream);
+        if (rc) return rc;
+    }
+    if (timing) CK(ev_rec(c->ev[1], c->stream));
+    CK(launch_pair_any(c, cell, flags, energy));
+    CK(kt_mark(c, "pair"));
+    if (timing) CK(ev_rec(c->ev[2], c->stream));
+    CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+    if (timing) CK(ev_rec(c->ev[5], c->stream));
+    CK(launch_water_finish(c, d_force, energy, (flags & PINYB200_DISTRIB_GHOSTS) != 0, c->pme_full_records));
+    CK(kt_mark(c, "finish (intra, force sum, out)"));
+    if (timing) {
+        CK(ev_rec(c->ev[3], c->stream));
+        CK(ev_rec(c->ev[4], c->stream));
+    }
+    if (energy && h_acc)
+        CK(cudaMemcpyAsync(h_acc, c->d_acc, (size_t)c->P * S_NSLOT * sizeof(double), cudaMemcpyDeviceToHost,
+                           c->stream));
+    return PINYB200_OK;
+}
+
 // One evaluation from device-resident positions to device-resident forces,
 // enqueued on c->stream without host synchronisation (see evaluate_enqueue).
 int pinyb200::enqueue_device(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, const Cell &cell, int flags,
@@ -968,6 +1113,7 @@ int pinyb200::enqueue_device(pinyb200_ctx *c, const double *d_pos, const double 
 {
     c->kt_n = 0;
     CK(kt_mark(c, nullptr));
+    if (c->water_ok && !c->pme_full_records) return water_enqueue(c, d_pos, d_xmod, cell, flags, d_force, timing, h_acc);
     int rc = stage_positions(c, d_pos, d_xmod, cell, flags);
     if (rc) return rc;
     CK(kt_mark(c, "transpose_in"));
@@ -1081,7 +1227,7 @@ int pinyb200_energy_force_device(pinyb200_ctx *c, const double *d_pos, const dou
     CK(cudaEventElapsedTime(&c->last_ms[0], c->ev[0], c->ev[4]));
     CK(cudaEventElapsedTime(&c->last_ms[1], c->ev[1], c->ev[2]));
     CK(cudaEventElapsedTime(&c->last_ms[2], c->ev_pme[0], c->ev_pme[1]));
-    CK(cudaEventElapsedTime(&c->last_ms[3], c->ev[2], c->ev[3]));
+    CK(cudaEventElapsedTime(&c->last_ms[3], c->ev[5], c->ev[3]));
     evaluate_finish(c, cell, flags, acc, e);
     if (energy && e && !std::isfinite(e->vintert + e->vintrat))
         return fail(c, PINYB200_ERR_NAN, "non-finite energy: check the positions (forces were written)");
@@ -1108,6 +1254,12 @@ int pinyb200_energy_force(pinyb200_ctx *c, const double *pos, const double *xmod
     double *acc = energy ? c->h_acc_pin : nullptr;  // pinned: the copy is queued, not waited for
     int rc = run_eval_graph(c, eval_key(c, 2, c->d_pos_aos, xmod ? c->d_xmod : nullptr, c->d_force_aos, hmat, flags),
                             [&]() {
+                                if (c->water_ok) {
+                                    c->kt_n = 0;
+                                    CK(kt_mark(c, nullptr));
+                                    return water_enqueue(c, c->d_pos_aos, xmod ? c->d_xmod : nullptr, cell, flags & ~PINYB200_UPDATE_LIST,
+                                                         c->d_force_aos, true, acc);
+                                }
                                 CK(launch_transpose_in(c, c->d_pos_aos));
                                 if (c->P > 1 && !xmod) {
                                     const long long n = (long long)c->sys.natm * 3;
@@ -1127,7 +1279,7 @@ int pinyb200_energy_force(pinyb200_ctx *c, const double *pos, const double *xmod
     CK(cudaEventElapsedTime(&c->last_ms[0], c->ev[0], c->ev[4]));
     CK(cudaEventElapsedTime(&c->last_ms[1], c->ev[1], c->ev[2]));
     CK(cudaEventElapsedTime(&c->last_ms[2], c->ev_pme[0], c->ev_pme[1]));
-    CK(cudaEventElapsedTime(&c->last_ms[3], c->ev[2], c->ev[3]));
+    CK(cudaEventElapsedTime(&c->last_ms[3], c->ev[5], c->ev[3]));
     CK(cudaEventElapsedTime(&c->last_ms[4], c->ev[6], c->ev[7]));
     evaluate_finish(c, cell, flags, acc, e);
     if (energy && e && !std::isfinite(e->vintert + e->vintrat))

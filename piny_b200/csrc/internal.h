@@ -38,8 +38,10 @@ struct Cell {
 // Table kinds in the coefficient arrays.
 enum TabKind { T_CV0 = 0, T_CDV0 = 1, T_CV0C = 2, T_CDV0C = 3 };
 
-// Molecule pairs per warp chunk of the molecule-pair kernel (per lane group
-// when P < 32): the i sites are loaded and their forces flushed once per chunk.
+// Most molecule pairs per chunk of the molecule-pair kernels (per lane group
+// when P < 32): the i sites are loaded and their forces flushed once per
+// chunk.  A list's own figure (pinyb200_ctx::mol_iters) is smaller where
+// chunks of this size would not give every resident warp two.
 #ifndef PINYB200_MOL_CHUNK
 #define PINYB200_MOL_CHUNK 8
 #endif
@@ -164,7 +166,7 @@ struct pinyb200_ctx {
     int pair_blocks_per_sm = 16;        // grid cap of the pair kernels, blocks per SM
     bool pme_full_records = false;      // forward PME writes the full weight records (the adjoint reads them)
     int pair_carveout = 25;             // shared-memory share (%) the MIXED molecule-pair kernel asks for
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_pme[2] = {nullptr, nullptr};
+    cudaEvent_t ev_fork = nullptr, ev_stage = nullptr, ev_join = nullptr, ev_pme[2] = {nullptr, nullptr};
     pinyb200::DeviceSystem sys;
     // host copies needed for energy bookkeeping
     std::vector<double> h_charge;
@@ -192,6 +194,10 @@ struct pinyb200_ctx {
     float4 *d_tabfe = nullptr;  // [2][nuniq][nsplin][2] vdW / Coulomb force and energy rows side by side
     float mix_rc2 = 0, mix_dri = 0, mix_rmd = 0, mix_tmax = 0;
     bool mol_ok = false;       // the current molecule list matches the site list
+    // identical molecules of sites O H H (M) whose bonds, bend, exclusion
+    // corrections and M site are water's: the fused staging and finishing serve them
+    bool water_ok = false, water_q0 = false;  // q0: the first site is charged
+    int water_bond = 0, water_bend = 0;       // their bond and bend type
     int nmol = 0, mol_ns = 0;
     int *d_mstart = nullptr;   // [nmol+1]
     int *d_mcount = nullptr;   // [nmol]
@@ -219,6 +225,7 @@ struct pinyb200_ctx {
     long long *d_ctot = nullptr;  // [1] scan total
     long long mlist_cap = 0, nmp = 0;
     int nchunk = 0;
+    int mol_iters = PINYB200_MOL_CHUNK;  // molecule pairs per chunk and lane group, set by the host build
     int *d_chunk = nullptr;    // [chunk_cap][3]
     long long chunk_cap = 0;
     int *d_nchunk = nullptr;   // device copy of the chunk count (the pair kernel reads it)
@@ -316,7 +323,12 @@ cudaError_t launch_scan(pinyb200_ctx *c, const int *gate, int n, int K, const in
 cudaError_t launch_mol_pair(pinyb200_ctx *c, const Cell &cell, bool energy);
 cudaError_t launch_mol_pair_mixed(pinyb200_ctx *c, const Cell &cell, bool energy);
 cudaError_t launch_site_from_mol(pinyb200_ctx *c, int pass, const int *gate = nullptr, cudaStream_t st = nullptr);
-cudaError_t launch_pme(pinyb200_ctx *c, const Cell &cell, bool energy);
+// staged: the grid is already zero and the charges are binned
+cudaError_t launch_pme(pinyb200_ctx *c, const Cell &cell, bool energy, bool staged = false);
+cudaError_t launch_pme_clear(pinyb200_ctx *c);
+// water molecules (pinyb200_ctx::water_ok): staging and finishing kernels
+cudaError_t launch_water_stage(pinyb200_ctx *c, const Cell &cell, const double *d_pos, const double *d_xmod);
+cudaError_t launch_water_finish(pinyb200_ctx *c, double *d_out, bool energy, bool distrib, bool keep_site_forces);
 cudaError_t launch_pme_force_add(pinyb200_ctx *c);
 
 // evaluation steps (capi.cu): device work of one evaluation enqueued on

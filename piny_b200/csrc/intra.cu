@@ -15,37 +15,9 @@
 
 #include "boxtab.cuh"
 #include "common.cuh"
+#include "intra.cuh"
 
 namespace pinyb200 {
-
-// Per-thread energy/virial sums v of a 256-thread block, thread t holding
-// bead t % P (P a power of two up to 64), added to acc[bead][slot]: lanes of
-// one bead by shuffles, then the block's warps through shared memory, then
-// one global atomic per (bead, slot).  Every thread of the block must call
-// it.  (Shared FP64 atomics instead of the shuffles serialise: with one bead
-// all 256 threads of a block met at 7 addresses, and each of the three
-// intramolecular kernels took 35-41 us of the 256- and 4096-molecule boxes;
-// now 3-5 us.)
-template <int NV>
-__device__ __forceinline__ void block_acc(double *acc, int P, const int *slot, const double *v)
-{
-    __shared__ double sh[NV][8][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int G = P < 32 ? P : 32;
-#pragma unroll
-    for (int c = 0; c < NV; c++) {
-        const double t = warp_sum_strided(v[c], G);
-        if (lane < G) sh[c][w][lane] = t;
-    }
-    __syncthreads();
-    const int wstep = P > 32 ? P / 32 : 1;  // warps w, w + wstep, ... hold the same beads
-    for (int i = threadIdx.x; i < P * NV; i += blockDim.x) {
-        const int c = i / P, b = i - c * P;
-        double t = 0.0;
-        for (int k = b >> 5; k < 8; k += wstep) t += sh[c][k][b & 31];
-        if (t != 0.0) atomicAdd(&acc[(size_t)b * S_NSLOT + slot[c]], t);
-    }
-}
 
 // out[c][r] = in[r][c] for an rows x cols matrix of doubles, through a
 // 32 x 32 shared tile (padded against bank conflicts): both the global reads
@@ -200,15 +172,7 @@ __global__ void __launch_bounds__(256) bond_kernel(const __grid_constant__ Intra
     bond_body(a, nbond, bj, eq, cc, dc, hw_blk());
 }
 
-// One bend of one bead (bend.c:186-330): forces on the outer atoms f1, f3
-// (the middle atom takes -(f1 + f3)), the bond vectors for the virial, and
-// the energy.
-struct BendTerm {
-    double dx12, dy12, dz12, dx23, dy23, dz23;
-    double fx1, fy1, fz1, fx3, fy3, fz3;
-    double v;
-};
-
+// One bend of one bead from the position array.
 __device__ __forceinline__ void bend_term(const double *posT, int P, int a1, int a2, int a3, int b,
                                           const double *c, const double *s, const double *dc, const double *ds,
                                           BendTerm &t)
@@ -217,35 +181,7 @@ __device__ __forceinline__ void bend_term(const double *posT, int P, int a1, int
     load_x(posT, P, a1, b, x1, y1, z1);
     load_x(posT, P, a2, b, x2, y2, z2);
     load_x(posT, P, a3, b, x3, y3, z3);
-    const double dx12 = x1 - x2, dy12 = y1 - y2, dz12 = z1 - z2;
-    const double dx23 = x3 - x2, dy23 = y3 - y2, dz23 = z3 - z2;
-    const double r122i = 1.0 / (dx12 * dx12 + dy12 * dy12 + dz12 * dz12);
-    const double r12i = sqrt(r122i);
-    const double r322i = 1.0 / (dx23 * dx23 + dy23 * dy23 + dz23 * dz23);
-    const double r32i = sqrt(r322i);
-    const double rpmag = r12i * r32i;
-    double cost = (dx12 * dx23 + dy12 * dy23 + dz12 * dz23) * rpmag;
-    cost = cost < 1.0 ? cost : 1.0;
-    cost = cost > -1.0 ? cost : -1.0;
-    double sint = sqrt(1.0 - cost * cost);
-    sint = sint > 1.0e-8 ? sint : 1.0e-8;
-    const double cos122 = cost * r122i, cos322 = cost * r322i;
-    const double vc = ((((((c[6] * cost + c[5]) * cost + c[4]) * cost + c[3]) * cost + c[2]) * cost + c[1]) * cost +
-                       c[0]);
-    const double sisum = (((((s[6] * sint + s[5]) * sint + s[4]) * sint + s[3]) * sint + s[2]) * sint);
-    t.v = vc + (sisum * cost + s[1] * sint);
-    const double dvc = (((((dc[6] * cost + dc[5]) * cost + dc[4]) * cost + dc[3]) * cost + dc[2]) * cost + dc[1]);
-    double dvs = ((((ds[6] * sint + ds[5]) * sint + ds[4]) * sint + ds[3]) * sint + ds[2]);
-    dvs = dvs * cost + ds[1];
-    const double pre = -(dvc + sisum - dvs * cost / sint);
-    t.fx1 = (dx23 * rpmag - dx12 * cos122) * pre;
-    t.fy1 = (dy23 * rpmag - dy12 * cos122) * pre;
-    t.fz1 = (dz23 * rpmag - dz12 * cos122) * pre;
-    t.fx3 = (dx12 * rpmag - dx23 * cos322) * pre;
-    t.fy3 = (dy12 * rpmag - dy23 * cos322) * pre;
-    t.fz3 = (dz12 * rpmag - dz23 * cos322) * pre;
-    t.dx12 = dx12; t.dy12 = dy12; t.dz12 = dz12;
-    t.dx23 = dx23; t.dy23 = dy23; t.dz23 = dz23;
+    bend_eval(x1, y1, z1, x2, y2, z2, x3, y3, z3, c, s, dc, ds, t);
 }
 
 __device__ __forceinline__ void bend_body(const IntraArgs &a, int nbend, const int *__restrict__ bj,
@@ -302,14 +238,11 @@ __device__ __forceinline__ void ecor_body(const IntraArgs &a, int necor, const i
         load_x(a.posT, a.P, j2, b, x2, y2, z2);
         const double dx = x1 - x2, dy = y1 - y2, dz = z1 - z2;
         const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
-        int k = __double2int_rz(__dadd_rn(__dmul_rn(__dsub_rn(r, rmin), dri), 0.5)) + 3;
-        k = k < nsplin - 2 ? k : nsplin - 2;
-        k = k > 3 ? k : 3;
-        const double rsp = __dadd_rn(__dmul_rn((double)(k - 3), dr), rmin);
-        const double del = __dmul_rn(__dsub_rn(r, rsp), dri);
+        double ev, edv;
+        ecor_eval(r, nsplin, rmin, dr, dri, tab, ev, edv);
         const double q12 = a.charge[j1] * a.charge[j2];
-        v += spline_eval<double4, double>(tab[k - 1], del) * q12;
-        const double dvt = spline_eval<double4, double>(tab[nsplin + k - 1], del) * q12;
+        v += ev * q12;
+        const double dvt = edv * q12;
         const double fx = dx * dvt, fy = dy * dvt, fz = dz * dvt;
         add_f(a.forceT, a.P, j1, b, fx, fy, fz);
         add_f(a.forceT, a.P, j2, b, -fx, -fy, -fz);

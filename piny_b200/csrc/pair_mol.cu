@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <map>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 #include <cmath>
 #include <cstddef>
@@ -903,49 +904,55 @@ __device__ __forceinline__ bool site_pair(const typename Vec4<R>::T *__restrict_
     return true;
 }
 
-// One molecule pair whose site-0 separation is within twice the molecular
-// extent of half a box, so that its site pairs may take different images:
-// every site pair gets its own period_pimd shift (period.c:163-176) and its
-// separation in FP64; forces go straight to the force array.  Kept out of
-// line: it is rare in large boxes and would otherwise burden the main
-// loop with its registers.
-template <typename R, int P, int NS, bool FAST, bool ENERGY>
-__device__ __noinline__ void mol_pair_near(const double *__restrict__ posT, const double *__restrict__ xmod,
-                                           double *__restrict__ forceT, const PairConst<R> *pc,
-                                           const typename Vec4<R>::T *__restrict__ tab, size_t tstride, int nsm2,
-                                           int i0, int j0, unsigned mask, int b, double hx, double hy, double hz,
-                                           double hix, double hiy, double hiz, double *sacc)
+// Site pairs of a molecule pair whose images differ from the site-0 pair's
+// (possible only when the site-0 separation is within twice the molecular
+// extent of half a box along some axis): bit si * NS + sj of up / dn along
+// axis d says that PINY's own shift of that site pair (period_pimd,
+// period.c:163-176) is one cell edge above / below the site-0 shift sh0.
+// The G lanes of a pair share the work and then hold the same masks; every
+// lane of the group calls it.
+struct NearImages {
+    unsigned w[3];  // axis d: up in the low half, dn in the high half
+    __device__ __forceinline__ int shift(int d, int sp) const
+    {
+        return (int)((w[d] >> sp) & 1u) - (int)((w[d] >> (16 + sp)) & 1u);
+    }
+};
+
+// x + n h for n = -1, 0, 1 in FP32: h in two parts, so that the sum of a
+// separation near h and -h keeps the separation's own rounding.
+__device__ __forceinline__ float add_cells(float x, int n, double h)
 {
-    const double hd[3] = {hx, hy, hz}, hid[3] = {hix, hiy, hiz};
-    R evs = 0, ecs = 0, pvs[6] = {0, 0, 0, 0, 0, 0};
-    for (unsigned m = mask; m; m &= m - 1u) {
-        const int sp = __ffs(m) - 1;
-        const int si = sp / NS, sj = sp % NS;
-        const int i = i0 + si, j = j0 + sj;
-        double r[3];
+    const float hh = (float)h, hl = (float)(h - (double)hh);
+    return n == 0 ? x : (n > 0 ? (x + hh) + hl : (x - hh) - hl);
+}
+__device__ __forceinline__ double add_cells(double x, int n, double h) { return x + (double)n * h; }
+
+template <int NS, int G>
+__device__ __forceinline__ NearImages near_images(const double *__restrict__ xmod, int i0, int j0, int ni,
+                                                  const double *sh0, const Cell &cell, int lane)
+{
+    NearImages n = {{0u, 0u, 0u}};
+    for (int sp = lane % G; sp < NS * NS; sp += G) {
+        const int si = sp / NS, sj = sp - si * NS;
+        if (si >= ni || sj >= ni) continue;
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            const double sh = shift_exact(__dsub_rn(xmod[3 * (size_t)i + d], xmod[3 * (size_t)j + d]), hid[d]);
-            r[d] = __dadd_rn(__dsub_rn(posT[(3 * (size_t)i + d) * P + b], posT[(3 * (size_t)j + d) * P + b]),
-                             __dmul_rn(sh, hd[d]));
-        }
-        R fx, fy, fz;
-        if (site_pair<R, FAST, ENERGY>(tab, tstride, nsm2, *pc, sp, (R)r[0], (R)r[1], (R)r[2], fx, fy, fz, evs, ecs,
-                                       pvs)) {
-            atomicAdd(&forceT[(3 * (size_t)i + 0) * P + b], (double)fx);
-            atomicAdd(&forceT[(3 * (size_t)i + 1) * P + b], (double)fy);
-            atomicAdd(&forceT[(3 * (size_t)i + 2) * P + b], (double)fz);
-            atomicAdd(&forceT[(3 * (size_t)j + 0) * P + b], -(double)fx);
-            atomicAdd(&forceT[(3 * (size_t)j + 1) * P + b], -(double)fy);
-            atomicAdd(&forceT[(3 * (size_t)j + 2) * P + b], -(double)fz);
+            const double sh = shift_exact(__dsub_rn(__ldg(xmod + 3 * (size_t)(i0 + si) + d),
+                                                    __ldg(xmod + 3 * (size_t)(j0 + sj) + d)),
+                                          cell.hi[4 * d]);
+            if (sh > sh0[d]) n.w[d] |= 1u << sp;
+            if (sh < sh0[d]) n.w[d] |= 1u << (16 + sp);
         }
     }
-    if (ENERGY) {
-        sacc[0] += (double)evs;
-        sacc[128] += (double)ecs;
+    if (G > 1) {
+        const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane / G * G);
 #pragma unroll
-        for (int c = 0; c < 6; c++) sacc[128 * (2 + c)] += (double)pvs[c];
+        for (int o = G / 2; o >= 1; o >>= 1)
+#pragma unroll
+            for (int d = 0; d < 3; d++) n.w[d] |= __shfl_xor_sync(mask, n.w[d], o);
     }
+    return n;
 }
 
 // A 128-thread block's energy and virial sums (sacc[k][t], thread t holding
@@ -1072,12 +1079,6 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
                     near |= fabs(t + sh0[d]) > 0.5 - ext2 * hid;
                 }
             }
-            if (near) {
-                mol_pair_near<R, P, NS, FAST, ENERGY>(posT, a.xmod, a.forceT, &pc, tab, tstride, nsm2, i0, j0, mask, b,
-                                                      cell.h[0], cell.h[4], cell.h[8], cell.hi[0], cell.hi[4],
-                                                      cell.hi[8], &sacc[0][threadIdx.x]);
-                continue;
-            }
             R d0[3], ej[NS][3];
             if (FAST) {
 #pragma unroll
@@ -1087,64 +1088,80 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
 #pragma unroll
                     for (int d = 0; d < 3; d++) ej[s][d] = (R)(xj[s][d] - xj[0][d]);
             }
-            // j sites in a warp-uniform loop (for P >= 32 the mask is the
-            // same in every lane); i sites unrolled so their offsets and
-            // forces stay in fixed registers
+            auto site_pairs = [&](auto near_tag, const NearImages &nim) {
+                constexpr bool NEAR = decltype(near_tag)::value;
+                // j sites in a warp-uniform loop (for P >= 32 the mask is the
+                // same in every lane); i sites unrolled so their offsets and
+                // forces stay in fixed registers
 #pragma unroll 1
-            for (int sj = 0; sj < NS; sj++) {
-                unsigned col = 0;
+                for (int sj = 0; sj < NS; sj++) {
+                    unsigned col = 0;
 #pragma unroll
-                for (int si = 0; si < NS; si++) col |= ((mask >> (si * NS + sj)) & 1u) << si;
-                if (!col) continue;
-                // j-site position: MIXED d0 - e_j, FP64 x_j
-                R djx = 0, djy = 0, djz = 0;
-                double xjx = 0, xjy = 0, xjz = 0;
+                    for (int si = 0; si < NS; si++) col |= ((mask >> (si * NS + sj)) & 1u) << si;
+                    if (!col) continue;
+                    // j-site position: MIXED d0 - e_j, FP64 x_j
+                    R djx = 0, djy = 0, djz = 0;
+                    double xjx = 0, xjy = 0, xjz = 0;
 #pragma unroll
-                for (int s2 = 0; s2 < NS; s2++)
-                    if (sj == s2) {
+                    for (int s2 = 0; s2 < NS; s2++)
+                        if (sj == s2) {
+                            if (FAST) {
+                                djx = d0[0] - ej[s2][0];
+                                djy = d0[1] - ej[s2][1];
+                                djz = d0[2] - ej[s2][2];
+                            } else {
+                                xjx = xj[s2][0];
+                                xjy = xj[s2][1];
+                                xjz = xj[s2][2];
+                            }
+                        }
+                    R fjx = 0, fjy = 0, fjz = 0;
+#pragma unroll
+                    for (int si = 0; si < NS; si++) {
+                        if (!((col >> si) & 1u)) continue;
+                        // away from half a box every site pair takes the site-0 image
+                        R rx, ry, rz;
                         if (FAST) {
-                            djx = d0[0] - ej[s2][0];
-                            djy = d0[1] - ej[s2][1];
-                            djz = d0[2] - ej[s2][2];
+                            rx = djx + ei[si][0];
+                            ry = djy + ei[si][1];
+                            rz = djz + ei[si][2];
+                            if constexpr (NEAR) {
+                                rx = add_cells(rx, nim.shift(0, si * NS + sj), cell.h[0]);
+                                ry = add_cells(ry, nim.shift(1, si * NS + sj), cell.h[4]);
+                                rz = add_cells(rz, nim.shift(2, si * NS + sj), cell.h[8]);
+                            }
                         } else {
-                            xjx = xj[s2][0];
-                            xjy = xj[s2][1];
-                            xjz = xj[s2][2];
+                            double sx = sh0[0], sy = sh0[1], sz = sh0[2];
+                            if constexpr (NEAR) {
+                                sx += (double)nim.shift(0, si * NS + sj);
+                                sy += (double)nim.shift(1, si * NS + sj);
+                                sz += (double)nim.shift(2, si * NS + sj);
+                            }
+                            rx = (R)__dadd_rn(__dsub_rn(xi[si][0], xjx), __dmul_rn(sx, cell.h[0]));
+                            ry = (R)__dadd_rn(__dsub_rn(xi[si][1], xjy), __dmul_rn(sy, cell.h[4]));
+                            rz = (R)__dadd_rn(__dsub_rn(xi[si][2], xjz), __dmul_rn(sz, cell.h[8]));
+                        }
+                        R fx, fy, fz;
+                        if (site_pair<R, FAST, ENERGY>(tab, tstride, nsm2, pc, si * NS + sj, rx, ry, rz, fx, fy, fz, evs,
+                                                       ecs, pvs)) {
+                            fi[si][0] += fx;
+                            fi[si][1] += fy;
+                            fi[si][2] += fz;
+                            fjx -= fx;
+                            fjy -= fy;
+                            fjz -= fz;
                         }
                     }
-                R fjx = 0, fjy = 0, fjz = 0;
-#pragma unroll
-                for (int si = 0; si < NS; si++) {
-                    if (!((col >> si) & 1u)) continue;
-                    // away from half a box every site pair takes the site-0 image
-                    R rx, ry, rz;
-                    if (FAST) {
-                        rx = djx + ei[si][0];
-                        ry = djy + ei[si][1];
-                        rz = djz + ei[si][2];
-                    } else {
-                        rx = (R)__dadd_rn(__dsub_rn(xi[si][0], xjx), __dmul_rn(sh0[0], cell.h[0]));
-                        ry = (R)__dadd_rn(__dsub_rn(xi[si][1], xjy), __dmul_rn(sh0[1], cell.h[4]));
-                        rz = (R)__dadd_rn(__dsub_rn(xi[si][2], xjz), __dmul_rn(sh0[2], cell.h[8]));
-                    }
-                    R fx, fy, fz;
-                    if (site_pair<R, FAST, ENERGY>(tab, tstride, nsm2, pc, si * NS + sj, rx, ry, rz, fx, fy, fz, evs,
-                                                   ecs, pvs)) {
-                        fi[si][0] += fx;
-                        fi[si][1] += fy;
-                        fi[si][2] += fz;
-                        fjx -= fx;
-                        fjy -= fy;
-                        fjz -= fz;
+                    if (fjx != (R)0 || fjy != (R)0 || fjz != (R)0) {
+                        const int j = j0 + sj;
+                        atomicAdd(&a.forceT[(3 * (size_t)j + 0) * P + b], (double)fjx);
+                        atomicAdd(&a.forceT[(3 * (size_t)j + 1) * P + b], (double)fjy);
+                        atomicAdd(&a.forceT[(3 * (size_t)j + 2) * P + b], (double)fjz);
                     }
                 }
-                if (fjx != (R)0 || fjy != (R)0 || fjz != (R)0) {
-                    const int j = j0 + sj;
-                    atomicAdd(&a.forceT[(3 * (size_t)j + 0) * P + b], (double)fjx);
-                    atomicAdd(&a.forceT[(3 * (size_t)j + 1) * P + b], (double)fjy);
-                    atomicAdd(&a.forceT[(3 * (size_t)j + 2) * P + b], (double)fjz);
-                }
-            }
+            };
+            if (near) site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, ni, sh0, cell, lane));
+            else site_pairs(std::false_type{}, NearImages{{0u, 0u, 0u}});
         }
         // i-site forces: sum the lane groups that hold the same bead
 #pragma unroll
@@ -1189,8 +1206,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
 //   * molecules are uniform runs of sites: the j site index is mj * stride,
 //     not a load.
 // Pairs whose site-0 separation is within twice the molecular extent of half
-// a box go through mol_pair_near (per-site-pair FP64 image), as in
-// mol_pair_kernel.
+// a box add each site pair's own image (near_images), as in mol_pair_kernel.
 
 // Table row load that asks L1 to keep the line (evict_last): the four
 // tables a water system reads stay resident while positions stream past.
@@ -1215,14 +1231,8 @@ __device__ __forceinline__ void ldg_keep_pair(const float4 *p, float4 &f, float4
 struct MixArgs {
     const int *nchunk, *chunk, *bad, *mj;
     const unsigned *mask;
-    const int *mstart;
     const double *posT, *xmod;
     const unsigned long long *ext;  // extent bound of the evaluation (mol_extent_kernel), or nullptr
-    const int *atm_typ;
-    const double *charge;
-    const int *inter_map;
-    const double *cutoff, *rmin, *dri;
-    const int *has_vdw;
     const float4 *tab;   // [4][nuniq][nsplin] interval coefficients (TabKind order)
     const float4 *tabfe; // [2][nuniq][nsplin][2]: vdW then Coulomb; force and energy rows interleaved
     double *forceT;
@@ -1261,24 +1271,7 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
 {
     constexpr int G = P >= 32 ? 32 : P;  // lanes per molecule pair
     constexpr int JPI = 32 / G;          // molecule pairs per warp step
-    __shared__ PairConst<float> pc;      // per-kind constants of the near path
     __shared__ double sacc[8][128];
-    if (threadIdx.x < NS * NS) {
-        const int si = threadIdx.x / NS, sj = threadIdx.x % NS;
-        const int nm0 = a.mstart[1];
-        const int ia = si < nm0 ? si : 0, ja = sj < nm0 ? sj : 0;
-        const int p = pair_type(a.atm_typ[ia], a.atm_typ[ja], m.ntyp);
-        const int u = a.inter_map[p];
-        const double q2 = a.charge[ia] * a.charge[ja];
-        float4 c;
-        c.x = (float)(a.cutoff[p] * a.cutoff[p]);
-        c.y = (float)a.rmin[u];
-        c.z = (float)a.dri[u];
-        c.w = (float)q2;
-        pc.c[threadIdx.x] = c;
-        pc.q2[threadIdx.x] = (float)q2;
-        pc.o[threadIdx.x] = make_int2(u * m.nsplin, a.has_vdw[u]);
-    }
     if (ENERGY)
         for (int c = 0; c < 8; c++) sacc[c][threadIdx.x] = 0.0;
     __syncthreads();
@@ -1327,13 +1320,6 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                 sh0[d] = -nint_rn(t);
                 near |= fabs(t + sh0[d]) > 0.5 - ext2 * hid;
             }
-            if (near) {
-                mol_pair_near<float, P, NS, true, ENERGY>(posT, a.xmod, a.forceT, &pc, a.tab,
-                                                           (size_t)m.nuniq * m.nsplin, m.nsplin - 2, i0, j0, mask, b,
-                                                           cell.h[0], cell.h[4], cell.h[8], cell.hi[0], cell.hi[4],
-                                                           cell.hi[8], &sacc[0][threadIdx.x]);
-                continue;
-            }
             unsigned jm = 1u;
 #pragma unroll
             for (int si = 0; si < NS; si++) jm |= (mask >> (si * NS)) & ((1u << NS) - 1u);
@@ -1355,81 +1341,105 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                         dj[s][d] = dj[0][d] - (float)(__ldcg(posT + (3 * (size_t)j + d) * P + b) - xj0[d]);
                 }
             }
+            // the site pairs; NEAR adds each pair's own image, in a copy of the
+            // loop so that pairs away from half a box pay nothing for it
+            auto site_pairs = [&](auto near_tag, const NearImages &nim) {
+                constexpr bool NEAR = decltype(near_tag)::value;
 #pragma unroll
-            for (int sj = 0; sj < NS; sj++) {
-                if (!((jm >> sj) & 1u)) continue;
-                float fjx = 0.0f, fjy = 0.0f, fjz = 0.0f;
+                for (int sj = 0; sj < NS; sj++) {
+                    if (!((jm >> sj) & 1u)) continue;
+                    float fjx = 0.0f, fjy = 0.0f, fjz = 0.0f;
 #pragma unroll
-                for (int si = 0; si < NS; si++) {
-                    const int sp = si * NS + sj;
-                    const bool coul = CM == kAnyPair ? (m.eflag[sp] & 2) != 0 : ((CM >> sp) & 1u) != 0;
-                    const bool vdw = VM == kAnyPair ? (m.eflag[sp] & 1) != 0 : ((VM >> sp) & 1u) != 0;
-                    if (CM != kAnyPair && !coul && !vdw) continue;  // a pair the masks never hold
-                    if (!((mask >> sp) & 1u)) continue;
-                    const float rx = dj[sj][0] + ei[si][0];
-                    const float ry = dj[sj][1] + ei[si][1];
-                    const float rz = dj[sj][2] + ei[si][2];
-                    const float r2 = rx * rx + ry * ry + rz * rz;
-                    if (r2 < rc2) {
-                        const float r = r2 * rsqrtf(r2);
-                        const float t = fminf(fmaxf(fmaf(r, dri, -rmd), 0.0f), tmax);
-                        const float tr = __fadd_rn(t, kRound);
-                        const int kn = __float_as_int(tr) - __float_as_int(kRound);
-                        const float del = t - __fsub_rn(tr, kRound);
-                        // with energies: the force and energy rows of an interval
-                        // sit side by side (one cache line for both loads)
-                        const float4 *row = tab + (m.toff[sp] + kn);
-                        const float4 *rfe = a.tabfe + 2 * (m.toff[sp] + kn);
-                        float dv = 0.0f;
-                        float4 ecf = make_float4(0.f, 0.f, 0.f, 0.f), evf = ecf;
-                        if (coul) {
-                            float4 cf;
-                            if (ENERGY) {
-                                ldg_keep_pair(rfe + 2 * m.tstride, cf, ecf);
-                            } else {
-                                cf = ldg_keep(row + T_CDV0C * m.tstride);
-                            }
-                            dv = m.q2[sp] * (cf.x + del * (cf.y + del * (cf.z + del * cf.w)));
+                    for (int si = 0; si < NS; si++) {
+                        const int sp = si * NS + sj;
+                        const bool coul = CM == kAnyPair ? (m.eflag[sp] & 2) != 0 : ((CM >> sp) & 1u) != 0;
+                        const bool vdw = VM == kAnyPair ? (m.eflag[sp] & 1) != 0 : ((VM >> sp) & 1u) != 0;
+                        if (CM != kAnyPair && !coul && !vdw) continue;  // a pair the masks never hold
+                        if (!((mask >> sp) & 1u)) continue;
+                        float rx = dj[sj][0] + ei[si][0];
+                        float ry = dj[sj][1] + ei[si][1];
+                        float rz = dj[sj][2] + ei[si][2];
+                        if constexpr (NEAR) {
+                            rx = add_cells(rx, nim.shift(0, sp), cell.h[0]);
+                            ry = add_cells(ry, nim.shift(1, sp), cell.h[4]);
+                            rz = add_cells(rz, nim.shift(2, sp), cell.h[8]);
                         }
-                        if (vdw) {
-                            float4 cf;
-                            if (ENERGY) {
-                                ldg_keep_pair(rfe, cf, evf);
-                            } else {
-                                cf = ldg_keep(row + T_CDV0 * m.tstride);
+                        const float r2 = rx * rx + ry * ry + rz * rz;
+                        if (r2 < rc2) {
+                            const float r = r2 * rsqrtf(r2);
+                            const float t = fminf(fmaxf(fmaf(r, dri, -rmd), 0.0f), tmax);
+                            const float tr = __fadd_rn(t, kRound);
+                            const int kn = __float_as_int(tr) - __float_as_int(kRound);
+                            const float del = t - __fsub_rn(tr, kRound);
+                            // with energies: the force and energy rows of an interval
+                            // sit side by side (one cache line for both loads)
+                            const float4 *row = tab + (m.toff[sp] + kn);
+                            const float4 *rfe = a.tabfe + 2 * (m.toff[sp] + kn);
+                            float dv = 0.0f;
+                            float4 ecf = make_float4(0.f, 0.f, 0.f, 0.f), evf = ecf;
+                            if (coul) {
+                                float4 cf;
+                                if (ENERGY) {
+                                    ldg_keep_pair(rfe + 2 * m.tstride, cf, ecf);
+                                } else {
+                                    cf = ldg_keep(row + T_CDV0C * m.tstride);
+                                }
+                                dv = m.q2[sp] * (cf.x + del * (cf.y + del * (cf.z + del * cf.w)));
                             }
-                            dv += cf.x + del * (cf.y + del * (cf.z + del * cf.w));
-                        }
-                        const float fx = rx * dv, fy = ry * dv, fz = rz * dv;
-                        fi[si][0] += fx;
-                        fi[si][1] += fy;
-                        fi[si][2] += fz;
-                        fjx -= fx;
-                        fjy -= fy;
-                        fjz -= fz;
-                        if (ENERGY) {
-                            if (vdw) evs += evf.x + del * (evf.y + del * (evf.z + del * evf.w));
-                            if (coul) ecs += m.q2[sp] * (ecf.x + del * (ecf.y + del * (ecf.z + del * ecf.w)));
+                            if (vdw) {
+                                float4 cf;
+                                if (ENERGY) {
+                                    ldg_keep_pair(rfe, cf, evf);
+                                } else {
+                                    cf = ldg_keep(row + T_CDV0 * m.tstride);
+                                }
+                                dv += cf.x + del * (cf.y + del * (cf.z + del * cf.w));
+                            }
+                            const float fx = rx * dv, fy = ry * dv, fz = rz * dv;
+                            fi[si][0] += fx;
+                            fi[si][1] += fy;
+                            fi[si][2] += fz;
+                            fjx -= fx;
+                            fjy -= fy;
+                            fjz -= fz;
+                            if (ENERGY && NEAR) {
+                                // the cell edges in r = dj + e_i + n h: their part of the virial
+                                const float cx = (float)nim.shift(0, sp) * (float)cell.h[0],
+                                            cy = (float)nim.shift(1, sp) * (float)cell.h[4],
+                                            cz = (float)nim.shift(2, sp) * (float)cell.h[8];
+                                pvs[0] += cx * fx;
+                                pvs[1] += cy * fy;
+                                pvs[2] += cz * fz;
+                                pvs[3] += cx * fy;
+                                pvs[4] += cx * fz;
+                                pvs[5] += cy * fz;
+                            }
+                            if (ENERGY) {
+                                if (vdw) evs += evf.x + del * (evf.y + del * (evf.z + del * evf.w));
+                                if (coul) ecs += m.q2[sp] * (ecf.x + del * (ecf.y + del * (ecf.z + del * ecf.w)));
+                            }
                         }
                     }
+                    // virial: r = dj + e_i, so sum r (x) f = dj (x) sum_i f (= -fj here)
+                    // + e_i (x) f_i, the latter once per chunk below
+                    if (ENERGY) {
+                        pvs[0] -= dj[sj][0] * fjx;
+                        pvs[1] -= dj[sj][1] * fjy;
+                        pvs[2] -= dj[sj][2] * fjz;
+                        pvs[3] -= dj[sj][0] * fjy;
+                        pvs[4] -= dj[sj][0] * fjz;
+                        pvs[5] -= dj[sj][1] * fjz;
+                    }
+                    if (fjx != 0.0f || fjy != 0.0f || fjz != 0.0f) {
+                        const int j = j0 + sj;
+                        atomicAdd(&a.forceT[(3 * (size_t)j + 0) * P + b], (double)fjx);
+                        atomicAdd(&a.forceT[(3 * (size_t)j + 1) * P + b], (double)fjy);
+                        atomicAdd(&a.forceT[(3 * (size_t)j + 2) * P + b], (double)fjz);
+                    }
                 }
-                // virial: r = dj + e_i, so sum r (x) f = dj (x) sum_i f (= -fj here)
-                // + e_i (x) f_i, the latter once per chunk below
-                if (ENERGY) {
-                    pvs[0] -= dj[sj][0] * fjx;
-                    pvs[1] -= dj[sj][1] * fjy;
-                    pvs[2] -= dj[sj][2] * fjz;
-                    pvs[3] -= dj[sj][0] * fjy;
-                    pvs[4] -= dj[sj][0] * fjz;
-                    pvs[5] -= dj[sj][1] * fjz;
-                }
-                if (fjx != 0.0f || fjy != 0.0f || fjz != 0.0f) {
-                    const int j = j0 + sj;
-                    atomicAdd(&a.forceT[(3 * (size_t)j + 0) * P + b], (double)fjx);
-                    atomicAdd(&a.forceT[(3 * (size_t)j + 1) * P + b], (double)fjy);
-                    atomicAdd(&a.forceT[(3 * (size_t)j + 2) * P + b], (double)fjz);
-                }
-            }
+            };
+            if (near) site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, ni, sh0, cell, lane));
+            else site_pairs(std::false_type{}, NearImages{{0u, 0u, 0u}});
         }
         if (ENERGY) {
             // the e_i (x) f_i part of the virial: e_i is fixed over the chunk
@@ -1828,17 +1838,9 @@ static MixArgs mix_args(pinyb200_ctx *c)
     a.bad = c->d_ls ? (const int *)((const char *)c->d_ls + offsetof(ListState, overflow)) : nullptr;
     a.mj = c->d_mj;
     a.mask = c->d_mmask;
-    a.mstart = c->d_mstart;
     a.posT = c->d_posT;
     a.xmod = c->P > 1 ? c->d_xmod : c->d_posT;
     a.ext = (const unsigned long long *)(c->d_acc + S_EXT);
-    a.atm_typ = s.atm_typ;
-    a.charge = s.charge;
-    a.inter_map = s.inter_map;
-    a.cutoff = s.cutoff;
-    a.rmin = s.rmin;
-    a.dri = s.dri;
-    a.has_vdw = s.has_vdw;
     a.tab = s.tab32;
     a.tabfe = c->d_tabfe;
     a.forceT = c->d_forceT;
@@ -1935,8 +1937,8 @@ static cudaError_t launch_mix_batch_t(const std::vector<pinyb200_ctx *> &box, co
 {
     BoxTabBuilder<MixBox> tb;
     const MixSite m = mix_site(box[0]);  // one model per group (launch_mol_pair_mixed_batch)
-    // Blocks of each box's own grid-stride loop over its chunks: about 16
-    // chunks' worth of 32-bead work per warp (a warp takes 32 / P molecule
+    // Blocks of each box's own grid-stride loop over its chunks: about 128
+    // molecule pairs' worth of 32-bead work per warp (a warp takes 32 / P molecule
     // pairs at a time below 32 beads), so that a block's set-up (site-pair
     // constants) and energy flush (FP64 atomics per bead and slot) are
     // spread over enough molecule pairs; more, down to 2 chunks per warp,
@@ -1945,7 +1947,7 @@ static cudaError_t launch_mix_batch_t(const std::vector<pinyb200_ctx *> &box, co
     std::vector<long long> vb(box.size());
     long long tot = 0;
     for (size_t i = 0; i < box.size(); i++) {
-        vb[i] = std::max<long long>(1, (box[i]->chunk_cap * G + 4LL * 16 * 32 - 1) / (4LL * 16 * 32));
+        vb[i] = std::max<long long>(1, (box[i]->chunk_cap * box[i]->mol_iters * G + 4LL * 128 * 32 - 1) / (4LL * 128 * 32));
         tot += vb[i] * (P > 32 ? P / 32 : 1);
     }
     const long long want = 2LL * sm_count * PINYB200_MIX_BATCH_BLOCKS;
@@ -1954,7 +1956,7 @@ static cudaError_t launch_mix_batch_t(const std::vector<pinyb200_ctx *> &box, co
         pinyb200_ctx *c = box[i];
         const long long v = std::min(vb[i] * scale, std::max<long long>(1, (c->chunk_cap + 7) / 8));
         tb.add(MixBox{mix_args(c), cells[i]}, (int)std::min<long long>(v, 1 << 20), P > 32 ? P / 32 : 1,
-               (double)c->chunk_cap * P);
+               (double)c->chunk_cap * c->mol_iters * P);
     }
     const void *fn = energy ? (const void *)mol_pair_mixed_batch_kernel<P, NS, true, CM, VM>
                             : (const void *)mol_pair_mixed_batch_kernel<P, NS, false, CM, VM>;

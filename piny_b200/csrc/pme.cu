@@ -27,6 +27,7 @@
 //               inverse FFT along a, real potential out
 //   gather      per (tile, bead): forces from a shared copy of the tile's
 //               potential
+#include <algorithm>
 #include <map>
 #include <tuple>
 #include <vector>
@@ -34,20 +35,9 @@
 #include "boxtab.cuh"
 #include "common.cuh"
 #include "fft.cuh"
+#include "pme_bin.cuh"
 
 namespace pinyb200 {
-
-struct PmeArgs {
-    int natm, P, nchrg;
-    const int *ichrg;
-    const double *charge;
-    const double *posT;
-    int Na, Nb, Nc, n;
-    void *grid;  // real [P][Nc][Nb][Na]
-    double *forceP;  // PME forces [nchrg][3][P]
-    int4 *rhead;  // per (charge, bead) records, see RecGeom
-    void *rw;
-};
 
 // B-spline weights of order NI at the fractional offset f (ewald3d_pme.c:
 // 301-338).  m[j], j = 1..NI as in PINY (index 0 unused); dm[] are the
@@ -76,51 +66,18 @@ __device__ __forceinline__ void bspline(R f, R *m, R *dm)
     }
 }
 
-// Scaled coordinate of one charge along one axis, wrapped to (0,1] and
-// multiplied by the grid size; returns floor and fraction (FP64, PINY order).
-__device__ __forceinline__ void scaled(double s, int N, int &i0, double &frac)
-{
-    s = __dsub_rn(s, nint_rn(__dsub_rn(s, 0.5)));
-    double xs = __dmul_rn(s, (double)N);
-    i0 = (int)xs;
-    frac = __dsub_rn(xs, (double)i0);
-    // s == 1 exactly (a coordinate on a cell face) and non-finite positions
-    // would index outside the grid; keep every access in bounds.
-    if (i0 == N) i0 = 0;
-    if (!(i0 >= 0 && i0 < N)) { i0 = 0; frac = 0.0; }
-}
-
-// First grid index per axis of one charge's stencil and the fractional
-// offsets.  PINY's points ia-(j-2), j = 1..n, are the n consecutive indices
-// ia-n+1 .. ia (wrapped), and point j carries weight m[j]; so grid index
-// lo + t (t = 0..n-1) carries m[n - t].  The binning and both tile kernels
-// call this same FP64 code, so they agree on every charge's tile.
+// Stencil of one charge and bead from the position array.
 __device__ __forceinline__ void stencil_origin(const PmeArgs &a, const Cell &cell, int at, int b, int ni, int &la,
                                                int &lb, int &lc, double &fa, double &fb, double &fc)
 {
-    const double x = a.posT[(3 * (size_t)at + 0) * a.P + b];
-    const double y = a.posT[(3 * (size_t)at + 1) * a.P + b];
-    const double z = a.posT[(3 * (size_t)at + 2) * a.P + b];
-    const double sa = __dadd_rn(__dadd_rn(__dmul_rn(x, cell.hi[0]), __dmul_rn(y, cell.hi[3])), __dmul_rn(z, cell.hi[6]));
-    const double sb = __dadd_rn(__dadd_rn(__dmul_rn(x, cell.hi[1]), __dmul_rn(y, cell.hi[4])), __dmul_rn(z, cell.hi[7]));
-    const double sc = __dadd_rn(__dadd_rn(__dmul_rn(x, cell.hi[2]), __dmul_rn(y, cell.hi[5])), __dmul_rn(z, cell.hi[8]));
-    int ia, ib, ic;
-    scaled(sa, a.Na, ia, fa);
-    scaled(sb, a.Nb, ib, fb);
-    scaled(sc, a.Nc, ic, fc);
-    la = ia - ni + 1;
-    if (la < 0) la += a.Na;
-    lb = ib - ni + 1;
-    if (lb < 0) lb += a.Nb;
-    lc = ic - ni + 1;
-    if (lc < 0) lc += a.Nc;
+    stencil_of(a, cell, a.posT[(3 * (size_t)at + 0) * a.P + b], a.posT[(3 * (size_t)at + 1) * a.P + b],
+               a.posT[(3 * (size_t)at + 2) * a.P + b], ni, la, lb, lc, fa, fb, fc);
 }
 
-// Charges binned by the grid tile that holds their stencil origin, per bead.
 // Largest value of the order-n cardinal B-spline (PINY's m[] over the
 // fractional offset, ewald3d_pme.c:301-338), sampled finely: a bound for the
 // fixed-point spread.
-static double bspline_peak(int n)
+static double bspline_peak_of(int n)
 {
     double best = 0.0;
     for (int k = 0; k <= 1024; k++) {
@@ -138,15 +95,16 @@ static double bspline_peak(int n)
     }
     return best * (1.0 + 1e-6);
 }
-
-struct TileArgs {
-    int T;  // tile edge (grid points)
-    float qfix, qfix_inv;  // FP32 spread: fixed-point scale 2^S of the shared tile, and 2^-S
-    int nta, ntb, ntc, ntile, cap;
-    int *cnt;  // [P][ntile], then the overflow count
-    int *bin;  // [P][ntile][cap] record numbers k*P + b
-    int *ovf;  // [nchrg * P] record numbers that did not fit their bin
-};
+static double bspline_peak(int n)
+{
+    // once per order: 1025 samples of the recursion are 50 us of host time
+    static const std::vector<double> peak = [] {
+        std::vector<double> p(13, 0.0);
+        for (int k = 3; k <= 12; k++) p[k] = bspline_peak_of(k);
+        return p;
+    }();
+    return peak[std::min(12, std::max(3, n))];
+}
 
 // Per (charge k, bead b) record, number idx = k*P + b, written by the bin
 // kernel and read by spread and gather:
@@ -708,21 +666,8 @@ __device__ __forceinline__ void pme_bin_compact_body(const PmeArgs &a, const Cel
     const int b = (int)(idx % a.P);
     const int k = (int)(idx / a.P);
     const int at = a.ichrg[k];
-    int la, lb, lc;
-    double fa, fb, fc;
-    stencil_origin(a, cell, at, b, NI, la, lb, lc, fa, fb, fc);
-    typename Vec4<R>::T fr;
-    fr.x = (R)fa;
-    fr.y = (R)fb;
-    fr.z = (R)fc;
-    fr.w = (R)a.charge[at];
-    ((typename Vec4<R>::T *)a.rw)[idx] = fr;
-    a.rhead[idx] = make_int4(at, la, lb, lc);
-    const int T = t.T;
-    const int tile = ((lc / T) * t.ntb + lb / T) * t.nta + la / T;
-    const int slot = atomicAdd(&t.cnt[b * t.ntile + tile], 1);
-    if (slot < t.cap) t.bin[((size_t)b * t.ntile + tile) * t.cap + slot] = (int)idx;
-    else t.ovf[atomicAdd(&t.cnt[a.P * t.ntile], 1)] = (int)idx;
+    pme_file_record<R>(a, t, cell, at, k, b, a.posT[(3 * (size_t)at + 0) * a.P + b],
+                       a.posT[(3 * (size_t)at + 1) * a.P + b], a.posT[(3 * (size_t)at + 2) * a.P + b]);
 }
 
 template <typename R, int NI>
@@ -792,7 +737,7 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
     for (int i = threadIdx.x; i < TG::NPT; i += blockDim.x) tl[i] = (R)0;
     pt.fill(false);
     __syncthreads();
-    const int tile = vb.x, b = vb.y;
+    const int tile = vb.x, b = vb.y / t.nshare, z = vb.y - b * t.nshare;
     const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int la8 = lane & 7, lb4 = lane >> 3;
@@ -801,16 +746,17 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
     R *g = (R *)a.grid + (size_t)b * a.Na * a.Nb * a.Nc;
     int4 hn = make_int4(0, 0, 0, 0);
     R4 fn = {};
-    if (warp < n) {
-        const int idx = list[warp];
+    const int e0 = z * nwarp + warp, estep = nwarp * t.nshare;
+    if (e0 < n) {
+        const int idx = list[e0];
         hn = a.rhead[idx];
         fn = load_frac<R>(a.rw, idx);
     }
-    for (int e = warp; e < n; e += nwarp) {
+    for (int e = e0; e < n; e += estep) {
         const int4 h = hn;
         const R4 fr = fn;
-        if (e + nwarp < n) {
-            const int idx = list[e + nwarp];
+        if (e + estep < n) {
+            const int idx = list[e + estep];
             hn = a.rhead[idx];
             fn = load_frac<R>(a.rw, idx);
         }
@@ -831,15 +777,13 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
                     for (int i = 0; i < NTB; i++) {
                         if (lb4 + 4 * i >= NI) continue;
                         const int o = off0 + (tc * TG::E + 4 * i) * TG::PA + 8 * s;
-                        if constexpr (sizeof(R) == 4) {
+                        {
                             // fixed point: v 2^S + 1.5 2^23 is exact to the nearest
                             // integer for |v 2^S| < 2^22, whose bits less those of
                             // 1.5 2^23 are that integer; integer shared atomics run
                             // at twice the rate of FP32 ones
                             const float y = fmaf(cq * w.mb[i], t.qfix, 12582912.0f);
                             atomicAdd((int *)tl + o, __float_as_int(y) - 0x4B400000);
-                        } else {
-                            atomicAdd(tl + o, cq * w.mb[i]);
                         }
                     }
                 }
@@ -881,12 +825,124 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
             const int cz = row / TG::E, by = row - cz * TG::E;
             R *dst = g + ((size_t)wrapi(tc0 + cz, a.Nc) * a.Nb + wrapi(tb0 + by, a.Nb)) * a.Na;
             for (int ax = lane; ax < TG::E; ax += 32) {
-                R v;
-                if constexpr (sizeof(R) == 4) v = (R)((float)((const int *)tl)[row * TG::PA + ax] * t.qfix_inv);
-                else v = tl[row * TG::PA + ax];
+                const R v = (float)((const int *)tl)[row * TG::PA + ax] * t.qfix_inv;
                 if (v != (R)0) atomicAdd(dst + wrapi(ta0 + ax, a.Na), v);
             }
         }
+    }
+}
+
+// FP64 spread: shared FP64 atomics are compare-and-swap loops, so here every
+// c plane of the shared tile belongs to one warp (plane c to warp c mod 8)
+// and is added to by plain loads and stores.  The block stages 32 records'
+// weights at a time in shared memory (8 threads a record, one barrier a
+// batch); each warp then walks the records, whose stencil holds one plane of
+// its own for every order up to 8, and adds its 8 a x 8 b points, 32 at a
+// time.  4096 TIP4P/F x 32 beads, 64^3, order 8: 525 us with atomics.
+template <int NI, int TT>
+constexpr size_t spread_own_smem()
+{
+    return sizeof(double) * ((size_t)TileGeom<NI, TT>::NPT + 2 * 32 * 3 * RecGeom<NI>::NIP);
+}
+
+template <int NI, int TT>
+__global__ void __launch_bounds__(256, 2) spread_own_kernel(const __grid_constant__ PmeArgs a,
+                                                            const __grid_constant__ TileArgs t)
+{
+    typedef TileGeom<NI, TT> TG;
+    constexpr int NIP = RecGeom<NI>::NIP, NTB = (NI + 3) / 4, NS8 = (NI + 7) / 8;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *tl = (double *)smem_raw;
+    double *wst = tl + TG::NPT;  // [2][32][3][NIP]: M_a, M_b, q M_c by stencil point
+    __shared__ __align__(16) PolyTab<double, NI> pt;
+    __shared__ int4 org[2][32];  // stencil origin in the tile, record number (~record: outside the tile)
+    for (int i = threadIdx.x; i < TG::NPT; i += 256) tl[i] = 0.0;
+    pt.fill(false);
+    __syncthreads();
+    const int tile = blockIdx.x, b = blockIdx.y / t.nshare, z = blockIdx.y - b * t.nshare;
+    const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int la8 = lane & 7, lb4 = lane >> 3;
+    const int n = min(t.cnt[b * t.ntile + tile], t.cap);
+    const int *list = t.bin + ((size_t)b * t.ntile + tile) * t.cap;
+    double *g = (double *)a.grid + (size_t)b * a.Na * a.Nb * a.Nc;
+    int buf = 0;
+    for (int e0 = 32 * z; e0 < n; e0 += 32 * t.nshare, buf ^= 1) {
+        const int nb = min(32, n - e0);
+        {
+            const int r = threadIdx.x >> 3, j0 = threadIdx.x & 7;
+            if (r < nb) {
+                const int idx = list[e0 + r];
+                const double4 fr = load_frac<double>(a.rw, idx);
+                double *w = wst + (buf * 32 + r) * 3 * NIP;
+#pragma unroll
+                for (int s = 0; s < NS8; s++) {
+                    const int j = j0 + 8 * s;
+                    if (j >= NI) break;
+                    w[j] = poly_eval<double, NI>(pt.m[NI - 1 - j], fr.x);
+                    w[NIP + j] = poly_eval<double, NI>(pt.m[NI - 1 - j], fr.y);
+                    w[2 * NIP + j] = fr.w * poly_eval<double, NI>(pt.m[NI - 1 - j], fr.z);
+                }
+                if (j0 == 0) {
+                    const int4 h = a.rhead[idx];
+                    const int oa = h.y - ta0, ob = h.z - tb0, oc = h.w - tc0;
+                    const bool in = oa >= 0 && oa < TG::T && ob >= 0 && ob < TG::T && oc >= 0 && oc < TG::T;
+                    org[buf][r] = make_int4(oa, ob, oc, in ? idx : ~idx);
+                }
+            }
+        }
+        __syncthreads();  // the other buffer's readers are done when its writers come back
+        for (int r = 0; r < nb; r++) {
+            const int4 o = org[buf][r];
+            const double *w = wst + (buf * 32 + r) * 3 * NIP;
+            if (o.w >= 0) {
+#pragma unroll
+                for (int s8 = 0; s8 < NS8; s8++) {
+                    const int p = ((warp - o.z) & 7) + 8 * s8;
+                    if (p >= NI) break;
+                    const double mc = w[2 * NIP + p];
+                    double *row = tl + ((o.z + p) * TG::E + o.y + lb4) * TG::PA + o.x + la8;
+#pragma unroll
+                    for (int s = 0; s < NS8; s++) {
+                        if (la8 + 8 * s >= NI) break;
+                        const double ca = mc * w[la8 + 8 * s];
+#pragma unroll
+                        for (int i = 0; i < NTB; i++)
+                            if (lb4 + 4 * i < NI) row[4 * i * TG::PA + 8 * s] += ca * w[NIP + lb4 + 4 * i];
+                    }
+                }
+            } else if (warp == 0) {
+                // origin outside the tile (none is expected): straight into the grid
+                const int idx = ~o.w;
+                const int4 h = a.rhead[idx];
+                const double4 fr = load_frac<double>(a.rw, idx);
+                SpreadW<double, NI> sw;
+                sw.eval(pt, fr, lane);
+                spread_warp_global<double, NI>(a, g, h.y, h.z, h.w, sw, fr.w, lane);
+            }
+            __syncwarp();
+        }
+    }
+    // overflow records: one warp each, straight into the grid
+    const int nov = t.cnt[a.P * t.ntile];
+    const int gid = blockIdx.y * gridDim.x + blockIdx.x, nblk = gridDim.x * gridDim.y;
+    for (int e = gid * 8 + warp; e < nov; e += nblk * 8) {
+        const int idx = t.ovf[e];
+        const int4 h = a.rhead[idx];
+        const double4 fr = load_frac<double>(a.rw, idx);
+        SpreadW<double, NI> sw;
+        sw.eval(pt, fr, lane);
+        spread_warp_global<double, NI>(a, (double *)a.grid + (size_t)(idx % a.P) * a.Na * a.Nb * a.Nc, h.y, h.z, h.w,
+                                       sw, fr.w, lane);
+    }
+    __syncthreads();
+    constexpr int NROW = TG::E * TG::E;
+    for (int i = threadIdx.x; i < NROW * TG::PA; i += 256) {
+        const double v = tl[i];
+        if (v == 0.0) continue;
+        const int row = i / TG::PA, ax = i - row * TG::PA;
+        const int cz = row / TG::E, by = row - cz * TG::E;
+        atomicAdd(g + ((size_t)wrapi(tc0 + cz, a.Nc) * a.Nb + wrapi(tb0 + by, a.Nb)) * a.Na + wrapi(ta0 + ax, a.Na), v);
     }
 }
 
@@ -946,12 +1002,13 @@ __device__ __forceinline__ void gather_tile_c_body(const PmeArgs &a, const Cell 
     R *tl = (R *)smem_raw;
     __shared__ __align__(16) PolyTab<R, NI> pt;
     pt.fill(true);
-    const int tile = vb.x, b = vb.y;
+    const int tile = vb.x, b = vb.y / t.nshare, z = vb.y - b * t.nshare;
     const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
     const R *g = (const R *)a.grid + (size_t)b * a.Na * a.Nb * a.Nc;
     const int n = min(t.cnt[b * t.ntile + tile], t.cap);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    if (n > 0) {
+    const int grp = threadIdx.x >> 3, l8 = threadIdx.x & 7, ngrp = blockDim.x >> 3;
+    if (n > z * ngrp) {
         constexpr int NROW = TG::E * TG::E;
         if (sizeof(R) == 4 && (a.Na & 3) == 0) {
             constexpr int NQ = TG::PA / 4;
@@ -975,25 +1032,25 @@ __device__ __forceinline__ void gather_tile_c_body(const PmeArgs &a, const Cell 
         }
     }
     __syncthreads();
-    const int grp = threadIdx.x >> 3, l8 = threadIdx.x & 7, ngrp = blockDim.x >> 3;
     const int *list = t.bin + ((size_t)b * t.ntile + tile) * t.cap;
-    const int nr = (n + ngrp - 1) / ngrp;  // same trip count in every group of a warp (shuffles)
+    const int eb = z * ngrp, estep = ngrp * t.nshare;
+    const int nr = n > eb ? (n - eb + estep - 1) / estep : 0;  // same trip count in every group of a warp (shuffles)
     int4 hn = make_int4(0, 0, 0, 0);
     R4 fn = {};
     int in = 0;
-    if (grp < n) {
-        in = list[grp];
+    if (eb + grp < n) {
+        in = list[eb + grp];
         hn = a.rhead[in];
         fn = load_frac<R>(a.rw, in);
     }
     for (int r = 0; r < nr; r++) {
-        const int e = r * ngrp + grp;
+        const int e = eb + r * estep + grp;
         const bool act = e < n;
         const int idx = in;
         const int4 h = hn;
         const R4 fr = fn;
-        if (e + ngrp < n) {
-            in = list[e + ngrp];
+        if (e + estep < n) {
+            in = list[e + estep];
             hn = a.rhead[in];
             fn = load_frac<R>(a.rw, in);
         }
@@ -1495,7 +1552,7 @@ static cudaError_t launch_fft_rt(pinyb200_ctx *c, const PmeArgs &a, const Cell &
 }
 
 // Kernel arguments of a context's PME mesh.
-static PmeArgs pme_args_of(pinyb200_ctx *c)
+PmeArgs pme_args_of(pinyb200_ctx *c)
 {
     const DeviceSystem &s = c->sys;
     PmeArgs a;
@@ -1543,9 +1600,18 @@ static cudaError_t launch_fft(pinyb200_ctx *c, const PmeArgs &a, const Cell &cel
     return launch_fft_rt<R>(c, a, cell, spec, filt, tw, sp, ss, energy);
 }
 
+// Zeroes the charge grid.
+cudaError_t launch_pme_clear(pinyb200_ctx *c)
+{
+    if (c->sys.nchrg == 0 || c->sys.nktot == 0) return cudaSuccess;
+    const size_t G = (size_t)c->sys.ngrid[0] * c->sys.ngrid[1] * c->sys.ngrid[2];
+    return cudaMemsetAsync(c->d_grid, 0, (c->precision == PINYB200_FP64 ? sizeof(double) : sizeof(float)) * G * c->P,
+                           c->stream);
+}
+
 // Tile binning arguments of a context's PME mesh for spline order NI and
 // tile edge TT.
-static TileArgs tile_args_of(pinyb200_ctx *c, int NI, int TT)
+TileArgs tile_args_of(pinyb200_ctx *c, int NI, int TT)
 {
     TileArgs t;
     t.T = TT;
@@ -1562,6 +1628,10 @@ static TileArgs tile_args_of(pinyb200_ctx *c, int NI, int TT)
         t.qfix = (float)std::ldexp(1.0, S);
         t.qfix_inv = (float)std::ldexp(1.0, -S);
     }
+    // few bins (small meshes of few beads): several blocks per bin, each with
+    // at least 16 of its records on average
+    const int bins = c->pme_ntile * c->P, mean = c->sys.nchrg / std::max(1, c->pme_ntile);
+    t.nshare = std::max(1, std::min(std::min(4, 2 * c->sm_count / std::max(1, bins)), mean / 16));
     t.nta = c->pme_nt[0];
     t.ntb = c->pme_nt[1];
     t.ntc = c->pme_nt[2];
@@ -1574,29 +1644,37 @@ static TileArgs tile_args_of(pinyb200_ctx *c, int NI, int TT)
 }
 
 template <typename R, int NI, int TT>
-static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy)
+static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy, bool staged)
 {
     typedef typename Cplx<R>::T C2;
     const PmeArgs a = pme_args_of(c);
     const size_t G = (size_t)a.Na * a.Nb * a.Nc;
-    const bool f64 = sizeof(R) == 8;
-    cudaError_t err = cudaMemsetAsync(c->d_grid, 0, sizeof(R) * G * c->P, c->stream);
-    if (err != cudaSuccess) return err;
-    if ((err = kt_mark(c, "pme_grid_clear (memset)")) != cudaSuccess) return err;
+    constexpr bool f64 = sizeof(R) == 8;
     const TileArgs t = tile_args_of(c, NI, TT);
-    err = cudaMemsetAsync(t.cnt, 0, ((size_t)a.P * t.ntile + 1) * sizeof(int), c->stream);
-    if (err != cudaSuccess) return err;
-    const long long nt = (long long)a.nchrg * a.P;
-    const int threads = 256;
     // the parameter adjoint reads the full weight records of the forward pass
     const bool full = c->pme_full_records;
-    if (full) pme_bin_kernel<R, NI><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
-    else pme_bin_compact_kernel<R, NI><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
-    if ((err = kt_mark(c, "pme_bin")) != cudaSuccess) return err;
+    cudaError_t err = cudaSuccess;
+    if (!staged) {
+        err = launch_pme_clear(c);
+        if (err != cudaSuccess) return err;
+        if ((err = kt_mark(c, "pme_grid_clear (memset)")) != cudaSuccess) return err;
+        err = cudaMemsetAsync(t.cnt, 0, ((size_t)a.P * t.ntile + 1) * sizeof(int), c->stream);
+        if (err != cudaSuccess) return err;
+        const long long nt = (long long)a.nchrg * a.P;
+        const int threads = 256;
+        if (full) pme_bin_kernel<R, NI><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
+        else pme_bin_compact_kernel<R, NI><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
+        if ((err = kt_mark(c, "pme_bin")) != cudaSuccess) return err;
+    }
     const size_t st = (size_t)TileGeom<NI, TT>::NPT * sizeof(R), ss_spread = spread_smem<R, NI, TT>();
     if (ss_spread > 48 * 1024 - sizeof(PolyTab<R, NI>)) {
         err = smem_optin((const void *)spread_tile_kernel<R, NI, TT>, (int)ss_spread);
-        if (err == cudaSuccess) err = smem_optin((const void *)spread_tile_c_kernel<R, NI, TT>, (int)ss_spread);
+        if constexpr (!f64)
+            if (err == cudaSuccess) err = smem_optin((const void *)spread_tile_c_kernel<R, NI, TT>, (int)ss_spread);
+        if (err != cudaSuccess) return err;
+    }
+    if constexpr (f64) {
+        err = smem_optin((const void *)spread_own_kernel<NI, TT>, (int)spread_own_smem<NI, TT>());
         if (err != cudaSuccess) return err;
     }
     if (st > 48 * 1024 - sizeof(PolyTab<R, NI>)) {
@@ -1604,8 +1682,10 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy)
         if (err == cudaSuccess) err = smem_optin((const void *)gather_tile_c_kernel<R, NI, TT>, (int)st);
         if (err != cudaSuccess) return err;
     }
-    const dim3 tgrid((unsigned)t.ntile, (unsigned)a.P);
-    if (full) spread_tile_kernel<R, NI, TT><<<tgrid, 256, ss_spread, c->stream>>>(a, t);
+    const dim3 tgrid((unsigned)t.ntile, (unsigned)(a.P * t.nshare));
+    const dim3 tgrid1((unsigned)t.ntile, (unsigned)a.P);  // the full-record kernels: one block per bin
+    if (full) spread_tile_kernel<R, NI, TT><<<tgrid1, 256, ss_spread, c->stream>>>(a, t);
+    else if constexpr (f64) spread_own_kernel<NI, TT><<<tgrid, 256, spread_own_smem<NI, TT>(), c->stream>>>(a, t);
     else spread_tile_c_kernel<R, NI, TT><<<tgrid, 256, ss_spread, c->stream>>>(a, t);
     if ((err = kt_mark(c, "pme_spread")) != cudaSuccess) return err;
     const R *twbase = (const R *)(f64 ? (const void *)c->d_twiddle64 : (const void *)c->d_twiddle32);
@@ -1615,30 +1695,31 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy)
     const R *filt = f64 ? (const R *)c->d_filter : (const R *)((const double *)c->d_filter + G);
     err = launch_fft<R>(c, a, cell, spec, filt, tw, sp, ss, energy);
     if (err != cudaSuccess) return err;
-    if (full) gather_tile_kernel<R, NI, TT><<<tgrid, 256, st, c->stream>>>(a, cell, t);
+    if (full) gather_tile_kernel<R, NI, TT><<<tgrid1, 256, st, c->stream>>>(a, cell, t);
     else gather_tile_c_kernel<R, NI, TT><<<tgrid, 256, st, c->stream>>>(a, cell, t);
     if ((err = kt_mark(c, "pme_gather")) != cudaSuccess) return err;
     return cudaGetLastError();
 }
 
 template <typename R, int TT>
-static cudaError_t launch_pme_rt(pinyb200_ctx *c, const Cell &cell, bool energy)
+static cudaError_t launch_pme_rt(pinyb200_ctx *c, const Cell &cell, bool energy, bool staged)
 {
     switch (c->sys.n_interp) {
-    case 4: return launch_pme_t<R, 4, TT>(c, cell, energy);
-    case 5: return launch_pme_t<R, 5, TT>(c, cell, energy);
-    case 6: return launch_pme_t<R, 6, TT>(c, cell, energy);
-    case 7: return launch_pme_t<R, 7, TT>(c, cell, energy);
-    case 8: return launch_pme_t<R, 8, TT>(c, cell, energy);
-    case 10: return launch_pme_t<R, 10, TT>(c, cell, energy);
+    case 4: return launch_pme_t<R, 4, TT>(c, cell, energy, staged);
+    case 5: return launch_pme_t<R, 5, TT>(c, cell, energy, staged);
+    case 6: return launch_pme_t<R, 6, TT>(c, cell, energy, staged);
+    case 7: return launch_pme_t<R, 7, TT>(c, cell, energy, staged);
+    case 8: return launch_pme_t<R, 8, TT>(c, cell, energy, staged);
+    case 10: return launch_pme_t<R, 10, TT>(c, cell, energy, staged);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename R>
-static cudaError_t launch_pme_r(pinyb200_ctx *c, const Cell &cell, bool energy)
+static cudaError_t launch_pme_r(pinyb200_ctx *c, const Cell &cell, bool energy, bool staged)
 {
-    return c->pme_tile == 8 ? launch_pme_rt<R, 8>(c, cell, energy) : launch_pme_rt<R, 16>(c, cell, energy);
+    return c->pme_tile == 8 ? launch_pme_rt<R, 8>(c, cell, energy, staged)
+                            : launch_pme_rt<R, 16>(c, cell, energy, staged);
 }
 
 cudaError_t launch_pme_force_add(pinyb200_ctx *c)
@@ -1660,7 +1741,7 @@ cudaError_t launch_pme_force_add_scaled(pinyb200_ctx *c, double w, double *targe
     return cudaGetLastError();
 }
 
-cudaError_t launch_pme(pinyb200_ctx *c, const Cell &cell, bool energy)
+cudaError_t launch_pme(pinyb200_ctx *c, const Cell &cell, bool energy, bool staged)
 {
     if (c->sys.nchrg == 0 || c->sys.nktot == 0) return cudaSuccess;
     const size_t G = (size_t)c->sys.ngrid[0] * c->sys.ngrid[1] * c->sys.ngrid[2];
@@ -1673,8 +1754,8 @@ cudaError_t launch_pme(pinyb200_ctx *c, const Cell &cell, bool energy)
         for (int i = 0; i < 9; i++) c->filter_h[i] = cell.h[i];
         c->filter_ok = true;
     }
-    if (c->precision == PINYB200_FP64) return launch_pme_r<double>(c, cell, energy);
-    return launch_pme_r<float>(c, cell, energy);
+    if (c->precision == PINYB200_FP64) return launch_pme_r<double>(c, cell, energy, staged);
+    return launch_pme_r<float>(c, cell, energy, staged);
 }
 
 // ---------------------------------------------------------------------------
@@ -1776,7 +1857,7 @@ static cudaError_t pme_batch_tiles(const std::vector<PmeBox> &bx, const std::vec
     for (size_t i = 0; i < bx.size(); i++) {
         const double work = (double)bx[i].a.nchrg * P[i];
         if (stage == 0) tb.add(bx[i], (int)(((long long)bx[i].a.nchrg * P[i] + 255) / 256), 1, work);
-        else tb.add(bx[i], bx[i].t.ntile, P[i], work);
+        else tb.add(bx[i], bx[i].t.ntile, P[i] * bx[i].t.nshare, work);
     }
     if (stage == 0)
         return launch_tables(tb, (const void *)pme_bin_batch_kernel<R, NI>, 256, 0, sm_count,
@@ -2031,121 +2112,155 @@ __global__ void __launch_bounds__(256) pme_dipole_spread_kernel(PmeArgs a, Cell 
     }
 }
 
-// Gathers phi, grad phi, chi, grad chi (and grad grad phi at sites with a
-// ghost tangent) per record and contracts them with every channel.
+// Value and gradient of a potential g at one record, this lane's a points:
+// s[0] = sum M M M phi, s[1..3] with the derivative along a, b, c.
 template <typename R, int NI>
-__global__ void __launch_bounds__(128) pme_adjoint_gather_kernel(PmeArgs a, Cell cell, GradArgs g,
+__device__ __forceinline__ void adjoint_lane(const PmeArgs &a, const R *g, const int4 &h, const LaneW<R, NI, true> &lw,
+                                             int l8, double *s)
+{
+    s[0] = s[1] = s[2] = s[3] = 0.0;
+#pragma unroll
+    for (int j = 0; j < (NI > 8 ? 2 : 1); j++) {
+        if (l8 + 8 * j >= NI) break;
+        const int ga = wrapi(h.y + l8 + 8 * j, a.Na);
+        R smm = 0, sdm = 0, smd = 0;
+#pragma unroll
+        for (int tc = 0; tc < NI; tc++) {
+            const R *pc = g + (size_t)wrapi(h.w + tc, a.Nc) * a.Nb * a.Na + ga;
+            R um = 0, ud = 0;
+#pragma unroll
+            for (int tb = 0; tb < NI; tb++) {
+                const R p = __ldg(pc + (size_t)wrapi(h.z + tb, a.Nb) * a.Na);
+                um += lw.mb[tb] * p;
+                ud += lw.db[tb] * p;
+            }
+            smm += lw.mc[tc] * um;
+            sdm += lw.mc[tc] * ud;
+            smd += lw.dc[tc] * um;
+        }
+        const R wa = j ? lw.wa1 : lw.wa0, da = j ? lw.da1 : lw.da0;
+        s[0] += (double)(wa * smm);
+        s[1] += (double)(da * smm);
+        s[2] += (double)(wa * sdm);
+        s[3] += (double)(wa * smd);
+    }
+}
+
+// Gathers phi, grad phi, chi, grad chi (and grad grad phi at sites with a
+// ghost tangent) per record and contracts them with every channel.  Blocks
+// take a bin's records (tile, bead, one of gridDim.z shares), whose stencils
+// overlap in L1; 8 lanes a record, a lane an a point, as in the gather: the
+// weights along a factor out and a row is one 32-byte sector.  Bound: L1/L2
+// sector reads, 128 per record.  1024 TIP4P/F x 16 beads, 32^3, FP32: 277 us
+// as one thread per record in record order.
+template <typename R, int NI>
+__global__ void __launch_bounds__(256) pme_adjoint_gather_kernel(const __grid_constant__ PmeArgs a,
+                                                                 const __grid_constant__ Cell cell,
+                                                                 const __grid_constant__ TileArgs t,
+                                                                 const __grid_constant__ GradArgs g,
                                                                  const R *__restrict__ phi, const R *__restrict__ chi)
 {
-    typedef RecGeom<NI> RG;
     __shared__ double sh[2 * PINYB200_MAX_TAN];
     double acc[2 * PINYB200_MAX_TAN];
     for (int k = 0; k < 2 * g.K; k++) acc[k] = 0.0;
-    const long long nrec = (long long)a.nchrg * a.P;
     const size_t G = (size_t)a.Na * a.Nb * a.Nc;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < nrec;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(idx % a.P);
-        const int4 h = a.rhead[idx];
-        const int at = h.x;
-        R m[6][RG::NIP];
-        const R *w = (const R *)a.rw + (size_t)idx * RG::NW;
-#pragma unroll
-        for (int j = 0; j < 6; j++) load4<RG::NIP>(m[j], w + j * RG::NIP);
-        const R *pg = phi + (size_t)b * G, *cg = chi + (size_t)b * G;
-        double P0 = 0, Pa = 0, Pb = 0, Pc = 0, X0 = 0, Xa = 0, Xb = 0, Xc = 0;
-#pragma unroll 1
-        for (int tc = 0; tc < NI; tc++) {
-            const int gc = wrapi(h.w + tc, a.Nc);
-            R p0 = 0, pa = 0, pb = 0, pc = 0, x0 = 0, xa = 0, xb = 0, xc = 0;
-#pragma unroll
-            for (int tb = 0; tb < NI; tb++) {
-                const size_t row = ((size_t)gc * a.Nb + wrapi(h.z + tb, a.Nb)) * a.Na;
-                R sp = 0, sdp = 0, sx = 0, sdx = 0;
-#pragma unroll
-                for (int t_a = 0; t_a < NI; t_a++) {
-                    const int ga = wrapi(h.y + t_a, a.Na);
-                    const R pv = pg[row + ga], xv = cg[row + ga];
-                    sp += m[0][t_a] * pv;
-                    sdp += m[3][t_a] * pv;
-                    sx += m[0][t_a] * xv;
-                    sdx += m[3][t_a] * xv;
+    const int l8 = threadIdx.x & 7, grp = threadIdx.x >> 3, ngrp = blockDim.x >> 3;
+    // one record (idx of bead b) by the 8 lanes of a group; every lane of the
+    // warp calls it (shuffles)
+    auto record = [&](bool act, int idx, int b) {
+        int4 h = make_int4(0, 0, 0, 0);
+        LaneW<R, NI, true> lw;
+        double s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, hs[6] = {0, 0, 0, 0, 0, 0};
+        bool need_h = false;
+        if (act) {
+            h = a.rhead[idx];
+            lw.load((const R *)a.rw, idx, l8);
+            adjoint_lane<R, NI>(a, phi + (size_t)b * G, h, lw, l8, s);
+            adjoint_lane<R, NI>(a, chi + (size_t)b * G, h, lw, l8, s + 4);
+            // the ghost-position tangents of this site, if any
+            for (int k = 0; k < g.K; k++)
+                if (g.ch[k].w) {
+                    const double *wv = g.ch[k].w + (3 * (size_t)h.x) * a.P + b;
+                    need_h |= wv[0] != 0.0 || wv[a.P] != 0.0 || wv[2 * a.P] != 0.0;
                 }
-                p0 += m[1][tb] * sp;
-                pa += m[1][tb] * sdp;
-                pb += m[4][tb] * sp;
-                x0 += m[1][tb] * sx;
-                xa += m[1][tb] * sdx;
-                xb += m[4][tb] * sx;
-                (void)pc;
-                (void)xc;
-            }
-            P0 += (double)(m[2][tc] * p0);
-            Pa += (double)(m[2][tc] * pa);
-            Pb += (double)(m[2][tc] * pb);
-            Pc += (double)(m[5][tc] * p0);
-            X0 += (double)(m[2][tc] * x0);
-            Xa += (double)(m[2][tc] * xa);
-            Xb += (double)(m[2][tc] * xb);
-            Xc += (double)(m[5][tc] * x0);
         }
+        if (act && need_h) {
+            int la, lb, lc;
+            double fa, fb, fc;
+            stencil_origin(a, cell, h.x, b, NI, la, lb, lc, fa, fb, fc);
+            R d2[NI + 1], d2b[NI], d2c[NI];
+            bspline_d2<R, NI>((R)fb, d2);
+#pragma unroll
+            for (int k = 0; k < NI; k++) d2b[k] = d2[NI - k];  // grid order: point lo + t carries index NI - t
+            bspline_d2<R, NI>((R)fc, d2);
+#pragma unroll
+            for (int k = 0; k < NI; k++) d2c[k] = d2[NI - k];
+            bspline_d2<R, NI>((R)fa, d2);
+            const R *pg = phi + (size_t)b * G;
+#pragma unroll
+            for (int j = 0; j < (NI > 8 ? 2 : 1); j++) {
+                const int ta = l8 + 8 * j;
+                if (ta >= NI) break;
+                R d2a = 0;
+#pragma unroll
+                for (int k = 0; k < NI; k++)
+                    if (k == ta) d2a = d2[NI - k];
+                const int ga = wrapi(h.y + ta, a.Na);
+                double smm = 0, s2m = 0, sm2 = 0, sdm = 0, smd = 0, sdd = 0;  // b and c weights
+#pragma unroll
+                for (int tc = 0; tc < NI; tc++) {
+                    const R *pc = pg + (size_t)wrapi(h.w + tc, a.Nc) * a.Nb * a.Na + ga;
+                    double um = 0, ud = 0, u2 = 0;
+#pragma unroll
+                    for (int tb = 0; tb < NI; tb++) {
+                        const double p = (double)__ldg(pc + (size_t)wrapi(h.z + tb, a.Nb) * a.Na);
+                        um += (double)lw.mb[tb] * p;
+                        ud += (double)lw.db[tb] * p;
+                        u2 += (double)d2b[tb] * p;
+                    }
+                    smm += (double)lw.mc[tc] * um;
+                    s2m += (double)lw.mc[tc] * u2;
+                    sm2 += (double)d2c[tc] * um;
+                    sdm += (double)lw.mc[tc] * ud;
+                    smd += (double)lw.dc[tc] * um;
+                    sdd += (double)lw.dc[tc] * ud;
+                }
+                const double wa = j ? lw.wa1 : lw.wa0, da = j ? lw.da1 : lw.da0;
+                hs[0] += (double)d2a * smm;
+                hs[1] += wa * s2m;
+                hs[2] += wa * sm2;
+                hs[3] += da * sdm;
+                hs[4] += da * smd;
+                hs[5] += wa * sdd;
+            }
+        }
+#pragma unroll
+        for (int o = 4; o >= 1; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        }
+        if (__any_sync(0xffffffffu, need_h)) {
+#pragma unroll
+            for (int o = 4; o >= 1; o >>= 1) {
+#pragma unroll
+                for (int k = 0; k < 6; k++) hs[k] += __shfl_xor_sync(0xffffffffu, hs[k], o);
+            }
+        }
+        if (!act || l8 != 0) return;
+        const int at = h.x;
         const double ux = g.uT[(3 * (size_t)at + 0) * a.P + b], uy = g.uT[(3 * (size_t)at + 1) * a.P + b],
                      uz = g.uT[(3 * (size_t)at + 2) * a.P + b];
         double ut[3];
         scaled_vec(a, cell, ux, uy, uz, ut);
-        const double udphi = ut[0] * Pa + ut[1] * Pb + ut[2] * Pc;
+        const double udphi = ut[0] * s[1] + ut[1] * s[2] + ut[2] * s[3];
         const double q = a.charge[at];
-        // the ghost-position tangents of this site, if any
-        bool need_h = false;
-        for (int k = 0; k < g.K; k++)
-            if (g.ch[k].w) {
-                const double *wv = g.ch[k].w;
-                if (wv[(3 * (size_t)at) * a.P + b] != 0.0 || wv[(3 * (size_t)at + 1) * a.P + b] != 0.0 ||
-                    wv[(3 * (size_t)at + 2) * a.P + b] != 0.0)
-                    need_h = true;
-            }
-        double H[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        if (need_h) {
-            int la, lb, lc;
-            double fa, fb, fc;
-            stencil_origin(a, cell, at, b, NI, la, lb, lc, fa, fb, fc);
-            R d2[3][NI + 1];
-            bspline_d2<R, NI>((R)fa, d2[0]);
-            bspline_d2<R, NI>((R)fb, d2[1]);
-            bspline_d2<R, NI>((R)fc, d2[2]);
-            // grid order: point lo + t carries index NI - t
-            double haa = 0, hbb = 0, hcc = 0, hab = 0, hac = 0, hbc = 0;
-            for (int tc = 0; tc < NI; tc++) {
-                const int gc = wrapi(h.w + tc, a.Nc);
-                for (int tb = 0; tb < NI; tb++) {
-                    const size_t row = ((size_t)gc * a.Nb + wrapi(h.z + tb, a.Nb)) * a.Na;
-                    for (int t_a = 0; t_a < NI; t_a++) {
-                        const double pv = (double)pg[row + wrapi(h.y + t_a, a.Na)];
-                        const double ma = m[0][t_a], mb = m[1][tb], mc = m[2][tc];
-                        const double da = m[3][t_a], db = m[4][tb], dc = m[5][tc];
-                        haa += (double)d2[0][NI - t_a] * mb * mc * pv;
-                        hbb += ma * (double)d2[1][NI - tb] * mc * pv;
-                        hcc += ma * mb * (double)d2[2][NI - tc] * pv;
-                        hab += da * db * mc * pv;
-                        hac += da * mb * dc * pv;
-                        hbc += ma * db * dc * pv;
-                    }
-                }
-            }
-            H[0][0] = haa;
-            H[1][1] = hbb;
-            H[2][2] = hcc;
-            H[0][1] = H[1][0] = hab;
-            H[0][2] = H[2][0] = hac;
-            H[1][2] = H[2][1] = hbc;
-        }
         for (int k = 0; k < g.K; k++) {
             const GradChan &ch = g.ch[k];
             if (ch.dq) {
                 const double dq = ch.dq[at];
                 if (dq != 0.0) {
-                    acc[2 * k] += dq * P0 / (double)a.P;
-                    acc[2 * k + 1] += -dq * (udphi + X0);
+                    acc[2 * k] += dq * s[0] / (double)a.P;
+                    acc[2 * k + 1] += -dq * (udphi + s[4]);
                 }
             }
             if (ch.w && need_h) {
@@ -2153,18 +2268,37 @@ __global__ void __launch_bounds__(128) pme_adjoint_gather_kernel(PmeArgs a, Cell
                              wz = ch.w[(3 * (size_t)at + 2) * a.P + b];
                 double wt[3];
                 scaled_vec(a, cell, wx, wy, wz, wt);
-                double uhw = 0;
-                for (int d = 0; d < 3; d++)
-                    for (int e = 0; e < 3; e++) uhw += ut[d] * H[d][e] * wt[e];
-                acc[2 * k + 1] += -q * (wt[0] * Xa + wt[1] * Xb + wt[2] * Xc + uhw);
+                const double uhw = ut[0] * (hs[0] * wt[0] + hs[3] * wt[1] + hs[4] * wt[2]) +
+                                   ut[1] * (hs[3] * wt[0] + hs[1] * wt[1] + hs[5] * wt[2]) +
+                                   ut[2] * (hs[4] * wt[0] + hs[5] * wt[1] + hs[2] * wt[2]);
+                acc[2 * k + 1] += -q * (wt[0] * s[5] + wt[1] * s[6] + wt[2] * s[7] + uhw);
             }
         }
+    };
+    const int tile = blockIdx.x, b = blockIdx.y;
+    const int n = min(t.cnt[b * t.ntile + tile], t.cap);
+    const int *list = t.bin + ((size_t)b * t.ntile + tile) * t.cap;
+    const int step = ngrp * gridDim.z;
+    for (int e0 = ngrp * blockIdx.z; e0 < n; e0 += step) {
+        const int e = e0 + grp;
+        record(e < n, e < n ? list[e] : 0, b);
     }
-    // block flush
+    const int nov = t.cnt[a.P * t.ntile];
+    const int gid = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    const int nblk = gridDim.x * gridDim.y * gridDim.z;
+    for (int e0 = gid * ngrp; e0 < nov; e0 += nblk * ngrp) {
+        const int e = e0 + grp, idx = e < nov ? t.ovf[e] : 0;
+        record(e < nov, idx, idx % a.P);
+    }
+    // block flush: warp sums (lanes other than a group's first hold zeros)
     for (int i = threadIdx.x; i < 2 * g.K; i += blockDim.x) sh[i] = 0.0;
     __syncthreads();
-    for (int i = 0; i < 2 * g.K; i++)
-        if (acc[i] != 0.0) atomicAdd(&sh[i], acc[i]);
+    for (int i = 0; i < 2 * g.K; i++) {
+        const double v = acc[i];
+        if (!__any_sync(0xffffffffu, v != 0.0)) continue;
+        const double w = warp_sum(v);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&sh[i], w);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * g.K; i += blockDim.x)
         if (sh[i] != 0.0) atomicAdd(&g.gacc[i], sh[i]);
@@ -2205,10 +2339,12 @@ static cudaError_t launch_pme_adjoint_t(pinyb200_ctx *c, const Cell &cell, const
     const R *filt = f64 ? (const R *)c->d_filter : (const R *)((const double *)c->d_filter + G);
     err = launch_fft<R>(c, a, cell, spec, filt, tw, sp, ss, false);
     if (err != cudaSuccess) return err;
-    long long gb = (nrec + 127) / 128;
-    if (gb > (long long)c->sm_count * 8) gb = (long long)c->sm_count * 8;
-    pme_adjoint_gather_kernel<R, NI><<<(unsigned)(gb < 1 ? 1 : gb), 128, 0, c->stream>>>(
-        a, cell, g, (const R *)c->d_grid, (const R *)c->grad.d_grid2);
+    const TileArgs t = tile_args_of(c, NI, c->pme_tile);
+    // a bin's records shared by as many blocks as give every SM some eight
+    const long long bins = (long long)t.ntile * a.P;
+    const unsigned split = (unsigned)std::max(1LL, std::min(16LL, (8LL * c->sm_count + bins - 1) / bins));
+    pme_adjoint_gather_kernel<R, NI><<<dim3((unsigned)t.ntile, (unsigned)a.P, split), 256, 0, c->stream>>>(
+        a, cell, t, g, (const R *)c->d_grid, (const R *)c->grad.d_grid2);
     return cudaGetLastError();
 }
 

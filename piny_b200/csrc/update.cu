@@ -166,7 +166,7 @@ int list_update_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_xm
             (e = launch_site_from_mol(c, 1, gate, st)) != cudaSuccess)
             return record_error(c, PINYB200_ERR_CUDA, cudaGetErrorString(e));
         const int jpi = c->P >= 32 ? 1 : 32 / c->P;
-        const int ch = PINYB200_MOL_CHUNK * jpi;
+        const int ch = c->mol_iters * jpi;
         const int blocks = (c->nmol + 255) / 256;
         ls_chunk_count_kernel<<<blocks, 256, 0, st>>>(gate, c->nmol, c->d_mrow, ch, c->d_mchunk);
         if ((e = launch_scan(c, gate, c->nmol, 1, c->d_mchunk, c->d_mchunk + c->nmol, nullptr, chunk_tot, st)) !=

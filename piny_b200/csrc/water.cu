@@ -1,0 +1,134 @@
+// Launchers of the staging and finishing kernels (water.cuh).
+#include "water.cuh"
+
+namespace pinyb200 {
+
+// The per-bead sums and the bin counters to zero.
+__global__ void __launch_bounds__(256) water_clear_kernel(double *__restrict__ acc, int nacc, int *__restrict__ cnt,
+                                                          int ncnt)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
+    for (int i = t; i < nacc; i += n) acc[i] = 0.0;
+    for (int i = t; i < ncnt; i += n) cnt[i] = 0;
+}
+
+template <typename R, int NS, bool Q0>
+__global__ void __launch_bounds__(256) water_stage_kernel(const __grid_constant__ StageArgs a,
+                                                          const __grid_constant__ PmeArgs pm,
+                                                          const __grid_constant__ TileArgs t,
+                                                          const __grid_constant__ Cell cell)
+{
+    water_stage_body<R, NS, Q0>(a, pm, t, cell, hw_blk());
+}
+
+template <int NS, bool Q0>
+__global__ void __launch_bounds__(256, 2) water_finish_kernel(const __grid_constant__ FinishArgs a)
+{
+    water_finish_body<NS, Q0>(a, hw_blk());
+}
+
+// Threads per block: 256, fewer (down to 64, and a bead each) while that
+// leaves SMs without a block.
+static int water_threads(const pinyb200_ctx *c)
+{
+    int t = 256;
+    while (t > 64 && t > c->P && (long long)c->nmol * c->P < (long long)t * c->sm_count) t /= 2;
+    return t;
+}
+static size_t water_smem(const pinyb200_ctx *c, int threads)
+{
+    return sizeof(double) * (size_t)c->P * (threads / c->P * 3 * c->mol_stride + 1);
+}
+
+template <typename R>
+static cudaError_t launch_stage_r(pinyb200_ctx *c, const StageArgs &a, const PmeArgs &pm, const TileArgs &t,
+                                  const Cell &cell)
+{
+    const int th = water_threads(c), mb = th / c->P;
+    const unsigned g = (unsigned)((c->nmol + mb - 1) / mb);
+    const size_t sm = water_smem(c, th);
+    if (c->mol_stride == 4) water_stage_kernel<R, 4, false><<<g, th, sm, c->stream>>>(a, pm, t, cell);
+    else if (c->water_q0) water_stage_kernel<R, 3, true><<<g, th, sm, c->stream>>>(a, pm, t, cell);
+    else water_stage_kernel<R, 3, false><<<g, th, sm, c->stream>>>(a, pm, t, cell);
+    return cudaGetLastError();
+}
+
+// Positions (and mode-1 positions d_xmod, nullptr: the bead centroid) staged,
+// sums and bins cleared, charges binned; enqueued on c->stream.
+cudaError_t launch_water_stage(pinyb200_ctx *c, const Cell &cell, const double *d_pos, const double *d_xmod)
+{
+    const bool pme = c->sys.nchrg > 0 && c->sys.nktot > 0;
+    StageArgs a;
+    a.natm = c->sys.natm;
+    a.nmol = c->nmol;
+    a.P = c->P;
+    a.pos = d_pos;
+    a.posT = c->d_posT;
+    a.forceT = c->d_forceT;
+    a.xm_src = c->P > 1 ? d_xmod : nullptr;
+    a.xm_dst = c->d_xmod;
+    a.ext = (unsigned long long *)(c->d_acc + S_EXT);
+    a.gcoef = c->sys.ghost_coef;
+    a.bin = pme ? 1 : 0;
+    PmeArgs pm = {};
+    TileArgs t = {};
+    int ncnt = 0;
+    if (pme) {
+        pm = pme_args_of(c);
+        t = tile_args_of(c, c->sys.n_interp, c->pme_tile);
+        ncnt = c->P * c->pme_ntile + 1;
+    }
+    const int nacc = c->P * S_NSLOT;
+    const int blocks = std::max(1, std::min((std::max(ncnt, nacc) + 255) / 256, c->sm_count));
+    water_clear_kernel<<<blocks, 256, 0, c->stream>>>(c->d_acc, nacc, t.cnt, ncnt);
+    if (c->precision == PINYB200_FP64) return launch_stage_r<double>(c, a, pm, t, cell);
+    return launch_stage_r<float>(c, a, pm, t, cell);
+}
+
+// Intramolecular terms, the sum of all forces and their way out to d_out;
+// keep_site_forces: the complete site forces are kept in c->d_forceT too.
+cudaError_t launch_water_finish(pinyb200_ctx *c, double *d_out, bool energy, bool distrib, bool keep_site_forces)
+{
+    const DeviceSystem &s = c->sys;
+    FinishArgs a;
+    a.natm = s.natm;
+    a.nmol = c->nmol;
+    a.P = c->P;
+    a.posT = c->d_posT;
+    a.forceT = c->d_forceT;
+    a.forceP = s.nchrg > 0 && s.nktot > 0 ? c->d_forceP : nullptr;
+    a.forceT_out = keep_site_forces ? c->d_forceT : nullptr;
+    a.out = d_out;
+    a.acc = c->d_acc;
+    a.energy = energy ? 1 : 0;
+    a.distrib = distrib ? 1 : 0;
+    a.bond_eq = s.bond_eq + c->water_bond;
+    a.bond_c = s.bond_c + 7 * c->water_bond;
+    a.bond_dc = s.bond_dc + 7 * c->water_bond;
+    a.bend_c = s.bend_c + 7 * c->water_bend;
+    a.bend_s = s.bend_s + 7 * c->water_bend;
+    a.bend_dc = s.bend_dc + 7 * c->water_bend;
+    a.bend_ds = s.bend_ds + 7 * c->water_bend;
+    a.ecor_nsplin = s.ecor_nsplin;
+    a.ecor_rmin = s.ecor_rmin;
+    a.ecor_dr = s.ecor_dr;
+    a.ecor_dri = s.ecor_dri;
+    a.ecor_tab = s.necor > 0 ? s.ecor_tab : nullptr;
+    for (int k = 0; k < 4; k++) a.q[k] = k < c->mol_stride ? c->h_charge[k] : 0.0;
+    a.gcoef = s.ghost_coef;
+    const int th = water_threads(c), mb = th / c->P;
+    const unsigned g = (unsigned)((c->nmol + mb - 1) / mb);
+    const size_t sm = water_smem(c, th);
+    auto go = [&](auto *kernel) {
+        // static and dynamic shared memory together may pass 48 KB
+        cudaError_t e = smem_optin((const void *)kernel, (int)sm);
+        if (e != cudaSuccess) return e;
+        kernel<<<g, th, sm, c->stream>>>(a);
+        return cudaGetLastError();
+    };
+    if (c->mol_stride == 4) return go(water_finish_kernel<4, false>);
+    if (c->water_q0) return go(water_finish_kernel<3, true>);
+    return go(water_finish_kernel<3, false>);
+}
+
+}  // namespace pinyb200
