@@ -123,7 +123,7 @@ bool fused_ok(const pinyb200_batch *bt, const double *const *hmat, int flags)
         const double *h = hmat[i];
         const bool ortho = h[1] == 0.0 && h[2] == 0.0 && h[3] == 0.0 && h[5] == 0.0 && h[6] == 0.0 && h[7] == 0.0;
         if (c->precision != PINYB200_MIXED || !c->use_mol || !c->mol_ok || !c->mix_ok || mix_pattern(c) == 0 ||
-            !ortho || c->pme_full_records || c->sm_count != bt->box[0]->sm_count)
+            !ortho || c->sm_count != bt->box[0]->sm_count)
             return false;
     }
     return true;

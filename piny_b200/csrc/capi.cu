@@ -252,12 +252,11 @@ static int pme_alloc(pinyb200_ctx *c, int nbeads, const int *ngrid, int n_interp
             if (rc2) return rc2;
         }
         CK(cudaMalloc(&c->d_pme_ovf, (size_t)std::max(1, d.nchrg) * nbeads * sizeof(int)));
-        // per (charge, bead) records: stencil origin and the six weight rows
-        const int nip = n_interp <= 4 ? 4 : (n_interp <= 8 ? 8 : 12);
+        // per (charge, bead) records: stencil origin, fractional offsets and charge
         const size_t nrec = (size_t)std::max(1, d.nchrg) * nbeads;
         CK(cudaMalloc(&c->d_pme_head, nrec * 4 * sizeof(int)));
         CK(cudaMalloc(&c->d_forceP, nrec * 3 * sizeof(double)));
-        CK(cudaMalloc(&c->d_pme_w, nrec * 6 * nip * rsz));
+        CK(cudaMalloc(&c->d_pme_w, nrec * 4 * rsz));
         // twiddles exp(2 pi i m / N) per axis, 256 entries each
         std::vector<double> tw(2 * 256 * 3, 0.0);
         std::vector<float> tw32(tw.size());
@@ -1053,7 +1052,7 @@ __global__ void centroid_kernel(const double *__restrict__ posT, double *__restr
 // The charge grid is cleared on the PME stream from the start, and PME waits
 // only for the staging, not for a list update.
 static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, const Cell &cell, int flags,
-                         double *d_force, bool timing, double *h_acc)
+                         double *d_force, bool timing, double *h_acc, bool keep)
 {
     const bool energy = !(flags & PINYB200_NO_ENERGY);
     cudaStream_t main_stream = c->stream;
@@ -1094,7 +1093,7 @@ static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_x
     if (timing) CK(ev_rec(c->ev[2], c->stream));
     CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
     if (timing) CK(ev_rec(c->ev[5], c->stream));
-    CK(launch_water_finish(c, d_force, energy, (flags & PINYB200_DISTRIB_GHOSTS) != 0, c->pme_full_records));
+    CK(launch_water_finish(c, d_force, energy, (flags & PINYB200_DISTRIB_GHOSTS) != 0, keep));
     CK(kt_mark(c, "finish (intra, force sum, out)"));
     if (timing) {
         CK(ev_rec(c->ev[3], c->stream));
@@ -1109,11 +1108,11 @@ static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_x
 // One evaluation from device-resident positions to device-resident forces,
 // enqueued on c->stream without host synchronisation (see evaluate_enqueue).
 int pinyb200::enqueue_device(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, const Cell &cell, int flags,
-                             double *d_force, bool timing, double *h_acc)
+                             double *d_force, bool timing, double *h_acc, bool keep)
 {
     c->kt_n = 0;
     CK(kt_mark(c, nullptr));
-    if (c->water_ok && !c->pme_full_records) return water_enqueue(c, d_pos, d_xmod, cell, flags, d_force, timing, h_acc);
+    if (c->water_ok) return water_enqueue(c, d_pos, d_xmod, cell, flags, d_force, timing, h_acc, keep);
     int rc = stage_positions(c, d_pos, d_xmod, cell, flags);
     if (rc) return rc;
     CK(kt_mark(c, "transpose_in"));
@@ -1258,7 +1257,7 @@ int pinyb200_energy_force(pinyb200_ctx *c, const double *pos, const double *xmod
                                     c->kt_n = 0;
                                     CK(kt_mark(c, nullptr));
                                     return water_enqueue(c, c->d_pos_aos, xmod ? c->d_xmod : nullptr, cell, flags & ~PINYB200_UPDATE_LIST,
-                                                         c->d_force_aos, true, acc);
+                                                         c->d_force_aos, true, acc, false);
                                 }
                                 CK(launch_transpose_in(c, c->d_pos_aos));
                                 if (c->P > 1 && !xmod) {

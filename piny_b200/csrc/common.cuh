@@ -130,6 +130,15 @@ template <> struct Idx<float> {
     }
 };
 
+// 16 bytes from global to shared memory without passing registers (both
+// addresses 16-byte aligned); cp_async_wait before the block's barrier.
+__device__ __forceinline__ void cp_async16(void *smem, const void *g)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Warp sum of a double over the lanes that share (lane mod stride); stride 32: v itself.
 __device__ __forceinline__ double warp_sum_strided(double v, int stride)
 {

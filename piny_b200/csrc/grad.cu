@@ -139,22 +139,13 @@ struct GradPairArgs {
     const void *tab;
 };
 
-// The channels one pass over the pairs serves: at most one with charge
-// tangents, one with ghost tangents and two with table tangents (the nine
-// q-TIP4P/F parameters have exactly these); number -1: none.
-struct GradPairSel {
-    int kq, kw, kt[2];
-    const double *dq, *w;
-    const void *tt[2];
-    unsigned tmask[2];  // tables with a non-zero tangent (bit u, u < 32)
-};
-
 // Pairs: a warp per row i and segment, lanes = beads x neighbours as in the
 // site kernel (pair.cu), one shared list for all beads; rows of a molecule go
 // to neighbouring warps, which find each other's j data in L1.  The channels'
 // sums stay in registers.  Bound: FP64 separations and conversions, and the
-// L2 reads of positions and u.  1024 TIP4P/F x 16 beads, FP32: 2164 us as one
-// thread per (row, bead) with a loop over all channels per pair.
+// L2 reads of positions and u.  1024 TIP4P/F x 16 beads, FP32: 405 us (2164
+// as one thread per (row, bead) with a loop over all channels per pair).
+// Serves FP64 and systems without the MIXED molecule-pair kernel.
 template <typename R>
 __global__ void __launch_bounds__(128) grad_pair_kernel(const __grid_constant__ GradPairArgs a,
                                                         const __grid_constant__ GradPairSel c,
@@ -511,7 +502,10 @@ cudaError_t launch_grad_terms(pinyb200_ctx *c, const Cell &cell, const GradArgs 
             sel.tt[t] = sel.kt[t] >= 0 ? g.ch[sel.kt[t]].ttab : nullptr;
             sel.tmask[t] = sel.kt[t] >= 0 ? c->grad.tmask[sel.kt[t]] : 0u;
         }
-        if (c->precision == PINYB200_FP64)
+        if (mol_grad_ok(c, cell)) {
+            cudaError_t e = launch_mol_pair_grad(c, cell, sel, g.uT, g.gacc);
+            if (e != cudaSuccess) return e;
+        } else if (c->precision == PINYB200_FP64)
             grad_pair_kernel<double><<<pgrid, 128, 0, st>>>(a, sel, cell, g.gacc);
         else
             grad_pair_kernel<float><<<pgrid, 128, 0, st>>>(a, sel, cell, g.gacc);
@@ -682,9 +676,7 @@ int pinyb200_grad(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, co
     const GradHost &gh = c->grad;
     const int K = gh.K;
     // forward: raw site forces (ghosts not distributed), potential grid, records
-    c->pme_full_records = true;
-    int rc = enqueue_device(c, d_pos, d_xmod, cell, 0, c->d_force_aos, false, nullptr);
-    c->pme_full_records = false;
+    int rc = enqueue_device(c, d_pos, d_xmod, cell, 0, c->d_force_aos, false, nullptr, true);
     if (rc) return rc;
     if (cudaMemsetAsync(gh.d_gacc, 0, (size_t)2 * PINYB200_MAX_TAN * sizeof(double), c->stream) != cudaSuccess)
         return record_error(c, PINYB200_ERR_CUDA, "grad: memset failed");

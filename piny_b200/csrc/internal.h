@@ -129,6 +129,19 @@ struct GradHost {
     void *d_grid2 = nullptr;            // PME: dipole spread of u, then its convolution
 };
 
+// The channels one pass over the pairs serves: at most one with charge
+// tangents, one with ghost tangents and two with table tangents (the nine
+// q-TIP4P/F parameters have exactly these); number -1: none.
+struct GradPairSel {
+    int kq, kw, kt[2];
+    const double *dq, *w;
+    const void *tt[2];
+    unsigned tmask[2];  // tables with a non-zero tangent (bit u, u < 32)
+};
+// Whether the molecule-pair form of the pair adjoint serves the context, and that pass.
+bool mol_grad_ok(const pinyb200_ctx *c, const Cell &cell);
+cudaError_t launch_mol_pair_grad(pinyb200_ctx *c, const Cell &cell, const GradPairSel &sel, const double *uT,
+                                 double *gacc);
 cudaError_t launch_pme_adjoint(pinyb200_ctx *c, const Cell &cell, const GradArgs &g);
 cudaError_t launch_grad_terms(pinyb200_ctx *c, const Cell &cell, const GradArgs &g, const double *d_fbar);
 
@@ -164,7 +177,6 @@ struct pinyb200_ctx {
     bool pme_overlap = true;            // false: PME on the main stream after the pair kernel
     int pair_variant = 0;               // 0 molecule-pair kernel (when available), 1 site-list kernel
     int pair_blocks_per_sm = 16;        // grid cap of the pair kernels, blocks per SM
-    bool pme_full_records = false;      // forward PME writes the full weight records (the adjoint reads them)
     int pair_carveout = 25;             // shared-memory share (%) the MIXED molecule-pair kernel asks for
     cudaEvent_t ev_fork = nullptr, ev_stage = nullptr, ev_join = nullptr, ev_pme[2] = {nullptr, nullptr};
     pinyb200::DeviceSystem sys;
@@ -253,7 +265,7 @@ struct pinyb200_ctx {
     int *d_pme_bin = nullptr;     // [P][ntile][cap] charge numbers (index into ichrg)
     int *d_pme_ovf = nullptr;     // [nchrg*P] overflowing (charge, bead) as k*P + b
     void *d_pme_head = nullptr;   // [nchrg*P] int4 stencil origin records
-    void *d_pme_w = nullptr;      // [nchrg*P][6][NIP] B-spline weight records
+    void *d_pme_w = nullptr;      // [nchrg*P][4] fractional offsets and charge
     double *d_twiddle64 = nullptr;  // per axis twiddles
     float *d_twiddle32 = nullptr;
     int *d_err = nullptr;
@@ -349,8 +361,9 @@ cudaError_t launch_keep_build_state(pinyb200_ctx *c, const int *gate, const doub
                                     const double *d_cs, cudaStream_t st);
 int stage_positions(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, const Cell &cell, int flags);
 void evaluate_finish(pinyb200_ctx *c, const Cell &cell, int flags, const double *acc, pinyb200_energies *e);
+// keep: the complete site forces stay in c->d_forceT too
 int enqueue_device(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, const Cell &cell, int flags,
-                   double *d_force, bool timing, double *h_acc);
+                   double *d_force, bool timing, double *h_acc, bool keep = false);
 Cell cell_from_hmat(const double *hmat);
 int pme_tiles_resize(pinyb200_ctx *c, int T);
 void pme_swap(pinyb200_ctx *c, PmeSet &p);

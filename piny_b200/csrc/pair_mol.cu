@@ -1481,6 +1481,170 @@ __global__ void __launch_bounds__(128, PINYB200_MIX_BLOCKS)
     mol_pair_mixed_body<P, NS, ENERGY, CM, VM>(a, m, cell, hw_blk());
 }
 
+// ---------------------------------------------------------------------------
+// Pair adjoint of the parameter gradient (grad.cu) on the molecule-pair list:
+// chunks, lanes, images, cutoffs and tables as mol_pair_mixed_body.  Per site
+// pair with u = u_i - u_j and separation r (FP32):
+//   charges  dE += tq S(cv0_c),  dF += (u . r) tq S(cdv0_c),  tq = dq_i q_j + q_i dq_j
+//   tables   dE += S(tangent cv0), dF += (u . r) S(tangent cdv0)
+//   ghosts   dF += (u . w) dv + (u . r)(r . w) dv' / r,  w = w_i - w_j; only the
+//            M site (the last of four) moves
+// A molecule pair's terms are summed in FP32, molecule pairs in FP64.  No
+// forces, so no atomics but a block's seven sums.
+template <int P, int NS, unsigned CM, unsigned VM>
+__global__ void __launch_bounds__(128, 4)
+    mol_pair_grad_kernel(const __grid_constant__ MixArgs a, const __grid_constant__ MixSite m,
+                         const __grid_constant__ Cell cell, const __grid_constant__ GradPairSel c,
+                         const __grid_constant__ float4 qs, const double *__restrict__ uT, double *__restrict__ gacc)
+{
+    constexpr int G = P >= 32 ? 32 : P, JPI = 32 / G;
+    constexpr int SM = NS == 4 ? 3 : -1;  // the M site
+    constexpr float kRound = 12582912.0f;
+    __shared__ double sh[7][4];
+    const int lane = threadIdx.x & 31, sub = lane / G;
+    const int warp = ((int)blockIdx.x * 128 + (int)threadIdx.x) >> 5, nwarps = (int)gridDim.x * 4;
+    const int b = (lane % G) + 32 * blockIdx.y;
+    const double *__restrict__ posT = a.posT;
+    const float q[4] = {qs.x, qs.y, qs.z, qs.w};
+    const bool gw = SM >= 0 && c.w;
+    double sum[7] = {0, 0, 0, 0, 0, 0, 0};  // eq, et0, et1, fq, ft0, ft1, fw
+    const double ext2 = ext2_of(a.ext);
+    const int nch = *a.nchunk;
+    for (int ch = warp; ch < nch; ch += nwarps) {
+        const int mi = a.chunk[3 * ch], beg = a.chunk[3 * ch + 1], end = a.chunk[3 * ch + 2];
+        const int i0 = mi * m.stride;
+        float ei[NS][3], ui[NS][3], wi[3] = {0, 0, 0};
+#pragma unroll
+        for (int s = 0; s < NS; s++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const size_t o = (3 * (size_t)(i0 + s) + d) * P + b;
+                ei[s][d] = (float)(posT[o] - posT[(3 * (size_t)i0 + d) * P + b]);
+                ui[s][d] = (float)uT[o];
+            }
+        if (gw)
+#pragma unroll
+            for (int d = 0; d < 3; d++) wi[d] = (float)c.w[(3 * (size_t)(i0 + NS - 1) + d) * P + b];
+        for (int k = beg + sub; k < end; k += JPI) {
+            const int mj = __ldcg(a.mj + k);
+            const unsigned mask = __ldcg(a.mask + k);
+            const int j0 = mj * m.stride;
+            double sh0[3];
+            bool near = false;
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const double hid = cell.hi[4 * d];
+                const double t = __dmul_rn(__dsub_rn(a.xmod[3 * (size_t)i0 + d], __ldcg(a.xmod + 3 * (size_t)j0 + d)), hid);
+                sh0[d] = -nint_rn(t);
+                near |= fabs(t + sh0[d]) > 0.5 - ext2 * hid;
+            }
+            float dj[NS][3], uj[NS][3], wj[3] = {0, 0, 0};
+            {
+                double xj0[3];
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    xj0[d] = __ldcg(posT + (3 * (size_t)j0 + d) * P + b);
+                    dj[0][d] = (float)(__dsub_rn(posT[(3 * (size_t)i0 + d) * P + b], xj0[d]) + sh0[d] * cell.h[4 * d]);
+                }
+#pragma unroll
+                for (int s = 0; s < NS; s++)
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        const size_t o = (3 * (size_t)(j0 + s) + d) * P + b;
+                        if (s > 0) dj[s][d] = dj[0][d] - (float)(__ldcg(posT + o) - xj0[d]);
+                        uj[s][d] = (float)__ldcg(uT + o);
+                    }
+                if (gw)
+#pragma unroll
+                    for (int d = 0; d < 3; d++) wj[d] = (float)__ldcg(c.w + (3 * (size_t)(j0 + NS - 1) + d) * P + b);
+            }
+            float eq = 0, et[2] = {0, 0}, fq = 0, ft[2] = {0, 0}, fw = 0;
+            auto site_pairs = [&](auto near_tag, const NearImages &nim) {
+                constexpr bool NEAR = decltype(near_tag)::value;
+#pragma unroll
+                for (int sj = 0; sj < NS; sj++) {
+#pragma unroll
+                    for (int si = 0; si < NS; si++) {
+                        const int sp = si * NS + sj;
+                        const bool coul = ((CM >> sp) & 1u) != 0, vdw = ((VM >> sp) & 1u) != 0;
+                        if (!coul && !vdw) continue;
+                        if (!((mask >> sp) & 1u)) continue;
+                        float rx = dj[sj][0] + ei[si][0], ry = dj[sj][1] + ei[si][1], rz = dj[sj][2] + ei[si][2];
+                        if constexpr (NEAR) {
+                            rx = add_cells(rx, nim.shift(0, sp), cell.h[0]);
+                            ry = add_cells(ry, nim.shift(1, sp), cell.h[4]);
+                            rz = add_cells(rz, nim.shift(2, sp), cell.h[8]);
+                        }
+                        const float r2 = rx * rx + ry * ry + rz * rz;
+                        if (!(r2 < m.rc2)) continue;
+                        const float ri = rsqrtf(r2);
+                        const float t = fminf(fmaxf(fmaf(r2 * ri, m.dri_f, -m.rmd), 0.0f), m.tmax);
+                        const float tr = __fadd_rn(t, kRound);
+                        const int kn = __float_as_int(tr) - __float_as_int(kRound);
+                        const float del = t - __fsub_rn(tr, kRound);
+                        const float ux = ui[si][0] - uj[sj][0], uy = ui[si][1] - uj[sj][1], uz = ui[si][2] - uj[sj][2];
+                        const float ur = ux * rx + uy * ry + uz * rz;
+                        const bool mv = gw && (si == SM || sj == SM);
+                        float dv = 0.0f, dvp = 0.0f;
+                        if (coul) {
+                            float4 cf, ef;
+                            ldg_keep_pair(a.tabfe + 2 * (m.toff[sp] + kn) + 2 * m.tstride, cf, ef);
+                            const float sc = spline_eval<float4, float>(cf, del);
+                            if (c.dq) {
+                                const float tq = (float)__ldg(c.dq + i0 + si) * q[sj] + q[si] * (float)__ldg(c.dq + j0 + sj);
+                                eq += tq * spline_eval<float4, float>(ef, del);
+                                fq += ur * (tq * sc);
+                            }
+                            if (mv) {
+                                dv = m.q2[sp] * sc;
+                                dvp = m.q2[sp] * (cf.y + del * (2.0f * cf.z + 3.0f * del * cf.w)) * m.dri_f;
+                            }
+                        }
+                        if (vdw) {
+#pragma unroll
+                            for (int n = 0; n < 2; n++)
+                                if (c.tt[n]) {
+                                    const float4 *tt = (const float4 *)c.tt[n] + m.toff[sp] + kn;
+                                    et[n] += spline_eval<float4, float>(__ldg(tt), del);
+                                    ft[n] += ur * spline_eval<float4, float>(__ldg(tt + m.tstride), del);
+                                }
+                            if (mv) {
+                                const float4 cv = __ldg(a.tab + m.toff[sp] + kn + T_CDV0 * m.tstride);
+                                dv += spline_eval<float4, float>(cv, del);
+                                dvp += (cv.y + del * (2.0f * cv.z + 3.0f * del * cv.w)) * m.dri_f;
+                            }
+                        }
+                        if (mv) {
+                            const float wx = (si == SM ? wi[0] : 0.0f) - (sj == SM ? wj[0] : 0.0f),
+                                        wy = (si == SM ? wi[1] : 0.0f) - (sj == SM ? wj[1] : 0.0f),
+                                        wz = (si == SM ? wi[2] : 0.0f) - (sj == SM ? wj[2] : 0.0f);
+                            fw += (ux * wx + uy * wy + uz * wz) * dv + ur * (rx * wx + ry * wy + rz * wz) * (dvp * ri);
+                        }
+                    }
+                }
+            };
+            if (near) site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, NS, sh0, cell, lane));
+            else site_pairs(std::false_type{}, NearImages{{0u, 0u, 0u}});
+            const float v[7] = {eq, et[0], et[1], fq, ft[0], ft[1], fw};
+#pragma unroll
+            for (int n = 0; n < 7; n++)
+                if (v[n] != 0.0f) sum[n] += (double)v[n];
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 7; n++) {
+        const double t = warp_sum(sum[n]);
+        if (lane == 0) sh[n][threadIdx.x >> 5] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        const int n = threadIdx.x;
+        const double t = (sh[n][0] + sh[n][1]) + (sh[n][2] + sh[n][3]);
+        const int k = n == 6 ? c.kw : (n % 3 == 0 ? c.kq : c.kt[n % 3 - 1]);
+        if (k >= 0 && t != 0.0) atomicAdd(&gacc[2 * k + (n >= 3)], n < 3 ? t / (double)P : t);
+    }
+}
+
 // Many boxes of one bead count and site pattern in one persistent launch.
 struct MixBox {
     MixArgs a;
@@ -1878,6 +2042,51 @@ cudaError_t launch_mol_pair_mixed(pinyb200_ctx *c, const Cell &cell, bool energy
     const MixSite m = mix_site(c);
     if (c->mol_ns == 3) return launch_mix_ns<3>(c, a, m, cell, energy);
     return launch_mix_ns<4>(c, a, m, cell, energy);
+}
+
+// The molecule-pair adjoint serves MIXED boxes of the two water patterns in
+// orthorhombic cells whose moving sites are the M sites (water_ok).
+bool mol_grad_ok(const pinyb200_ctx *c, const Cell &cell)
+{
+    const bool ortho = cell.h[1] == 0.0 && cell.h[2] == 0.0 && cell.h[3] == 0.0 && cell.h[5] == 0.0 &&
+                       cell.h[6] == 0.0 && cell.h[7] == 0.0;
+    return c->precision == PINYB200_MIXED && c->use_mol && c->mol_ok && c->mix_ok && c->water_ok && ortho &&
+           mix_pattern(c) != 0;
+}
+
+template <int P, int NS, unsigned CM, unsigned VM>
+static cudaError_t launch_grad_t(pinyb200_ctx *c, const Cell &cell, const GradPairSel &sel, const double *uT,
+                                 double *gacc)
+{
+    const float4 q = make_float4((float)c->h_charge[0], (float)c->h_charge[1], (float)c->h_charge[2],
+                                 NS == 4 ? (float)c->h_charge[3] : 0.0f);
+    const long long blocks = std::max<long long>(1, std::min<long long>((c->chunk_cap + 3) / 4, c->sm_count * 4LL));
+    const dim3 grid((unsigned)blocks, P > 32 ? P / 32 : 1);
+    mol_pair_grad_kernel<P, NS, CM, VM><<<grid, 128, 0, c->stream>>>(mix_args(c), mix_site(c), cell, sel, q, uT, gacc);
+    return cudaGetLastError();
+}
+
+template <int NS, unsigned CM, unsigned VM>
+static cudaError_t launch_grad_p(pinyb200_ctx *c, const Cell &cell, const GradPairSel &sel, const double *uT,
+                                 double *gacc)
+{
+    switch (c->P) {
+    case 1: return launch_grad_t<1, NS, CM, VM>(c, cell, sel, uT, gacc);
+    case 2: return launch_grad_t<2, NS, CM, VM>(c, cell, sel, uT, gacc);
+    case 4: return launch_grad_t<4, NS, CM, VM>(c, cell, sel, uT, gacc);
+    case 8: return launch_grad_t<8, NS, CM, VM>(c, cell, sel, uT, gacc);
+    case 16: return launch_grad_t<16, NS, CM, VM>(c, cell, sel, uT, gacc);
+    case 32: return launch_grad_t<32, NS, CM, VM>(c, cell, sel, uT, gacc);
+    case 64: return launch_grad_t<64, NS, CM, VM>(c, cell, sel, uT, gacc);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_mol_pair_grad(pinyb200_ctx *c, const Cell &cell, const GradPairSel &sel, const double *uT,
+                                 double *gacc)
+{
+    if (c->mol_ns == 4) return launch_grad_p<4, kTip4pCoul, kTip4pVdw>(c, cell, sel, uT, gacc);
+    return launch_grad_p<3, kSpcCoul, kSpcVdw>(c, cell, sel, uT, gacc);
 }
 
 // The molecule extent bound of this evaluation into the context's per-bead

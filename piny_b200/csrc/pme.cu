@@ -39,33 +39,6 @@
 
 namespace pinyb200 {
 
-// B-spline weights of order NI at the fractional offset f (ewald3d_pme.c:
-// 301-338).  m[j], j = 1..NI as in PINY (index 0 unused); dm[] are the
-// derivative weights formed at order NI-1 (:512-532).
-template <typename R, int NI, bool DERIV>
-__device__ __forceinline__ void bspline(R f, R *m, R *dm)
-{
-    R u[NI + 1];
-#pragma unroll
-    for (int j = 1; j <= NI; j++) u[j] = f + (R)(j - 1);
-    m[1] = (R)1 - fabs(u[1] - (R)1);
-    m[2] = (R)1 - fabs(u[2] - (R)1);
-#pragma unroll
-    for (int j = 3; j <= NI; j++) m[j] = (R)0;
-#pragma unroll
-    for (int nn = 3; nn <= NI; nn++) {
-        const R rn = (R)nn, rn1 = (R)1 / (R)(nn - 1);
-#pragma unroll
-        for (int j = nn; j >= 2; j--) m[j] = (u[j] * m[j] + (rn - u[j]) * m[j - 1]) * rn1;
-        m[1] = u[1] * m[1] * rn1;
-        if (DERIV && nn == NI - 1) {
-            dm[1] = m[1];
-#pragma unroll
-            for (int j = 2; j <= NI; j++) dm[j] = m[j] - m[j - 1];
-        }
-    }
-}
-
 // Stencil of one charge and bead from the position array.
 __device__ __forceinline__ void stencil_origin(const PmeArgs &a, const Cell &cell, int at, int b, int ni, int &la,
                                                int &lb, int &lc, double &fa, double &fb, double &fc)
@@ -106,15 +79,10 @@ static double bspline_peak(int n)
     return peak[std::min(12, std::max(3, n))];
 }
 
-// Per (charge k, bead b) record, number idx = k*P + b, written by the bin
-// kernel and read by spread and gather:
-//   head[idx] = (atom, la, lb, lc)  stencil origin per axis
-//   w[idx][j][t], j = 0..5 for M_a, M_b, M_c, dM_a, dM_b, dM_c, t = 0..NIP-1:
-//                 weight of grid point lo + t (PINY's m[NI - t]), zero for t >= NI
+// Stencil points per axis, padded.
 template <int NI>
 struct RecGeom {
     static constexpr int NIP = NI <= 4 ? 4 : (NI <= 8 ? 8 : 12);
-    static constexpr int NW = 6 * NIP;
 };
 
 // Tile geometry: T^3 grid points own the charges whose stencil starts in
@@ -137,72 +105,30 @@ __device__ __forceinline__ int wrapi(int i, int N)
     return i;
 }
 
-// Store n consecutive values of type R (n a multiple of 4) with vector stores.
-__device__ __forceinline__ void store4(float *dst, const float *v, int n)
+// The E^3 points of the tile with corner (ta0, tb0, tc0) of grid g into the
+// block's shared copy: asynchronous 16-byte copies where the rows allow (all
+// in flight at once; the padding columns take what the grid holds there),
+// else plain loads.  The caller's barrier follows.
+template <typename R, typename TG>
+__device__ __forceinline__ void load_tile(R *tl, const R *g, int Na, int Nb, int Nc, int ta0, int tb0, int tc0)
 {
-    for (int i = 0; i < n; i += 4) *(float4 *)(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-}
-__device__ __forceinline__ void store4(double *dst, const double *v, int n)
-{
-    for (int i = 0; i < n; i += 2) *(double2 *)(dst + i) = make_double2(v[i], v[i + 1]);
-}
-template <int N>
-__device__ __forceinline__ void load4(float *v, const float *src)
-{
-#pragma unroll
-    for (int i = 0; i < N; i += 4) {
-        const float4 x = __ldg((const float4 *)(src + i));
-        v[i] = x.x;
-        v[i + 1] = x.y;
-        v[i + 2] = x.z;
-        v[i + 3] = x.w;
+    constexpr int NROW = TG::E * TG::E, V = 16 / sizeof(R), NQ = TG::PA / V;
+    if ((Na & (V - 1)) == 0) {
+        for (int i = threadIdx.x; i < NROW * NQ; i += blockDim.x) {
+            const int row = i / NQ, q = i - row * NQ;
+            const int cz = row / TG::E, by = row - cz * TG::E;
+            cp_async16(tl + row * TG::PA + V * q,
+                       g + ((size_t)wrapi(tc0 + cz, Nc) * Nb + wrapi(tb0 + by, Nb)) * Na + wrapi(ta0 + V * q, Na));
+        }
+        cp_async_wait();
+    } else {
+        for (int i = threadIdx.x; i < NROW * TG::PA; i += blockDim.x) {
+            const int row = i / TG::PA, ax = i - row * TG::PA;
+            const int cz = row / TG::E, by = row - cz * TG::E;
+            tl[i] = ax < TG::E ? g[((size_t)wrapi(tc0 + cz, Nc) * Nb + wrapi(tb0 + by, Nb)) * Na + wrapi(ta0 + ax, Na)]
+                               : (R)0;
+        }
     }
-}
-template <int N>
-__device__ __forceinline__ void load4(double *v, const double *src)
-{
-#pragma unroll
-    for (int i = 0; i < N; i += 2) {
-        const double2 x = __ldg((const double2 *)(src + i));
-        v[i] = x.x;
-        v[i + 1] = x.y;
-    }
-}
-
-// Bin kernel: one thread per (charge, bead).  Stencil origin in FP64 with
-// PINY's operation order, B-spline weights and derivatives in R, record
-// written in (charge, bead) order, record number filed under its tile.
-template <typename R, int NI>
-__global__ void __launch_bounds__(256) pme_bin_kernel(PmeArgs a, Cell cell, TileArgs t)
-{
-    typedef RecGeom<NI> RG;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)a.nchrg * a.P) return;
-    const int b = (int)(idx % a.P);
-    const int k = (int)(idx / a.P);
-    const int at = a.ichrg[k];
-    int la, lb, lc;
-    double fa, fb, fc;
-    stencil_origin(a, cell, at, b, NI, la, lb, lc, fa, fb, fc);
-    R m[NI + 1], d[NI + 1], w[RG::NIP];
-    R *out = (R *)a.rw + (size_t)idx * RG::NW;
-    const double fr[3] = {fa, fb, fc};
-#pragma unroll
-    for (int ax = 0; ax < 3; ax++) {
-        bspline<R, NI, true>((R)fr[ax], m, d);
-#pragma unroll
-        for (int s = 0; s < RG::NIP; s++) w[s] = s < NI ? m[NI - s] : (R)0;
-        store4(out + ax * RG::NIP, w, RG::NIP);
-#pragma unroll
-        for (int s = 0; s < RG::NIP; s++) w[s] = s < NI ? d[NI - s] : (R)0;
-        store4(out + (3 + ax) * RG::NIP, w, RG::NIP);
-    }
-    a.rhead[idx] = make_int4(at, la, lb, lc);
-    const int T = t.T;
-    const int tile = ((lc / T) * t.ntb + lb / T) * t.nta + la / T;
-    const int slot = atomicAdd(&t.cnt[b * t.ntile + tile], 1);
-    if (slot < t.cap) t.bin[((size_t)b * t.ntile + tile) * t.cap + slot] = (int)idx;
-    else t.ovf[atomicAdd(&t.cnt[a.P * t.ntile], 1)] = (int)idx;
 }
 
 // Weights of one record that a lane of an 8-lane group needs: its own a
@@ -212,143 +138,13 @@ struct LaneW {
     typedef RecGeom<NI> RG;
     R wa0, wa1, da0, da1;
     R mb[RG::NIP], mc[RG::NIP], db[DERIV ? RG::NIP : 1], dc[DERIV ? RG::NIP : 1];
-    __device__ __forceinline__ void load(const R *rw, int idx, int l8)
-    {
-        const R *w = rw + (size_t)idx * RG::NW;
-        wa0 = l8 < NI ? w[l8] : (R)0;
-        wa1 = (NI > 8 && l8 + 8 < NI) ? w[l8 + 8] : (R)0;
-        load4<RG::NIP>(mb, w + RG::NIP);
-        load4<RG::NIP>(mc, w + 2 * RG::NIP);
-        if (DERIV) {
-            da0 = l8 < NI ? w[3 * RG::NIP + l8] : (R)0;
-            da1 = (NI > 8 && l8 + 8 < NI) ? w[3 * RG::NIP + l8 + 8] : (R)0;
-            load4<RG::NIP>(db, w + 4 * RG::NIP);
-            load4<RG::NIP>(dc, w + 5 * RG::NIP);
-        }
-    }
 };
 
-// Spread one record straight into the global grid (overflow entries).
-template <typename R, int NI>
-__device__ __forceinline__ void spread_global(const PmeArgs &a, R *g, int la, int lb, int lc,
-                                              const LaneW<R, NI, false> &lw, R q, int l8)
-{
-    const int ga0 = wrapi(la + l8, a.Na), ga1 = wrapi(la + l8 + 8, a.Na);
-#pragma unroll
-    for (int tc = 0; tc < NI; tc++) {
-        const int gc = wrapi(lc + tc, a.Nc);
-        const R qc = q * lw.mc[tc];
-#pragma unroll
-        for (int tb = 0; tb < NI; tb++) {
-            const int gb = wrapi(lb + tb, a.Nb);
-            const R w = lw.mb[tb] * qc;
-            R *row = g + ((size_t)gc * a.Nb + gb) * a.Na;
-            if (l8 < NI) atomicAdd(row + ga0, lw.wa0 * w);
-            if (NI > 8 && l8 + 8 < NI) atomicAdd(row + ga1, lw.wa1 * w);
-        }
-    }
-}
-
-// Spread: one block per (tile, bead), one warp per record.  A warp adds its
-// record's stencil to a shared copy of the tile with shared-memory atomics;
-// its 32 lanes cover 8 a points x 4 b rows, so the 32 addresses of one
-// atomic are distinct and, with rows padded to PA = 0 mod 8 floats,
-// fall in distinct banks.  The copy is then added to the grid once, with
-// 16-byte vector atomics where the rows allow.  Records whose origin lies
-// outside the tile (none are expected) and overflow records go straight to
-// the grid.
+// Shared copy of a tile.
 template <typename R, int NI, int TT>
 size_t spread_smem()
 {
     return (size_t)TileGeom<NI, TT>::NPT * sizeof(R);
-}
-
-template <typename R, int NI, int TT>
-__global__ void __launch_bounds__(256) spread_tile_kernel(PmeArgs a, TileArgs t)
-{
-    typedef TileGeom<NI, TT> TG;
-    typedef RecGeom<NI> RG;
-    constexpr int NIP = RG::NIP;
-    constexpr int NTB = (NI + 3) / 4;  // b rows per lane
-    extern __shared__ unsigned char smem_raw[];
-    R *tl = (R *)smem_raw;
-    for (int i = threadIdx.x; i < TG::NPT; i += blockDim.x) tl[i] = (R)0;
-    __syncthreads();
-    const int tile = blockIdx.x, b = blockIdx.y;
-    const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    const int la8 = lane & 7, lb4 = lane >> 3;
-    const int n = min(t.cnt[b * t.ntile + tile], t.cap);
-    const int *list = t.bin + ((size_t)b * t.ntile + tile) * t.cap;
-    const R *rw = (const R *)a.rw;
-    R *g = (R *)a.grid + (size_t)b * a.Na * a.Nb * a.Nc;
-    for (int e = warp; e < n; e += nwarp) {
-        const int idx = list[e];
-        const int4 h = a.rhead[idx];
-        const int oa = h.y - ta0, ob = h.z - tb0, oc = h.w - tc0;
-        const R q = (R)a.charge[h.x];
-        const R *w = rw + (size_t)idx * RG::NW;
-        if (oa >= 0 && oa < TG::T && ob >= 0 && ob < TG::T && oc >= 0 && oc < TG::T) {
-            R mc[NIP];
-            load4<NIP>(mc, w + 2 * NIP);
-            R mbl[NTB];
-#pragma unroll
-            for (int i = 0; i < NTB; i++) mbl[i] = lb4 + 4 * i < NI ? w[NIP + lb4 + 4 * i] : (R)0;
-            R *base = tl + (oc * TG::E + ob + lb4) * TG::PA + oa + la8;
-#pragma unroll
-            for (int sa = 0; sa < NI; sa += 8) {
-                if (la8 + sa >= NI) break;
-                const R qa = q * w[la8 + sa];
-#pragma unroll
-                for (int tc = 0; tc < NI; tc++) {
-                    const R cq = qa * mc[tc];
-#pragma unroll
-                    for (int i = 0; i < NTB; i++)
-                        if (lb4 + 4 * i < NI) atomicAdd(base + (tc * TG::E + 4 * i) * TG::PA + sa, cq * mbl[i]);
-                }
-            }
-        } else if (lane < 8) {
-            LaneW<R, NI, false> lw;
-            lw.load(rw, idx, lane);
-            spread_global<R, NI>(a, g, h.y, h.z, h.w, lw, q, lane);
-        }
-    }
-    const int grp = threadIdx.x >> 3, l8 = threadIdx.x & 7, ngrp = blockDim.x >> 3;
-    const int nov = t.cnt[a.P * t.ntile];
-    const int gid = blockIdx.y * gridDim.x + blockIdx.x, nblk = gridDim.x * gridDim.y;
-    for (int e = gid * ngrp + grp; e < nov; e += nblk * ngrp) {
-        const int idx = t.ovf[e];
-        const int4 h = a.rhead[idx];
-        LaneW<R, NI, false> lw;
-        lw.load(rw, idx, l8);
-        R *g2 = (R *)a.grid + (size_t)(idx % a.P) * a.Na * a.Nb * a.Nc;
-        spread_global<R, NI>(a, g2, h.y, h.z, h.w, lw, (R)a.charge[h.x], l8);
-    }
-    __syncthreads();
-    // add the shared copy to the grid, a warp per row (or rows)
-    constexpr int NROW = TG::E * TG::E;
-    if (sizeof(R) == 4 && (a.Na & 3) == 0) {
-        constexpr int NQ = TG::PA / 4;
-        constexpr int RPI = 32 / NQ;  // rows per warp step
-        for (int r0 = warp * RPI; r0 < NROW; r0 += nwarp * RPI) {
-            const int row = r0 + lane / NQ, q4 = lane % NQ;
-            if (lane >= RPI * NQ || row >= NROW) continue;
-            const float4 v = ((const float4 *)tl)[row * NQ + q4];
-            if (v.x == 0.f && v.y == 0.f && v.z == 0.f && v.w == 0.f) continue;
-            const int cz = row / TG::E, by = row - cz * TG::E;
-            const int gc = wrapi(tc0 + cz, a.Nc), gb = wrapi(tb0 + by, a.Nb), ga = wrapi(ta0 + 4 * q4, a.Na);
-            atomicAdd((float4 *)((float *)g + ((size_t)gc * a.Nb + gb) * a.Na + ga), v);
-        }
-    } else {
-        for (int row = warp; row < NROW; row += nwarp) {
-            const int cz = row / TG::E, by = row - cz * TG::E;
-            R *dst = g + ((size_t)wrapi(tc0 + cz, a.Nc) * a.Nb + wrapi(tb0 + by, a.Nb)) * a.Na;
-            for (int ax = lane; ax < TG::E; ax += 32) {
-                const R v = tl[row * TG::PA + ax];
-                if (v != (R)0) atomicAdd(dst + wrapi(ta0 + ax, a.Na), v);
-            }
-        }
-    }
 }
 
 // Gather sums of one record for lane l8: d/ds_a, d/ds_b, d/ds_c of
@@ -450,122 +246,17 @@ __global__ void __launch_bounds__(256) pme_force_add_scaled_kernel(int nchrg, in
     fT[(3 * (size_t)ichrg[k] + d) * P + b] += fP[t] * w;
 }
 
-// Gather: one block per (tile, bead); the tile's potential (with the
-// stencil reach) is copied to shared memory once and the bin's records read
-// it there.  Overflow records read the grid directly.  Every (charge, bead)
-// is handled by exactly one 8-lane group, so the force update needs no
-// atomics.
-template <typename R, int NI, int TT>
-__global__ void __launch_bounds__(256) gather_tile_kernel(PmeArgs a, Cell cell, TileArgs t)
-{
-    typedef TileGeom<NI, TT> TG;
-    extern __shared__ unsigned char smem_raw[];
-    R *tl = (R *)smem_raw;
-    const int tile = blockIdx.x, b = blockIdx.y;
-    const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
-    const R *g = (const R *)a.grid + (size_t)b * a.Na * a.Nb * a.Nc;
-    const int n = min(t.cnt[b * t.ntile + tile], t.cap);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    if (n > 0) {
-        constexpr int NROW = TG::E * TG::E;
-        if (sizeof(R) == 4 && (a.Na & 3) == 0) {
-            // 16-byte chunks; the padding column takes whatever the grid holds there
-            constexpr int NQ = TG::PA / 4;
-            constexpr int RPI = 32 / NQ;
-            for (int r0 = warp * RPI; r0 < NROW; r0 += nwarp * RPI) {
-                const int row = r0 + lane / NQ, q4 = lane % NQ;
-                if (lane >= RPI * NQ || row >= NROW) continue;
-                const int cz = row / TG::E, by = row - cz * TG::E;
-                const float *src = (const float *)g +
-                                   ((size_t)wrapi(tc0 + cz, a.Nc) * a.Nb + wrapi(tb0 + by, a.Nb)) * a.Na +
-                                   wrapi(ta0 + 4 * q4, a.Na);
-                ((float4 *)tl)[row * NQ + q4] = __ldg((const float4 *)src);
-            }
-        } else {
-            for (int row = warp; row < NROW; row += nwarp) {
-                const int cz = row / TG::E, by = row - cz * TG::E;
-                const R *src = g + ((size_t)wrapi(tc0 + cz, a.Nc) * a.Nb + wrapi(tb0 + by, a.Nb)) * a.Na;
-                for (int ax = lane; ax < TG::PA; ax += 32)
-                    tl[row * TG::PA + ax] = ax < TG::E ? src[wrapi(ta0 + ax, a.Na)] : (R)0;
-            }
-        }
-    }
-    __syncthreads();
-    const int grp = threadIdx.x >> 3, l8 = threadIdx.x & 7, ngrp = blockDim.x >> 3;
-    const int *list = t.bin + ((size_t)b * t.ntile + tile) * t.cap;
-    const R *rw = (const R *)a.rw;
-    // every lane of a warp takes part in the group reductions: loop to the
-    // same trip count in all groups of the warp
-    const int nr = (n + ngrp - 1) / ngrp;
-    for (int r = 0; r < nr; r++) {
-        const int e = r * ngrp + grp;
-        const bool act = e < n;
-        int at = 0, idx = 0;
-        double ea = 0, eb = 0, ec = 0;
-        if (act) {
-            idx = list[e];
-            const int4 h = a.rhead[idx];
-            at = h.x;
-            LaneW<R, NI, true> lw;
-            lw.load(rw, idx, l8);
-            const int oa = h.y - ta0, ob = h.z - tb0, oc = h.w - tc0;
-            if (oa >= 0 && oa < TG::T && ob >= 0 && ob < TG::T && oc >= 0 && oc < TG::T) {
-                const R *base = tl + (oc * TG::E + ob) * TG::PA + oa;
-                gather_lane<R, NI>([&](int tc, int tb, int ta) { return base[(tc * TG::E + tb) * TG::PA + ta]; }, lw,
-                                   l8, ea, eb, ec);
-            } else {
-                const int la = h.y, lb = h.z, lc = h.w;
-                gather_lane<R, NI>(
-                    [&](int tc, int tb, int ta) {
-                        return g[((size_t)wrapi(lc + tc, a.Nc) * a.Nb + wrapi(lb + tb, a.Nb)) * a.Na +
-                                 wrapi(la + ta, a.Na)];
-                    },
-                    lw, l8, ea, eb, ec);
-            }
-        }
-        gather_store(a, cell, at, idx, ea, eb, ec, act ? l8 : 1);
-    }
-    const int nov = t.cnt[a.P * t.ntile];
-    const int gid = blockIdx.y * gridDim.x + blockIdx.x, nblk = gridDim.x * gridDim.y;
-    const int nr2 = (nov + nblk * ngrp - 1) / (nblk * ngrp);
-    for (int r = 0; r < nr2; r++) {
-        const int e = (r * nblk + gid) * ngrp + grp;
-        const bool act = e < nov;
-        int at = 0, b2 = 0, idx = 0;
-        double ea = 0, eb = 0, ec = 0;
-        if (act) {
-            idx = t.ovf[e];
-            const int4 h = a.rhead[idx];
-            b2 = idx % a.P;
-            at = h.x;
-            LaneW<R, NI, true> lw;
-            lw.load(rw, idx, l8);
-            const R *g2 = (const R *)a.grid + (size_t)b2 * a.Na * a.Nb * a.Nc;
-            const int la = h.y, lb = h.z, lc = h.w;
-            gather_lane<R, NI>(
-                [&](int tc, int tb, int ta) {
-                    return g2[((size_t)wrapi(lc + tc, a.Nc) * a.Nb + wrapi(lb + tb, a.Nb)) * a.Na +
-                              wrapi(la + ta, a.Na)];
-                },
-                lw, l8, ea, eb, ec);
-        }
-        gather_store(a, cell, at, idx, ea, eb, ec, act ? l8 : 1);
-    }
-}
-
 // ---------------------------------------------------------------------------
-// Compact forward path: bin, spread and gather without weight records.
-//
 // B-spline weights as polynomials of the fractional offset.  PINY's
 // recursion (ewald3d_pme.c:301-338) makes the weight m[j] of order NI (at
 // u = f + j - 1) a polynomial of degree NI - 1 in f on [0, 1), and the
 // derivative weight dm[j] = m'[j] - m'[j - 1] formed from the order NI - 1
 // splines (:512-532) one of degree NI - 2.  BsplinePoly runs that recursion
 // on coefficient arrays at compile time; the kernels evaluate each lane's
-// weights by Horner from a shared-memory copy.  The bin kernel writes, per
-// (charge, bead), only the stencil origin and the three fractional offsets
-// with the charge (32 bytes in FP32) instead of the 6 x NIP weights, and
-// spread and gather read the next record while they work on the current one.
+// weights by Horner.  The bin kernel writes, per (charge, bead), the stencil
+// origin and the three fractional offsets with the charge (32 bytes in
+// FP32), and spread and gather read the next record while they work on the
+// current one.
 template <int NI>
 struct BsplinePoly {
     double m[NI][NI];   // m[p][d]: coefficient of f^d of PINY's m[p + 1]
@@ -647,6 +338,50 @@ __device__ __forceinline__ R poly_eval(const R (&row)[PolyTab<R, NI>::NP4], R f)
     return w;
 }
 
+// The piece of one stencil point (t of a lane of an 8-lane group, order up to
+// 8) in registers: its weight at f, and the weight's derivative (which is
+// dm: the difference of the order n - 1 splines is the derivative of the
+// order n one) from the same Horner pass.
+template <typename R, int NI>
+struct Piece {
+    R c[NI];
+    __device__ __forceinline__ void load(int t)
+    {
+        const int p = NI - 1 - (t < NI ? t : NI - 1);
+#pragma unroll
+        for (int d = 0; d < NI; d++) c[d] = t < NI ? (R)kBspline<NI>.m[p][d] : (R)0;
+    }
+    __device__ __forceinline__ R value(R f) const
+    {
+        R w = c[NI - 1];
+#pragma unroll
+        for (int d = NI - 2; d >= 0; d--) w = w * f + c[d];
+        return w;
+    }
+    // second derivative
+    __device__ __forceinline__ R second(R f) const
+    {
+        R w = c[NI - 1], dw = (R)0, d2 = (R)0;
+#pragma unroll
+        for (int d = NI - 2; d >= 0; d--) {
+            d2 = d2 * f + dw;
+            dw = dw * f + w;
+            w = w * f + c[d];
+        }
+        return (R)2 * d2;
+    }
+    __device__ __forceinline__ void both(R f, R &w, R &dw) const
+    {
+        w = c[NI - 1];
+        dw = (R)0;
+#pragma unroll
+        for (int d = NI - 2; d >= 0; d--) {
+            dw = dw * f + w;
+            w = w * f + c[d];
+        }
+    }
+};
+
 template <typename R>
 __device__ __forceinline__ typename Vec4<R>::T load_frac(const void *rw, int idx)
 {
@@ -655,7 +390,7 @@ __device__ __forceinline__ typename Vec4<R>::T load_frac(const void *rw, int idx
 }
 
 // Bin kernel of the compact path: one thread per (charge, bead), stencil
-// origin in FP64 with PINY's operation order (as pme_bin_kernel), record
+// origin in FP64 with PINY's operation order, record
 // (atom, la, lb, lc) + (fa, fb, fc, q), record number filed under its tile.
 template <typename R, int NI>
 __device__ __forceinline__ void pme_bin_compact_body(const PmeArgs &a, const Cell &cell, const TileArgs &t,
@@ -679,22 +414,47 @@ __global__ void __launch_bounds__(256) pme_bin_compact_kernel(const __grid_const
 }
 
 // Weights one spread lane needs (lanes = 8 a points x 4 b rows): its a
-// points la8 (+8), its b rows lb4 + 4 i, and all c points, the latter
-// evaluated by lanes 0..NI-1 and shuffled.  Every lane of the warp calls it.
+// points la8 (+8), its b rows lb4 + 4 i, and all c points.  Up to order 8 a
+// lane evaluates the three axes at point la8 from its piece in registers and
+// the b and c weights are shuffled from lanes 0..7 (weights from a shared
+// table took 12 of the 60 shared-memory wavefronts of a record); order 10
+// evaluates from the table.  Every lane of the warp calls it.
+template <typename R, int NI>
+struct SpreadPoly {
+    PolyTab<R, NI> *pt;
+    Piece<R, NI <= 8 ? NI : 4> piece;
+    __device__ __forceinline__ void init(PolyTab<R, NI> *tab, int lane)
+    {
+        pt = tab;
+        if constexpr (NI <= 8) piece.load(lane & 7);
+    }
+};
 template <typename R, int NI>
 struct SpreadW {
     static constexpr int NTB = (NI + 3) / 4, NSA = (NI + 7) / 8;
     R wa[NSA], mb[NTB], mc[NI];
-    __device__ __forceinline__ void eval(const PolyTab<R, NI> &pt, const typename Vec4<R>::T &fr, int lane)
+    __device__ __forceinline__ void eval(const SpreadPoly<R, NI> &sp, const typename Vec4<R>::T &fr, int lane)
     {
         const int la8 = lane & 7, lb4 = lane >> 3;
+        if constexpr (NI <= 8) {
+            wa[0] = sp.piece.value(fr.x);
+            const R wb = sp.piece.value(fr.y), wc = sp.piece.value(fr.z);
 #pragma unroll
-        for (int s = 0; s < NSA; s++) wa[s] = la8 + 8 * s < NI ? poly_eval<R, NI>(pt.m[NI - 1 - (la8 + 8 * s)], fr.x) : (R)0;
+            for (int i = 0; i < NTB; i++) mb[i] = __shfl_sync(0xffffffffu, wb, (lb4 + 4 * i) & 7);
 #pragma unroll
-        for (int i = 0; i < NTB; i++) mb[i] = lb4 + 4 * i < NI ? poly_eval<R, NI>(pt.m[NI - 1 - (lb4 + 4 * i)], fr.y) : (R)0;
-        const R mcl = lane < NI ? poly_eval<R, NI>(pt.m[NI - 1 - lane], fr.z) : (R)0;
+            for (int tc = 0; tc < NI; tc++) mc[tc] = __shfl_sync(0xffffffffu, wc, tc);
+        } else {
+            const PolyTab<R, NI> &pt = *sp.pt;
 #pragma unroll
-        for (int tc = 0; tc < NI; tc++) mc[tc] = __shfl_sync(0xffffffffu, mcl, tc);
+            for (int s = 0; s < NSA; s++)
+                wa[s] = la8 + 8 * s < NI ? poly_eval<R, NI>(pt.m[NI - 1 - (la8 + 8 * s)], fr.x) : (R)0;
+#pragma unroll
+            for (int i = 0; i < NTB; i++)
+                mb[i] = lb4 + 4 * i < NI ? poly_eval<R, NI>(pt.m[NI - 1 - (lb4 + 4 * i)], fr.y) : (R)0;
+            const R mcl = lane < NI ? poly_eval<R, NI>(pt.m[NI - 1 - lane], fr.z) : (R)0;
+#pragma unroll
+            for (int tc = 0; tc < NI; tc++) mc[tc] = __shfl_sync(0xffffffffu, mcl, tc);
+        }
     }
 };
 
@@ -735,7 +495,9 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
     R *tl = (R *)smem_raw;
     __shared__ __align__(16) PolyTab<R, NI> pt;
     for (int i = threadIdx.x; i < TG::NPT; i += blockDim.x) tl[i] = (R)0;
-    pt.fill(false);
+    if (NI > 8) pt.fill(false);
+    SpreadPoly<R, NI> sp;
+    sp.init(&pt, threadIdx.x & 31);
     __syncthreads();
     const int tile = vb.x, b = vb.y / t.nshare, z = vb.y - b * t.nshare;
     const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
@@ -761,7 +523,7 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
             fn = load_frac<R>(a.rw, idx);
         }
         SpreadW<R, NI> w;
-        w.eval(pt, fr, lane);
+        w.eval(sp, fr, lane);
         const R q = fr.w;
         const int oa = h.y - ta0, ob = h.z - tb0, oc = h.w - tc0;
         if (oa >= 0 && oa < TG::T && ob >= 0 && ob < TG::T && oc >= 0 && oc < TG::T) {
@@ -800,7 +562,7 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
         const int4 h = a.rhead[idx];
         const R4 fr = load_frac<R>(a.rw, idx);
         SpreadW<R, NI> w;
-        w.eval(pt, fr, lane);
+        w.eval(sp, fr, lane);
         R *g2 = (R *)a.grid + (size_t)(idx % a.P) * a.Na * a.Nb * a.Nc;
         spread_warp_global<R, NI>(a, g2, h.y, h.z, h.w, w, fr.w, lane);
     }
@@ -834,15 +596,16 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
 
 // FP64 spread: shared FP64 atomics are compare-and-swap loops, so here every
 // c plane of the shared tile belongs to one warp (plane c to warp c mod 8)
-// and is added to by plain loads and stores.  The block stages 32 records'
+// and is added to by plain loads and stores.  The block stages 16 records'
 // weights at a time in shared memory (8 threads a record, one barrier a
 // batch); each warp then walks the records, whose stencil holds one plane of
 // its own for every order up to 8, and adds its 8 a x 8 b points, 32 at a
 // time.  4096 TIP4P/F x 32 beads, 64^3, order 8: 525 us with atomics.
+constexpr int kOwnBatch = 16;  // two blocks of 16-point tiles still fit an SM
 template <int NI, int TT>
 constexpr size_t spread_own_smem()
 {
-    return sizeof(double) * ((size_t)TileGeom<NI, TT>::NPT + 2 * 32 * 3 * RecGeom<NI>::NIP);
+    return sizeof(double) * ((size_t)TileGeom<NI, TT>::NPT + 2 * kOwnBatch * 3 * RecGeom<NI>::NIP);
 }
 
 template <int NI, int TT>
@@ -853,11 +616,13 @@ __global__ void __launch_bounds__(256, 2) spread_own_kernel(const __grid_constan
     constexpr int NIP = RecGeom<NI>::NIP, NTB = (NI + 3) / 4, NS8 = (NI + 7) / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *tl = (double *)smem_raw;
-    double *wst = tl + TG::NPT;  // [2][32][3][NIP]: M_a, M_b, q M_c by stencil point
+    double *wst = tl + TG::NPT;  // [2][kOwnBatch][3][NIP]: M_a, M_b, q M_c by stencil point
     __shared__ __align__(16) PolyTab<double, NI> pt;
-    __shared__ int4 org[2][32];  // stencil origin in the tile, record number (~record: outside the tile)
+    __shared__ int4 org[2][kOwnBatch];  // stencil origin in the tile, record number (~record: outside the tile)
     for (int i = threadIdx.x; i < TG::NPT; i += 256) tl[i] = 0.0;
     pt.fill(false);
+    SpreadPoly<double, NI> sp;
+    sp.init(&pt, threadIdx.x & 31);
     __syncthreads();
     const int tile = blockIdx.x, b = blockIdx.y / t.nshare, z = blockIdx.y - b * t.nshare;
     const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
@@ -867,14 +632,14 @@ __global__ void __launch_bounds__(256, 2) spread_own_kernel(const __grid_constan
     const int *list = t.bin + ((size_t)b * t.ntile + tile) * t.cap;
     double *g = (double *)a.grid + (size_t)b * a.Na * a.Nb * a.Nc;
     int buf = 0;
-    for (int e0 = 32 * z; e0 < n; e0 += 32 * t.nshare, buf ^= 1) {
-        const int nb = min(32, n - e0);
+    for (int e0 = kOwnBatch * z; e0 < n; e0 += kOwnBatch * t.nshare, buf ^= 1) {
+        const int nb = min(kOwnBatch, n - e0);
         {
             const int r = threadIdx.x >> 3, j0 = threadIdx.x & 7;
             if (r < nb) {
                 const int idx = list[e0 + r];
                 const double4 fr = load_frac<double>(a.rw, idx);
-                double *w = wst + (buf * 32 + r) * 3 * NIP;
+                double *w = wst + (buf * kOwnBatch + r) * 3 * NIP;
 #pragma unroll
                 for (int s = 0; s < NS8; s++) {
                     const int j = j0 + 8 * s;
@@ -894,7 +659,7 @@ __global__ void __launch_bounds__(256, 2) spread_own_kernel(const __grid_constan
         __syncthreads();  // the other buffer's readers are done when its writers come back
         for (int r = 0; r < nb; r++) {
             const int4 o = org[buf][r];
-            const double *w = wst + (buf * 32 + r) * 3 * NIP;
+            const double *w = wst + (buf * kOwnBatch + r) * 3 * NIP;
             if (o.w >= 0) {
 #pragma unroll
                 for (int s8 = 0; s8 < NS8; s8++) {
@@ -917,7 +682,7 @@ __global__ void __launch_bounds__(256, 2) spread_own_kernel(const __grid_constan
                 const int4 h = a.rhead[idx];
                 const double4 fr = load_frac<double>(a.rw, idx);
                 SpreadW<double, NI> sw;
-                sw.eval(pt, fr, lane);
+                sw.eval(sp, fr, lane);
                 spread_warp_global<double, NI>(a, g, h.y, h.z, h.w, sw, fr.w, lane);
             }
             __syncwarp();
@@ -931,7 +696,7 @@ __global__ void __launch_bounds__(256, 2) spread_own_kernel(const __grid_constan
         const int4 h = a.rhead[idx];
         const double4 fr = load_frac<double>(a.rw, idx);
         SpreadW<double, NI> sw;
-        sw.eval(pt, fr, lane);
+        sw.eval(sp, fr, lane);
         spread_warp_global<double, NI>(a, (double *)a.grid + (size_t)(idx % a.P) * a.Na * a.Nb * a.Nc, h.y, h.z, h.w,
                                        sw, fr.w, lane);
     }
@@ -955,26 +720,34 @@ __global__ void __launch_bounds__(256) spread_tile_c_kernel(const __grid_constan
 
 // Gather weights of one record for lane l8 of an 8-lane group: its a
 // points (l8, l8 + 8) with derivatives, and all b and c points, evaluated by
-// lane t % 8 of the group and shuffled.  Every lane of the warp calls it.
+// lane t % 8 of the group and shuffled; up to order 8 from the lane's piece
+// in registers.  Every lane of the warp calls it.
 template <typename R, int NI>
-__device__ __forceinline__ void gather_weights(const PolyTab<R, NI> &pt, const typename Vec4<R>::T &fr, int l8,
-                                               LaneW<R, NI, true> &lw)
+__device__ __forceinline__ void gather_weights(const PolyTab<R, NI> &pt, const Piece<R, NI <= 8 ? NI : 4> &piece,
+                                               const typename Vec4<R>::T &fr, int l8, LaneW<R, NI, true> &lw)
 {
-    const bool t0 = l8 < NI, t1 = NI > 8 && l8 + 8 < NI;
-    const int p0 = NI - 1 - (t0 ? l8 : 0), p1 = NI - 1 - (t1 ? l8 + 8 : 0);
-    lw.wa0 = t0 ? poly_eval<R, NI>(pt.m[p0], fr.x) : (R)0;
-    lw.da0 = t0 ? poly_eval<R, NI>(pt.dm[p0], fr.x) : (R)0;
-    lw.wa1 = t1 ? poly_eval<R, NI>(pt.m[p1], fr.x) : (R)0;
-    lw.da1 = t1 ? poly_eval<R, NI>(pt.dm[p1], fr.x) : (R)0;
     R ob[2], odb[2], oc[2], odc[2];
-    ob[0] = t0 ? poly_eval<R, NI>(pt.m[p0], fr.y) : (R)0;
-    odb[0] = t0 ? poly_eval<R, NI>(pt.dm[p0], fr.y) : (R)0;
-    oc[0] = t0 ? poly_eval<R, NI>(pt.m[p0], fr.z) : (R)0;
-    odc[0] = t0 ? poly_eval<R, NI>(pt.dm[p0], fr.z) : (R)0;
-    ob[1] = t1 ? poly_eval<R, NI>(pt.m[p1], fr.y) : (R)0;
-    odb[1] = t1 ? poly_eval<R, NI>(pt.dm[p1], fr.y) : (R)0;
-    oc[1] = t1 ? poly_eval<R, NI>(pt.m[p1], fr.z) : (R)0;
-    odc[1] = t1 ? poly_eval<R, NI>(pt.dm[p1], fr.z) : (R)0;
+    if constexpr (NI <= 8) {
+        piece.both(fr.x, lw.wa0, lw.da0);
+        piece.both(fr.y, ob[0], odb[0]);
+        piece.both(fr.z, oc[0], odc[0]);
+        lw.wa1 = lw.da1 = ob[1] = odb[1] = oc[1] = odc[1] = (R)0;
+    } else {
+        const bool t0 = l8 < NI, t1 = NI > 8 && l8 + 8 < NI;
+        const int p0 = NI - 1 - (t0 ? l8 : 0), p1 = NI - 1 - (t1 ? l8 + 8 : 0);
+        lw.wa0 = t0 ? poly_eval<R, NI>(pt.m[p0], fr.x) : (R)0;
+        lw.da0 = t0 ? poly_eval<R, NI>(pt.dm[p0], fr.x) : (R)0;
+        lw.wa1 = t1 ? poly_eval<R, NI>(pt.m[p1], fr.x) : (R)0;
+        lw.da1 = t1 ? poly_eval<R, NI>(pt.dm[p1], fr.x) : (R)0;
+        ob[0] = t0 ? poly_eval<R, NI>(pt.m[p0], fr.y) : (R)0;
+        odb[0] = t0 ? poly_eval<R, NI>(pt.dm[p0], fr.y) : (R)0;
+        oc[0] = t0 ? poly_eval<R, NI>(pt.m[p0], fr.z) : (R)0;
+        odc[0] = t0 ? poly_eval<R, NI>(pt.dm[p0], fr.z) : (R)0;
+        ob[1] = t1 ? poly_eval<R, NI>(pt.m[p1], fr.y) : (R)0;
+        odb[1] = t1 ? poly_eval<R, NI>(pt.dm[p1], fr.y) : (R)0;
+        oc[1] = t1 ? poly_eval<R, NI>(pt.m[p1], fr.z) : (R)0;
+        odc[1] = t1 ? poly_eval<R, NI>(pt.dm[p1], fr.z) : (R)0;
+    }
 #pragma unroll
     for (int s = 0; s < RecGeom<NI>::NIP; s++) {
         if (s >= NI) {
@@ -998,39 +771,18 @@ __device__ __forceinline__ void gather_tile_c_body(const PmeArgs &a, const Cell 
 {
     typedef TileGeom<NI, TT> TG;
     typedef typename Vec4<R>::T R4;
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     R *tl = (R *)smem_raw;
     __shared__ __align__(16) PolyTab<R, NI> pt;
-    pt.fill(true);
+    if (NI > 8) pt.fill(true);
+    Piece<R, NI <= 8 ? NI : 4> piece;
+    piece.load(threadIdx.x & 7);
     const int tile = vb.x, b = vb.y / t.nshare, z = vb.y - b * t.nshare;
     const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
     const R *g = (const R *)a.grid + (size_t)b * a.Na * a.Nb * a.Nc;
     const int n = min(t.cnt[b * t.ntile + tile], t.cap);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int grp = threadIdx.x >> 3, l8 = threadIdx.x & 7, ngrp = blockDim.x >> 3;
-    if (n > z * ngrp) {
-        constexpr int NROW = TG::E * TG::E;
-        if (sizeof(R) == 4 && (a.Na & 3) == 0) {
-            constexpr int NQ = TG::PA / 4;
-            constexpr int RPI = 32 / NQ;
-            for (int r0 = warp * RPI; r0 < NROW; r0 += nwarp * RPI) {
-                const int row = r0 + lane / NQ, q4 = lane % NQ;
-                if (lane >= RPI * NQ || row >= NROW) continue;
-                const int cz = row / TG::E, by = row - cz * TG::E;
-                const float *src = (const float *)g +
-                                   ((size_t)wrapi(tc0 + cz, a.Nc) * a.Nb + wrapi(tb0 + by, a.Nb)) * a.Na +
-                                   wrapi(ta0 + 4 * q4, a.Na);
-                ((float4 *)tl)[row * NQ + q4] = __ldg((const float4 *)src);
-            }
-        } else {
-            for (int row = warp; row < NROW; row += nwarp) {
-                const int cz = row / TG::E, by = row - cz * TG::E;
-                const R *src = g + ((size_t)wrapi(tc0 + cz, a.Nc) * a.Nb + wrapi(tb0 + by, a.Nb)) * a.Na;
-                for (int ax = lane; ax < TG::PA; ax += 32)
-                    tl[row * TG::PA + ax] = ax < TG::E ? src[wrapi(ta0 + ax, a.Na)] : (R)0;
-            }
-        }
-    }
+    if (n > z * ngrp) load_tile<R, TG>(tl, g, a.Na, a.Nb, a.Nc, ta0, tb0, tc0);
     __syncthreads();
     const int *list = t.bin + ((size_t)b * t.ntile + tile) * t.cap;
     const int eb = z * ngrp, estep = ngrp * t.nshare;
@@ -1055,7 +807,7 @@ __device__ __forceinline__ void gather_tile_c_body(const PmeArgs &a, const Cell 
             fn = load_frac<R>(a.rw, in);
         }
         LaneW<R, NI, true> lw;
-        gather_weights<R, NI>(pt, fr, l8, lw);
+        gather_weights<R, NI>(pt, piece, fr, l8, lw);
         double ea = 0, eb = 0, ec = 0;
         if (act) {
             const int oa = h.y - ta0, ob = h.z - tb0, oc = h.w - tc0;
@@ -1089,7 +841,7 @@ __device__ __forceinline__ void gather_tile_c_body(const PmeArgs &a, const Cell 
             fr = load_frac<R>(a.rw, idx);
         }
         LaneW<R, NI, true> lw;
-        gather_weights<R, NI>(pt, fr, l8, lw);
+        gather_weights<R, NI>(pt, piece, fr, l8, lw);
         double ea = 0, eb = 0, ec = 0;
         if (act) {
             const R *g2 = (const R *)a.grid + (size_t)(idx % a.P) * a.Na * a.Nb * a.Nc;
@@ -1651,8 +1403,6 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy, 
     const size_t G = (size_t)a.Na * a.Nb * a.Nc;
     constexpr bool f64 = sizeof(R) == 8;
     const TileArgs t = tile_args_of(c, NI, TT);
-    // the parameter adjoint reads the full weight records of the forward pass
-    const bool full = c->pme_full_records;
     cudaError_t err = cudaSuccess;
     if (!staged) {
         err = launch_pme_clear(c);
@@ -1662,15 +1412,12 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy, 
         if (err != cudaSuccess) return err;
         const long long nt = (long long)a.nchrg * a.P;
         const int threads = 256;
-        if (full) pme_bin_kernel<R, NI><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
-        else pme_bin_compact_kernel<R, NI><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
+        pme_bin_compact_kernel<R, NI><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
         if ((err = kt_mark(c, "pme_bin")) != cudaSuccess) return err;
     }
     const size_t st = (size_t)TileGeom<NI, TT>::NPT * sizeof(R), ss_spread = spread_smem<R, NI, TT>();
     if (ss_spread > 48 * 1024 - sizeof(PolyTab<R, NI>)) {
-        err = smem_optin((const void *)spread_tile_kernel<R, NI, TT>, (int)ss_spread);
-        if constexpr (!f64)
-            if (err == cudaSuccess) err = smem_optin((const void *)spread_tile_c_kernel<R, NI, TT>, (int)ss_spread);
+        if constexpr (!f64) err = smem_optin((const void *)spread_tile_c_kernel<R, NI, TT>, (int)ss_spread);
         if (err != cudaSuccess) return err;
     }
     if constexpr (f64) {
@@ -1678,14 +1425,11 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy, 
         if (err != cudaSuccess) return err;
     }
     if (st > 48 * 1024 - sizeof(PolyTab<R, NI>)) {
-        err = smem_optin((const void *)gather_tile_kernel<R, NI, TT>, (int)st);
-        if (err == cudaSuccess) err = smem_optin((const void *)gather_tile_c_kernel<R, NI, TT>, (int)st);
+        err = smem_optin((const void *)gather_tile_c_kernel<R, NI, TT>, (int)st);
         if (err != cudaSuccess) return err;
     }
     const dim3 tgrid((unsigned)t.ntile, (unsigned)(a.P * t.nshare));
-    const dim3 tgrid1((unsigned)t.ntile, (unsigned)a.P);  // the full-record kernels: one block per bin
-    if (full) spread_tile_kernel<R, NI, TT><<<tgrid1, 256, ss_spread, c->stream>>>(a, t);
-    else if constexpr (f64) spread_own_kernel<NI, TT><<<tgrid, 256, spread_own_smem<NI, TT>(), c->stream>>>(a, t);
+    if constexpr (f64) spread_own_kernel<NI, TT><<<tgrid, 256, spread_own_smem<NI, TT>(), c->stream>>>(a, t);
     else spread_tile_c_kernel<R, NI, TT><<<tgrid, 256, ss_spread, c->stream>>>(a, t);
     if ((err = kt_mark(c, "pme_spread")) != cudaSuccess) return err;
     const R *twbase = (const R *)(f64 ? (const void *)c->d_twiddle64 : (const void *)c->d_twiddle32);
@@ -1695,8 +1439,7 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy, 
     const R *filt = f64 ? (const R *)c->d_filter : (const R *)((const double *)c->d_filter + G);
     err = launch_fft<R>(c, a, cell, spec, filt, tw, sp, ss, energy);
     if (err != cudaSuccess) return err;
-    if (full) gather_tile_kernel<R, NI, TT><<<tgrid1, 256, st, c->stream>>>(a, cell, t);
-    else gather_tile_c_kernel<R, NI, TT><<<tgrid, 256, st, c->stream>>>(a, cell, t);
+    gather_tile_c_kernel<R, NI, TT><<<tgrid, 256, st, c->stream>>>(a, cell, t);
     if ((err = kt_mark(c, "pme_gather")) != cudaSuccess) return err;
     return cudaGetLastError();
 }
@@ -1922,7 +1665,6 @@ static cudaError_t pme_batch_tiles_group(const std::pair<int, int> &key, const s
 // one: grids and bin counters cleared, charges binned, spread, transformed,
 // convolved (energies and virials into each context's per-bead sums when
 // `energy`), transformed back and gathered into each context's PME forces.
-// The contexts' meshes use the compact records (pme_full_records off).
 cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<Cell> &cells, bool energy,
                              int sm_count, cudaStream_t st)
 {
@@ -1933,7 +1675,7 @@ cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::
     for (size_t i = 0; i < box.size(); i++) {
         pinyb200_ctx *c = box[i];
         if (c->sys.nchrg == 0 || c->sys.nktot == 0) continue;
-        if (c->precision != PINYB200_MIXED || c->pme_full_records) return cudaErrorInvalidValue;
+        if (c->precision != PINYB200_MIXED) return cudaErrorInvalidValue;
         const Cell &cell = cells[i];
         const size_t G = (size_t)c->sys.ngrid[0] * c->sys.ngrid[1] * c->sys.ngrid[2];
         bool same = c->filter_ok;
@@ -2073,64 +1815,96 @@ __device__ __forceinline__ void scaled_vec(const PmeArgs &a, const Cell &cell, d
 
 // Q_u: one warp per record, lanes 8 a points x 4 b rows, FP32/FP64 atomics.
 template <typename R, int NI>
-__global__ void __launch_bounds__(256) pme_dipole_spread_kernel(PmeArgs a, Cell cell, const double *__restrict__ uT,
-                                                                R *__restrict__ grid2)
+__global__ void __launch_bounds__(256) pme_dipole_spread_kernel(const __grid_constant__ PmeArgs a,
+                                                                const __grid_constant__ Cell cell,
+                                                                const double *__restrict__ uT, R *__restrict__ grid2)
 {
-    typedef RecGeom<NI> RG;
-    const int lane = threadIdx.x & 31;
-    const int ta = lane & 7, tq = lane >> 3;
+    constexpr int NTB = (NI + 3) / 4, NSA = (NI + 7) / 8;
+    __shared__ __align__(16) PolyTab<R, NI> pt;
+    if (NI > 8) pt.fill(true);
+    Piece<R, NI <= 8 ? NI : 4> piece;
+    piece.load(threadIdx.x & 7);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, la8 = lane & 7, lb4 = lane >> 3;
     const long long nrec = (long long)a.nchrg * a.P;
     const size_t G = (size_t)a.Na * a.Nb * a.Nc;
     for (long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; idx < nrec;
          idx += ((long long)gridDim.x * blockDim.x) >> 5) {
         const int b = (int)(idx % a.P);
         const int4 h = a.rhead[idx];
+        const typename Vec4<R>::T fr = load_frac<R>(a.rw, (int)idx);
         const int at = h.x;
         const double ux = uT[(3 * (size_t)at + 0) * a.P + b], uy = uT[(3 * (size_t)at + 1) * a.P + b],
                      uz = uT[(3 * (size_t)at + 2) * a.P + b];
         if (ux == 0.0 && uy == 0.0 && uz == 0.0) continue;
         double ut[3];
         scaled_vec(a, cell, ux, uy, uz, ut);
-        const R q = (R)a.charge[at];
-        const R *w = (const R *)a.rw + (size_t)idx * RG::NW;
+        R wa[NSA], da[NSA], mb[NTB], db[NTB], mcl = 0, dcl = 0;
+        if constexpr (NI <= 8) {
+            R wb, eb;
+            piece.both(fr.x, wa[0], da[0]);
+            piece.both(fr.y, wb, eb);
+            piece.both(fr.z, mcl, dcl);
+#pragma unroll
+            for (int i = 0; i < NTB; i++) {
+                mb[i] = __shfl_sync(0xffffffffu, wb, (lb4 + 4 * i) & 7);
+                db[i] = __shfl_sync(0xffffffffu, eb, (lb4 + 4 * i) & 7);
+            }
+        } else {
+#pragma unroll
+            for (int s = 0; s < NSA; s++) {
+                const int p = NI - 1 - min(la8 + 8 * s, NI - 1);
+                wa[s] = poly_eval<R, NI>(pt.m[p], fr.x);
+                da[s] = poly_eval<R, NI>(pt.dm[p], fr.x);
+            }
+#pragma unroll
+            for (int i = 0; i < NTB; i++) {
+                const int p = NI - 1 - min(lb4 + 4 * i, NI - 1);
+                mb[i] = poly_eval<R, NI>(pt.m[p], fr.y);
+                db[i] = poly_eval<R, NI>(pt.dm[p], fr.y);
+            }
+            const int p = NI - 1 - min(lane, NI - 1);
+            mcl = poly_eval<R, NI>(pt.m[p], fr.z);
+            dcl = poly_eval<R, NI>(pt.dm[p], fr.z);
+        }
+        const R q = fr.w;
         R *g = grid2 + (size_t)b * G;
-        for (int sa = 0; sa < NI; sa += 8) {
-            const int t_a = ta + sa;
-            if (t_a >= NI) break;
-            const R ma = w[t_a], da = w[3 * RG::NIP + t_a];
-            const int ga = wrapi(h.y + t_a, a.Na);
-            for (int tb = tq; tb < NI; tb += 4) {
-                const R mb = w[RG::NIP + tb], db = w[4 * RG::NIP + tb];
-                const int gb = wrapi(h.z + tb, a.Nb);
-                const R cab = q * ((R)ut[0] * da * mb + (R)ut[1] * ma * db), cc = q * (R)ut[2] * ma * mb;
-                for (int tc = 0; tc < NI; tc++) {
-                    const R val = cab * w[2 * RG::NIP + tc] + cc * w[5 * RG::NIP + tc];
-                    atomicAdd(g + ((size_t)wrapi(h.w + tc, a.Nc) * a.Nb + gb) * a.Na + ga, val);
-                }
+#pragma unroll
+        for (int tc = 0; tc < NI; tc++) {
+            const R mc = __shfl_sync(0xffffffffu, mcl, tc), dc = __shfl_sync(0xffffffffu, dcl, tc);
+            R *pc = g + (size_t)wrapi(h.w + tc, a.Nc) * a.Nb * a.Na;
+#pragma unroll
+            for (int s = 0; s < NSA; s++) {
+                if (la8 + 8 * s >= NI) continue;
+                const R ma = q * wa[s], ga = q * da[s];
+                const R cm = (R)ut[0] * ga * mc + (R)ut[2] * ma * dc, cd = (R)ut[1] * ma * mc;
+                const int ia = wrapi(h.y + la8 + 8 * s, a.Na);
+#pragma unroll
+                for (int i = 0; i < NTB; i++)
+                    if (lb4 + 4 * i < NI)
+                        atomicAdd(pc + (size_t)wrapi(h.z + lb4 + 4 * i, a.Nb) * a.Na + ia, cm * mb[i] + cd * db[i]);
             }
         }
     }
 }
 
-// Value and gradient of a potential g at one record, this lane's a points:
-// s[0] = sum M M M phi, s[1..3] with the derivative along a, b, c.
-template <typename R, int NI>
-__device__ __forceinline__ void adjoint_lane(const PmeArgs &a, const R *g, const int4 &h, const LaneW<R, NI, true> &lw,
-                                             int l8, double *s)
+// Sums of one potential at one record over this lane's a points: value and
+// derivatives along a, b, c; phi(tc, tb, ta) reads the potential.
+template <typename R, int NI, typename PHI>
+__device__ __forceinline__ void adjoint_lane(PHI phi, const LaneW<R, NI, true> &lw, int l8, double *s)
 {
     s[0] = s[1] = s[2] = s[3] = 0.0;
 #pragma unroll
     for (int j = 0; j < (NI > 8 ? 2 : 1); j++) {
-        if (l8 + 8 * j >= NI) break;
-        const int ga = wrapi(h.y + l8 + 8 * j, a.Na);
+        const int ta = l8 + 8 * j;
+        if (ta >= NI) break;
         R smm = 0, sdm = 0, smd = 0;
 #pragma unroll
         for (int tc = 0; tc < NI; tc++) {
-            const R *pc = g + (size_t)wrapi(h.w + tc, a.Nc) * a.Nb * a.Na + ga;
             R um = 0, ud = 0;
 #pragma unroll
             for (int tb = 0; tb < NI; tb++) {
-                const R p = __ldg(pc + (size_t)wrapi(h.z + tb, a.Nb) * a.Na);
+                const R p = phi(tc, tb, ta);
                 um += lw.mb[tb] * p;
                 ud += lw.db[tb] * p;
             }
@@ -2146,149 +1920,198 @@ __device__ __forceinline__ void adjoint_lane(const PmeArgs &a, const R *g, const
     }
 }
 
+// Second derivatives aa, bb, cc, ab, ac, bc of one potential at one record,
+// this lane's share, in FP64; the 8 lanes of the group call it together.
+template <typename R, int NI, typename PHI>
+__device__ __forceinline__ void adjoint_hessian(PHI phi, const Piece<R, NI <= 8 ? NI : 4> &piece,
+                                                const typename Vec4<R>::T &fr, const LaneW<R, NI, true> &lw, int l8,
+                                                double *hs)
+{
+    R d2a[2] = {0, 0}, d2b[NI], d2c[NI];
+    if constexpr (NI <= 8) {
+        const unsigned mask = 0xffu << (threadIdx.x & 24);
+        d2a[0] = piece.second(fr.x);
+        const R sb = piece.second(fr.y), sc = piece.second(fr.z);
+#pragma unroll
+        for (int k = 0; k < NI; k++) {
+            d2b[k] = __shfl_sync(mask, sb, k, 8);
+            d2c[k] = __shfl_sync(mask, sc, k, 8);
+        }
+    } else {
+        R d2[NI + 1];  // grid order: point lo + t carries index NI - t
+        bspline_d2<R, NI>(fr.y, d2);
+#pragma unroll
+        for (int k = 0; k < NI; k++) d2b[k] = d2[NI - k];
+        bspline_d2<R, NI>(fr.z, d2);
+#pragma unroll
+        for (int k = 0; k < NI; k++) d2c[k] = d2[NI - k];
+        bspline_d2<R, NI>(fr.x, d2);
+#pragma unroll
+        for (int k = 0; k < NI; k++) {
+            if (k == l8) d2a[0] = d2[NI - k];
+            if (k == l8 + 8) d2a[1] = d2[NI - k];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < (NI > 8 ? 2 : 1); j++) {
+        const int ta = l8 + 8 * j;
+        if (ta >= NI) break;
+        double smm = 0, s2m = 0, sm2 = 0, sdm = 0, smd = 0, sdd = 0;  // b and c weights
+#pragma unroll
+        for (int tc = 0; tc < NI; tc++) {
+            double um = 0, ud = 0, u2 = 0;
+#pragma unroll
+            for (int tb = 0; tb < NI; tb++) {
+                const double p = (double)phi(tc, tb, ta);
+                um += (double)lw.mb[tb] * p;
+                ud += (double)lw.db[tb] * p;
+                u2 += (double)d2b[tb] * p;
+            }
+            smm += (double)lw.mc[tc] * um;
+            s2m += (double)lw.mc[tc] * u2;
+            sm2 += (double)d2c[tc] * um;
+            sdm += (double)lw.mc[tc] * ud;
+            smd += (double)lw.dc[tc] * um;
+            sdd += (double)lw.dc[tc] * ud;
+        }
+        const double wa = j ? lw.wa1 : lw.wa0, da = j ? lw.da1 : lw.da0;
+        hs[0] += (double)d2a[j] * smm;
+        hs[1] += wa * s2m;
+        hs[2] += wa * sm2;
+        hs[3] += da * sdm;
+        hs[4] += da * smd;
+        hs[5] += wa * sdd;
+    }
+}
+
 // Gathers phi, grad phi, chi, grad chi (and grad grad phi at sites with a
-// ghost tangent) per record and contracts them with every channel.  Blocks
-// take a bin's records (tile, bead, one of gridDim.z shares), whose stencils
-// overlap in L1; 8 lanes a record, a lane an a point, as in the gather: the
-// weights along a factor out and a row is one 32-byte sector.  Bound: L1/L2
-// sector reads, 128 per record.  1024 TIP4P/F x 16 beads, 32^3, FP32: 277 us
-// as one thread per record in record order.
-template <typename R, int NI>
-__global__ void __launch_bounds__(256) pme_adjoint_gather_kernel(const __grid_constant__ PmeArgs a,
+// ghost tangent) per record and contracts them with every channel.  As the
+// gather: a block per (tile, bead, share), the tile's potential in shared
+// memory (phi, then chi in its place), 8 lanes a record.  The contraction is
+// linear, so each potential's terms are added on their own.  Bound:
+// shared-memory reads, 128 a record and lane.  1024 TIP4P/F x 16 beads, 32^3,
+// FP32: 277 us as one thread per record reading global memory.
+template <typename R, int NI, int TT>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 && NI <= 8 ? 2 : 1) pme_adjoint_gather_kernel(const __grid_constant__ PmeArgs a,
                                                                  const __grid_constant__ Cell cell,
                                                                  const __grid_constant__ TileArgs t,
                                                                  const __grid_constant__ GradArgs g,
                                                                  const R *__restrict__ phi, const R *__restrict__ chi)
 {
+    typedef TileGeom<NI, TT> TG;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    R *tl = (R *)smem_raw;
+    __shared__ __align__(16) PolyTab<R, NI> pt;
     __shared__ double sh[2 * PINYB200_MAX_TAN];
+    if (NI > 8) pt.fill(true);
+    Piece<R, NI <= 8 ? NI : 4> piece;
+    piece.load(threadIdx.x & 7);
     double acc[2 * PINYB200_MAX_TAN];
     for (int k = 0; k < 2 * g.K; k++) acc[k] = 0.0;
     const size_t G = (size_t)a.Na * a.Nb * a.Nc;
     const int l8 = threadIdx.x & 7, grp = threadIdx.x >> 3, ngrp = blockDim.x >> 3;
-    // one record (idx of bead b) by the 8 lanes of a group; every lane of the
-    // warp calls it (shuffles)
-    auto record = [&](bool act, int idx, int b) {
-        int4 h = make_int4(0, 0, 0, 0);
-        LaneW<R, NI, true> lw;
-        double s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, hs[6] = {0, 0, 0, 0, 0, 0};
-        bool need_h = false;
-        if (act) {
-            h = a.rhead[idx];
-            lw.load((const R *)a.rw, idx, l8);
-            adjoint_lane<R, NI>(a, phi + (size_t)b * G, h, lw, l8, s);
-            adjoint_lane<R, NI>(a, chi + (size_t)b * G, h, lw, l8, s + 4);
-            // the ghost-position tangents of this site, if any
-            for (int k = 0; k < g.K; k++)
-                if (g.ch[k].w) {
-                    const double *wv = g.ch[k].w + (3 * (size_t)h.x) * a.P + b;
-                    need_h |= wv[0] != 0.0 || wv[a.P] != 0.0 || wv[2 * a.P] != 0.0;
-                }
-        }
-        if (act && need_h) {
-            int la, lb, lc;
-            double fa, fb, fc;
-            stencil_origin(a, cell, h.x, b, NI, la, lb, lc, fa, fb, fc);
-            R d2[NI + 1], d2b[NI], d2c[NI];
-            bspline_d2<R, NI>((R)fb, d2);
-#pragma unroll
-            for (int k = 0; k < NI; k++) d2b[k] = d2[NI - k];  // grid order: point lo + t carries index NI - t
-            bspline_d2<R, NI>((R)fc, d2);
-#pragma unroll
-            for (int k = 0; k < NI; k++) d2c[k] = d2[NI - k];
-            bspline_d2<R, NI>((R)fa, d2);
-            const R *pg = phi + (size_t)b * G;
-#pragma unroll
-            for (int j = 0; j < (NI > 8 ? 2 : 1); j++) {
-                const int ta = l8 + 8 * j;
-                if (ta >= NI) break;
-                R d2a = 0;
-#pragma unroll
-                for (int k = 0; k < NI; k++)
-                    if (k == ta) d2a = d2[NI - k];
-                const int ga = wrapi(h.y + ta, a.Na);
-                double smm = 0, s2m = 0, sm2 = 0, sdm = 0, smd = 0, sdd = 0;  // b and c weights
-#pragma unroll
-                for (int tc = 0; tc < NI; tc++) {
-                    const R *pc = pg + (size_t)wrapi(h.w + tc, a.Nc) * a.Nb * a.Na + ga;
-                    double um = 0, ud = 0, u2 = 0;
-#pragma unroll
-                    for (int tb = 0; tb < NI; tb++) {
-                        const double p = (double)__ldg(pc + (size_t)wrapi(h.z + tb, a.Nb) * a.Na);
-                        um += (double)lw.mb[tb] * p;
-                        ud += (double)lw.db[tb] * p;
-                        u2 += (double)d2b[tb] * p;
-                    }
-                    smm += (double)lw.mc[tc] * um;
-                    s2m += (double)lw.mc[tc] * u2;
-                    sm2 += (double)d2c[tc] * um;
-                    sdm += (double)lw.mc[tc] * ud;
-                    smd += (double)lw.dc[tc] * um;
-                    sdd += (double)lw.dc[tc] * ud;
-                }
-                const double wa = j ? lw.wa1 : lw.wa0, da = j ? lw.da1 : lw.da0;
-                hs[0] += (double)d2a * smm;
-                hs[1] += wa * s2m;
-                hs[2] += wa * sm2;
-                hs[3] += da * sdm;
-                hs[4] += da * smd;
-                hs[5] += wa * sdd;
+    const int lane = threadIdx.x & 31;
+    const int tile = blockIdx.x, b0 = blockIdx.y / t.nshare, z = blockIdx.y - b0 * t.nshare;
+    const int ta0 = (tile % t.nta) * TG::T, tb0 = ((tile / t.nta) % t.ntb) * TG::T, tc0 = (tile / (t.nta * t.ntb)) * TG::T;
+    const int n = min(t.cnt[b0 * t.ntile + tile], t.cap);
+    const int *list = t.bin + ((size_t)b0 * t.ntile + tile) * t.cap;
+    const int nov = t.cnt[a.P * t.ntile];
+    const int gid = blockIdx.y * gridDim.x + blockIdx.x, nblk = gridDim.x * gridDim.y;
+    bool any_w = false;
+    for (int k = 0; k < g.K; k++) any_w |= g.ch[k].w != nullptr;
+
+    for (int which = 0; which < 2; which++) {  // 0 phi, 1 chi
+        const R *pot = which ? chi : phi;
+        if (n > z * ngrp) load_tile<R, TG>(tl, pot + (size_t)b0 * G, a.Na, a.Nb, a.Nc, ta0, tb0, tc0);
+        __syncthreads();
+        // one record by the 8 lanes of a group; every lane of the warp calls it
+        auto record = [&](bool act, int idx, bool binned) {
+            const int b = idx % a.P;
+            int4 h = make_int4(0, 0, 0, 0);
+            typename Vec4<R>::T fr = {};
+            if (act) {
+                h = a.rhead[idx];
+                fr = load_frac<R>(a.rw, idx);
             }
-        }
-#pragma unroll
-        for (int o = 4; o >= 1; o >>= 1) {
-#pragma unroll
-            for (int k = 0; k < 8; k++) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-        }
-        if (__any_sync(0xffffffffu, need_h)) {
+            LaneW<R, NI, true> lw;
+            gather_weights<R, NI>(pt, piece, fr, l8, lw);
+            double s[4] = {0, 0, 0, 0}, hs[6] = {0, 0, 0, 0, 0, 0};
+            bool need_h = false;  // a ghost-position tangent at this site
+            if (act && any_w)
+                for (int k = 0; k < g.K; k++)
+                    if (g.ch[k].w) {
+                        const double *wv = g.ch[k].w + (3 * (size_t)h.x) * a.P + b;
+                        need_h |= wv[0] != 0.0 || wv[a.P] != 0.0 || wv[2 * a.P] != 0.0;
+                    }
+            const bool hess = need_h && which == 0;
+            const int oa = h.y - ta0, ob = h.z - tb0, oc = h.w - tc0;
+            if (act && binned && oa >= 0 && oa < TG::T && ob >= 0 && ob < TG::T && oc >= 0 && oc < TG::T) {
+                const R *base = tl + (oc * TG::E + ob) * TG::PA + oa;
+                auto get = [&](int tc, int tb, int ta) { return base[(tc * TG::E + tb) * TG::PA + ta]; };
+                adjoint_lane<R, NI>(get, lw, l8, s);
+                if (hess) adjoint_hessian<R, NI>(get, piece, fr, lw, l8, hs);
+            } else if (act) {
+                const R *gb = pot + (size_t)b * G;
+                auto get = [&](int tc, int tb, int ta) {
+                    return gb[((size_t)wrapi(h.w + tc, a.Nc) * a.Nb + wrapi(h.z + tb, a.Nb)) * a.Na +
+                              wrapi(h.y + ta, a.Na)];
+                };
+                adjoint_lane<R, NI>(get, lw, l8, s);
+                if (hess) adjoint_hessian<R, NI>(get, piece, fr, lw, l8, hs);
+            }
 #pragma unroll
             for (int o = 4; o >= 1; o >>= 1) {
 #pragma unroll
-                for (int k = 0; k < 6; k++) hs[k] += __shfl_xor_sync(0xffffffffu, hs[k], o);
+                for (int k = 0; k < 4; k++) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
             }
-        }
-        if (!act || l8 != 0) return;
-        const int at = h.x;
-        const double ux = g.uT[(3 * (size_t)at + 0) * a.P + b], uy = g.uT[(3 * (size_t)at + 1) * a.P + b],
-                     uz = g.uT[(3 * (size_t)at + 2) * a.P + b];
-        double ut[3];
-        scaled_vec(a, cell, ux, uy, uz, ut);
-        const double udphi = ut[0] * s[1] + ut[1] * s[2] + ut[2] * s[3];
-        const double q = a.charge[at];
-        for (int k = 0; k < g.K; k++) {
-            const GradChan &ch = g.ch[k];
-            if (ch.dq) {
-                const double dq = ch.dq[at];
-                if (dq != 0.0) {
-                    acc[2 * k] += dq * s[0] / (double)a.P;
-                    acc[2 * k + 1] += -dq * (udphi + s[4]);
+            if (__any_sync(0xffffffffu, hess)) {
+#pragma unroll
+                for (int o = 4; o >= 1; o >>= 1) {
+#pragma unroll
+                    for (int k = 0; k < 6; k++) hs[k] += __shfl_xor_sync(0xffffffffu, hs[k], o);
                 }
             }
-            if (ch.w && need_h) {
-                const double wx = ch.w[(3 * (size_t)at) * a.P + b], wy = ch.w[(3 * (size_t)at + 1) * a.P + b],
-                             wz = ch.w[(3 * (size_t)at + 2) * a.P + b];
-                double wt[3];
-                scaled_vec(a, cell, wx, wy, wz, wt);
-                const double uhw = ut[0] * (hs[0] * wt[0] + hs[3] * wt[1] + hs[4] * wt[2]) +
-                                   ut[1] * (hs[3] * wt[0] + hs[1] * wt[1] + hs[5] * wt[2]) +
-                                   ut[2] * (hs[4] * wt[0] + hs[5] * wt[1] + hs[2] * wt[2]);
-                acc[2 * k + 1] += -q * (wt[0] * s[5] + wt[1] * s[6] + wt[2] * s[7] + uhw);
+            if (!act || l8 != 0) return;
+            const int at = h.x;
+            double ut[3] = {0, 0, 0};
+            if (which == 0)
+                scaled_vec(a, cell, g.uT[(3 * (size_t)at + 0) * a.P + b], g.uT[(3 * (size_t)at + 1) * a.P + b],
+                           g.uT[(3 * (size_t)at + 2) * a.P + b], ut);
+            const double q = a.charge[at];
+            for (int k = 0; k < g.K; k++) {
+                const GradChan &ch = g.ch[k];
+                if (ch.dq) {
+                    const double dq = ch.dq[at];
+                    if (dq != 0.0) {
+                        if (which == 0) {
+                            acc[2 * k] += dq * s[0] / (double)a.P;
+                            acc[2 * k + 1] -= dq * (ut[0] * s[1] + ut[1] * s[2] + ut[2] * s[3]);
+                        } else {
+                            acc[2 * k + 1] -= dq * s[0];
+                        }
+                    }
+                }
+                if (ch.w && need_h) {
+                    double wt[3];
+                    scaled_vec(a, cell, ch.w[(3 * (size_t)at) * a.P + b], ch.w[(3 * (size_t)at + 1) * a.P + b],
+                               ch.w[(3 * (size_t)at + 2) * a.P + b], wt);
+                    const double v = which ? wt[0] * s[1] + wt[1] * s[2] + wt[2] * s[3]
+                                           : ut[0] * (hs[0] * wt[0] + hs[3] * wt[1] + hs[4] * wt[2]) +
+                                                 ut[1] * (hs[3] * wt[0] + hs[1] * wt[1] + hs[5] * wt[2]) +
+                                                 ut[2] * (hs[4] * wt[0] + hs[5] * wt[1] + hs[2] * wt[2]);
+                    acc[2 * k + 1] -= q * v;
+                }
             }
+        };
+        for (int e0 = ngrp * z; e0 < n; e0 += ngrp * t.nshare) {
+            const int e = e0 + grp;
+            record(e < n, e < n ? list[e] : 0, true);
         }
-    };
-    const int tile = blockIdx.x, b = blockIdx.y;
-    const int n = min(t.cnt[b * t.ntile + tile], t.cap);
-    const int *list = t.bin + ((size_t)b * t.ntile + tile) * t.cap;
-    const int step = ngrp * gridDim.z;
-    for (int e0 = ngrp * blockIdx.z; e0 < n; e0 += step) {
-        const int e = e0 + grp;
-        record(e < n, e < n ? list[e] : 0, b);
-    }
-    const int nov = t.cnt[a.P * t.ntile];
-    const int gid = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    const int nblk = gridDim.x * gridDim.y * gridDim.z;
-    for (int e0 = gid * ngrp; e0 < nov; e0 += nblk * ngrp) {
-        const int e = e0 + grp, idx = e < nov ? t.ovf[e] : 0;
-        record(e < nov, idx, idx % a.P);
+        for (int e0 = gid * ngrp; e0 < nov; e0 += nblk * ngrp) {
+            const int e = e0 + grp;
+            record(e < nov, e < nov ? t.ovf[e] : 0, false);
+        }
+        __syncthreads();
     }
     // block flush: warp sums (lanes other than a group's first hold zeros)
     for (int i = threadIdx.x; i < 2 * g.K; i += blockDim.x) sh[i] = 0.0;
@@ -2297,33 +2120,34 @@ __global__ void __launch_bounds__(256) pme_adjoint_gather_kernel(const __grid_co
         const double v = acc[i];
         if (!__any_sync(0xffffffffu, v != 0.0)) continue;
         const double w = warp_sum(v);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&sh[i], w);
+        if (lane == 0) atomicAdd(&sh[i], w);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * g.K; i += blockDim.x)
         if (sh[i] != 0.0) atomicAdd(&g.gacc[i], sh[i]);
 }
 
+template <typename R, int NI, int TT>
+static cudaError_t launch_adjoint_gather(pinyb200_ctx *c, const PmeArgs &a, const Cell &cell, const GradArgs &g)
+{
+    TileArgs t = tile_args_of(c, NI, TT);
+    // two passes of loads and a wide inner loop: more blocks per bin than the gather
+    const int bins = t.ntile * a.P;
+    t.nshare = std::max(1, std::min(8, (4 * c->sm_count + bins - 1) / bins));
+    const size_t st = (size_t)TileGeom<NI, TT>::NPT * sizeof(R);
+    cudaError_t err = smem_optin((const void *)pme_adjoint_gather_kernel<R, NI, TT>, (int)st);
+    if (err != cudaSuccess) return err;
+    pme_adjoint_gather_kernel<R, NI, TT><<<dim3((unsigned)t.ntile, (unsigned)(a.P * t.nshare)), 256, st, c->stream>>>(
+        a, cell, t, g, (const R *)c->d_grid, (const R *)c->grad.d_grid2);
+    return cudaGetLastError();
+}
+
 template <typename R, int NI>
 static cudaError_t launch_pme_adjoint_t(pinyb200_ctx *c, const Cell &cell, const GradArgs &g)
 {
     typedef typename Cplx<R>::T C2;
-    const DeviceSystem &s = c->sys;
-    PmeArgs a;
-    a.natm = s.natm;
-    a.P = c->P;
-    a.nchrg = s.nchrg;
-    a.ichrg = s.ichrg;
-    a.charge = s.charge;
-    a.posT = c->d_posT;
-    a.Na = s.ngrid[0];
-    a.Nb = s.ngrid[1];
-    a.Nc = s.ngrid[2];
-    a.n = s.n_interp;
+    PmeArgs a = pme_args_of(c);
     a.grid = c->grad.d_grid2;
-    a.forceP = c->d_forceP;
-    a.rhead = (int4 *)c->d_pme_head;
-    a.rw = c->d_pme_w;
     const size_t G = (size_t)a.Na * a.Nb * a.Nc;
     const bool f64 = sizeof(R) == 8;
     cudaError_t err = cudaMemsetAsync(c->grad.d_grid2, 0, sizeof(R) * G * c->P, c->stream);
@@ -2339,13 +2163,7 @@ static cudaError_t launch_pme_adjoint_t(pinyb200_ctx *c, const Cell &cell, const
     const R *filt = f64 ? (const R *)c->d_filter : (const R *)((const double *)c->d_filter + G);
     err = launch_fft<R>(c, a, cell, spec, filt, tw, sp, ss, false);
     if (err != cudaSuccess) return err;
-    const TileArgs t = tile_args_of(c, NI, c->pme_tile);
-    // a bin's records shared by as many blocks as give every SM some eight
-    const long long bins = (long long)t.ntile * a.P;
-    const unsigned split = (unsigned)std::max(1LL, std::min(16LL, (8LL * c->sm_count + bins - 1) / bins));
-    pme_adjoint_gather_kernel<R, NI><<<dim3((unsigned)t.ntile, (unsigned)a.P, split), 256, 0, c->stream>>>(
-        a, cell, t, g, (const R *)c->d_grid, (const R *)c->grad.d_grid2);
-    return cudaGetLastError();
+    return c->pme_tile == 8 ? launch_adjoint_gather<R, NI, 8>(c, a, cell, g) : launch_adjoint_gather<R, NI, 16>(c, a, cell, g);
 }
 
 template <typename R>

@@ -66,9 +66,9 @@ struct TileArgs {
 
 // One (charge k, bead b) record, number k P + b, at position (x, y, z):
 // stencil origin in FP64 with PINY's operation order and the fractional
-// offsets with the charge in R; its number filed under its origin's tile.
+// offsets with the charge in R; returns the bin (bead and tile of its origin).
 template <typename R>
-__device__ __forceinline__ void pme_file_record(const PmeArgs &a, const TileArgs &t, const Cell &cell, int at, int k,
+__device__ __forceinline__ int pme_write_record(const PmeArgs &a, const TileArgs &t, const Cell &cell, int at, int k,
                                                 int b, double x, double y, double z)
 {
     const int idx = k * a.P + b;
@@ -82,11 +82,23 @@ __device__ __forceinline__ void pme_file_record(const PmeArgs &a, const TileArgs
     fr.w = (R)a.charge[at];
     ((typename Vec4<R>::T *)a.rw)[idx] = fr;
     a.rhead[idx] = make_int4(at, la, lb, lc);
-    const int T = t.T;
-    const int tile = ((lc / T) * t.ntb + lb / T) * t.nta + la / T;
-    const int slot = atomicAdd(&t.cnt[b * t.ntile + tile], 1);
-    if (slot < t.cap) t.bin[((size_t)b * t.ntile + tile) * t.cap + slot] = idx;
+    const int sh = t.T == 8 ? 3 : 4;  // tile edges are 8 or 16
+    return b * t.ntile + ((lc >> sh) * t.ntb + (lb >> sh)) * t.nta + (la >> sh);
+}
+
+// Record idx into place `slot` of its bin, or the overflow list.
+__device__ __forceinline__ void pme_put_record(const PmeArgs &a, const TileArgs &t, int bin, int slot, int idx)
+{
+    if (slot < t.cap) t.bin[(size_t)bin * t.cap + slot] = idx;
     else t.ovf[atomicAdd(&t.cnt[a.P * t.ntile], 1)] = idx;
+}
+
+template <typename R>
+__device__ __forceinline__ void pme_file_record(const PmeArgs &a, const TileArgs &t, const Cell &cell, int at, int k,
+                                                int b, double x, double y, double z)
+{
+    const int bin = pme_write_record<R>(a, t, cell, at, k, b, x, y, z);
+    pme_put_record(a, t, bin, atomicAdd(&t.cnt[bin], 1), k * a.P + b);
 }
 
 // Kernel arguments of a context's mesh, and of its tile bins for spline order

@@ -89,12 +89,19 @@ __device__ __forceinline__ void water_stage_body(const StageArgs &a, const PmeAr
             for (int k = 3; k < NC; k++) ext = fmax(ext, fabs(x[k] - x[k % 3]));
         }
         if (a.bin) {
+            // the counters' replies are waited for together
             constexpr int NQ = Q0 ? NS : NS - 1, S0 = Q0 ? 0 : 1;
+            int bin[NQ], slot[NQ];
 #pragma unroll
             for (int q = 0; q < NQ; q++) {
-                const int s = S0 + q, k = m * NQ + q, at = m * NS + s;
-                pme_file_record<R>(pm, tl, cell, at, k, b, x[3 * s], x[3 * s + 1], x[3 * s + 2]);
+                const int s = S0 + q;
+                bin[q] = pme_write_record<R>(pm, tl, cell, m * NS + s, m * NQ + q, b, x[3 * s], x[3 * s + 1],
+                                             x[3 * s + 2]);
             }
+#pragma unroll
+            for (int q = 0; q < NQ; q++) slot[q] = atomicAdd(&tl.cnt[bin[q]], 1);
+#pragma unroll
+            for (int q = 0; q < NQ; q++) pme_put_record(pm, tl, bin[q], slot[q], (m * NQ + q) * P + b);
         }
     }
     if (P > 1) {
