@@ -586,7 +586,8 @@ __global__ void __launch_bounds__(256, 2) mol_list_cell_kernel(const int *__rest
     const int home = blockIdx.x;
     const int ha = home % na, hb = (home / na) % nb, hc = home / (na * nb);
     const int h0 = coff[home], nhome = coff[home + 1] - h0;
-    if (nhome == 0) return;
+    // gridDim.y blocks share a cell's molecules, eight at a time
+    if (nhome <= nwarp * (int)blockIdx.y) return;
     mol_site_tables<NS>(a, tcs2, tact);
     if (threadIdx.x < 125) {
         const int k = threadIdx.x;
@@ -623,7 +624,7 @@ __global__ void __launch_bounds__(256, 2) mol_list_cell_kernel(const int *__rest
             sx[e] = v;
         }
         __syncthreads();
-        for (int hk = warp; hk < nhome; hk += nwarp) {
+        for (int hk = warp + nwarp * (int)blockIdx.y; hk < nhome; hk += nwarp * (int)gridDim.y) {
             const int mi = cmol[h0 + hk];
             const int i0 = a.mstart[mi], ni = a.mstart[mi + 1] - i0;
             const float4 si = a.msf[mi];
@@ -654,7 +655,8 @@ __global__ void __launch_bounds__(256, 2) mol_list_cell_kernel(const int *__rest
     }
     __syncthreads();
     if (!FILL)
-        for (int hk = threadIdx.x; hk < nhome; hk += blockDim.x) a.count[cmol[h0 + hk]] = hcnt[hk];
+        for (int hk = threadIdx.x; hk < nhome; hk += blockDim.x)
+            if (hk / nwarp % (int)gridDim.y == (int)blockIdx.y) a.count[cmol[h0 + hk]] = hcnt[hk];
     if (FILL) {
         for (int o = 16; o >= 1; o >>= 1) sites += __shfl_xor_sync(0xffffffffu, sites, o);
         if (lane == 0) atomicAdd(a.nsite, sites);
@@ -1747,12 +1749,18 @@ cudaError_t launch_mol_list(pinyb200_ctx *c, const Cell &cell, const double *d_p
         }
     }
     const int cell_smem = PINYB200_CELL_BATCH * (int)sizeof(float4);
+    // a cell's molecules, eight to a block at a time, go to as many blocks as
+    // fill the SMs' block slots some four times (343 cells of 23 at 8000
+    // TIP4P/F: one block a cell left the second wave nearly empty, 372 us)
+    const int csplit = ncell > 0 ? std::max(1, std::min(std::min(4, (c->nmol / ncell + 7) / 8),
+                                                        (8 * c->sm_count + ncell - 1) / ncell))
+                                 : 1;
 #define MOL_LIST(NSV, FILLV, XMV)                                                                                 \
     {                                                                                                             \
         if (cells) {                                                                                              \
             if ((e = smem_optin((const void *)mol_list_cell_kernel<FILLV, NSV, XMV>, cell_smem)) != cudaSuccess)  \
                 return e;                                                                                         \
-            mol_list_cell_kernel<FILLV, NSV, XMV><<<ncell, 256, cell_smem, st>>>(                                 \
+            mol_list_cell_kernel<FILLV, NSV, XMV><<<dim3(ncell, csplit), 256, cell_smem, st>>>(                   \
                 gate, cellok, c->cell_n[0], c->cell_n[1], c->cell_n[2], c->d_coff, c->d_cmol + c->nmol, pl, cell,  \
                 a);                                                                                               \
         }                                                                                                         \
