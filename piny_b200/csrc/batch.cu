@@ -113,8 +113,8 @@ int bfail(pinyb200_batch *bt, int code, const std::string &msg)
     } while (0)
 
 // Whether the multi-box kernels cover every box of the call: MIXED
-// molecule-pair kernel with a known site pattern, orthorhombic cells,
-// compact PME records, flags they serve.
+// molecule-pair kernel with a known site pattern, water molecules as the
+// staging and finishing kernels take them, orthorhombic cells, flags they serve.
 bool fused_ok(const pinyb200_batch *bt, const double *const *hmat, int flags)
 {
     if (flags & (PINYB200_UPDATE_LIST | PINYB200_SITE_PAIRS | PINYB200_BATCH_BRANCHES)) return false;
@@ -122,7 +122,7 @@ bool fused_ok(const pinyb200_batch *bt, const double *const *hmat, int flags)
         const pinyb200_ctx *c = bt->box[i];
         const double *h = hmat[i];
         const bool ortho = h[1] == 0.0 && h[2] == 0.0 && h[3] == 0.0 && h[5] == 0.0 && h[6] == 0.0 && h[7] == 0.0;
-        if (c->precision != PINYB200_MIXED || !c->use_mol || !c->mol_ok || !c->mix_ok || mix_pattern(c) == 0 ||
+        if (c->precision != PINYB200_MIXED || !c->water_ok || !c->use_mol || !c->mol_ok || !c->mix_ok || mix_pattern(c) == 0 ||
             !ortho || c->sm_count != bt->box[0]->sm_count)
             return false;
     }
@@ -142,34 +142,31 @@ int fused_enqueue(pinyb200_batch *bt, const double *const *d_pos, const double *
     std::vector<const double *> pos;
     std::vector<double *> force;
     std::vector<std::pair<void *, size_t>> zero;
-    std::vector<CopySeg> xm, acc;
+    std::vector<CopySeg> acc;
+    std::vector<const double *> xm;
     for (int i = 0; i < nbox; i++) {
         pinyb200_ctx *c = bt->box[i];
         cells.push_back(cell_from_hmat(hmat[i]));
         pos.push_back(d_pos[i]);
         force.push_back(d_force[i]);
-        const size_t nb = (size_t)c->sys.natm * 3 * c->P;
-        zero.emplace_back(c->d_forceT, nb * sizeof(double));
+        xm.push_back(c->P > 1 && d_xmod ? d_xmod[i] : nullptr);
         zero.emplace_back(c->d_acc, (size_t)c->P * S_NSLOT * sizeof(double));
-        if (c->P > 1) {
-            const double *src = d_xmod ? d_xmod[i] : nullptr;
-            if (src != c->d_xmod) xm.push_back(CopySeg{src, c->d_posT, c->d_xmod, (long long)c->sys.natm * 3, c->P});
+        if (c->sys.nchrg > 0 && c->sys.nktot > 0) {
+            const size_t G = (size_t)c->sys.ngrid[0] * c->sys.ngrid[1] * c->sys.ngrid[2];
+            zero.emplace_back(c->d_pme_cnt, ((size_t)c->P * c->pme_ntile + 1) * sizeof(int));
+            zero.emplace_back(c->d_grid, sizeof(float) * G * c->P);
         }
         if (energy)
-            acc.push_back(CopySeg{c->d_acc, nullptr, bt->h_acc + bt->acc_off[i], (long long)c->P * S_NSLOT, 1});
+            acc.push_back(CopySeg{c->d_acc, bt->h_acc + bt->acc_off[i], (long long)c->P * S_NSLOT});
     }
     cudaError_t e = launch_zero_batch(zero, sm, st);
-    if (e == cudaSuccess) e = launch_transpose_in_batch(bt->box, pos, sm, st);
-    if (e == cudaSuccess && !xm.empty()) e = launch_copy_batch(xm, sm, st);
-    if (e == cudaSuccess) e = launch_ghost_batch(bt->box, false, sm, st);
-    if (e == cudaSuccess) e = launch_mol_extent_batch(bt->box, sm, st);
+    if (e == cudaSuccess) e = launch_water_stage_batch(bt->box, cells, pos, xm, sm, st);
     // The force terms as parallel branches: one per PME shape group (order,
     // tile edge, mesh: its whole chain of launches), one per pair-kernel
-    // group (bead count, site pattern), one for the intramolecular terms;
-    // heaviest first.  Independent groups overlap, so no launch's tail
+    // group (bead count, site pattern); heaviest first.  Independent groups overlap, so no launch's tail
     // leaves the GPU idle while other groups still have work.
     struct Branch {
-        int kind;  // 0 PME, 1 pair, 2 intramolecular
+        int kind;  // 0 PME, 1 pair
         std::vector<pinyb200_ctx *> box;
         std::vector<Cell> cell;
         double work;
@@ -194,7 +191,6 @@ int fused_enqueue(pinyb200_batch *bt, const double *const *d_pos, const double *
     }
     std::vector<Branch> br;
     for (auto &kv : groups) br.push_back(kv.second);
-    br.push_back(Branch{2, bt->box, cells, 0.0});
     std::stable_sort(br.begin(), br.end(), [](const Branch &x, const Branch &y) { return x.work > y.work; });
     const size_t npool = 12;
     while (e == cudaSuccess && bt->gstream.size() < std::min(npool, br.size())) {
@@ -213,14 +209,12 @@ int fused_enqueue(pinyb200_batch *bt, const double *const *d_pos, const double *
         e = cudaStreamWaitEvent(s, bt->pfork, 0);
         if (e != cudaSuccess) break;
         if (br[k].kind == 0) e = launch_pme_batch(br[k].box, br[k].cell, energy, sm, s);
-        else if (br[k].kind == 1) e = launch_mol_pair_mixed_batch(br[k].box, br[k].cell, energy, sm, s);
-        else e = launch_intra_batch(br[k].box, energy, sm, s);
+        else e = launch_mol_pair_mixed_batch(br[k].box, br[k].cell, energy, sm, s);
         if (e == cudaSuccess) e = cudaEventRecord(bt->gjoin[k], s);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, bt->gjoin[k], 0);
     }
-    if (e == cudaSuccess) e = launch_pme_force_add_batch(bt->box, sm, st);
-    if (e == cudaSuccess && (flags & PINYB200_DISTRIB_GHOSTS)) e = launch_ghost_batch(bt->box, true, sm, st);
-    if (e == cudaSuccess) e = launch_transpose_out_batch(bt->box, force, sm, st);
+    if (e == cudaSuccess)
+        e = launch_water_finish_batch(bt->box, force, energy, (flags & PINYB200_DISTRIB_GHOSTS) != 0, sm, st);
     // per-bead sums straight into the pinned host buffer
     if (e == cudaSuccess && energy) e = launch_copy_batch(acc, sm, st);
     if (e != cudaSuccess) return bfail(bt, PINYB200_ERR_CUDA, std::string("batch kernels: ") + cudaGetErrorString(e));

@@ -486,7 +486,7 @@ int pinyb200_destroy(pinyb200_ctx *c)
     cudaSetDevice(c->device);
     pme_res_free(c);
     free_sys(c->sys);
-    void *ptrs[] = {c->d_row, c->d_col, c->d_rowA, c->d_colA, c->d_count, c->d_tot, c->d_posT, c->d_forceT,
+    void *ptrs[] = {c->d_row, c->d_col, c->d_rowA, c->d_colA, c->d_count, c->d_tot, c->d_posT, c->d_offT, c->d_forceT,
                     c->d_xmod, c->d_pos_aos, c->d_force_aos, c->d_acc, c->d_grid, c->d_spec, c->d_filter, c->d_twiddle64,
                     c->d_twiddle32, c->d_err, c->d_mstart, c->d_mcount, c->d_mrow, c->d_mj, c->d_mmask, c->d_chunk,
                     c->d_pme_cnt, c->d_pme_bin, c->d_pme_ovf, c->d_x0, c->d_forceP,
@@ -653,6 +653,7 @@ int pinyb200_create(const pinyb200_system *s, int nbeads, int precision, pinyb20
     }
     const size_t nb = (size_t)natm * 3 * nbeads;
     CK(cudaMalloc(&c->d_posT, nb * sizeof(double)));
+    if (precision == PINYB200_MIXED) CK(cudaMalloc(&c->d_offT, nb * sizeof(float)));
     CK(cudaMalloc(&c->d_forceT, nb * sizeof(double)));
     CK(cudaMalloc(&c->d_pos_aos, nb * sizeof(double)));
     CK(cudaMalloc(&c->d_force_aos, nb * sizeof(double)));
@@ -902,12 +903,14 @@ int pinyb200_get_list(pinyb200_ctx *c, int *pi, int *pj, long cap, long *npairs)
 }  // extern "C"
 
 // The pair kernel the system, cell, flags and tuning ask for.
-static cudaError_t launch_pair_any(pinyb200_ctx *c, const Cell &cell, int flags, bool energy)
+static cudaError_t launch_pair_any(pinyb200_ctx *c, const Cell &cell, int flags, bool energy, bool staged)
 {
     const bool ortho = cell.h[1] == 0.0 && cell.h[2] == 0.0 && cell.h[3] == 0.0 && cell.h[5] == 0.0 &&
                        cell.h[6] == 0.0 && cell.h[7] == 0.0;
-    if (c->use_mol && c->mol_ok && ortho && c->pair_variant == 0 && !(flags & PINYB200_SITE_PAIRS) && c->mix_ok)
-        return launch_mol_pair_mixed(c, cell, energy);
+    if (c->use_mol && c->mol_ok && ortho && c->pair_variant == 0 && !(flags & PINYB200_SITE_PAIRS) && c->mix_ok) {
+        const cudaError_t e = staged ? cudaSuccess : launch_mol_offsets(c);
+        return e != cudaSuccess ? e : launch_mol_pair_mixed(c, cell, energy);
+    }
     if (c->use_mol && c->mol_ok && ortho && c->pair_variant != 1 && !(flags & PINYB200_SITE_PAIRS))
         return launch_mol_pair(c, cell, energy);
     return launch_pair(c, cell, energy);
@@ -948,7 +951,7 @@ int pinyb200::evaluate_enqueue(pinyb200_ctx *c, const Cell &cell, int flags, boo
         c->stream = main_stream;
         CK(perr);
     }
-    CK(launch_pair_any(c, cell, flags, energy));
+    CK(launch_pair_any(c, cell, flags, energy, false));
     CK(kt_mark(c, "pair"));
     if (respa_w) {
         // RESPA outer level: the weighted pair forces from the plain ones
@@ -1088,7 +1091,7 @@ static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_x
         if (rc) return rc;
     }
     if (timing) CK(ev_rec(c->ev[1], c->stream));
-    CK(launch_pair_any(c, cell, flags, energy));
+    CK(launch_pair_any(c, cell, flags, energy, true));
     CK(kt_mark(c, "pair"));
     if (timing) CK(ev_rec(c->ev[2], c->stream));
     CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));

@@ -137,6 +137,11 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *g)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g)
                  : "memory");
 }
+__device__ __forceinline__ void cp_async8(void *smem, const void *g)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Warp sum of a double over the lanes that share (lane mod stride); stride 32: v itself.

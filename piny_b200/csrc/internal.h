@@ -247,6 +247,7 @@ struct pinyb200_ctx {
     int *d_mchunk = nullptr;   // [nmol] chunks per molecule row, then [nmol + 1] offsets
     // work buffers
     double *d_posT = nullptr;     // [natm][3][P]
+    float *d_offT = nullptr;      // [natm][3][P] site offsets from site 0 of the molecule (MIXED pair kernel)
     double *d_forceT = nullptr;   // [natm][3][P]
     double *d_xmod = nullptr;     // [natm][3]
     double *d_x0 = nullptr;       // [natm][3] bead-1 positions at the last list build
@@ -334,6 +335,7 @@ cudaError_t launch_scan(pinyb200_ctx *c, const int *gate, int n, int K, const in
                         long long *tot, cudaStream_t st);
 cudaError_t launch_mol_pair(pinyb200_ctx *c, const Cell &cell, bool energy);
 cudaError_t launch_mol_pair_mixed(pinyb200_ctx *c, const Cell &cell, bool energy);
+cudaError_t launch_mol_offsets(pinyb200_ctx *c);  // before it, unless launch_water_stage staged the positions
 cudaError_t launch_site_from_mol(pinyb200_ctx *c, int pass, const int *gate = nullptr, cudaStream_t st = nullptr);
 // staged: the grid is already zero and the charges are binned
 cudaError_t launch_pme(pinyb200_ctx *c, const Cell &cell, bool energy, bool staged = false);
@@ -458,28 +460,22 @@ namespace pinyb200 {
 // boxes that share a kernel's compile-time shape (boxtab.cuh).
 int mix_pattern(const pinyb200_ctx *c);
 cudaError_t launch_mol_extent(pinyb200_ctx *c);
-cudaError_t launch_mol_extent_batch(const std::vector<pinyb200_ctx *> &box, int sm_count, cudaStream_t st);
 cudaError_t launch_mol_pair_mixed_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<Cell> &cells,
                                         bool energy, int sm_count, cudaStream_t st);
 cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<Cell> &cells, bool energy,
                              int sm_count, cudaStream_t st);
-cudaError_t launch_pme_force_add_batch(const std::vector<pinyb200_ctx *> &box, int sm_count, cudaStream_t st);
 // zero byte ranges (pointer, bytes; 4-byte multiples) in one launch
 cudaError_t launch_zero_batch(const std::vector<std::pair<void *, size_t>> &seg, int sm_count, cudaStream_t st);
-// copies of n doubles src -> dst (device or pinned host memory); src null:
-// dst = the bead centroid of posT [n][P]
+// copies of n doubles src -> dst (device or pinned host memory)
 struct CopySeg {
     const double *src;
-    const double *posT;
     double *dst;
     long long n;
-    int P;
 };
 cudaError_t launch_copy_batch(const std::vector<CopySeg> &seg, int sm_count, cudaStream_t st);
-cudaError_t launch_transpose_in_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<const double *> &d_pos,
-                                      int sm_count, cudaStream_t st);
-cudaError_t launch_transpose_out_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<double *> &d_force,
-                                       int sm_count, cudaStream_t st);
-cudaError_t launch_ghost_batch(const std::vector<pinyb200_ctx *> &box, bool distrib, int sm_count, cudaStream_t st);
-cudaError_t launch_intra_batch(const std::vector<pinyb200_ctx *> &box, bool energy, int sm_count, cudaStream_t st);
+cudaError_t launch_water_stage_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<Cell> &cells,
+                                     const std::vector<const double *> &pos, const std::vector<const double *> &xmod,
+                                     int sm_count, cudaStream_t st);
+cudaError_t launch_water_finish_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<double *> &out,
+                                      bool energy, bool distrib, int sm_count, cudaStream_t st);
 }  // namespace pinyb200

@@ -465,8 +465,8 @@ cudaError_t launch_ecor_weighted(pinyb200_ctx *c, double w, double *target, int 
 
 
 // ---------------------------------------------------------------------------
-// Many boxes per launch (the batched evaluation): staging, intramolecular
-// terms and the finishing steps of every box in a few persistent launches.
+// Many boxes per launch (the batched evaluation): ranges cleared and sums
+// copied for every box in one persistent launch each.
 
 struct ZeroBox {
     unsigned *p;
@@ -495,66 +495,7 @@ __global__ void __launch_bounds__(256) copy_batch_kernel(const __grid_constant__
     PINYB200_BOX_LOOP(t, i, vb, {
         const CopySeg &c = t.arg[i];
         const long long k = (long long)vb.x * blockDim.x + threadIdx.x;
-        if (k < c.n) {
-            if (c.src) {
-                c.dst[k] = c.src[k];
-            } else {
-                double v = 0.0;
-                for (int b = 0; b < c.P; b++) v += c.posT[k * c.P + b];
-                c.dst[k] = v / (double)c.P;
-            }
-        }
-    });
-}
-
-struct TrBox {
-    const double *in;
-    double *out;
-    int rows;
-    long long cols;
-};
-
-__global__ void __launch_bounds__(256) transpose_batch_kernel(const __grid_constant__ BoxTab<TrBox> t)
-{
-    PINYB200_BOX_LOOP(t, i, vb, (transpose_tiled_body(t.arg[i].in, t.arg[i].out, t.arg[i].rows, t.arg[i].cols, vb)));
-}
-
-struct GhostBox {
-    double *x;  // positions (placement) or forces (distribution)
-    int P, nghost, ncomp;
-    const int *gatom, *gcomp;
-    const double *gcoef;
-};
-
-template <bool DISTRIB>
-__global__ void __launch_bounds__(256) ghost_batch_kernel(const __grid_constant__ BoxTab<GhostBox> t)
-{
-    PINYB200_BOX_LOOP(t, i, vb, {
-        const GhostBox &g = t.arg[i];
-        if (DISTRIB) ghost_distrib_body(g.x, g.P, g.nghost, g.ncomp, g.gatom, g.gcomp, g.gcoef, vb);
-        else ghost_pos_body(g.x, g.P, g.nghost, g.ncomp, g.gatom, g.gcomp, g.gcoef, vb);
-    });
-}
-
-// One intramolecular term of one box: kind 0 bonds, 1 bends, 2 excluded-pair
-// correction; the three kinds of every box share one launch (a typed work list).
-struct IntraBox {
-    IntraArgs a;
-    int kind, n;
-    const int *j1, *j2;
-    const double *c0, *c1, *c2, *c3;
-    int nsplin;
-    double rmin, dr, dri;
-    const double4 *tab;
-};
-
-__global__ void __launch_bounds__(256) intra_batch_kernel(const __grid_constant__ BoxTab<IntraBox> t)
-{
-    PINYB200_BOX_LOOP(t, i, vb, {
-        const IntraBox &x = t.arg[i];
-        if (x.kind == 0) bond_body(x.a, x.n, x.j1, x.c0, x.c1, x.c2, vb);
-        else if (x.kind == 1) bend_body(x.a, x.n, x.j1, x.c0, x.c1, x.c2, x.c3, vb);
-        else ecor_body(x.a, x.n, x.j1, x.j2, x.nsplin, x.rmin, x.dr, x.dri, x.tab, vb);
+        if (k < c.n) c.dst[k] = c.src[k];
     });
 }
 
@@ -572,111 +513,9 @@ cudaError_t launch_zero_batch(const std::vector<std::pair<void *, size_t>> &seg,
 cudaError_t launch_copy_batch(const std::vector<CopySeg> &seg, int sm_count, cudaStream_t st)
 {
     BoxTabBuilder<CopySeg> tb;
-    for (const CopySeg &c : seg) tb.add(c, (int)((c.n + 255) / 256), 1, (double)c.n * (c.src ? 1 : c.P));
+    for (const CopySeg &c : seg) tb.add(c, (int)((c.n + 255) / 256), 1, (double)c.n);
     return launch_tables(tb, (const void *)copy_batch_kernel, 256, 0, sm_count,
                          [&](const BoxTab<CopySeg> &t, int g) { copy_batch_kernel<<<g, 256, 0, st>>>(t); });
-}
-
-// Positions of every box into its [atom][xyz][bead] layout (from d_pos[i],
-// PINY's [bead][atom][xyz]).
-cudaError_t launch_transpose_in_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<const double *> &d_pos,
-                                      int sm_count, cudaStream_t st)
-{
-    BoxTabBuilder<TrBox> tb;
-    for (size_t i = 0; i < box.size(); i++) {
-        pinyb200_ctx *c = box[i];
-        const long long M = (long long)c->sys.natm * 3;
-        tb.add(TrBox{d_pos[i], c->d_posT, c->P, M}, (int)((M + 31) / 32), (c->P + 31) / 32, (double)M * c->P);
-    }
-    return launch_tables(tb, (const void *)transpose_batch_kernel, 256, 0, sm_count,
-                         [&](const BoxTab<TrBox> &t, int g) { transpose_batch_kernel<<<g, 256, 0, st>>>(t); });
-}
-
-// Site forces of every box out to d_force[i] in PINY's order.
-cudaError_t launch_transpose_out_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<double *> &d_force,
-                                       int sm_count, cudaStream_t st)
-{
-    BoxTabBuilder<TrBox> tb;
-    for (size_t i = 0; i < box.size(); i++) {
-        pinyb200_ctx *c = box[i];
-        const long long M = (long long)c->sys.natm * 3;
-        tb.add(TrBox{c->d_forceT, d_force[i], (int)M, c->P}, (c->P + 31) / 32,
-               (int)std::min<long long>((M + 31) / 32, 65535), (double)M * c->P);
-    }
-    return launch_tables(tb, (const void *)transpose_batch_kernel, 256, 0, sm_count,
-                         [&](const BoxTab<TrBox> &t, int g) { transpose_batch_kernel<<<g, 256, 0, st>>>(t); });
-}
-
-cudaError_t launch_ghost_batch(const std::vector<pinyb200_ctx *> &box, bool distrib, int sm_count, cudaStream_t st)
-{
-    BoxTabBuilder<GhostBox> tb;
-    for (pinyb200_ctx *c : box) {
-        const DeviceSystem &s = c->sys;
-        if (s.nghost == 0) continue;
-        const long long n = (long long)s.nghost * c->P;
-        tb.add(GhostBox{distrib ? c->d_forceT : c->d_posT, c->P, s.nghost, s.ghost_ncomp, s.ghost_atom, s.ghost_comp,
-                        s.ghost_coef},
-               (int)((n + 255) / 256), 1, (double)n);
-    }
-    if (distrib)
-        return launch_tables(tb, (const void *)ghost_batch_kernel<true>, 256, 0, sm_count,
-                             [&](const BoxTab<GhostBox> &t, int g) { ghost_batch_kernel<true><<<g, 256, 0, st>>>(t); });
-    return launch_tables(tb, (const void *)ghost_batch_kernel<false>, 256, 0, sm_count,
-                         [&](const BoxTab<GhostBox> &t, int g) { ghost_batch_kernel<false><<<g, 256, 0, st>>>(t); });
-}
-
-// Bonds, bends and excluded-pair corrections of every box in one launch.
-cudaError_t launch_intra_batch(const std::vector<pinyb200_ctx *> &box, bool energy, int sm_count, cudaStream_t st)
-{
-    BoxTabBuilder<IntraBox> tb;
-    for (pinyb200_ctx *c : box) {
-        const DeviceSystem &s = c->sys;
-        IntraBox x;
-        memset(&x, 0, sizeof(x));
-        x.a.natm = s.natm;
-        x.a.P = c->P;
-        x.a.posT = c->d_posT;
-        x.a.forceT = c->d_forceT;
-        x.a.acc = c->d_acc;
-        x.a.charge = s.charge;
-        x.a.energy = energy ? 1 : 0;
-        if (s.nbond) {
-            IntraBox b = x;
-            b.kind = 0;
-            b.n = s.nbond;
-            b.j1 = s.bond_j;
-            b.c0 = s.bond_eq;
-            b.c1 = s.bond_c;
-            b.c2 = s.bond_dc;
-            tb.add(b, (int)nblk_gs(c, (long long)s.nbond * c->P), 1, (double)s.nbond * c->P);
-        }
-        if (s.nbend) {
-            IntraBox b = x;
-            b.kind = 1;
-            b.n = s.nbend;
-            b.j1 = s.bend_j;
-            b.c0 = s.bend_c;
-            b.c1 = s.bend_s;
-            b.c2 = s.bend_dc;
-            b.c3 = s.bend_ds;
-            tb.add(b, (int)nblk_gs(c, (long long)s.nbend * c->P), 1, 2.0 * s.nbend * c->P);
-        }
-        if (s.necor) {
-            IntraBox b = x;
-            b.kind = 2;
-            b.n = s.necor;
-            b.j1 = s.ecor_j1;
-            b.j2 = s.ecor_j2;
-            b.nsplin = s.ecor_nsplin;
-            b.rmin = s.ecor_rmin;
-            b.dr = s.ecor_dr;
-            b.dri = s.ecor_dri;
-            b.tab = s.ecor_tab;
-            tb.add(b, (int)nblk_gs(c, (long long)s.necor * c->P), 1, (double)s.necor * c->P);
-        }
-    }
-    return launch_tables(tb, (const void *)intra_batch_kernel, 256, 0, sm_count,
-                         [&](const BoxTab<IntraBox> &t, int g) { intra_batch_kernel<<<g, 256, 0, st>>>(t); });
 }
 
 }  // namespace pinyb200

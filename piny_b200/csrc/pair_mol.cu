@@ -1234,6 +1234,7 @@ struct MixArgs {
     const int *nchunk, *chunk, *bad, *mj;
     const unsigned *mask;
     const double *posT, *xmod;
+    const float *offT;  // [natm][3][P] offsets of the sites from their molecule's first, FP32
     const unsigned long long *ext;  // extent bound of the evaluation (mol_extent_kernel), or nullptr
     const float4 *tab;   // [4][nuniq][nsplin] interval coefficients (TabKind order)
     const float4 *tabfe; // [2][nuniq][nsplin][2]: vdW then Coulomb; force and energy rows interleaved
@@ -1273,6 +1274,13 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
 {
     constexpr int G = P >= 32 ? 32 : P;  // lanes per molecule pair
     constexpr int JPI = 32 / G;          // molecule pairs per warp step
+    // One or two beads: a lane's own loads and reductions would touch a
+    // sector each, so the warp copies its molecules' positions through shared
+    // memory and hands the j forces back the same way, whole molecules (3 NS P
+    // consecutive values) at a time; rows are padded by one against conflicts.
+    constexpr bool COOP = P <= 2 && CM != kAnyPair;
+    constexpr int NR = 3 * NS * P;
+    __shared__ double stage[COOP ? 4 : 1][COOP ? JPI * (NR + 1) : 1];
     __shared__ double sacc[8][128];
     if (ENERGY)
         for (int c = 0; c < 8; c++) sacc[c][threadIdx.x] = 0.0;
@@ -1302,15 +1310,30 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
             const int i = i0 + (s < ni ? s : 0);
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                ei[s][d] = (float)(posT[(3 * (size_t)i + d) * P + b] - posT[(3 * (size_t)i0 + d) * P + b]);
+                ei[s][d] = s == 0 ? 0.0f : a.offT[(3 * (size_t)i + d) * P + b];
                 fi[s][d] = 0.0f;
             }
         }
         float evs = 0.0f, ecs = 0.0f, pvs[6] = {0, 0, 0, 0, 0, 0};
-        for (int k = beg + sub; k < end; k += JPI) {
-            const int mj = __ldcg(a.mj + k);
-            const unsigned mask = __ldcg(a.mask + k);
+        double *st = stage[COOP ? (threadIdx.x >> 5) : 0];
+        for (int kb = beg; kb < end; kb += JPI) {
+            const int k = kb + sub;
+            const bool act = k < end;
+            if (!COOP && !act) break;
+            const int mj = act ? __ldcg(a.mj + k) : 0;
+            const unsigned mask = act ? __ldcg(a.mask + k) : 0u;
             const int j0 = mj * m.stride;
+            double *sx = st + sub * (NR + 1) + (lane & (P - 1));
+            if constexpr (COOP) {
+                __syncwarp();
+                for (int e = lane; e < 32 * 3 * NS; e += 32) {
+                    const int slot = e / NR, o = e - slot * NR;
+                    const int ms = __shfl_sync(0xffffffffu, mj, slot * G);
+                    cp_async8(st + slot * (NR + 1) + o, posT + (size_t)ms * NR + o);
+                }
+                cp_async_wait();
+                __syncwarp();
+            }
             // site-0 image from the mode-1 separation (FP64) and whether site
             // pairs may take other images
             double sh0[3];
@@ -1318,7 +1341,9 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
 #pragma unroll
             for (int d = 0; d < 3; d++) {
                 const double hid = cell.hi[4 * d];
-                const double t = __dmul_rn(__dsub_rn(a.xmod[3 * (size_t)i0 + d], __ldcg(a.xmod + 3 * (size_t)j0 + d)), hid);
+                // (one bead: the mode-1 positions are the staged ones)
+                const double xmj = COOP && P == 1 ? sx[d] : __ldcg(a.xmod + 3 * (size_t)j0 + d);
+                const double t = __dmul_rn(__dsub_rn(a.xmod[3 * (size_t)i0 + d], xmj), hid);
                 sh0[d] = -nint_rn(t);
                 near |= fabs(t + sh0[d]) > 0.5 - ext2 * hid;
             }
@@ -1328,20 +1353,33 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
             // dj[s] = x_i0 - x_j(s) + image, in FP32 from the FP64 site-0 separation
             float dj[NS][3];
             {
-                // the i anchor is re-read (an L1 hit) rather than held over the chunk
+                // the i anchor is re-read (an L1 hit) rather than held over the
+                // chunk; the sites' FP32 offsets from site 0 are as staged with
+                // the positions (an FP64 row is twice the bytes, and L2 traffic
+                // bounds this kernel: 3 FP64 and 9 FP32 rows of j against 12)
                 double xj0[3];
 #pragma unroll
-                for (int d = 0; d < 3; d++) xj0[d] = __ldcg(posT + (3 * (size_t)j0 + d) * P + b);
-#pragma unroll
-                for (int d = 0; d < 3; d++)
+                for (int d = 0; d < 3; d++) {
+                    xj0[d] = COOP ? sx[d * P] : __ldcg(posT + (3 * (size_t)j0 + d) * P + b);
                     dj[0][d] = (float)(__dsub_rn(posT[(3 * (size_t)i0 + d) * P + b], xj0[d]) + sh0[d] * cell.h[4 * d]);
+                }
 #pragma unroll
                 for (int s = 1; s < NS; s++) {
                     const int j = j0 + (((jm >> s) & 1u) ? s : 0);
 #pragma unroll
-                    for (int d = 0; d < 3; d++)
-                        dj[s][d] = dj[0][d] - (float)(__ldcg(posT + (3 * (size_t)j + d) * P + b) - xj0[d]);
+                    for (int d = 0; d < 3; d++) {
+                        const float e = COOP ? (float)(sx[(3 * s + d) * P] - xj0[d])
+                                             : __ldcg(a.offT + (3 * (size_t)j + d) * P + b);
+                        dj[s][d] = dj[0][d] - e;
+                    }
                 }
+            }
+            // j forces of the staged molecules, in the positions' place
+            float *sf = (float *)st + sub * (NR + 1) + (lane & (P - 1));
+            if constexpr (COOP) {
+                __syncwarp();
+#pragma unroll
+                for (int o = 0; o < 3 * NS; o++) sf[o * P] = 0.0f;
             }
             // the site pairs; NEAR adds each pair's own image, in a copy of the
             // loop so that pairs away from half a box pay nothing for it
@@ -1432,7 +1470,11 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                         pvs[4] -= dj[sj][0] * fjz;
                         pvs[5] -= dj[sj][1] * fjz;
                     }
-                    if (fjx != 0.0f || fjy != 0.0f || fjz != 0.0f) {
+                    if constexpr (COOP) {
+                        sf[(3 * sj) * P] = fjx;
+                        sf[(3 * sj + 1) * P] = fjy;
+                        sf[(3 * sj + 2) * P] = fjz;
+                    } else if (fjx != 0.0f || fjy != 0.0f || fjz != 0.0f) {
                         const int j = j0 + sj;
                         atomicAdd(&a.forceT[(3 * (size_t)j + 0) * P + b], (double)fjx);
                         atomicAdd(&a.forceT[(3 * (size_t)j + 1) * P + b], (double)fjy);
@@ -1440,8 +1482,17 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                     }
                 }
             };
-            if (near) site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, ni, sh0, cell, lane));
+            if (near && act) site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, ni, sh0, cell, lane));
             else site_pairs(std::false_type{}, NearImages{{0u, 0u, 0u}});
+            if constexpr (COOP) {
+                __syncwarp();
+                for (int e = lane; e < 32 * 3 * NS; e += 32) {
+                    const int slot = e / NR, o = e - slot * NR;
+                    const int ms = __shfl_sync(0xffffffffu, mj, slot * G);
+                    const float v = ((const float *)st)[slot * (NR + 1) + o];
+                    if (v != 0.0f) atomicAdd(&a.forceT[(size_t)ms * NR + o], (double)v);
+                }
+            }
         }
         if (ENERGY) {
             // the e_i (x) f_i part of the virial: e_i is fixed over the chunk
@@ -1521,7 +1572,7 @@ __global__ void __launch_bounds__(128, 4)
 #pragma unroll
             for (int d = 0; d < 3; d++) {
                 const size_t o = (3 * (size_t)(i0 + s) + d) * P + b;
-                ei[s][d] = (float)(posT[o] - posT[(3 * (size_t)i0 + d) * P + b]);
+                ei[s][d] = s == 0 ? 0.0f : a.offT[o];
                 ui[s][d] = (float)uT[o];
             }
         if (gw)
@@ -1553,7 +1604,7 @@ __global__ void __launch_bounds__(128, 4)
 #pragma unroll
                     for (int d = 0; d < 3; d++) {
                         const size_t o = (3 * (size_t)(j0 + s) + d) * P + b;
-                        if (s > 0) dj[s][d] = dj[0][d] - (float)(__ldcg(posT + o) - xj0[d]);
+                        if (s > 0) dj[s][d] = dj[0][d] - __ldcg(a.offT + o);
                         uj[s][d] = (float)__ldcg(uT + o);
                     }
                 if (gw)
@@ -1953,10 +2004,10 @@ static void launch_mix_pattern(pinyb200_ctx *c, const MixArgs &a, const MixSite 
 {
     const int threads = 128;
     if (energy) {
-        carveout_pref((const void *)mol_pair_mixed_kernel<P, NS, true, CM, VM>, c->pair_carveout);
+        carveout_pref((const void *)mol_pair_mixed_kernel<P, NS, true, CM, VM>, P <= 2 ? 50 : c->pair_carveout);
         mol_pair_mixed_kernel<P, NS, true, CM, VM><<<grid, threads, 0, c->stream>>>(a, m, cell);
     } else {
-        carveout_pref((const void *)mol_pair_mixed_kernel<P, NS, false, CM, VM>, c->pair_carveout);
+        carveout_pref((const void *)mol_pair_mixed_kernel<P, NS, false, CM, VM>, P <= 2 ? 50 : c->pair_carveout);
         mol_pair_mixed_kernel<P, NS, false, CM, VM><<<grid, threads, 0, c->stream>>>(a, m, cell);
     }
 }
@@ -2012,6 +2063,7 @@ static MixArgs mix_args(pinyb200_ctx *c)
     a.mask = c->d_mmask;
     a.posT = c->d_posT;
     a.xmod = c->P > 1 ? c->d_xmod : c->d_posT;
+    a.offT = c->d_offT;
     a.ext = (const unsigned long long *)(c->d_acc + S_EXT);
     a.tab = s.tab32;
     a.tabfe = c->d_tabfe;
@@ -2041,6 +2093,26 @@ static MixSite mix_site(const pinyb200_ctx *c)
     m.rmd = c->mix_rmd;
     m.tmax = c->mix_tmax;
     return m;
+}
+
+// Offsets of every site from its molecule's first, for evaluations that the
+// water staging kernel did not stage.
+__global__ void __launch_bounds__(256) mol_offsets_kernel(const double *__restrict__ posT, float *__restrict__ offT,
+                                                          int stride, int P, long long n)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const long long row = t / P;
+    const int b = (int)(t - row * P), d = (int)(row % 3);
+    const long long i0 = row / 3 / stride * stride;
+    offT[t] = (float)(posT[t] - posT[(3 * i0 + d) * P + b]);
+}
+
+cudaError_t launch_mol_offsets(pinyb200_ctx *c)
+{
+    const long long n = (long long)c->sys.natm * 3 * c->P;
+    mol_offsets_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->d_posT, c->d_offT, c->mol_stride, c->P, n);
+    return cudaGetLastError();
 }
 
 // The MIXED kernel with combined per-site-pair tables (pinyb200_ctx::mix_ok).
@@ -2109,32 +2181,8 @@ cudaError_t launch_mol_extent(pinyb200_ctx *c)
     return cudaGetLastError();
 }
 
-struct ExtBox {
-    const int *mstart;
-    int nmol;
-    const double *xm;
-    unsigned long long *out;
-};
-
-__global__ void __launch_bounds__(256) mol_extent_batch_kernel(const __grid_constant__ BoxTab<ExtBox> t)
-{
-    PINYB200_BOX_LOOP(t, i, vb, (mol_extent_body(t.arg[i].mstart, t.arg[i].nmol, t.arg[i].xm, t.arg[i].out, vb)));
-}
-
-cudaError_t launch_mol_extent_batch(const std::vector<pinyb200_ctx *> &box, int sm_count, cudaStream_t st)
-{
-    BoxTabBuilder<ExtBox> tb;
-    for (pinyb200_ctx *c : box) {
-        if (!c->use_mol || c->nmol == 0) continue;
-        tb.add(ExtBox{c->d_mstart, c->nmol, c->P > 1 ? c->d_xmod : c->d_posT, (unsigned long long *)(c->d_acc + S_EXT)},
-               (c->nmol + 255) / 256, 1, (double)c->nmol);
-    }
-    return launch_tables(tb, (const void *)mol_extent_batch_kernel, 256, 0, sm_count,
-                         [&](const BoxTab<ExtBox> &t, int g) { mol_extent_batch_kernel<<<g, 256, 0, st>>>(t); });
-}
-
-// Site-pair table pattern of a context: 1 q-TIP4P/F-like (4 sites), 2
-// q-SPC/Fw-like (3 sites), 0 another pattern.
+// Site pattern of a context's MIXED pair kernel: 1 q-TIP4P/F-like (4 sites),
+// 2 q-SPC/Fw-like (3 sites), 0 another pattern.
 int mix_pattern(const pinyb200_ctx *c)
 {
     unsigned cm = 0, vm = 0;
@@ -2177,7 +2225,7 @@ static cudaError_t launch_mix_batch_t(const std::vector<pinyb200_ctx *> &box, co
     }
     const void *fn = energy ? (const void *)mol_pair_mixed_batch_kernel<P, NS, true, CM, VM>
                             : (const void *)mol_pair_mixed_batch_kernel<P, NS, false, CM, VM>;
-    cudaError_t err = carveout_pref(fn, box.empty() ? 25 : box[0]->pair_carveout);
+    cudaError_t err = carveout_pref(fn, P <= 2 ? 50 : (box.empty() ? 25 : box[0]->pair_carveout));
     if (err != cudaSuccess) return err;
     return launch_tables(tb, fn, 128, 0, sm_count, [&](const BoxTab<MixBox> &t, int g) {
         if (energy) mol_pair_mixed_batch_kernel<P, NS, true, CM, VM><<<g, 128, 0, st>>>(t, m);

@@ -1530,19 +1530,6 @@ struct FftBox {
     int energy;
 };
 
-struct AddBox {
-    int nchrg, P;
-    const int *ichrg;
-    const double *fP;
-    double *fT;
-};
-
-template <typename R, int NI>
-__global__ void __launch_bounds__(256) pme_bin_batch_kernel(const __grid_constant__ BoxTab<PmeBox> t)
-{
-    PINYB200_BOX_LOOP(t, i, vb, (pme_bin_compact_body<R, NI>(t.arg[i].a, t.arg[i].cell, t.arg[i].t, vb)));
-}
-
 template <typename R, int NI, int TT>
 __global__ void __launch_bounds__(256) spread_batch_kernel(const __grid_constant__ BoxTab<PmeBox> t)
 {
@@ -1584,13 +1571,7 @@ __global__ void __launch_bounds__(256) plane_inv_batch_kernel(const __grid_const
                                              t.arg[i].Nc, (const R *)t.arg[i].tw[0], (const R *)t.arg[i].tw[1], vb)));
 }
 
-__global__ void __launch_bounds__(256) pme_force_add_batch_kernel(const __grid_constant__ BoxTab<AddBox> t)
-{
-    PINYB200_BOX_LOOP(t, i, vb,
-                      (pme_force_add_body(t.arg[i].nchrg, t.arg[i].P, t.arg[i].ichrg, t.arg[i].fP, t.arg[i].fT, vb)));
-}
-
-// stage 0 bin, 1 spread, 2 gather for the boxes of one (order, tile edge) group
+// stage 0 spread, 1 gather for the boxes of one (order, tile edge) group
 template <int NI, int TT>
 static cudaError_t pme_batch_tiles(const std::vector<PmeBox> &bx, const std::vector<int> &P, int sm_count,
                                    cudaStream_t st, int stage)
@@ -1599,13 +1580,9 @@ static cudaError_t pme_batch_tiles(const std::vector<PmeBox> &bx, const std::vec
     BoxTabBuilder<PmeBox> tb;
     for (size_t i = 0; i < bx.size(); i++) {
         const double work = (double)bx[i].a.nchrg * P[i];
-        if (stage == 0) tb.add(bx[i], (int)(((long long)bx[i].a.nchrg * P[i] + 255) / 256), 1, work);
-        else tb.add(bx[i], bx[i].t.ntile, P[i] * bx[i].t.nshare, work);
+        tb.add(bx[i], bx[i].t.ntile, P[i] * bx[i].t.nshare, work);
     }
-    if (stage == 0)
-        return launch_tables(tb, (const void *)pme_bin_batch_kernel<R, NI>, 256, 0, sm_count,
-                             [&](const BoxTab<PmeBox> &t, int g) { pme_bin_batch_kernel<R, NI><<<g, 256, 0, st>>>(t); });
-    if (stage == 1) {
+    if (stage == 0) {
         const size_t ss = spread_smem<R, NI, TT>();
         return launch_tables(tb, (const void *)spread_batch_kernel<R, NI, TT>, 256, ss, sm_count,
                              [&](const BoxTab<PmeBox> &t, int g) { spread_batch_kernel<R, NI, TT><<<g, 256, ss, st>>>(t); });
@@ -1662,7 +1639,7 @@ static cudaError_t pme_batch_tiles_group(const std::pair<int, int> &key, const s
 }
 
 // Forward PME of many MIXED contexts on stream st, as launch_pme does for
-// one: grids and bin counters cleared, charges binned, spread, transformed,
+// one whose grids are clear and charges binned: spread, transformed,
 // convolved (energies and virials into each context's per-bead sums when
 // `energy`), transformed back and gathered into each context's PME forces.
 cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::vector<Cell> &cells, bool energy,
@@ -1671,7 +1648,6 @@ cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::
     // groups: tiles by (order, tile edge), FFTs by mesh
     std::map<std::pair<int, int>, std::pair<std::vector<PmeBox>, std::vector<int>>> tiles;
     std::map<std::tuple<int, int, int>, std::pair<std::vector<FftBox>, std::vector<int>>> ffts;
-    std::vector<std::pair<void *, size_t>> zero;
     for (size_t i = 0; i < box.size(); i++) {
         pinyb200_ctx *c = box[i];
         if (c->sys.nchrg == 0 || c->sys.nktot == 0) continue;
@@ -1712,15 +1688,12 @@ cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::
         auto &fg = ffts[std::make_tuple(fb.Na, fb.Nb, fb.Nc)];
         fg.first.push_back(fb);
         fg.second.push_back(c->P);
-        zero.emplace_back(c->d_grid, sizeof(float) * G * c->P);
-        zero.emplace_back(c->d_pme_cnt, ((size_t)c->P * c->pme_ntile + 1) * sizeof(int));
     }
-    cudaError_t err = launch_zero_batch(zero, sm_count, st);
-    for (int stage = 0; stage < 2 && err == cudaSuccess; stage++)
-        for (auto &kv : tiles) {
-            err = pme_batch_tiles_group(kv.first, kv.second.first, kv.second.second, sm_count, st, stage);
-            if (err != cudaSuccess) break;
-        }
+    cudaError_t err = cudaSuccess;
+    for (auto &kv : tiles) {
+        err = pme_batch_tiles_group(kv.first, kv.second.first, kv.second.second, sm_count, st, 0);
+        if (err != cudaSuccess) break;
+    }
     for (int stage = 0; stage < 3 && err == cudaSuccess; stage++)
         for (auto &kv : ffts) {
             const int Na = std::get<0>(kv.first), Nb = std::get<1>(kv.first), Nc = std::get<2>(kv.first);
@@ -1746,23 +1719,9 @@ cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::
         }
     for (auto &kv : tiles) {
         if (err != cudaSuccess) break;
-        err = pme_batch_tiles_group(kv.first, kv.second.first, kv.second.second, sm_count, st, 2);
+        err = pme_batch_tiles_group(kv.first, kv.second.first, kv.second.second, sm_count, st, 1);
     }
     return err;
-}
-
-// PME forces of many contexts added to their site forces.
-cudaError_t launch_pme_force_add_batch(const std::vector<pinyb200_ctx *> &box, int sm_count, cudaStream_t st)
-{
-    BoxTabBuilder<AddBox> tb;
-    for (pinyb200_ctx *c : box) {
-        if (c->sys.nchrg == 0 || c->sys.nktot == 0) continue;
-        const long long n = (long long)c->sys.nchrg * 3 * c->P;
-        tb.add(AddBox{c->sys.nchrg, c->P, c->sys.ichrg, c->d_forceP, c->d_forceT}, (int)((n + 255) / 256), 1,
-               (double)n);
-    }
-    return launch_tables(tb, (const void *)pme_force_add_batch_kernel, 256, 0, sm_count,
-                         [&](const BoxTab<AddBox> &t, int g) { pme_force_add_batch_kernel<<<g, 256, 0, st>>>(t); });
 }
 
 }  // namespace pinyb200

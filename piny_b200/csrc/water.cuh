@@ -27,6 +27,7 @@ struct StageArgs {
     int natm, nmol, P;
     const double *pos;     // [P][natm][3]
     double *posT, *forceT; // [natm][3][P]
+    float *offT;           // [natm][3][P] FP32 offsets from the first site, or nullptr
     const double *xm_src;  // mode-1 positions [natm][3], or nullptr: the bead centroid (P > 1)
     double *xm_dst;        // kept copy (may be xm_src itself)
     unsigned long long *ext;
@@ -84,6 +85,10 @@ __device__ __forceinline__ void water_stage_body(const StageArgs &a, const PmeAr
             a.posT[o + (size_t)k * P] = x[k];
             a.forceT[o + (size_t)k * P] = 0.0;
         }
+        if (a.offT) {
+#pragma unroll
+            for (int k = 3; k < NC; k++) a.offT[o + (size_t)k * P] = (float)(x[k] - x[k % 3]);
+        }
         if (P == 1) {
 #pragma unroll
             for (int k = 3; k < NC; k++) ext = fmax(ext, fabs(x[k] - x[k % 3]));
@@ -114,9 +119,18 @@ __device__ __forceinline__ void water_stage_body(const StageArgs &a, const PmeAr
             ext = fmax(ext, fabs(r[k] - r[k % 3]));
         }
     }
+    // one atomic per block, and only where it raises the bound: thousands of
+    // warps meeting at this address took most of the kernel's time
+    __shared__ double bext[8];
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) ext = fmax(ext, __shfl_xor_sync(0xffffffffu, ext, o));
-    if ((threadIdx.x & 31) == 0 && ext > 0.0) atomicMax(a.ext, (unsigned long long)__double_as_longlong(ext));
+    if ((threadIdx.x & 31) == 0) bext[threadIdx.x >> 5] = ext;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) ext = fmax(ext, bext[w]);
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(ext);
+        if (ext > 0.0 && bits > __ldcg(a.ext)) atomicMax(a.ext, bits);
+    }
 }
 
 struct FinishArgs {
