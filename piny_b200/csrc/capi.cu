@@ -550,6 +550,10 @@ int pinyb200_create(const pinyb200_system *s, int nbeads, int precision, pinyb20
     CK(upload(&d.atm_typ, s->atm_typ, natm));
     CK(upload(&d.charge, s->charge, natm));
     c->h_charge.assign(s->charge, s->charge + natm);
+    for (double q : c->h_charge) {
+        c->q2_sum += q * q;
+        c->q_sum += q;
+    }
     c->h_cutoff.assign(s->cutoff, s->cutoff + s->ntyp * (s->ntyp + 1) / 2);
     c->skin = s->skin;
     c->nbond_typ = s->nbond_typ;
@@ -1012,8 +1016,7 @@ void pinyb200::evaluate_finish(pinyb200_ctx *c, const Cell &cell, int flags, con
             double s[S_NSLOT] = {0};
             for (int b = 0; b < c->P; b++)
                 for (int k = 0; k < S_NSLOT; k++) s[k] += acc[(size_t)b * S_NSLOT + k];
-            double q2 = 0, q1 = 0;
-            for (double q : c->h_charge) { q2 += q * q; q1 += q; }
+            const double q2 = c->q2_sum, q1 = c->q_sum;
             const bool ewald = c->sys.nktot > 0 && c->sys.nchrg > 0;
             e->vself = ewald ? -q2 * c->alp_ewd * c->self_erf / sqrt(M_PI) : 0.0;
             e->vbgr = ewald ? -0.5 * q1 * q1 * M_PI / (c->alp_ewd * c->alp_ewd * cell.vol) : 0.0;

@@ -693,8 +693,7 @@ int pinyb200_grad(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, co
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return record_error(c, PINYB200_ERR_CUDA, std::string("grad: ") + cudaGetErrorString(e));
     // terms without forces: Ewald self and background (ewald3d_self_bgr.c:28-80), LJ tail
-    double q1 = 0;
-    for (double q : c->h_charge) q1 += q;
+    const double q1 = c->q_sum;
     const bool ewald = c->sys.nktot > 0 && c->sys.nchrg > 0;
     for (int k = 0; k < K; k++) {
         double de = h[2 * k];

@@ -541,7 +541,7 @@ int pimd_finish(pinyb200_pimd *pm, pinyb200_ctx *c, const pinyb200::Cell &cell, 
         cudaEventElapsedTime(&c->last_ms[0], c->ev[0], c->ev[4]);
         cudaEventElapsedTime(&c->last_ms[1], c->ev[1], c->ev[2]);
         cudaEventElapsedTime(&c->last_ms[2], c->ev_pme[0], c->ev_pme[1]);
-        cudaEventElapsedTime(&c->last_ms[3], c->ev[2], c->ev[3]);
+        cudaEventElapsedTime(&c->last_ms[3], c->ev[5], c->ev[3]);
     }
     pinyb200_energies fe;
     pinyb200::evaluate_finish(c, cell, PINYB200_DISTRIB_GHOSTS, pm->h_facc, &fe);
