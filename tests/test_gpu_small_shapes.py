@@ -1,0 +1,169 @@
+"""Kernels at the sizes where they can go wrong, against the oracle: every mesh
+edge the mesh transforms are compiled for, tiles of both edges, bead counts and
+molecule counts around the pair kernels' chunks, boxes in which most molecule
+pairs are near half a box, and the water staging and finishing kernels against
+the general ones."""
+import numpy as np
+import pytest
+
+from piny_b200 import params, system, water
+
+pytestmark = pytest.mark.gpu
+
+# FP64 follows the oracle's operation order up to summation order; MIXED
+# evaluates pairs and mesh in FP32 (2^-24 per operation, a few hundred terms
+# per force): the bounds of the parity tests
+TOL = {"fp64": (1e-12, 1e-11), "mixed": (1e-5, 1e-6)}
+
+
+def _box(model, nmol, beads, grid, order, seed=11, cutoff=None, edge=None):
+    L = water.density_box_edge(nmol) if edge is None else edge
+    spec = water.BoxSpec(model, nmol, L, beads, 298.0, seed, cutoff=cutoff or min(9.0, 0.47 * L), grid=grid,
+                         order=order)
+    pos = water.build_positions(spec) / water.BOHR
+    return spec, system.build_system(spec, pos), pos, (pos.mean(axis=0) if beads > 1 else None)
+
+
+def _oracle(oracle, S, pos, xmod, distribute=False):
+    pi, pj = oracle.verlist(S, pos[0], xmod, S["hmat"], S["cutskin2"])
+    f, e = oracle.energy_force(S, pos, xmod, S["hmat"], pi, pj, distribute_ghosts=distribute)
+    return f, e
+
+
+def _device(S, pos, xmod, precision, tuning=None, distribute=False):
+    from piny_b200.lib import DeviceBox
+    box = DeviceBox(S, pos.shape[0], precision)
+    box.build_list(pos[0], xmod, S["hmat"], S["cutskin2"])
+    if tuning:
+        ch = box.tuning()
+        for k, v in tuning.items():
+            ch[k] = v
+        box.set_tuning(ch)
+    f, e = box.energy_force(pos, xmod, S["hmat"], distribute_ghosts=distribute)
+    box.close()
+    return f, e
+
+
+def _check(precision, f, e, fref, eref):
+    ftol, etol = TOL[precision]
+    assert np.linalg.norm(f - fref) <= ftol * np.linalg.norm(fref)
+    scale = abs(eref["vvdw"]) + abs(eref["vcoul"]) + abs(eref["vself"])
+    for k in ("vintert", "vrecip", "vecor", "vbond", "vbend"):
+        assert abs(e[k] - eref[k]) <= etol * scale, k
+    assert np.abs(e["pvten"] - eref["pvten"]).max() <= 10 * etol * scale * f.shape[0]
+
+
+@pytest.mark.parametrize("grid", [16, 20, 24, 32, 36, 40, 48, 60, 64, 72, 80, 96, 100, 108, 120, 128])
+def test_mesh_edges(oracle, grid):
+    spec, S, pos, xmod = _box(water.SPC_FW, 27, 1, grid, 6, edge=12.4, cutoff=5.5)
+    assert S["ngrid_a"] == grid
+    fref, eref = _oracle(oracle, S, pos, xmod)
+    # FP64 planes above 117 x 117 points do not fit a block's shared memory
+    for precision in ("fp64", "mixed") if grid <= 108 else ("mixed",):
+        f, e = _device(S, pos, xmod, precision)
+        _check(precision, f, e, fref, eref)
+
+
+@pytest.mark.parametrize("order", [4, 5, 6, 7, 8, 10])
+@pytest.mark.parametrize("tile", [8, 16])
+def test_orders_and_tiles(oracle, order, tile):
+    spec, S, pos, xmod = _box(water.TIP4P_F, 65, 2, 32, order)
+    fref, eref = _oracle(oracle, S, pos, xmod)
+    for precision in ("fp64", "mixed"):
+        f, e = _device(S, pos, xmod, precision, tuning={0: tile})
+        _check(precision, f, e, fref, eref)
+
+
+@pytest.mark.parametrize("beads", [1, 2, 8, 32, 64])
+@pytest.mark.parametrize("model, nmol, cutoff", [(water.TIP4P_F, 33, 4.5), (water.TIP4P_F, 64, 9.0),
+                                                 (water.SPC_FW, 65, 9.0)])
+def test_pairs_near_half_a_box(oracle, model, nmol, cutoff, beads):
+    """Boxes of 10 to 12.5 Angstrom: with a cutoff beyond half the box every
+    image decision matters, and each site pair has to get its own."""
+    spec, S, pos, xmod = _box(model, nmol, beads, 16, 6, cutoff=cutoff)
+    fref, eref = _oracle(oracle, S, pos, xmod, distribute=True)
+    for precision in ("fp64", "mixed"):
+        for variant in (0, 2):
+            f, e = _device(S, pos, xmod, precision, tuning={1: variant}, distribute=True)
+            _check(precision, f, e, fref, eref)
+
+
+def _two_types(S):
+    """The same box with its second half's bonds and bends under a second type
+    of equal constants: not the one-type water of the fused kernels."""
+    T = dict(S)
+    T["nbond_typ"] = T["nbend_typ"] = 2
+    T["bond_typ"] = np.array(S["bond_typ"]).copy()
+    T["bond_typ"][len(T["bond_typ"]) // 2:] = 1
+    T["bend_typ"] = np.array(S["bend_typ"]).copy()
+    T["bend_typ"][len(T["bend_typ"]) // 2:] = 1
+    for k in ("bond_eq", "bond_c", "bond_dc", "bend_eq", "bend_c", "bend_s", "bend_dc", "bend_ds"):
+        T[k] = np.concatenate([S[k], S[k]])
+    return T
+
+
+def _turned(S):
+    """The same box with bonds, bends and exclusion pairs listed backwards and turned round."""
+    T = dict(S)
+    for a, b in (("bond_j1", "bond_j2"), ("bend_j1", "bend_j3"), ("ecor_j1", "ecor_j2")):
+        T[a], T[b] = np.ascontiguousarray(S[b][::-1]), np.ascontiguousarray(S[a][::-1])
+    T["bend_j2"] = np.ascontiguousarray(S["bend_j2"][::-1])
+    return T
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("model, nmol, beads", [(water.TIP4P_F, 65, 1), (water.TIP4P_F, 33, 4), (water.SPC_FW, 65, 2),
+                                                (water.SPC_FW, 27, 64), (water.TIP4P_F, 27, 32)])
+def test_water_kernels_equal_the_general_ones(model, nmol, beads, precision):
+    import torch
+
+    from piny_b200.lib import DeviceBox
+    spec, S, pos, xmod = _box(model, nmol, beads, 20, 6)
+    got = []
+    for T in (S, _two_types(S), _turned(S)):
+        for distribute in (False, True):
+            got.append(_device(T, pos, xmod, precision, distribute=distribute))
+        # without mode-1 positions: the bead centroid
+        box = DeviceBox(T, beads, precision)
+        box.build_list(pos[0], xmod, S["hmat"], S["cutskin2"])
+        d = torch.from_numpy(pos).cuda()
+        f = torch.full_like(d, float("nan"))
+        e = box.energy_force_device(d.data_ptr(), None, S["hmat"], f.data_ptr(), distribute_ghosts=True, energy=False)
+        got.append((f.cpu().numpy(), e))
+        box.close()
+    # FP64 sums in another order; in MIXED the same FP32 terms summed in FP64
+    tol = 1e-13 if precision == "fp64" else 1e-9
+    for k in range(3, 9):
+        f0, e0 = got[k % 3]
+        f, e = got[k]
+        assert np.linalg.norm(f - f0) <= tol * np.linalg.norm(f0)
+        scale = abs(e0["vreal"]) + abs(e0["vself"]) + 1.0
+        assert abs(e["vintert"] - e0["vintert"]) <= 10 * tol * scale
+        assert np.abs(e["pvten"] - e0["pvten"]).max() <= 100 * tol * scale * beads
+
+
+@pytest.mark.parametrize("nmol, beads, cutoff", [(65, 1, None), (64, 4, 9.0), (130, 16, None), (27, 64, None)])
+def test_gradient_pair_kernels(nmol, beads, cutoff):
+    """The molecule-pair adjoint (MIXED), the site-list one (MIXED, two bond
+    types) and FP64 give the same derivatives."""
+    import torch
+
+    from piny_b200.lib import DeviceBox
+    spec, S, pos, xmod = _box(water.TIP4P_F, nmol, beads, 20, 6, cutoff=cutoff)
+    tan = params.tangents(spec, params.theta_of(spec.model), S)
+    tan2 = [{k: (np.concatenate([v, v]) if k.startswith(("dbond", "dbend")) else v) for k, v in t.items()}
+            for t in tan]
+    rng = np.random.default_rng(3)
+    d, x = torch.from_numpy(pos).cuda(), None if xmod is None else torch.from_numpy(xmod).cuda()
+    fbar = torch.from_numpy(rng.normal(size=pos.shape)).cuda()
+    out = []
+    for T, t, precision in ((S, tan, "fp64"), (S, tan, "mixed"), (_two_types(S), tan2, "mixed")):
+        box = DeviceBox(T, beads, precision)
+        box.build_list(pos[0], xmod, S["hmat"], S["cutskin2"])
+        box.grad_prepare(t)
+        out.append(box.grad(d.data_ptr(), None if x is None else x.data_ptr(), S["hmat"], fbar.data_ptr()))
+        box.close()
+    for dE, dF in out[1:]:
+        # FP32 pair and mesh terms: 1e-6 of the largest component, single ones within 1e-3 of it as elsewhere
+        assert np.abs(dE - out[0][0]).max() <= 1e-5 * np.abs(out[0][0]).max()
+        assert np.abs(dF - out[0][1]).max() <= 1e-5 * np.abs(out[0][1]).max()
