@@ -553,6 +553,7 @@ int pinyb200_create(const pinyb200_system *s, int nbeads, int precision, pinyb20
     for (double q : c->h_charge) {
         c->q2_sum += q * q;
         c->q_sum += q;
+        c->q_max = std::max(c->q_max, std::fabs(q));
     }
     c->h_cutoff.assign(s->cutoff, s->cutoff + s->ntyp * (s->ntyp + 1) / 2);
     c->skin = s->skin;

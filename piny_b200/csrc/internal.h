@@ -274,7 +274,7 @@ struct pinyb200_ctx {
     bool filter_ok = false;
     cudaEvent_t ev[8];
     float last_ms[5] = {0, 0, 0, 0, 0};
-    double q_sum = 0, q2_sum = 0; // sums of the charges and of their squares
+    double q_sum = 0, q2_sum = 0, q_max = 0;  // sum of the charges, of their squares, largest magnitude
     // per-kernel timing (pinyb200_set_kernel_timing): an event after every
     // kernel of a serialised evaluation, named by the kernel it closes
     // cached CUDA graph of one evaluation (the single-box entry points)

@@ -1372,9 +1372,7 @@ TileArgs tile_args_of(pinyb200_ctx *c, int NI, int TT)
     // after scaling, the range the rounding trick is exact in; at most 2^24
     // (a resolution of 6e-8 against contributions of up to ~0.15)
     {
-        double qmax = 0.0;
-        for (double q : c->h_charge) qmax = std::max(qmax, std::fabs(q));
-        const double bmax = bspline_peak(NI);
+        const double qmax = c->q_max, bmax = bspline_peak(NI);
         int S = 24;
         while (S > 8 && std::ldexp(qmax * bmax * bmax * bmax, S) >= 0.99 * std::ldexp(1.0, 22)) S--;
         t.qfix = (float)std::ldexp(1.0, S);
