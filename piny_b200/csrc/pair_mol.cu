@@ -593,14 +593,39 @@ __global__ void __launch_bounds__(256, 2) mol_list_cell_kernel(const int *__rest
         const int k = threadIdx.x;
         const int da = k % 5 - 2, db = (k / 5) % 5 - 2, dc = k / 25 - 2;
         const int cid = ((hc + dc + nc) % nc * nb + (hb + db + nb) % nb) * na + (ha + da + na) % na;
-        nbase[k] = coff[cid];
-        nstart[k + 1] = coff[cid + 1] - coff[cid];
+        // a cell's molecules ascend: only those below the home cell's last can
+        // be in a home row (half of them where indices follow the box)
+        const int last = cmol[h0 + nhome - 1], beg = coff[cid];
+        int lo = beg, hi = coff[cid + 1];
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (cmol[mid] < last) lo = mid + 1;
+            else hi = mid;
+        }
+        nbase[k] = beg;
+        nstart[k + 1] = lo - beg;
     }
     for (int k = threadIdx.x; k < PINYB200_CELL_HOME; k += blockDim.x) hcnt[k] = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        nstart[0] = 0;
-        for (int k = 1; k <= 125; k++) nstart[k] += nstart[k - 1];
+    if (warp == 0) {
+        // running sums of the 125 counts, four to a lane
+        int c[4], t = 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int k = 4 * lane + u;
+            t += k < 125 ? nstart[k + 1] : 0;
+            c[u] = t;
+        }
+        int p = t;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, p, o);
+            if (lane >= o) p += v;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (4 * lane + u < 125) nstart[4 * lane + u + 1] = p - t + c[u];
+        if (lane == 0) nstart[0] = 0;
     }
     __syncthreads();
     const int total = nstart[125];
@@ -716,6 +741,8 @@ __global__ void __launch_bounds__(256) site_fill_kernel(const int *__restrict__ 
                                                         int *__restrict__ col, int *__restrict__ colA, long long cap)
 {
     if (gate && *gate == 0) return;
+    __shared__ int bufs[8][2][NS][32 * NS];  // a warp's entries of each row, written out in whole lines
+    int(*const buf)[NS][32 * NS] = bufs[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -723,38 +750,61 @@ __global__ void __launch_bounds__(256) site_fill_kernel(const int *__restrict__ 
     for (int mi = warp; mi < nmol; mi += nwarps) {
         const int i0 = mstart[mi], ni = mstart[mi + 1] - i0;
         const int k1 = (int)(mrow[mi + 1] < mcap ? mrow[mi + 1] : mcap);
-        for (int si = 0; si < ni; si++) {
-            long long wf = row[i0 + si], wa = rowA[i0 + si];
-            for (int k0 = mrow[mi]; k0 < k1; k0 += 32) {
-                const int k = k0 + lane;
-                unsigned f = 0, a = 0;
-                int j0 = 0;
-                if (k < k1) {
-                    f = (maskf[k] >> (si * NS)) & RM;
-                    a = (mask[k] >> (si * NS)) & RM;
-                    j0 = mstart[mj[k]];
-                }
-                // exclusive prefix sums of the per-lane counts
-                int nf = __popc(f), na = __popc(a), pf = nf, pa = na;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int tf = __shfl_up_sync(0xffffffffu, pf, o), ta = __shfl_up_sync(0xffffffffu, pa, o);
-                    if (lane >= o) {
-                        pf += tf;
-                        pa += ta;
-                    }
-                }
-                long long qf = wf + pf - nf, qa = wa + pa - na;
-                for (unsigned m = f; m; m &= m - 1u) {
-                    if (qf < cap) col[qf] = j0 + __ffs(m) - 1;
-                    qf++;
-                }
-                for (unsigned m = a; m; m &= m - 1u) {
-                    if (qa < cap) colA[qa] = j0 + __ffs(m) - 1;
-                    qa++;
-                }
-                wf += __shfl_sync(0xffffffffu, pf, 31);
-                wa += __shfl_sync(0xffffffffu, pa, 31);
+        long long wf[NS], wa[NS];
+#pragma unroll
+        for (int si = 0; si < NS; si++) {
+            wf[si] = si < ni ? row[i0 + si] : 0;
+            wa[si] = si < ni ? rowA[i0 + si] : 0;
+        }
+        for (int k0 = mrow[mi]; k0 < k1; k0 += 32) {
+            const int k = k0 + lane;
+            unsigned f = 0, a = 0;
+            int j0 = 0;
+            if (k < k1) {
+                f = maskf[k];
+                a = mask[k];
+                j0 = mstart[mj[k]];
             }
+            // exclusive prefix sums of the per-lane counts, a byte per i site
+            // (at most 32 * 4 in all)
+            unsigned nf = 0, na = 0;
+#pragma unroll
+            for (int si = 0; si < NS; si++) {
+                nf |= (unsigned)__popc((f >> (si * NS)) & RM) << (8 * si);
+                na |= (unsigned)__popc((a >> (si * NS)) & RM) << (8 * si);
+            }
+            unsigned pf = nf, pa = na;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned tf = __shfl_up_sync(0xffffffffu, pf, o), ta = __shfl_up_sync(0xffffffffu, pa, o);
+                if (lane >= o) {
+                    pf += tf;
+                    pa += ta;
+                }
+            }
+            const unsigned allf = __shfl_sync(0xffffffffu, pf, 31), alla = __shfl_sync(0xffffffffu, pa, 31);
+            pf -= nf;
+            pa -= na;
+#pragma unroll
+            for (int si = 0; si < NS; si++) {
+                int qf = (pf >> (8 * si)) & 255u, qa = (pa >> (8 * si)) & 255u;
+#pragma unroll
+                for (int sj = 0; sj < NS; sj++) {
+                    if ((f >> (si * NS + sj)) & 1u) buf[0][si][qf++] = j0 + sj;
+                    if ((a >> (si * NS + sj)) & 1u) buf[1][si][qa++] = j0 + sj;
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int si = 0; si < NS; si++) {
+                const int tf = (allf >> (8 * si)) & 255u, ta = (alla >> (8 * si)) & 255u;
+                for (int q = lane; q < tf; q += 32)
+                    if (wf[si] + q < cap) col[wf[si] + q] = buf[0][si][q];
+                for (int q = lane; q < ta; q += 32)
+                    if (wa[si] + q < cap) colA[wa[si] + q] = buf[1][si][q];
+                wf[si] += tf;
+                wa[si] += ta;
+            }
+            __syncwarp();
         }
     }
 }
