@@ -425,6 +425,18 @@ static void mixed_setup(pinyb200_ctx *c, const pinyb200_system *s, int n0)
             c->mix_q2[sp] = (float)q2;
             c->mix_toff[sp] = (int)((size_t)u * per + 2);  // knot k = nint(t) + 3, coefficients at k - 1
         }
+    // one Coulomb table for every charged pair (the shared-memory kernel's condition)
+    c->mix_coul_u = -1;
+    bool one = true;
+    for (int sp = 0; sp < NS * NS; sp++) {
+        if (!(c->mix_eflag[sp] & 2)) continue;
+        const int u = (int)((c->mix_toff[sp] - 2) / (long long)per);
+        if (c->mix_coul_u < 0) c->mix_coul_u = u;
+        const size_t o = (size_t)u * per, o0 = (size_t)c->mix_coul_u * per;
+        one = one && s->cv0_c && s->cdv0_c && memcmp(s->cv0_c + o, s->cv0_c + o0, per * sizeof(double)) == 0 &&
+              memcmp(s->cdv0_c + o, s->cdv0_c + o0, per * sizeof(double)) == 0;
+    }
+    if (!one) c->mix_coul_u = -1;
     const int u0 = s->inter_map[p0];
     c->mix_rc2 = (float)(s->cutoff[p0] * s->cutoff[p0]);
     c->mix_dri = (float)s->dri_spl[u0];

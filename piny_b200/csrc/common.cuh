@@ -111,7 +111,11 @@ template <> struct Idx<double> {
     }
     static __device__ __forceinline__ double dist(double dx, double dy, double dz)
     {
-        return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+        return __dsqrt_rn(dist2(dx, dy, dz));
+    }
+    static __device__ __forceinline__ double dist2(double dx, double dy, double dz)
+    {
+        return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
     }
 };
 template <> struct Idx<float> {

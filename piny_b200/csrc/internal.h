@@ -23,6 +23,7 @@ enum Slot {
     S_VBOND,
     S_VBEND,
     S_PXX, S_PYY, S_PZZ, S_PXY, S_PXZ, S_PYZ,  // bead pressure tensor
+    S_NEXT = 14,  // first bead of a launch's bead group: chunks its pair kernel has handed out
     S_EXT = 15,   // bead 0 only: molecule extent bound of the evaluation (bits of a double >= 0)
     S_NSLOT = 16
 };
@@ -202,6 +203,7 @@ struct pinyb200_ctx {
     // site pair of the molecule shares one cutoff and spline grid
     bool mix_ok = false;
     int mix_toff[16] = {0}, mix_eflag[16] = {0};
+    int mix_coul_u = -1;  // table whose Coulomb rows every charged pair reads, or -1
     float mix_q2[16] = {0};
     float4 *d_tabfe = nullptr;  // [2][nuniq][nsplin][2] vdW / Coulomb force and energy rows side by side
     float mix_rc2 = 0, mix_dri = 0, mix_rmd = 0, mix_tmax = 0;

@@ -843,6 +843,7 @@ template <typename R>
 struct PairConst {
     typename Vec4<R>::T c[16];
     R q2[16];
+    R lim[16];  // FP64: r^2 beyond which sqrt(r^2) cannot round below the cutoff
     int2 o[16];
 };
 
@@ -912,8 +913,11 @@ __device__ __forceinline__ int knot32(float r, float rmin, float dri, int nsm2, 
 
 // One site pair of one bead: force -dV/dr * r_vec / r on i (returned in
 // f), energies and virial accumulated.  r holds the separation i - j.
-// The sum is force_npol's: q2 * Coulomb table + vdW table.
-template <typename R, bool FAST, bool ENERGY>
+// The sum is force_npol's: q2 * Coulomb table + vdW table.  Half of a list's
+// site pairs lie between the cutoff and the skin: with one molecule pair to a
+// warp (PRE) FP64 tells most of them by r^2, without the square root (1202 ->
+// 1167 us at 4096 TIP4P/F x 32).
+template <typename R, bool FAST, bool ENERGY, bool PRE>
 __device__ __forceinline__ bool site_pair(const typename Vec4<R>::T *__restrict__ tab, size_t tstride, int nsm2,
                                           const PairConst<R> &pc, int sp, R rx, R ry, R rz, R &fx, R &fy, R &fz,
                                           R &evs, R &ecs, R *pvs)
@@ -931,7 +935,9 @@ __device__ __forceinline__ bool site_pair(const typename Vec4<R>::T *__restrict_
         kk = knot32(r, c.y, c.z, nsm2, del);
         q2 = c.w;
     } else {
-        const R r = Idx<R>::dist(rx, ry, rz);
+        const R r2 = Idx<double>::dist2(rx, ry, rz);
+        if (PRE && !(r2 <= pc.lim[sp])) return false;
+        const R r = __dsqrt_rn(r2);
         if (!(r < c.x)) return false;
         kk = Idx<R>::knot(r, c.y, c.z, c.w, nsm2, del);
         q2 = pc.q2[sp];
@@ -1007,31 +1013,55 @@ __device__ __forceinline__ NearImages near_images(const double *__restrict__ xmo
     return n;
 }
 
+// Chunks of mol_pair_kernel after each warp's first, handed out in order where
+// there are more than two to a warp: with a static stride over 16 blocks per
+// SM the last ones finished alone (FP64, 5.5 chunks a warp: 1167 -> 1051 us at
+// 4096 TIP4P/F x 32; at one chunk a warp the counter only costs, 2 to 3 us of
+// 35 to 240).  The counter lies with the energy
+// sums (cleared with them); the next chunk is asked for before the current one
+// is worked on.  The MIXED kernels gain nothing from it (359 against 366 us;
+// 45 against 49 us with one bead): their grid is one wave of resident blocks.
+struct ChunkQueue {
+    unsigned *next;
+    int first, got;
+    __device__ __forceinline__ ChunkQueue(double *acc, int group, int nwarps)
+        : next((unsigned *)(acc + (size_t)32 * group * S_NSLOT + S_NEXT)), first(nwarps), got(0)
+    {
+    }
+    __device__ __forceinline__ void ask(int lane)
+    {
+        if (lane == 0) got = first + (int)atomicAdd(next, 1u);
+    }
+    __device__ __forceinline__ int take() { return __shfl_sync(0xffffffffu, got, 0); }
+};
+
 // A 128-thread block's energy and virial sums (sacc[k][t], thread t holding
 // bead t % G) added to acc[bead][slot], summed over the block first: an
 // atomic per bead, sum and block instead of one per warp (or lane group).
 // Every thread of the block must call it.
-template <int G>
-__device__ __forceinline__ void pair_energy_flush(const double (*sacc)[128], double *acc)
+template <int G, int BT = 128>
+__device__ __forceinline__ void pair_energy_flush(const double (*sacc)[BT], double *acc)
 {
     __syncthreads();
     const int lane = threadIdx.x & 31;
+    for (int c = threadIdx.x >> 5; c < 8; c += BT / 32) {
+        double t = 0.0;
 #pragma unroll
-    for (int c = threadIdx.x >> 5; c < 8; c += 4) {
-        double t = (sacc[c][lane] + sacc[c][lane + 32]) + (sacc[c][lane + 64] + sacc[c][lane + 96]);
+        for (int k = lane; k < BT; k += 32) t += sacc[c][k];
         if (G < 32) t = warp_sum_strided(t, G);
         // sums 0, 1: S_VVDW, S_VCOUL; 2..7: S_PXX..S_PYZ
         if (lane < G && t != 0.0) atomicAdd(&acc[(size_t)lane * S_NSLOT + (c < 2 ? S_VVDW + c : S_PXX + c - 2)], t);
     }
 }
 
-template <typename R, int P, int NS, bool FAST, bool ENERGY>
+template <typename R, int P, int NS, bool ENERGY>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : PINYB200_MOL_BLOCKS64)
     mol_pair_kernel(MolArgs a, Cell cell)
 {
     typedef typename Vec4<R>::T V;
     constexpr int G = P >= 32 ? 32 : P;  // lanes per molecule pair
     constexpr int JPI = 32 / G;          // molecule pairs per warp step
+    constexpr bool FAST = sizeof(R) == 4;  // MIXED: offsets and r^2 in FP32; else PINY's order in FP64
     __shared__ PairConst<R> pc;
     __shared__ double sacc[8][128];      // per-thread energy / virial sums
     if (threadIdx.x < NS * NS) {
@@ -1056,6 +1086,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
         }
         pc.c[threadIdx.x] = c;
         pc.q2[threadIdx.x] = (R)q2;
+        pc.lim[threadIdx.x] = (R)(a.cutoff[p] * a.cutoff[p] * (1.0 + 1e-14));
         pc.o[threadIdx.x] = make_int2(u * a.nsplin, a.has_vdw[u]);
     }
     if (ENERGY)
@@ -1079,7 +1110,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
 
     const double ext2 = ext2_of(a.ext);  // image test margin of this evaluation
     const int nch = *a.nchunk;
-    for (int ch = warp; ch < nch; ch += nwarps) {
+    ChunkQueue q(a.acc, blockIdx.y, nwarps);
+    const bool queue = nch > 2 * nwarps;
+    for (int ch = warp; ch < nch; ch = queue ? q.take() : ch + nwarps) {
+        if (queue) q.ask(lane);
         const int mi = a.chunk[3 * ch], beg = a.chunk[3 * ch + 1], end = a.chunk[3 * ch + 2];
         const int i0 = a.mstart[mi], ni = a.mstart[mi + 1] - i0;
         double xi[NS][3];  // FP64 positions (MIXED keeps site 0 only live)
@@ -1194,7 +1228,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
                             rz = (R)__dadd_rn(__dsub_rn(xi[si][2], xjz), __dmul_rn(sz, cell.h[8]));
                         }
                         R fx, fy, fz;
-                        if (site_pair<R, FAST, ENERGY>(tab, tstride, nsm2, pc, si * NS + sj, rx, ry, rz, fx, fy, fz, evs,
+                        if (site_pair<R, FAST, ENERGY, P >= 32>(tab, tstride, nsm2, pc, si * NS + sj, rx, ry, rz, fx, fy, fz, evs,
                                                        ecs, pvs)) {
                             fi[si][0] += fx;
                             fi[si][1] += fy;
@@ -1301,6 +1335,7 @@ struct MixSite {
     float q2[16];        // charge product of the site pair
     int eflag[16];       // tables the site pair uses: 1 vdW, 2 Coulomb
     int tstride;         // nuniq * nsplin, the distance between table kinds
+    int coul;            // first row of the one Coulomb table
     float rc2, dri_f, rmd, tmax;  // cutoff^2, 1/dr, rmin/dr, last interval
 };
 
@@ -1318,7 +1353,7 @@ constexpr unsigned kAnyPair = 0xffffffffu;
 constexpr unsigned kTip4pCoul = 0xEEE0u, kTip4pVdw = 0x1u;  // O H H M: H, M charged; LJ on O-O
 constexpr unsigned kSpcCoul = 0x1FFu, kSpcVdw = 0x1u;       // O H H: all charged; LJ on O-O
 
-template <int P, int NS, bool ENERGY, unsigned CM, unsigned VM>
+template <int P, int NS, bool ENERGY, unsigned CM, unsigned VM, int BT = 128, bool ST = false>
 __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixSite &m, const Cell &cell,
                                                     const VBlk vb)
 {
@@ -1330,10 +1365,24 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
     // consecutive values) at a time; rows are padded by one against conflicts.
     constexpr bool COOP = P <= 2 && CM != kAnyPair;
     constexpr int NR = 3 * NS * P;
-    __shared__ double stage[COOP ? 4 : 1][COOP ? JPI * (NR + 1) : 1];
-    __shared__ double sacc[8][128];
+    constexpr int NST = COOP ? BT / 32 * JPI * (NR + 1) : 0;
+    // ST: the Coulomb rows, the sums and the staged molecules in dynamic shared
+    // memory (mix_shared_smem), otherwise the last two in static
+    extern __shared__ float4 mix_dyn[];
+    __shared__ double static_mem[ST ? 1 : 8 * BT + NST];
+    double *const smem = ST ? (double *)(mix_dyn + (ENERGY ? 2 : 1) * m.nsplin) : static_mem;
+    double(*const sacc)[BT] = (double(*)[BT])smem;
+    double *const stage = smem + 8 * BT;
     if (ENERGY)
         for (int c = 0; c < 8; c++) sacc[c][threadIdx.x] = 0.0;
+    if constexpr (ST) {
+        const float4 *src = ENERGY ? a.tabfe + 2 * (m.tstride + m.coul) : a.tab + T_CDV0C * m.tstride + m.coul;
+        for (int k = threadIdx.x; k < m.nsplin; k += BT) {
+            cp_async16(mix_dyn + k, src + (ENERGY ? 2 * k : k));
+            if (ENERGY) cp_async16(mix_dyn + m.nsplin + k, src + 2 * k + 1);
+        }
+        cp_async_wait();
+    }
     __syncthreads();
     if (a.bad && (a.bad[0] | a.bad[1])) {
         if (vb.x == 0 && vb.y == 0 && threadIdx.x == 0) a.acc[S_VVDW] = __longlong_as_double(0x7ff8000000000000LL);
@@ -1365,7 +1414,7 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
             }
         }
         float evs = 0.0f, ecs = 0.0f, pvs[6] = {0, 0, 0, 0, 0, 0};
-        double *st = stage[COOP ? (threadIdx.x >> 5) : 0];
+        double *st = stage + (COOP ? (threadIdx.x >> 5) * JPI * (NR + 1) : 0);
         for (int kb = beg; kb < end; kb += JPI) {
             const int k = kb + sub;
             const bool act = k < end;
@@ -1469,7 +1518,10 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                             float4 ecf = make_float4(0.f, 0.f, 0.f, 0.f), evf = ecf;
                             if (coul) {
                                 float4 cf;
-                                if (ENERGY) {
+                                if constexpr (ST) {
+                                    cf = mix_dyn[kn + 2];
+                                    if (ENERGY) ecf = mix_dyn[m.nsplin + kn + 2];
+                                } else if (ENERGY) {
                                     ldg_keep_pair(rfe + 2 * m.tstride, cf, ecf);
                                 } else {
                                     cf = ldg_keep(row + T_CDV0C * m.tstride);
@@ -1572,9 +1624,33 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
             for (int c = 0; c < 6; c++) sacc[2 + c][threadIdx.x] += (double)pvs[c];
         }
     }
-    if (ENERGY) pair_energy_flush<G>(sacc, a.acc + (size_t)32 * vb.y * S_NSLOT);
+    if (ENERGY) pair_energy_flush<G, BT>(sacc, a.acc + (size_t)32 * vb.y * S_NSLOT);
 }
 
+
+// One block of 20 warps per SM with the Coulomb force and energy rows in
+// shared memory.  32 beads' knots spread over some 30 cache lines, so a gather
+// through L1 costs a tag lookup for each; 16-byte shared loads cost bank
+// conflicts instead (about 10 wavefronts a load), never miss, and leave L1 to
+// the positions.  Pair phase, gathers through L1 -> shared rows: 393 -> 365 us
+// (4096 TIP4P/F x 32), 185 -> 160 (8000 x 4), 43 -> 35 (512 x 8), 80 -> 74
+// (1024 x 16).  What bounds it now: issue 63 %, L1 and shared memory 72 %, no
+// unit full at 20 warps per SM.
+constexpr int kMixShared = 640;
+template <int P, int NS, bool ENERGY, unsigned CM, unsigned VM>
+__global__ void __launch_bounds__(kMixShared, 1)
+    mol_pair_mixed_shared_kernel(const __grid_constant__ MixArgs a, const __grid_constant__ MixSite m, Cell cell)
+{
+    mol_pair_mixed_body<P, NS, ENERGY, CM, VM, kMixShared, true>(a, m, cell, hw_blk());
+}
+
+// Most dynamic shared memory it takes (tables of 4096 points with both rows),
+// so that L1 keeps some 60 KB.
+#define PINYB200_MIX_SHARED_MAX (168 * 1024)
+static size_t mix_shared_smem(int nsplin, bool energy)
+{
+    return (size_t)(energy ? 2 : 1) * nsplin * sizeof(float4) + 8 * kMixShared * sizeof(double);
+}
 
 template <int P, int NS, bool ENERGY, unsigned CM = kAnyPair, unsigned VM = kAnyPair>
 __global__ void __launch_bounds__(128, PINYB200_MIX_BLOCKS)
@@ -1973,7 +2049,7 @@ cudaError_t launch_site_from_mol(pinyb200_ctx *c, int pass, const int *gate, cud
 }
 
 template <typename R, int P, int NS>
-static void launch_mol_t(pinyb200_ctx *c, const MolArgs &a, const Cell &cell, bool fast)
+static void launch_mol_t(pinyb200_ctx *c, const MolArgs &a, const Cell &cell)
 {
     const int threads = 128;
     long long blocks = ((long long)c->chunk_cap * 32 + threads - 1) / threads;
@@ -1981,28 +2057,21 @@ static void launch_mol_t(pinyb200_ctx *c, const MolArgs &a, const Cell &cell, bo
     if (blocks > maxb) blocks = maxb;
     if (blocks < 1) blocks = 1;
     dim3 grid((unsigned)blocks, P > 32 ? P / 32 : 1);
-    if constexpr (sizeof(R) == 4) {
-        if (fast) {
-            if (a.energy) mol_pair_kernel<R, P, NS, true, true><<<grid, threads, 0, c->stream>>>(a, cell);
-            else mol_pair_kernel<R, P, NS, true, false><<<grid, threads, 0, c->stream>>>(a, cell);
-            return;
-        }
-    }
-    if (a.energy) mol_pair_kernel<R, P, NS, false, true><<<grid, threads, 0, c->stream>>>(a, cell);
-    else mol_pair_kernel<R, P, NS, false, false><<<grid, threads, 0, c->stream>>>(a, cell);
+    if (a.energy) mol_pair_kernel<R, P, NS, true><<<grid, threads, 0, c->stream>>>(a, cell);
+    else mol_pair_kernel<R, P, NS, false><<<grid, threads, 0, c->stream>>>(a, cell);
 }
 
 template <typename R, int NS>
-static cudaError_t launch_mol_ns(pinyb200_ctx *c, const MolArgs &a, const Cell &cell, bool fast)
+static cudaError_t launch_mol_ns(pinyb200_ctx *c, const MolArgs &a, const Cell &cell)
 {
     switch (c->P) {
-    case 1: launch_mol_t<R, 1, NS>(c, a, cell, fast); break;
-    case 2: launch_mol_t<R, 2, NS>(c, a, cell, fast); break;
-    case 4: launch_mol_t<R, 4, NS>(c, a, cell, fast); break;
-    case 8: launch_mol_t<R, 8, NS>(c, a, cell, fast); break;
-    case 16: launch_mol_t<R, 16, NS>(c, a, cell, fast); break;
-    case 32: launch_mol_t<R, 32, NS>(c, a, cell, fast); break;
-    case 64: launch_mol_t<R, 64, NS>(c, a, cell, fast); break;
+    case 1: launch_mol_t<R, 1, NS>(c, a, cell); break;
+    case 2: launch_mol_t<R, 2, NS>(c, a, cell); break;
+    case 4: launch_mol_t<R, 4, NS>(c, a, cell); break;
+    case 8: launch_mol_t<R, 8, NS>(c, a, cell); break;
+    case 16: launch_mol_t<R, 16, NS>(c, a, cell); break;
+    case 32: launch_mol_t<R, 32, NS>(c, a, cell); break;
+    case 64: launch_mol_t<R, 64, NS>(c, a, cell); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -2039,20 +2108,38 @@ cudaError_t launch_mol_pair(pinyb200_ctx *c, const Cell &cell, bool energy)
     a.energy = energy ? 1 : 0;
     if (c->precision == PINYB200_FP64) {
         a.tab = s.tab64;
-        if (c->mol_ns == 3) return launch_mol_ns<double, 3>(c, a, cell, false);
-        return launch_mol_ns<double, 4>(c, a, cell, false);
+        if (c->mol_ns == 3) return launch_mol_ns<double, 3>(c, a, cell);
+        return launch_mol_ns<double, 4>(c, a, cell);
     }
     a.tab = s.tab32;
-    if (c->mol_ns == 3) return launch_mol_ns<float, 3>(c, a, cell, true);
-    return launch_mol_ns<float, 4>(c, a, cell, true);
+    if (c->mol_ns == 3) return launch_mol_ns<float, 3>(c, a, cell);
+    return launch_mol_ns<float, 4>(c, a, cell);
 }
 
 
 template <int P, int NS, unsigned CM, unsigned VM>
-static void launch_mix_pattern(pinyb200_ctx *c, const MixArgs &a, const MixSite &m, const Cell &cell, bool energy,
+static cudaError_t launch_mix_pattern(pinyb200_ctx *c, const MixArgs &a, const MixSite &m, const Cell &cell, bool energy,
                                dim3 grid)
 {
     const int threads = 128;
+    // Tables in shared memory: every charged pair reads one Coulomb table, the
+    // rows fit, and the chunks fill 20 warps on every SM (below that the
+    // 128-thread blocks spread over more SMs).  Not with one or two beads, where
+    // the staged molecules need the space (45 us either way at 4096 x 1).
+    if constexpr (CM != kAnyPair && P > 2) {
+        const size_t sm = mix_shared_smem(m.nsplin, energy);
+        const long long full = ((long long)c->chunk_cap + 3) / 4 * grid.y;
+        if (c->mix_coul_u >= 0 && sm <= PINYB200_MIX_SHARED_MAX && full >= 5LL * c->sm_count) {
+            const void *fn = energy ? (const void *)mol_pair_mixed_shared_kernel<P, NS, true, CM, VM>
+                                    : (const void *)mol_pair_mixed_shared_kernel<P, NS, false, CM, VM>;
+            const cudaError_t e = smem_optin(fn, (int)sm);
+            if (e != cudaSuccess) return e;
+            grid.x = std::max(1, std::max(1, c->pair_blocks_per_sm / 5) * c->sm_count / (int)grid.y);
+            if (energy) mol_pair_mixed_shared_kernel<P, NS, true, CM, VM><<<grid, kMixShared, sm, c->stream>>>(a, m, cell);
+            else mol_pair_mixed_shared_kernel<P, NS, false, CM, VM><<<grid, kMixShared, sm, c->stream>>>(a, m, cell);
+            return cudaGetLastError();
+        }
+    }
     if (energy) {
         carveout_pref((const void *)mol_pair_mixed_kernel<P, NS, true, CM, VM>, P <= 2 ? 50 : c->pair_carveout);
         mol_pair_mixed_kernel<P, NS, true, CM, VM><<<grid, threads, 0, c->stream>>>(a, m, cell);
@@ -2060,10 +2147,11 @@ static void launch_mix_pattern(pinyb200_ctx *c, const MixArgs &a, const MixSite 
         carveout_pref((const void *)mol_pair_mixed_kernel<P, NS, false, CM, VM>, P <= 2 ? 50 : c->pair_carveout);
         mol_pair_mixed_kernel<P, NS, false, CM, VM><<<grid, threads, 0, c->stream>>>(a, m, cell);
     }
+    return cudaGetLastError();
 }
 
 template <int P, int NS>
-static void launch_mix_t(pinyb200_ctx *c, const MixArgs &a, const MixSite &m, const Cell &cell, bool energy)
+static cudaError_t launch_mix_t(pinyb200_ctx *c, const MixArgs &a, const MixSite &m, const Cell &cell, bool energy)
 {
     const int threads = 128;
     long long blocks = ((long long)c->chunk_cap * 32 + threads - 1) / threads;
@@ -2078,27 +2166,25 @@ static void launch_mix_t(pinyb200_ctx *c, const MixArgs &a, const MixSite &m, co
         if (c->mix_eflag[k] & 1) vm |= 1u << k;
     }
     if (NS == 4 && cm == kTip4pCoul && vm == kTip4pVdw)
-        launch_mix_pattern<P, NS, kTip4pCoul, kTip4pVdw>(c, a, m, cell, energy, grid);
-    else if (NS == 3 && cm == kSpcCoul && vm == kSpcVdw)
-        launch_mix_pattern<P, NS, kSpcCoul, kSpcVdw>(c, a, m, cell, energy, grid);
-    else
-        launch_mix_pattern<P, NS, kAnyPair, kAnyPair>(c, a, m, cell, energy, grid);
+        return launch_mix_pattern<P, NS, kTip4pCoul, kTip4pVdw>(c, a, m, cell, energy, grid);
+    if (NS == 3 && cm == kSpcCoul && vm == kSpcVdw)
+        return launch_mix_pattern<P, NS, kSpcCoul, kSpcVdw>(c, a, m, cell, energy, grid);
+    return launch_mix_pattern<P, NS, kAnyPair, kAnyPair>(c, a, m, cell, energy, grid);
 }
 
 template <int NS>
 static cudaError_t launch_mix_ns(pinyb200_ctx *c, const MixArgs &a, const MixSite &m, const Cell &cell, bool energy)
 {
     switch (c->P) {
-    case 1: launch_mix_t<1, NS>(c, a, m, cell, energy); break;
-    case 2: launch_mix_t<2, NS>(c, a, m, cell, energy); break;
-    case 4: launch_mix_t<4, NS>(c, a, m, cell, energy); break;
-    case 8: launch_mix_t<8, NS>(c, a, m, cell, energy); break;
-    case 16: launch_mix_t<16, NS>(c, a, m, cell, energy); break;
-    case 32: launch_mix_t<32, NS>(c, a, m, cell, energy); break;
-    case 64: launch_mix_t<64, NS>(c, a, m, cell, energy); break;
+    case 1: return launch_mix_t<1, NS>(c, a, m, cell, energy);
+    case 2: return launch_mix_t<2, NS>(c, a, m, cell, energy);
+    case 4: return launch_mix_t<4, NS>(c, a, m, cell, energy);
+    case 8: return launch_mix_t<8, NS>(c, a, m, cell, energy);
+    case 16: return launch_mix_t<16, NS>(c, a, m, cell, energy);
+    case 32: return launch_mix_t<32, NS>(c, a, m, cell, energy);
+    case 64: return launch_mix_t<64, NS>(c, a, m, cell, energy);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 // Arguments of the MIXED molecule-pair kernel for one context.
@@ -2138,6 +2224,7 @@ static MixSite mix_site(const pinyb200_ctx *c)
         m.eflag[k] = c->mix_eflag[k];
     }
     m.tstride = s.nuniq * s.nsplin;
+    m.coul = c->mix_coul_u * s.nsplin;
     m.rc2 = c->mix_rc2;
     m.dri_f = c->mix_dri;
     m.rmd = c->mix_rmd;

@@ -167,3 +167,28 @@ def test_gradient_pair_kernels(nmol, beads, cutoff):
         # FP32 pair and mesh terms: 1e-6 of the largest component, single ones within 1e-3 of it as elsewhere
         assert np.abs(dE - out[0][0]).max() <= 1e-5 * np.abs(out[0][0]).max()
         assert np.abs(dF - out[0][1]).max() <= 1e-5 * np.abs(out[0][1]).max()
+
+
+@pytest.mark.parametrize("nsplin", [2000, 4096, 4097, 9000])
+@pytest.mark.parametrize("model,nmol,beads", [(water.TIP4P_F, 700, 4), (water.SPC_FW, 300, 8), (water.TIP4P_F, 300, 16),
+                                              (water.TIP4P_F, 300, 32), (water.SPC_FW, 216, 64)])
+def test_pair_tables_in_shared_memory(oracle, model, nmol, beads, nsplin):
+    # boxes large enough for the one-block-per-SM kernel; tables that fit its shared memory up to the
+    # last point, and ones that do not
+    L = water.density_box_edge(nmol)
+    spec = water.BoxSpec(model, nmol, L, beads, 298.0, 5, cutoff=min(9.0, 0.45 * L), grid=24, order=6, nsplin=nsplin)
+    pos = water.build_positions(spec) / water.BOHR
+    S = system.build_system(spec, pos)
+    xmod = pos.mean(axis=0)
+    fref, eref = _oracle(oracle, S, pos, xmod)
+    f, e = _device(S, pos, xmod, "mixed")
+    _check("mixed", f, e, fref, eref)
+
+
+@pytest.mark.parametrize("nmol,beads", [(65, 32), (700, 32), (700, 64)])
+def test_fp64_pairs_by_chunk_queue(oracle, nmol, beads):
+    # fewer and more than two chunks to a warp
+    spec, S, pos, xmod = _box(water.TIP4P_F, nmol, beads, 24, 6)
+    fref, eref = _oracle(oracle, S, pos, xmod)
+    f, e = _device(S, pos, xmod, "fp64", tuning={2: 1})
+    _check("fp64", f, e, fref, eref)
