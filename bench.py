@@ -157,6 +157,10 @@ def kernel_bytes(S, P, precision, npairs, nmolp):
         "pme_force_add": 72.0 * nrec,
         "intra (bond, bend, ecor)": 72.0 * P * (2 * nb + 3 * nbe + 2 * nec),
         "transpose_out": 48.0 * N * P,
+        # water boxes: positions in and out, FP32 offsets (MIXED), forces cleared, PME records;
+        # positions, pair and mesh forces in, forces out
+        "stage": (72.0 + (12.0 if precision == "mixed" else 0.0)) * N * P + nrec * (rec + 4.0),
+        "finish (intra, force sum, out)": 72.0 * N * P + 24.0 * nrec,
     }
 
 

@@ -353,7 +353,9 @@ int pinyb200_autotune(pinyb200_ctx *c, const double *d_pos, const double *d_xmod
                     if (rc) return rc;
                     float tsum = 0;
                     for (int r = 0; r <= reps; r++) {
-                        rc = enqueue_device(c, d_pos, d_xmod, cell, eflags, c->d_force_aos, true, nullptr);
+                        cudaEventRecord(c->ev[0], c->stream);
+                        rc = enqueue_device(c, d_pos, d_xmod, cell, eflags, c->d_force_aos, false, nullptr);
+                        cudaEventRecord(c->ev[4], c->stream);
                         if (rc) return rc;
                         if (cudaStreamSynchronize(c->stream) != cudaSuccess)
                             return record_error(c, PINYB200_ERR_CUDA, "autotune: synchronize");

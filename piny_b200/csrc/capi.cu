@@ -676,7 +676,7 @@ int pinyb200_create(const pinyb200_system *s, int nbeads, int precision, pinyb20
     CK(cudaMalloc(&c->d_force_aos, nb * sizeof(double)));
     CK(cudaMalloc(&c->d_xmod, (size_t)natm * 3 * sizeof(double)));
     CK(cudaMalloc(&c->d_x0, (size_t)natm * 3 * sizeof(double)));
-    CK(cudaMalloc(&c->d_acc, (size_t)nbeads * S_NSLOT * sizeof(double)));
+    CK(cudaMalloc(&c->d_acc, ((size_t)nbeads * S_NSLOT + T_NSTAMP) * sizeof(double)));
     CK(cudaMalloc(&c->d_row, (size_t)(natm + 1) * sizeof(int)));
     CK(cudaMalloc(&c->d_rowA, (size_t)(natm + 1) * sizeof(int)));
     CK(cudaMalloc(&c->d_count, (size_t)2 * natm * sizeof(int)));
@@ -1056,6 +1056,27 @@ void pinyb200::evaluate_finish(pinyb200_ctx *c, const Cell &cell, int flags, con
     }
 }
 
+// Phase times of the evaluation just waited for: the stamps behind its sums
+// (water path), or the events around its phases.
+cudaError_t pinyb200::read_phase_times(pinyb200_ctx *c, const double *acc)
+{
+    if (c->water_ok) {
+        unsigned long long t[T_NSTAMP];
+        memcpy(t, acc + (size_t)c->P * S_NSLOT, sizeof(t));
+        auto ms = [&](int a, int b) { return t[a] && t[b] > t[a] ? (float)(1e-6 * (double)(t[b] - t[a])) : 0.0f; };
+        c->last_ms[0] = ms(T_BEG, T_END);
+        c->last_ms[1] = ms(T_PAIR0, T_PAIR1);
+        c->last_ms[2] = ms(T_PME0, T_PME1);
+        c->last_ms[3] = ms(T_FIN0, T_END);
+        return cudaSuccess;
+    }
+    cudaError_t e = cudaEventElapsedTime(&c->last_ms[0], c->ev[0], c->ev[4]);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&c->last_ms[1], c->ev[1], c->ev[2]);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&c->last_ms[2], c->ev_pme[0], c->ev_pme[1]);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&c->last_ms[3], c->ev[5], c->ev[3]);
+    return e;
+}
+
 // mode-1 positions for a PIMD call without xmod: the bead centroid
 __global__ void centroid_kernel(const double *__restrict__ posT, double *__restrict__ xm, int natm, int P)
 {
@@ -1069,7 +1090,8 @@ __global__ void centroid_kernel(const double *__restrict__ posT, double *__restr
 // The evaluation of a box of water molecules (pinyb200_ctx::water_ok): one
 // staging kernel, the pair kernel beside the PME chain, one finishing kernel.
 // The charge grid is cleared on the PME stream from the start, and PME waits
-// only for the staging, not for a list update.
+// only for the staging, not for a list update.  timing: h_acc has room for the
+// time stamps behind the sums, and takes them (with or without energies).
 static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, const Cell &cell, int flags,
                          double *d_force, bool timing, double *h_acc, bool keep)
 {
@@ -1083,7 +1105,6 @@ static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_x
         c->stream = main_stream;
         return e;
     };
-    if (timing) CK(ev_rec(c->ev[0], c->stream));
     CK(cudaEventRecord(c->ev_fork, c->stream));
     if (overlap) CK(cudaStreamWaitEvent(pme, c->ev_fork, 0));
     CK(on(pme, launch_pme_clear));
@@ -1094,9 +1115,7 @@ static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_x
     if (overlap) CK(cudaStreamWaitEvent(pme, c->ev_stage, 0));
     {
         c->stream = pme;
-        cudaError_t perr = timing ? ev_rec(c->ev_pme[0], c->stream) : cudaSuccess;
-        if (perr == cudaSuccess) perr = launch_pme(c, cell, energy, true);
-        if (perr == cudaSuccess && timing) perr = ev_rec(c->ev_pme[1], c->stream);
+        cudaError_t perr = launch_pme(c, cell, energy, true);
         if (perr == cudaSuccess) perr = cudaEventRecord(c->ev_join, c->stream);
         c->stream = main_stream;
         CK(perr);
@@ -1106,21 +1125,14 @@ static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_x
         int rc = list_update_enqueue(c, d_pos, c->P > 1 ? c->d_xmod : nullptr, cell, c->stream);
         if (rc) return rc;
     }
-    if (timing) CK(ev_rec(c->ev[1], c->stream));
     CK(launch_pair_any(c, cell, flags, energy, true));
     CK(kt_mark(c, "pair"));
-    if (timing) CK(ev_rec(c->ev[2], c->stream));
     CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
-    if (timing) CK(ev_rec(c->ev[5], c->stream));
     CK(launch_water_finish(c, d_force, energy, (flags & PINYB200_DISTRIB_GHOSTS) != 0, keep));
     CK(kt_mark(c, "finish (intra, force sum, out)"));
-    if (timing) {
-        CK(ev_rec(c->ev[3], c->stream));
-        CK(ev_rec(c->ev[4], c->stream));
-    }
-    if (energy && h_acc)
-        CK(cudaMemcpyAsync(h_acc, c->d_acc, (size_t)c->P * S_NSLOT * sizeof(double), cudaMemcpyDeviceToHost,
-                           c->stream));
+    const size_t nacc = (size_t)c->P * S_NSLOT, off = energy ? 0 : nacc, num = (energy ? nacc : 0) + (timing ? T_NSTAMP : 0);
+    if (h_acc && num)
+        CK(cudaMemcpyAsync(h_acc + off, c->d_acc + off, num * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     return PINYB200_OK;
 }
 
@@ -1236,16 +1248,13 @@ int pinyb200_energy_force_device(pinyb200_ctx *c, const double *d_pos, const dou
     } restore{c, own};
     Cell cell = make_cell(hmat);
     const bool energy = !(flags & PINYB200_NO_ENERGY);
-    if (energy && !c->h_acc_pin) CK(cudaMallocHost(&c->h_acc_pin, (size_t)c->P * S_NSLOT * sizeof(double)));
-    double *acc = energy ? c->h_acc_pin : nullptr;  // pinned: the copy can sit in the graph
+    if (!c->h_acc_pin) CK(cudaMallocHost(&c->h_acc_pin, ((size_t)c->P * S_NSLOT + T_NSTAMP) * sizeof(double)));
+    double *acc = c->h_acc_pin;  // pinned: the copy can sit in the graph
     int rc = run_eval_graph(c, eval_key(c, 1, d_pos, d_xmod, d_force, hmat, flags),
                             [&]() { return enqueue_device(c, d_pos, d_xmod, cell, flags, d_force, true, acc); });
     if (rc) return rc;
     CK(cudaStreamSynchronize(c->stream));
-    CK(cudaEventElapsedTime(&c->last_ms[0], c->ev[0], c->ev[4]));
-    CK(cudaEventElapsedTime(&c->last_ms[1], c->ev[1], c->ev[2]));
-    CK(cudaEventElapsedTime(&c->last_ms[2], c->ev_pme[0], c->ev_pme[1]));
-    CK(cudaEventElapsedTime(&c->last_ms[3], c->ev[5], c->ev[3]));
+    CK(read_phase_times(c, acc));
     evaluate_finish(c, cell, flags, acc, e);
     if (energy && e && !std::isfinite(e->vintert + e->vintrat))
         return fail(c, PINYB200_ERR_NAN, "non-finite energy: check the positions (forces were written)");
@@ -1268,8 +1277,8 @@ int pinyb200_energy_force(pinyb200_ctx *c, const double *pos, const double *xmod
     // everything enqueued, one wait: the forces come back right behind the
     // evaluation; the device part replays the context's graph
     const bool energy = !(flags & PINYB200_NO_ENERGY);
-    if (energy && !c->h_acc_pin) CK(cudaMallocHost(&c->h_acc_pin, (size_t)c->P * S_NSLOT * sizeof(double)));
-    double *acc = energy ? c->h_acc_pin : nullptr;  // pinned: the copy is queued, not waited for
+    if (!c->h_acc_pin) CK(cudaMallocHost(&c->h_acc_pin, ((size_t)c->P * S_NSLOT + T_NSTAMP) * sizeof(double)));
+    double *acc = c->h_acc_pin;  // pinned: the copy is queued, not waited for
     int rc = run_eval_graph(c, eval_key(c, 2, c->d_pos_aos, xmod ? c->d_xmod : nullptr, c->d_force_aos, hmat, flags),
                             [&]() {
                                 if (c->water_ok) {
@@ -1294,10 +1303,7 @@ int pinyb200_energy_force(pinyb200_ctx *c, const double *pos, const double *xmod
     CK(cudaMemcpyAsync(force, c->d_force_aos, nb * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaEventRecord(c->ev[7], c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    CK(cudaEventElapsedTime(&c->last_ms[0], c->ev[0], c->ev[4]));
-    CK(cudaEventElapsedTime(&c->last_ms[1], c->ev[1], c->ev[2]));
-    CK(cudaEventElapsedTime(&c->last_ms[2], c->ev_pme[0], c->ev_pme[1]));
-    CK(cudaEventElapsedTime(&c->last_ms[3], c->ev[5], c->ev[3]));
+    CK(read_phase_times(c, acc));
     CK(cudaEventElapsedTime(&c->last_ms[4], c->ev[6], c->ev[7]));
     evaluate_finish(c, cell, flags, acc, e);
     if (energy && e && !std::isfinite(e->vintert + e->vintrat))

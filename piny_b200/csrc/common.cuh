@@ -134,6 +134,23 @@ template <> struct Idx<float> {
     }
 };
 
+__device__ __forceinline__ unsigned long long clock_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// Stamp k of an evaluation (enum Stamp, behind its bead sums): the time the
+// grid's first block starts, the time its last one ends.
+__device__ __forceinline__ void stamp_start(unsigned long long *st, int k)
+{
+    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) st[k] = clock_ns();
+}
+__device__ __forceinline__ void stamp_end(unsigned long long *st, int k)
+{
+    if (threadIdx.x == 0) atomicMax(&st[k], clock_ns());
+}
+
 // 16 bytes from global to shared memory without passing registers (both
 // addresses 16-byte aligned); cp_async_wait before the block's barrier.
 __device__ __forceinline__ void cp_async16(void *smem, const void *g)

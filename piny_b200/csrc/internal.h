@@ -28,6 +28,11 @@ enum Slot {
     S_NSLOT = 16
 };
 
+// Times of one evaluation of the water path, behind the bead sums: its kernels
+// stamp them (a timing event between two kernels of a graph costs 5 us, eight
+// of them took 33 us of a call's 137 at 256 SPC/Fw, one bead).
+enum Stamp { T_BEG = 0, T_END, T_PAIR0, T_PAIR1, T_PME0, T_PME1, T_FIN0, T_NSTAMP = 8 };
+
 // Cell passed by value to kernels: h column-major, hi = h^-1 (gethinv).
 struct Cell {
     double h[9];
@@ -369,6 +374,8 @@ void evaluate_finish(pinyb200_ctx *c, const Cell &cell, int flags, const double 
 // keep: the complete site forces stay in c->d_forceT too
 int enqueue_device(pinyb200_ctx *c, const double *d_pos, const double *d_xmod, const Cell &cell, int flags,
                    double *d_force, bool timing, double *h_acc, bool keep = false);
+// last_ms of the evaluation just waited for; acc: its sums and stamps on the host
+cudaError_t read_phase_times(pinyb200_ctx *c, const double *acc);
 Cell cell_from_hmat(const double *hmat);
 int pme_tiles_resize(pinyb200_ctx *c, int T);
 void pme_swap(pinyb200_ctx *c, PmeSet &p);

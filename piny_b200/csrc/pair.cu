@@ -52,6 +52,8 @@ struct PairArgs {
 template <typename R, int P, bool RSP>
 __global__ void __launch_bounds__(256) pair_kernel(PairArgs a, Cell cell)
 {
+    unsigned long long *stamp = (unsigned long long *)(a.acc + (size_t)P * S_NSLOT);
+    if (!RSP) stamp_start(stamp, T_PAIR0);
     if (a.bad && (a.bad[0] | a.bad[1])) {
         // the list update could not hold the new list: fail loudly
         if (blockIdx.x == 0 && threadIdx.x == 0) a.acc[S_VVDW] = __longlong_as_double(0x7ff8000000000000LL);
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(256) pair_kernel(PairArgs a, Cell cell)
             }
         }
     }
+    if (!RSP) stamp_end(stamp, T_PAIR1);
 }
 
 template <typename R, int P, bool RSP>

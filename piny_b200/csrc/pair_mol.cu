@@ -1058,6 +1058,8 @@ template <typename R, int P, int NS, bool ENERGY>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : PINYB200_MOL_BLOCKS64)
     mol_pair_kernel(MolArgs a, Cell cell)
 {
+    unsigned long long *stamp = (unsigned long long *)(a.acc + (size_t)P * S_NSLOT);
+    stamp_start(stamp, T_PAIR0);
     typedef typename Vec4<R>::T V;
     constexpr int G = P >= 32 ? 32 : P;  // lanes per molecule pair
     constexpr int JPI = 32 / G;          // molecule pairs per warp step
@@ -1268,6 +1270,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
         }
     }
     if (ENERGY) pair_energy_flush<G>(sacc, a.acc + (size_t)32 * blockIdx.y * S_NSLOT);
+    stamp_end(stamp, T_PAIR1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1641,7 +1644,10 @@ template <int P, int NS, bool ENERGY, unsigned CM, unsigned VM>
 __global__ void __launch_bounds__(kMixShared, 1)
     mol_pair_mixed_shared_kernel(const __grid_constant__ MixArgs a, const __grid_constant__ MixSite m, Cell cell)
 {
+    unsigned long long *stamp = (unsigned long long *)(a.acc + (size_t)P * S_NSLOT);
+    stamp_start(stamp, T_PAIR0);
     mol_pair_mixed_body<P, NS, ENERGY, CM, VM, kMixShared, true>(a, m, cell, hw_blk());
+    stamp_end(stamp, T_PAIR1);
 }
 
 // Most dynamic shared memory it takes (tables of 4096 points with both rows),
@@ -1657,7 +1663,10 @@ __global__ void __launch_bounds__(128, PINYB200_MIX_BLOCKS)
     mol_pair_mixed_kernel(const __grid_constant__ MixArgs a, const __grid_constant__ MixSite m,
                           const __grid_constant__ Cell cell)
 {
+    unsigned long long *stamp = (unsigned long long *)(a.acc + (size_t)P * S_NSLOT);
+    stamp_start(stamp, T_PAIR0);
     mol_pair_mixed_body<P, NS, ENERGY, CM, VM>(a, m, cell, hw_blk());
+    stamp_end(stamp, T_PAIR1);
 }
 
 // ---------------------------------------------------------------------------

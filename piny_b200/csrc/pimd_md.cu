@@ -538,10 +538,7 @@ int pimd_finish(pinyb200_pimd *pm, pinyb200_ctx *c, const pinyb200::Cell &cell, 
 {
     PCK(cudaStreamSynchronize(st));
     if (!pm->graph_mode && pm->timed) {  // a replayed graph (or a RESPA step) records no phase events
-        cudaEventElapsedTime(&c->last_ms[0], c->ev[0], c->ev[4]);
-        cudaEventElapsedTime(&c->last_ms[1], c->ev[1], c->ev[2]);
-        cudaEventElapsedTime(&c->last_ms[2], c->ev_pme[0], c->ev_pme[1]);
-        cudaEventElapsedTime(&c->last_ms[3], c->ev[5], c->ev[3]);
+        pinyb200::read_phase_times(c, pm->h_facc);
     }
     pinyb200_energies fe;
     pinyb200::evaluate_finish(c, cell, PINYB200_DISTRIB_GHOSTS, pm->h_facc, &fe);
@@ -732,7 +729,7 @@ int pinyb200_pimd_create(const pinyb200_pimd_setup *s, pinyb200_pimd **out)
     CCK(cudaMalloc(&pm->d_acc, sizeof(double) * A_N));
     if (pm->nres[0] * pm->nres[1] * pm->nres[2] * pm->nres[3] > 1) CCK(cudaMalloc(&pm->d_ft, sizeof(double) * nb * 3));
     CCK(cudaMallocHost(&pm->h_acc, sizeof(double) * A_N));
-    CCK(cudaMallocHost(&pm->h_facc, sizeof(double) * (size_t)s->nbeads * pinyb200::S_NSLOT));
+    CCK(cudaMallocHost(&pm->h_facc, sizeof(double) * ((size_t)s->nbeads * pinyb200::S_NSLOT + pinyb200::T_NSTAMP)));
     CCK(cudaMemcpy(pm->d_mass, s->mass, sizeof(double) * na, cudaMemcpyHostToDevice));
     CCK(cudaMemcpy(pm->d_bmass, s->bead_mass, sizeof(double) * nb, cudaMemcpyHostToDevice));
     CCK(cudaMemcpy(pm->d_prekf, s->prekf, sizeof(double) * na, cudaMemcpyHostToDevice));

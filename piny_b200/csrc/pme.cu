@@ -612,6 +612,7 @@ template <int NI, int TT>
 __global__ void __launch_bounds__(256, 2) spread_own_kernel(const __grid_constant__ PmeArgs a,
                                                             const __grid_constant__ TileArgs t)
 {
+    stamp_start(a.stamp, T_PME0);
     typedef TileGeom<NI, TT> TG;
     constexpr int NIP = RecGeom<NI>::NIP, NTB = (NI + 3) / 4, NS8 = (NI + 7) / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -715,6 +716,7 @@ template <typename R, int NI, int TT>
 __global__ void __launch_bounds__(256) spread_tile_c_kernel(const __grid_constant__ PmeArgs a,
                                                             const __grid_constant__ TileArgs t)
 {
+    stamp_start(a.stamp, T_PME0);
     spread_tile_c_body<R, NI, TT>(a, t, hw_blk());
 }
 
@@ -870,6 +872,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 && NI <= 8 ? PINYB200_GATH
                                                             const __grid_constant__ TileArgs t)
 {
     gather_tile_c_body<R, NI, TT>(a, cell, t, hw_blk());
+    stamp_end(a.stamp, T_PME1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1322,6 +1325,7 @@ PmeArgs pme_args_of(pinyb200_ctx *c)
     a.forceP = c->d_forceP;
     a.rhead = (int4 *)c->d_pme_head;
     a.rw = c->d_pme_w;
+    a.stamp = (unsigned long long *)(c->d_acc + (size_t)c->P * S_NSLOT);
     return a;
 }
 

@@ -15,6 +15,7 @@ struct PmeArgs {
     double *forceP;  // PME forces [nchrg][3][P]
     int4 *rhead;  // per (charge, bead) records, see RecGeom
     void *rw;
+    unsigned long long *stamp;
 };
 
 // Scaled coordinate of one charge along one axis, wrapped to (0,1] and

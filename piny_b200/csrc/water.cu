@@ -4,11 +4,13 @@
 namespace pinyb200 {
 
 // The per-bead sums and the bin counters to zero.
+// acc: the bead sums and the time stamps behind them, nacc in all.
 __global__ void __launch_bounds__(256) water_clear_kernel(double *__restrict__ acc, int nacc, int *__restrict__ cnt,
                                                           int ncnt)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
-    for (int i = t; i < nacc; i += n) acc[i] = 0.0;
+    for (int i = t; i < nacc; i += n)
+        acc[i] = i == nacc - T_NSTAMP + T_BEG ? __longlong_as_double((long long)clock_ns()) : 0.0;
     for (int i = t; i < ncnt; i += n) cnt[i] = 0;
 }
 
@@ -24,7 +26,10 @@ __global__ void __launch_bounds__(256) water_stage_kernel(const __grid_constant_
 template <int NS, bool Q0>
 __global__ void __launch_bounds__(256, 2) water_finish_kernel(const __grid_constant__ FinishArgs a)
 {
+    unsigned long long *stamp = (unsigned long long *)(a.acc + (size_t)a.P * S_NSLOT);
+    stamp_start(stamp, T_FIN0);
     water_finish_body<NS, Q0>(a, hw_blk());
+    stamp_end(stamp, T_END);
 }
 
 // Threads per block: 256, fewer (down to 64, and a bead each) while that
@@ -117,7 +122,7 @@ cudaError_t launch_water_stage(pinyb200_ctx *c, const Cell &cell, const double *
         t = tile_args_of(c, c->sys.n_interp, c->pme_tile);
         ncnt = c->P * c->pme_ntile + 1;
     }
-    const int nacc = c->P * S_NSLOT;
+    const int nacc = c->P * S_NSLOT + T_NSTAMP;
     const int blocks = std::max(1, std::min((std::max(ncnt, nacc) + 255) / 256, c->sm_count));
     water_clear_kernel<<<blocks, 256, 0, c->stream>>>(c->d_acc, nacc, t.cnt, ncnt);
     if (c->precision == PINYB200_FP64) return launch_stage_r<double>(c, a, pm, t, cell);
