@@ -1285,7 +1285,7 @@ def main():
     kernels = kernel_profile(box, lambda: step(box, d_force), S, P, args.precision, npairs,
                              linfo.get("nmol_pairs", 0), flush, stream)
     # roofline of the dominant kernel by serialised time; its duration is
-    # the one measured inside the timed steps (pair phase events / PME phase)
+    # the one measured inside the timed steps (pair phase / PME phase)
     hbm, peak_kind = peaks()
     names = ["total", "pair", "pme", "intra"]
     dom_k = max(kernels, key=lambda k: k["ms"])
@@ -1313,8 +1313,8 @@ def main():
     roof = {"bound": "hbm", "kernel": dom_name, "achieved": achieved, "peak": hbm, "unit": "GB/s",
             "frac": achieved / hbm, "traffic": traffic, "peak_kind": peak_kind,
             "algorithmic_bytes_per_launch": alg_bytes, "bytes_model": unit_note,
-            "duration_ms": dom_ms, "duration_from": "pair-phase CUDA events of the timed steps (PME concurrent)"
-            if dom_name == "pair" else "PME-phase CUDA events of the timed steps",
+            "duration_ms": dom_ms, "duration_from": "pair phase of the timed steps (PME concurrent)"
+            if dom_name == "pair" else "PME phase of the timed steps",
             "phase_ms": {names[i]: float(phase[i]) for i in range(4)}}
 
     # against PINY itself: forces of the beads PINY's evaluation of this

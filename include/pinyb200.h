@@ -505,7 +505,8 @@ int pinyb200_grad(pinyb200_ctx *ctx, const double *d_pos, const double *d_xmod,
                   const double *hmat, const double *d_fbar, double *dE,
                   double *dF, void *stream);
 
-/* Milliseconds of the last evaluation, from CUDA events: 0 device work,
+/* Milliseconds of the last evaluation, from the kernels' time stamps (boxes of
+ * water molecules) or CUDA events (other systems): 0 device work,
  * 1 pair forces, 2 PME, 3 intramolecular, 4 the whole host-buffer call of
  * pinyb200_energy_force (copies included).  PME runs on a second stream of
  * the context, concurrently with 1 and 3, so 1 + 2 + 3 may exceed 0. */
