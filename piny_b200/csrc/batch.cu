@@ -6,9 +6,9 @@
 // out, energy sums to pinned host memory -- in one of two forms:
 //   multi-box kernels: each phase is one persistent launch per group of
 //     boxes that share its compile-time shape (boxtab.cuh); the groups'
-//     PME chains, pair launches and the intramolecular launch are parallel
-//     graph branches between the staging and the finishing launches -- a
-//     few dozen launches for any number of boxes;
+//     PME chains and pair launches are parallel graph branches between the
+//     staging and the finishing launches -- a few dozen launches for any
+//     number of boxes;
 //   branches: every box's own kernels as a parallel branch forked from and
 //     joined to one stream (for boxes the multi-box kernels do not cover).
 // The first call (and any call whose device pointers, cells or flags differ
