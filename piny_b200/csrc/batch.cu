@@ -514,6 +514,8 @@ int pinyb200_batch_energy_force_device(pinyb200_batch *bt, const double *const *
         bt->key_h = kh;
         bt->key_flags = flags;
     }
+    // a box may have been evaluated at another cell since the last call
+    for (int i = 0; i < nbox; i++) BCK(pme_filters_ready(bt->box[i], cell_from_hmat(hmat[i]), st));
     BCK(cudaEventRecord(bt->ev[0], st));
     BCK(cudaGraphLaunch(bt->exec, st));
     BCK(cudaEventRecord(bt->ev[1], st));

@@ -1186,10 +1186,13 @@ int pinyb200::stage_positions(pinyb200_ctx *c, const double *d_pos, const double
 // from the host: the first call with a key runs the work plainly (it sets
 // kernel attributes and builds the influence function outside any
 // capture), the second captures and launches it, later ones launch it.
-// Per-kernel timing runs plainly.
-static int run_eval_graph(pinyb200_ctx *c, const std::vector<double> &key, const std::function<int()> &body)
+// Per-kernel timing runs plainly.  The influence function is brought to the
+// call's cell first: another call may have used another cell since the capture.
+static int run_eval_graph(pinyb200_ctx *c, const Cell &cell, const std::vector<double> &key,
+                          const std::function<int()> &body)
 {
     if (c->kt_on || c->no_graph) return body();
+    CK(pme_filters_ready(c, cell, c->stream));
     if (c->eg_exec && key == c->eg_key) {
         CK(cudaGraphLaunch(c->eg_exec, c->stream));
         return PINYB200_OK;
@@ -1250,7 +1253,7 @@ int pinyb200_energy_force_device(pinyb200_ctx *c, const double *d_pos, const dou
     const bool energy = !(flags & PINYB200_NO_ENERGY);
     if (!c->h_acc_pin) CK(cudaMallocHost(&c->h_acc_pin, ((size_t)c->P * S_NSLOT + T_NSTAMP) * sizeof(double)));
     double *acc = c->h_acc_pin;  // pinned: the copy can sit in the graph
-    int rc = run_eval_graph(c, eval_key(c, 1, d_pos, d_xmod, d_force, hmat, flags),
+    int rc = run_eval_graph(c, cell, eval_key(c, 1, d_pos, d_xmod, d_force, hmat, flags),
                             [&]() { return enqueue_device(c, d_pos, d_xmod, cell, flags, d_force, true, acc); });
     if (rc) return rc;
     CK(cudaStreamSynchronize(c->stream));
@@ -1279,7 +1282,8 @@ int pinyb200_energy_force(pinyb200_ctx *c, const double *pos, const double *xmod
     const bool energy = !(flags & PINYB200_NO_ENERGY);
     if (!c->h_acc_pin) CK(cudaMallocHost(&c->h_acc_pin, ((size_t)c->P * S_NSLOT + T_NSTAMP) * sizeof(double)));
     double *acc = c->h_acc_pin;  // pinned: the copy is queued, not waited for
-    int rc = run_eval_graph(c, eval_key(c, 2, c->d_pos_aos, xmod ? c->d_xmod : nullptr, c->d_force_aos, hmat, flags),
+    int rc = run_eval_graph(c, cell,
+                            eval_key(c, 2, c->d_pos_aos, xmod ? c->d_xmod : nullptr, c->d_force_aos, hmat, flags),
                             [&]() {
                                 if (c->water_ok) {
                                     c->kt_n = 0;

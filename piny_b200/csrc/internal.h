@@ -348,6 +348,11 @@ cudaError_t launch_site_from_mol(pinyb200_ctx *c, int pass, const int *gate = nu
 // staged: the grid is already zero and the charges are binned
 cudaError_t launch_pme(pinyb200_ctx *c, const Cell &cell, bool energy, bool staged = false);
 cudaError_t launch_pme_clear(pinyb200_ctx *c);
+// The influence functions of the evaluation's mesh (and the RESPA mesh) for
+// this cell, built on st where the last call's cell was another one.  A context
+// has one of each, so a captured graph holds none of their kernels, and every
+// capture and replay is preceded by this.
+cudaError_t pme_filters_ready(pinyb200_ctx *c, const Cell &cell, cudaStream_t st);
 // water molecules (pinyb200_ctx::water_ok): staging and finishing kernels
 cudaError_t launch_water_stage(pinyb200_ctx *c, const Cell &cell, const double *d_pos, const double *d_xmod);
 cudaError_t launch_water_finish(pinyb200_ctx *c, double *d_out, bool energy, bool distrib, bool keep_site_forces);

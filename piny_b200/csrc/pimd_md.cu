@@ -838,6 +838,8 @@ int pinyb200_pimd_step(pinyb200_pimd *pm, pinyb200_ctx *c, double *d_x, double *
         pm->graph_mode = false;
         return pimd_finish(pm, c, cell, e, st);
     }
+    // the force context may have been used at another cell since the last step
+    PCK(pinyb200::pme_filters_ready(c, cell, st));
     if (!pm->exec) {
         if (!pm->cap) PCK(cudaStreamCreateWithFlags(&pm->cap, cudaStreamNonBlocking));
         PCK(cudaStreamBeginCapture(pm->cap, cudaStreamCaptureModeRelaxed));

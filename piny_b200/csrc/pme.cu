@@ -1489,19 +1489,39 @@ cudaError_t launch_pme_force_add_scaled(pinyb200_ctx *c, double w, double *targe
     return cudaGetLastError();
 }
 
+// The influence function of the context's mesh for this cell, on st, unless
+// it is the one already there.
+static cudaError_t launch_filter(pinyb200_ctx *c, const Cell &cell, cudaStream_t st)
+{
+    bool same = c->filter_ok;
+    for (int i = 0; i < 9 && same; i++) same = c->filter_h[i] == cell.h[i];
+    if (same) return cudaSuccess;
+    const size_t G = (size_t)c->sys.ngrid[0] * c->sys.ngrid[1] * c->sys.ngrid[2];
+    filter_kernel<<<(unsigned)((G + 255) / 256), 256, 0, st>>>(
+        c->sys.ngrid[0], c->sys.ngrid[1], c->sys.ngrid[2], c->sys.kmask, c->sys.kvec, c->sys.bweight, cell,
+        c->alp_ewd, (double *)c->d_filter, (float *)((double *)c->d_filter + G));
+    for (int i = 0; i < 9; i++) c->filter_h[i] = cell.h[i];
+    c->filter_ok = true;
+    return cudaGetLastError();
+}
+
+cudaError_t pme_filters_ready(pinyb200_ctx *c, const Cell &cell, cudaStream_t st)
+{
+    if (c->sys.nchrg == 0) return cudaSuccess;
+    cudaError_t e = c->sys.nktot > 0 ? launch_filter(c, cell, st) : cudaSuccess;
+    if (e == cudaSuccess && c->pme_res.on) {
+        pme_swap(c, c->pme_res);
+        e = launch_filter(c, cell, st);
+        pme_swap(c, c->pme_res);
+    }
+    return e;
+}
+
 cudaError_t launch_pme(pinyb200_ctx *c, const Cell &cell, bool energy, bool staged)
 {
     if (c->sys.nchrg == 0 || c->sys.nktot == 0) return cudaSuccess;
-    const size_t G = (size_t)c->sys.ngrid[0] * c->sys.ngrid[1] * c->sys.ngrid[2];
-    bool same = c->filter_ok;
-    for (int i = 0; i < 9 && same; i++) same = c->filter_h[i] == cell.h[i];
-    if (!same) {
-        filter_kernel<<<(unsigned)((G + 255) / 256), 256, 0, c->stream>>>(
-            c->sys.ngrid[0], c->sys.ngrid[1], c->sys.ngrid[2], c->sys.kmask, c->sys.kvec, c->sys.bweight, cell,
-            c->alp_ewd, (double *)c->d_filter, (float *)((double *)c->d_filter + G));
-        for (int i = 0; i < 9; i++) c->filter_h[i] = cell.h[i];
-        c->filter_ok = true;
-    }
+    const cudaError_t err = launch_filter(c, cell, c->stream);
+    if (err != cudaSuccess) return err;
     if (c->precision == PINYB200_FP64) return launch_pme_r<double>(c, cell, energy, staged);
     return launch_pme_r<float>(c, cell, energy, staged);
 }
@@ -1659,16 +1679,8 @@ cudaError_t launch_pme_batch(const std::vector<pinyb200_ctx *> &box, const std::
         if (c->precision != PINYB200_MIXED) return cudaErrorInvalidValue;
         const Cell &cell = cells[i];
         const size_t G = (size_t)c->sys.ngrid[0] * c->sys.ngrid[1] * c->sys.ngrid[2];
-        bool same = c->filter_ok;
-        for (int k = 0; k < 9 && same; k++) same = c->filter_h[k] == cell.h[k];
-        if (!same) {
-            // the influence function of this cell (normally built by the plain run before capture)
-            filter_kernel<<<(unsigned)((G + 255) / 256), 256, 0, st>>>(
-                c->sys.ngrid[0], c->sys.ngrid[1], c->sys.ngrid[2], c->sys.kmask, c->sys.kvec, c->sys.bweight, cell,
-                c->alp_ewd, (double *)c->d_filter, (float *)((double *)c->d_filter + G));
-            for (int k = 0; k < 9; k++) c->filter_h[k] = cell.h[k];
-            c->filter_ok = true;
-        }
+        const cudaError_t ef = launch_filter(c, cell, st);
+        if (ef != cudaSuccess) return ef;
         PmeBox pb;
         pb.a = pme_args_of(c);
         pb.t = tile_args_of(c, c->sys.n_interp, c->pme_tile);
