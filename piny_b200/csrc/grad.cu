@@ -502,7 +502,7 @@ cudaError_t launch_grad_terms(pinyb200_ctx *c, const Cell &cell, const GradArgs 
             sel.tt[t] = sel.kt[t] >= 0 ? g.ch[sel.kt[t]].ttab : nullptr;
             sel.tmask[t] = sel.kt[t] >= 0 ? c->grad.tmask[sel.kt[t]] : 0u;
         }
-        if (mol_grad_ok(c, cell)) {
+        if (mol_grad_ok(c, cell, sel)) {
             cudaError_t e = launch_mol_pair_grad(c, cell, sel, g.uT, g.gacc);
             if (e != cudaSuccess) return e;
         } else if (c->precision == PINYB200_FP64)

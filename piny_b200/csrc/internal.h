@@ -144,8 +144,9 @@ struct GradPairSel {
     const void *tt[2];
     unsigned tmask[2];  // tables with a non-zero tangent (bit u, u < 32)
 };
-// Whether the molecule-pair form of the pair adjoint serves the context, and that pass.
-bool mol_grad_ok(const pinyb200_ctx *c, const Cell &cell);
+// Whether the molecule-pair form of the pair adjoint serves the context and
+// these channels, and that pass.
+bool mol_grad_ok(const pinyb200_ctx *c, const Cell &cell, const GradPairSel &sel);
 cudaError_t launch_mol_pair_grad(pinyb200_ctx *c, const Cell &cell, const GradPairSel &sel, const double *uT,
                                  double *gacc);
 cudaError_t launch_pme_adjoint(pinyb200_ctx *c, const Cell &cell, const GradArgs &g);

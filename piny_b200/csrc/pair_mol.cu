@@ -2271,9 +2271,20 @@ cudaError_t launch_mol_pair_mixed(pinyb200_ctx *c, const Cell &cell, bool energy
 }
 
 // The molecule-pair adjoint serves MIXED boxes of the two water patterns in
-// orthorhombic cells whose moving sites are the M sites (water_ok).
-bool mol_grad_ok(const pinyb200_ctx *c, const Cell &cell)
+// orthorhombic cells whose moving sites are the M sites (water_ok), and table
+// tangents that vanish outside the tables of the site pairs with a vdW term:
+// it reads no others (a tangent on the table of, say, H-H is the slope along a
+// term not in the model yet).  The site-list kernel takes any (GradPairSel
+// knows the first 32 tables' tangents).
+bool mol_grad_ok(const pinyb200_ctx *c, const Cell &cell, const GradPairSel &sel)
 {
+    unsigned tables = 0;
+    for (int sp = 0; sp < 16; sp++) {
+        const int u = (c->mix_toff[sp] - 2) / c->sys.nsplin;
+        if ((c->mix_eflag[sp] & 1) && u < 32) tables |= 1u << u;
+    }
+    for (int t = 0; t < 2; t++)
+        if (sel.kt[t] >= 0 && (c->sys.nuniq > 32 || (sel.tmask[t] & ~tables))) return false;
     const bool ortho = cell.h[1] == 0.0 && cell.h[2] == 0.0 && cell.h[3] == 0.0 && cell.h[5] == 0.0 &&
                        cell.h[6] == 0.0 && cell.h[7] == 0.0;
     return c->precision == PINYB200_MIXED && c->use_mol && c->mol_ok && c->mix_ok && c->water_ok && ortho &&

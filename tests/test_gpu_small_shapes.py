@@ -192,3 +192,53 @@ def test_fp64_pairs_by_chunk_queue(oracle, nmol, beads):
     fref, eref = _oracle(oracle, S, pos, xmod)
     f, e = _device(S, pos, xmod, "fp64", tuning={2: 1})
     _check("fp64", f, e, fref, eref)
+
+
+@pytest.mark.parametrize("model, nmol, beads", [(water.SPC_FW, 65, 1), (water.SPC_FW, 64, 16), (water.TIP4P_F, 65, 1),
+                                                (water.TIP4P_F, 64, 16)])
+def test_gradient_of_tables_without_a_term(oracle, model, nmol, beads):
+    """A table tangent on the table that is zero in the model (the slope along a
+    term not there yet), alone and together with one on the O-O table: the same
+    derivatives in MIXED and FP64, and where every site pair is charged, so that
+    every one of them is listed, the oracle's difference quotient (energy and
+    forces are linear in the tables)."""
+    import torch
+
+    from piny_b200.lib import DeviceBox
+    spec, S, pos, xmod = _box(model, nmol, beads, 20, 6)
+    ns, nu = int(S["nsplin"]), int(S["ninter_unique"])
+    null = [u for u in range(nu) if not np.any(np.asarray(S["cv0"])[u * ns:(u + 1) * ns])]
+    assert len(null) == 1 and nu == 2
+    r = float(S["rmin_spl"][0]) + float(S["dr_spl"][0]) * np.arange(-2, ns - 2)
+    v, dv = np.exp(-0.3 * r), 0.3 * np.exp(-0.3 * r) / r
+
+    def on(tables):
+        return {"dcv0": np.concatenate([v if u in tables else 0 * v for u in range(nu)]),
+                "dcdv0": np.concatenate([dv if u in tables else 0 * v for u in range(nu)])}
+
+    tan = [on(null), on([0, 1]), on([1 - null[0]])]
+    d, x = torch.from_numpy(pos).cuda(), None if xmod is None else torch.from_numpy(xmod).cuda()
+    fbar = np.random.default_rng(3).normal(size=pos.shape)
+    dfbar = torch.from_numpy(fbar).cuda()
+    out = {}
+    for precision in ("fp64", "mixed"):
+        box = DeviceBox(S, beads, precision)
+        box.build_list(pos[0], xmod, S["hmat"], S["cutskin2"])
+        box.grad_prepare(tan)
+        out[precision] = box.grad(d.data_ptr(), None if x is None else x.data_ptr(), S["hmat"], dfbar.data_ptr())
+        box.close()
+    for got, ref in zip(out["mixed"], out["fp64"]):
+        assert np.all(ref != 0.0)
+        assert np.all(np.abs(got - ref) <= 1e-5 * np.abs(ref))
+    if model is not water.SPC_FW:
+        return
+    pi, pj = oracle.verlist(S, pos[0], xmod, S["hmat"], S["cutskin2"])
+    f0, e0 = oracle.energy_force(S, pos, xmod, S["hmat"], pi, pj, distribute_ghosts=True)
+    for k, t in enumerate(tan):
+        T = dict(S, cv0=np.asarray(S["cv0"]) + t["dcv0"], cdv0=np.asarray(S["cdv0"]) + t["dcdv0"])
+        f1, e1 = oracle.energy_force(T, pos, xmod, S["hmat"], pi, pj, distribute_ghosts=True)
+        dE, dF = e1["vintert"] - e0["vintert"], float(((f1 - f0) * fbar).sum())
+        # both are differences of sums of this size, to 1e-13 of it
+        escale = abs(e0["vreal"]) + abs(e0["vself"]) + abs(dE)
+        assert abs(out["fp64"][0][k] - dE) <= 1e-12 * escale
+        assert abs(out["fp64"][1][k] - dF) <= 1e-12 * np.abs(f1 * fbar).sum()
