@@ -966,7 +966,9 @@ __device__ __forceinline__ bool site_pair(const typename Vec4<R>::T *__restrict_
 // (possible only when the site-0 separation is within twice the molecular
 // extent of half a box along some axis): bit si * NS + sj of up / dn along
 // axis d says that PINY's own shift of that site pair (period_pimd,
-// period.c:163-176) is one cell edge above / below the site-0 shift sh0.
+// period.c:163-176) is one cell edge above / below the site-0 shift sh0; none
+// is further off unless far_images.  Separations of these pairs are formed in
+// FP64 also by the MIXED kernels.
 // The G lanes of a pair share the work and then hold the same masks; every
 // lane of the group calls it.
 struct NearImages {
@@ -977,14 +979,29 @@ struct NearImages {
     }
 };
 
-// x + n h for n = -1, 0, 1 in FP32: h in two parts, so that the sum of a
-// separation near h and -h keeps the separation's own rounding.
-__device__ __forceinline__ float add_cells(float x, int n, double h)
+// Whether a site pair's image may be further than one cell from its site-0
+// pair's: molecules that reach over half a box, as where a program wraps atoms
+// into the cell one by one.  Their shifts are taken site pair by site pair.
+__device__ __forceinline__ bool far_images(double ext2, const Cell &cell)
 {
-    const float hh = (float)h, hl = (float)(h - (double)hh);
-    return n == 0 ? x : (n > 0 ? (x + hh) + hl : (x - hh) - hl);
+    return ext2 * fmax(cell.hi[0], fmax(cell.hi[4], cell.hi[8])) > 0.99;
 }
-__device__ __forceinline__ double add_cells(double x, int n, double h) { return x + (double)n * h; }
+
+// PINY's shift of one site pair along axis d.
+__device__ __forceinline__ double site_shift(const double *__restrict__ xmod, int i, int j, int d, const Cell &cell)
+{
+    return shift_exact(__dsub_rn(__ldg(xmod + 3 * (size_t)i + d), __ldg(xmod + 3 * (size_t)j + d)), cell.hi[4 * d]);
+}
+
+// Separation of sites i and j of one bead at image shift sh (cells), in FP64
+// with PINY's operation order (period.c:163-176).
+template <int P>
+__device__ __forceinline__ double image_sep(const double *__restrict__ posT, int i, int j, int d, int b, double sh,
+                                            double h)
+{
+    return __dadd_rn(__dsub_rn(posT[(3 * (size_t)i + d) * P + b], __ldcg(posT + (3 * (size_t)j + d) * P + b)),
+                     __dmul_rn(sh, h));
+}
 
 template <int NS, int G>
 __device__ __forceinline__ NearImages near_images(const double *__restrict__ xmod, int i0, int j0, int ni,
@@ -1054,9 +1071,41 @@ __device__ __forceinline__ void pair_energy_flush(const double (*sacc)[BT], doub
     }
 }
 
+// One molecule pair under far_images: forces straight to the force array,
+// energies and virial to the thread's sums.  Out of line: a third copy of the
+// main loop costs the FP64 kernel 6 % in spills.
+template <typename R, int P, int NS, bool FAST, bool ENERGY>
+__device__ __noinline__ void mol_pair_far(const double *__restrict__ posT, const double *__restrict__ xmod,
+                                          double *__restrict__ forceT, const PairConst<R> *pc,
+                                          const typename Vec4<R>::T *__restrict__ tab, size_t tstride, int nsm2,
+                                          int i0, int j0, unsigned mask, int b, const Cell &cell, double *sacc)
+{
+    R evs = 0, ecs = 0, pvs[6] = {0, 0, 0, 0, 0, 0};
+    for (unsigned m = mask; m; m &= m - 1u) {
+        const int sp = __ffs(m) - 1, i = i0 + sp / NS, j = j0 + sp % NS;
+        R r[3], f[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            r[d] = (R)image_sep<P>(posT, i, j, d, b, site_shift(xmod, i, j, d, cell), cell.h[4 * d]);
+        if (site_pair<R, FAST, ENERGY, false>(tab, tstride, nsm2, *pc, sp, r[0], r[1], r[2], f[0], f[1], f[2], evs, ecs,
+                                              pvs))
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                atomicAdd(&forceT[(3 * (size_t)i + d) * P + b], (double)f[d]);
+                atomicAdd(&forceT[(3 * (size_t)j + d) * P + b], -(double)f[d]);
+            }
+    }
+    if (ENERGY) {
+        sacc[0] += (double)evs;
+        sacc[128] += (double)ecs;
+#pragma unroll
+        for (int c = 0; c < 6; c++) sacc[128 * (2 + c)] += (double)pvs[c];
+    }
+}
+
 template <typename R, int P, int NS, bool ENERGY>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : PINYB200_MOL_BLOCKS64)
-    mol_pair_kernel(MolArgs a, Cell cell)
+    mol_pair_kernel(const __grid_constant__ MolArgs a, const __grid_constant__ Cell cell)
 {
     unsigned long long *stamp = (unsigned long long *)(a.acc + (size_t)P * S_NSLOT);
     stamp_start(stamp, T_PAIR0);
@@ -1209,15 +1258,15 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
                         if (!((col >> si) & 1u)) continue;
                         // away from half a box every site pair takes the site-0 image
                         R rx, ry, rz;
-                        if (FAST) {
+                        if (FAST && NEAR) {
+                            const int sp = si * NS + sj;
+                            rx = (R)image_sep<P>(posT, i0 + si, j0 + sj, 0, b, sh0[0] + nim.shift(0, sp), cell.h[0]);
+                            ry = (R)image_sep<P>(posT, i0 + si, j0 + sj, 1, b, sh0[1] + nim.shift(1, sp), cell.h[4]);
+                            rz = (R)image_sep<P>(posT, i0 + si, j0 + sj, 2, b, sh0[2] + nim.shift(2, sp), cell.h[8]);
+                        } else if (FAST) {
                             rx = djx + ei[si][0];
                             ry = djy + ei[si][1];
                             rz = djz + ei[si][2];
-                            if constexpr (NEAR) {
-                                rx = add_cells(rx, nim.shift(0, si * NS + sj), cell.h[0]);
-                                ry = add_cells(ry, nim.shift(1, si * NS + sj), cell.h[4]);
-                                rz = add_cells(rz, nim.shift(2, si * NS + sj), cell.h[8]);
-                            }
                         } else {
                             double sx = sh0[0], sy = sh0[1], sz = sh0[2];
                             if constexpr (NEAR) {
@@ -1248,8 +1297,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
                     }
                 }
             };
-            if (near) site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, ni, sh0, cell, lane));
-            else site_pairs(std::false_type{}, NearImages{{0u, 0u, 0u}});
+            if (!near)
+                site_pairs(std::false_type{}, NearImages{{0u, 0u, 0u}});
+            else if (!far_images(ext2, cell))
+                site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, ni, sh0, cell, lane));
+            else
+                mol_pair_far<R, P, NS, FAST, ENERGY>(posT, a.xmod, a.forceT, &pc, tab, tstride, nsm2, i0, j0, mask, b,
+                                                     cell, &sacc[0][threadIdx.x]);
         }
         // i-site forces: sum the lane groups that hold the same bead
 #pragma unroll
@@ -1295,7 +1349,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
 //   * molecules are uniform runs of sites: the j site index is mj * stride,
 //     not a load.
 // Pairs whose site-0 separation is within twice the molecular extent of half
-// a box add each site pair's own image (near_images), as in mol_pair_kernel.
+// a box take each site pair's own image (mixed_near), as in mol_pair_kernel.
 
 // Table row load that asks L1 to keep the line (evict_last): the four
 // tables a water system reads stay resident while positions stream past.
@@ -1343,8 +1397,9 @@ struct MixSite {
 };
 
 // Resident blocks per SM of the MIXED molecule-pair kernel: 5 x 128
-// threads leave it 96 registers and no spills (at 6, 85 registers spilled
-// ~180 bytes per thread into L1, the cache its table gathers depend on).
+// threads leave it 96 registers and no spills for the two water patterns (at
+// 6, 85 registers spilled ~180 bytes per thread into L1, the cache its table
+// gathers depend on).
 #ifndef PINYB200_MIX_BLOCKS
 #define PINYB200_MIX_BLOCKS 5
 #endif
@@ -1355,6 +1410,90 @@ struct MixSite {
 constexpr unsigned kAnyPair = 0xffffffffu;
 constexpr unsigned kTip4pCoul = 0xEEE0u, kTip4pVdw = 0x1u;  // O H H M: H, M charged; LJ on O-O
 constexpr unsigned kSpcCoul = 0x1FFu, kSpcVdw = 0x1u;       // O H H: all charged; LJ on O-O
+
+// One molecule pair near half a box for the MIXED kernel: forces on the i sites
+// and energies into the chunk's sums, j forces to the force array.  Separations
+// and images in FP64, rounded once (sums of FP32 offsets and cell edges round
+// each of them), far images site pair by site pair.  The j sites are a loop, so
+// that the main loop keeps its registers.  Pair phase against a second unrolled
+// copy of the main loop with FP32 cell edges: 75 -> 62 us (256 SPC/Fw x 32),
+// 57 -> 44 (216 TIP4P/F x 32), 366 -> 369 (4096 TIP4P/F x 32, no such pairs).
+template <int P, int NS, bool ENERGY>
+__device__ __forceinline__ void mixed_near(const MixArgs &a, const MixSite &m, const Cell &cell, int i0, int j0,
+                                           unsigned mask, int b, int lane, bool far, const double *sh0,
+                                           const float (&ei)[NS][3], float (&fi)[NS][3], float &evs, float &ecs,
+                                           float (&pvs)[6])
+{
+    constexpr int G = P >= 32 ? 32 : P;
+    NearImages nim = {{0u, 0u, 0u}};
+    if (!far) nim = near_images<NS, G>(a.xmod, i0, j0, m.stride, sh0, cell, lane);
+#pragma unroll 1
+    for (int sj = 0; sj < NS; sj++) {
+        float fj[3] = {0, 0, 0};
+        double xj[3];
+        const int j = j0 + (sj < m.stride ? sj : 0);
+#pragma unroll
+        for (int d = 0; d < 3; d++) xj[d] = __ldcg(a.posT + (3 * (size_t)j + d) * P + b);
+#pragma unroll
+        for (int si = 0; si < NS; si++) {
+            const int sp = si * NS + sj;
+            if (!((mask >> sp) & 1u)) continue;
+            float r[3];
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const double sh = far ? site_shift(a.xmod, i0 + si, j, d, cell) : sh0[d] + nim.shift(d, sp);
+                r[d] = (float)__dadd_rn(__dsub_rn(a.posT[(3 * (size_t)(i0 + si) + d) * P + b], xj[d]),
+                                        __dmul_rn(sh, cell.h[4 * d]));
+            }
+            const float r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+            if (!(r2 < m.rc2)) continue;
+            const float t = fminf(fmaxf(fmaf(r2 * rsqrtf(r2), m.dri_f, -m.rmd), 0.0f), m.tmax);
+            const int kn = __float2int_rn(t);
+            const float del = t - (float)kn;
+            const float4 *row = a.tab + (m.toff[sp] + kn), *rfe = a.tabfe + 2 * (m.toff[sp] + kn);
+            float dv = 0.0f;
+            if (m.eflag[sp] & 2) {
+                float4 cf, ef;
+                if (ENERGY) {
+                    ldg_keep_pair(rfe + 2 * m.tstride, cf, ef);
+                    ecs += m.q2[sp] * spline_eval<float4, float>(ef, del);
+                } else {
+                    cf = ldg_keep(row + T_CDV0C * m.tstride);
+                }
+                dv = m.q2[sp] * spline_eval<float4, float>(cf, del);
+            }
+            if (m.eflag[sp] & 1) {
+                float4 cf, ef;
+                if (ENERGY) {
+                    ldg_keep_pair(rfe, cf, ef);
+                    evs += spline_eval<float4, float>(ef, del);
+                } else {
+                    cf = ldg_keep(row + T_CDV0 * m.tstride);
+                }
+                dv += spline_eval<float4, float>(cf, del);
+            }
+            float f[3], q[3];
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                f[d] = r[d] * dv;
+                fi[si][d] += f[d];
+                fj[d] -= f[d];
+                q[d] = r[d] - ei[si][d];  // the e_i (x) f_i part of the virial is added once per chunk
+            }
+            if (ENERGY) {
+                pvs[0] += q[0] * f[0];
+                pvs[1] += q[1] * f[1];
+                pvs[2] += q[2] * f[2];
+                pvs[3] += q[0] * f[1];
+                pvs[4] += q[0] * f[2];
+                pvs[5] += q[1] * f[2];
+            }
+        }
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            if (fj[d] != 0.0f) atomicAdd(&a.forceT[(3 * (size_t)j + d) * P + b], (double)fj[d]);
+    }
+}
 
 template <int P, int NS, bool ENERGY, unsigned CM, unsigned VM, int BT = 128, bool ST = false>
 __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixSite &m, const Cell &cell,
@@ -1449,6 +1588,11 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                 sh0[d] = -nint_rn(t);
                 near |= fabs(t + sh0[d]) > 0.5 - ext2 * hid;
             }
+            if (!COOP && __builtin_expect(near, 0)) {
+                mixed_near<P, NS, ENERGY>(a, m, cell, i0, j0, mask, b, lane, far_images(ext2, cell), sh0, ei, fi, evs,
+                                          ecs, pvs);
+                continue;
+            }
             unsigned jm = 1u;
 #pragma unroll
             for (int si = 0; si < NS; si++) jm |= (mask >> (si * NS)) & ((1u << NS) - 1u);
@@ -1483,10 +1627,10 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
 #pragma unroll
                 for (int o = 0; o < 3 * NS; o++) sf[o * P] = 0.0f;
             }
-            // the site pairs; NEAR adds each pair's own image, in a copy of the
-            // loop so that pairs away from half a box pay nothing for it
-            auto site_pairs = [&](auto near_tag, const NearImages &nim) {
-                constexpr bool NEAR = decltype(near_tag)::value;
+            if (COOP && near && act) {
+                mixed_near<P, NS, ENERGY>(a, m, cell, i0, j0, mask, b, lane, far_images(ext2, cell), sh0, ei, fi, evs,
+                                          ecs, pvs);
+            } else {
 #pragma unroll
                 for (int sj = 0; sj < NS; sj++) {
                     if (!((jm >> sj) & 1u)) continue;
@@ -1498,14 +1642,9 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                         const bool vdw = VM == kAnyPair ? (m.eflag[sp] & 1) != 0 : ((VM >> sp) & 1u) != 0;
                         if (CM != kAnyPair && !coul && !vdw) continue;  // a pair the masks never hold
                         if (!((mask >> sp) & 1u)) continue;
-                        float rx = dj[sj][0] + ei[si][0];
-                        float ry = dj[sj][1] + ei[si][1];
-                        float rz = dj[sj][2] + ei[si][2];
-                        if constexpr (NEAR) {
-                            rx = add_cells(rx, nim.shift(0, sp), cell.h[0]);
-                            ry = add_cells(ry, nim.shift(1, sp), cell.h[4]);
-                            rz = add_cells(rz, nim.shift(2, sp), cell.h[8]);
-                        }
+                        const float rx = dj[sj][0] + ei[si][0];
+                        const float ry = dj[sj][1] + ei[si][1];
+                        const float rz = dj[sj][2] + ei[si][2];
                         const float r2 = rx * rx + ry * ry + rz * rz;
                         if (r2 < rc2) {
                             const float r = r2 * rsqrtf(r2);
@@ -1547,18 +1686,6 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                             fjx -= fx;
                             fjy -= fy;
                             fjz -= fz;
-                            if (ENERGY && NEAR) {
-                                // the cell edges in r = dj + e_i + n h: their part of the virial
-                                const float cx = (float)nim.shift(0, sp) * (float)cell.h[0],
-                                            cy = (float)nim.shift(1, sp) * (float)cell.h[4],
-                                            cz = (float)nim.shift(2, sp) * (float)cell.h[8];
-                                pvs[0] += cx * fx;
-                                pvs[1] += cy * fy;
-                                pvs[2] += cz * fz;
-                                pvs[3] += cx * fy;
-                                pvs[4] += cx * fz;
-                                pvs[5] += cy * fz;
-                            }
                             if (ENERGY) {
                                 if (vdw) evs += evf.x + del * (evf.y + del * (evf.z + del * evf.w));
                                 if (coul) ecs += m.q2[sp] * (ecf.x + del * (ecf.y + del * (ecf.z + del * ecf.w)));
@@ -1586,9 +1713,7 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                         atomicAdd(&a.forceT[(3 * (size_t)j + 2) * P + b], (double)fjz);
                     }
                 }
-            };
-            if (near && act) site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, ni, sh0, cell, lane));
-            else site_pairs(std::false_type{}, NearImages{{0u, 0u, 0u}});
+            }
             if constexpr (COOP) {
                 __syncwarp();
                 for (int e = lane; e < 32 * 3 * NS; e += 32) {
@@ -1642,7 +1767,8 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
 constexpr int kMixShared = 640;
 template <int P, int NS, bool ENERGY, unsigned CM, unsigned VM>
 __global__ void __launch_bounds__(kMixShared, 1)
-    mol_pair_mixed_shared_kernel(const __grid_constant__ MixArgs a, const __grid_constant__ MixSite m, Cell cell)
+    mol_pair_mixed_shared_kernel(const __grid_constant__ MixArgs a, const __grid_constant__ MixSite m,
+                                 const __grid_constant__ Cell cell)
 {
     unsigned long long *stamp = (unsigned long long *)(a.acc + (size_t)P * S_NSLOT);
     stamp_start(stamp, T_PAIR0);
@@ -1670,6 +1796,67 @@ __global__ void __launch_bounds__(128, PINYB200_MIX_BLOCKS)
 }
 
 // ---------------------------------------------------------------------------
+// One molecule pair of mol_pair_grad_kernel near half a box, as mixed_near: its
+// seven sums.
+template <int P, int NS>
+__device__ __forceinline__ void grad_near(const MixArgs &a, const MixSite &m, const Cell &cell, const GradPairSel &c,
+                                          const float4 &qs, const double *__restrict__ uT, int i0, int j0,
+                                          unsigned mask, int b, int lane, bool far, const double *sh0, double (&sum)[7])
+{
+    constexpr int G = P >= 32 ? 32 : P;
+    const float *q = &qs.x;
+    NearImages nim = {{0u, 0u, 0u}};
+    if (!far) nim = near_images<NS, G>(a.xmod, i0, j0, NS, sh0, cell, lane);
+#pragma unroll 1
+    for (unsigned rem = mask; rem; rem &= rem - 1u) {
+        const int sp = __ffs(rem) - 1, si = sp / NS, sj = sp % NS, i = i0 + si, j = j0 + sj;
+        float r[3], u[3], w[3] = {0, 0, 0};
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const size_t oi = (3 * (size_t)i + d) * P + b, oj = (3 * (size_t)j + d) * P + b;
+            const double sh = far ? site_shift(a.xmod, i, j, d, cell) : sh0[d] + nim.shift(d, sp);
+            r[d] = (float)image_sep<P>(a.posT, i, j, d, b, sh, cell.h[4 * d]);
+            u[d] = (float)(uT[oi] - uT[oj]);
+            if (c.w) w[d] = (float)(c.w[oi] - c.w[oj]);
+        }
+        const float r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+        if (!(r2 < m.rc2)) continue;
+        const float ri = rsqrtf(r2);
+        const float t = fminf(fmaxf(fmaf(r2 * ri, m.dri_f, -m.rmd), 0.0f), m.tmax);
+        const int kn = __float2int_rn(t);
+        const float del = t - (float)kn;
+        const float ur = u[0] * r[0] + u[1] * r[1] + u[2] * r[2];
+        const float4 *row = a.tab + (m.toff[sp] + kn);
+        float dv = 0.0f, dvp = 0.0f;
+        if (m.eflag[sp] & 2) {
+            const float4 cf = __ldg(row + T_CDV0C * m.tstride);
+            const float sc = spline_eval<float4, float>(cf, del);
+            if (c.dq) {
+                const float tq = (float)__ldg(c.dq + i) * q[sj] + q[si] * (float)__ldg(c.dq + j);
+                sum[0] += (double)(tq * spline_eval<float4, float>(__ldg(row + T_CV0C * m.tstride), del));
+                sum[3] += (double)(ur * (tq * sc));
+            }
+            dv = m.q2[sp] * sc;
+            dvp = m.q2[sp] * (cf.y + del * (2.0f * cf.z + 3.0f * del * cf.w)) * m.dri_f;
+        }
+        if (m.eflag[sp] & 1) {
+#pragma unroll
+            for (int n = 0; n < 2; n++)
+                if (c.tt[n]) {
+                    const float4 *tt = (const float4 *)c.tt[n] + m.toff[sp] + kn;
+                    sum[1 + n] += (double)spline_eval<float4, float>(__ldg(tt), del);
+                    sum[4 + n] += (double)(ur * spline_eval<float4, float>(__ldg(tt + m.tstride), del));
+                }
+            const float4 cv = __ldg(row + T_CDV0 * m.tstride);
+            dv += spline_eval<float4, float>(cv, del);
+            dvp += (cv.y + del * (2.0f * cv.z + 3.0f * del * cv.w)) * m.dri_f;
+        }
+        if (c.w)
+            sum[6] += (double)((u[0] * w[0] + u[1] * w[1] + u[2] * w[2]) * dv +
+                               ur * (r[0] * w[0] + r[1] * w[1] + r[2] * w[2]) * (dvp * ri));
+    }
+}
+
 // Pair adjoint of the parameter gradient (grad.cu) on the molecule-pair list:
 // chunks, lanes, images, cutoffs and tables as mol_pair_mixed_body.  Per site
 // pair with u = u_i - u_j and separation r (FP32):
@@ -1726,6 +1913,10 @@ __global__ void __launch_bounds__(128, 4)
                 sh0[d] = -nint_rn(t);
                 near |= fabs(t + sh0[d]) > 0.5 - ext2 * hid;
             }
+            if (__builtin_expect(near, 0)) {
+                grad_near<P, NS>(a, m, cell, c, qs, uT, i0, j0, mask, b, lane, far_images(ext2, cell), sh0, sum);
+                continue;
+            }
             float dj[NS][3], uj[NS][3], wj[3] = {0, 0, 0};
             {
                 double xj0[3];
@@ -1747,72 +1938,62 @@ __global__ void __launch_bounds__(128, 4)
                     for (int d = 0; d < 3; d++) wj[d] = (float)__ldcg(c.w + (3 * (size_t)(j0 + NS - 1) + d) * P + b);
             }
             float eq = 0, et[2] = {0, 0}, fq = 0, ft[2] = {0, 0}, fw = 0;
-            auto site_pairs = [&](auto near_tag, const NearImages &nim) {
-                constexpr bool NEAR = decltype(near_tag)::value;
 #pragma unroll
-                for (int sj = 0; sj < NS; sj++) {
+            for (int sj = 0; sj < NS; sj++) {
 #pragma unroll
-                    for (int si = 0; si < NS; si++) {
-                        const int sp = si * NS + sj;
-                        const bool coul = ((CM >> sp) & 1u) != 0, vdw = ((VM >> sp) & 1u) != 0;
-                        if (!coul && !vdw) continue;
-                        if (!((mask >> sp) & 1u)) continue;
-                        float rx = dj[sj][0] + ei[si][0], ry = dj[sj][1] + ei[si][1], rz = dj[sj][2] + ei[si][2];
-                        if constexpr (NEAR) {
-                            rx = add_cells(rx, nim.shift(0, sp), cell.h[0]);
-                            ry = add_cells(ry, nim.shift(1, sp), cell.h[4]);
-                            rz = add_cells(rz, nim.shift(2, sp), cell.h[8]);
-                        }
-                        const float r2 = rx * rx + ry * ry + rz * rz;
-                        if (!(r2 < m.rc2)) continue;
-                        const float ri = rsqrtf(r2);
-                        const float t = fminf(fmaxf(fmaf(r2 * ri, m.dri_f, -m.rmd), 0.0f), m.tmax);
-                        const float tr = __fadd_rn(t, kRound);
-                        const int kn = __float_as_int(tr) - __float_as_int(kRound);
-                        const float del = t - __fsub_rn(tr, kRound);
-                        const float ux = ui[si][0] - uj[sj][0], uy = ui[si][1] - uj[sj][1], uz = ui[si][2] - uj[sj][2];
-                        const float ur = ux * rx + uy * ry + uz * rz;
-                        const bool mv = gw && (si == SM || sj == SM);
-                        float dv = 0.0f, dvp = 0.0f;
-                        if (coul) {
-                            float4 cf, ef;
-                            ldg_keep_pair(a.tabfe + 2 * (m.toff[sp] + kn) + 2 * m.tstride, cf, ef);
-                            const float sc = spline_eval<float4, float>(cf, del);
-                            if (c.dq) {
-                                const float tq = (float)__ldg(c.dq + i0 + si) * q[sj] + q[si] * (float)__ldg(c.dq + j0 + sj);
-                                eq += tq * spline_eval<float4, float>(ef, del);
-                                fq += ur * (tq * sc);
-                            }
-                            if (mv) {
-                                dv = m.q2[sp] * sc;
-                                dvp = m.q2[sp] * (cf.y + del * (2.0f * cf.z + 3.0f * del * cf.w)) * m.dri_f;
-                            }
-                        }
-                        if (vdw) {
-#pragma unroll
-                            for (int n = 0; n < 2; n++)
-                                if (c.tt[n]) {
-                                    const float4 *tt = (const float4 *)c.tt[n] + m.toff[sp] + kn;
-                                    et[n] += spline_eval<float4, float>(__ldg(tt), del);
-                                    ft[n] += ur * spline_eval<float4, float>(__ldg(tt + m.tstride), del);
-                                }
-                            if (mv) {
-                                const float4 cv = __ldg(a.tab + m.toff[sp] + kn + T_CDV0 * m.tstride);
-                                dv += spline_eval<float4, float>(cv, del);
-                                dvp += (cv.y + del * (2.0f * cv.z + 3.0f * del * cv.w)) * m.dri_f;
-                            }
+                for (int si = 0; si < NS; si++) {
+                    const int sp = si * NS + sj;
+                    const bool coul = ((CM >> sp) & 1u) != 0, vdw = ((VM >> sp) & 1u) != 0;
+                    if (!coul && !vdw) continue;
+                    if (!((mask >> sp) & 1u)) continue;
+                    const float rx = dj[sj][0] + ei[si][0], ry = dj[sj][1] + ei[si][1], rz = dj[sj][2] + ei[si][2];
+                    const float r2 = rx * rx + ry * ry + rz * rz;
+                    if (!(r2 < m.rc2)) continue;
+                    const float ri = rsqrtf(r2);
+                    const float t = fminf(fmaxf(fmaf(r2 * ri, m.dri_f, -m.rmd), 0.0f), m.tmax);
+                    const float tr = __fadd_rn(t, kRound);
+                    const int kn = __float_as_int(tr) - __float_as_int(kRound);
+                    const float del = t - __fsub_rn(tr, kRound);
+                    const float ux = ui[si][0] - uj[sj][0], uy = ui[si][1] - uj[sj][1], uz = ui[si][2] - uj[sj][2];
+                    const float ur = ux * rx + uy * ry + uz * rz;
+                    const bool mv = gw && (si == SM || sj == SM);
+                    float dv = 0.0f, dvp = 0.0f;
+                    if (coul) {
+                        float4 cf, ef;
+                        ldg_keep_pair(a.tabfe + 2 * (m.toff[sp] + kn) + 2 * m.tstride, cf, ef);
+                        const float sc = spline_eval<float4, float>(cf, del);
+                        if (c.dq) {
+                            const float tq = (float)__ldg(c.dq + i0 + si) * q[sj] + q[si] * (float)__ldg(c.dq + j0 + sj);
+                            eq += tq * spline_eval<float4, float>(ef, del);
+                            fq += ur * (tq * sc);
                         }
                         if (mv) {
-                            const float wx = (si == SM ? wi[0] : 0.0f) - (sj == SM ? wj[0] : 0.0f),
-                                        wy = (si == SM ? wi[1] : 0.0f) - (sj == SM ? wj[1] : 0.0f),
-                                        wz = (si == SM ? wi[2] : 0.0f) - (sj == SM ? wj[2] : 0.0f);
-                            fw += (ux * wx + uy * wy + uz * wz) * dv + ur * (rx * wx + ry * wy + rz * wz) * (dvp * ri);
+                            dv = m.q2[sp] * sc;
+                            dvp = m.q2[sp] * (cf.y + del * (2.0f * cf.z + 3.0f * del * cf.w)) * m.dri_f;
                         }
                     }
+                    if (vdw) {
+#pragma unroll
+                        for (int n = 0; n < 2; n++)
+                            if (c.tt[n]) {
+                                const float4 *tt = (const float4 *)c.tt[n] + m.toff[sp] + kn;
+                                et[n] += spline_eval<float4, float>(__ldg(tt), del);
+                                ft[n] += ur * spline_eval<float4, float>(__ldg(tt + m.tstride), del);
+                            }
+                        if (mv) {
+                            const float4 cv = __ldg(a.tab + m.toff[sp] + kn + T_CDV0 * m.tstride);
+                            dv += spline_eval<float4, float>(cv, del);
+                            dvp += (cv.y + del * (2.0f * cv.z + 3.0f * del * cv.w)) * m.dri_f;
+                        }
+                    }
+                    if (mv) {
+                        const float wx = (si == SM ? wi[0] : 0.0f) - (sj == SM ? wj[0] : 0.0f),
+                                    wy = (si == SM ? wi[1] : 0.0f) - (sj == SM ? wj[1] : 0.0f),
+                                    wz = (si == SM ? wi[2] : 0.0f) - (sj == SM ? wj[2] : 0.0f);
+                        fw += (ux * wx + uy * wy + uz * wz) * dv + ur * (rx * wx + ry * wy + rz * wz) * (dvp * ri);
+                    }
                 }
-            };
-            if (near) site_pairs(std::true_type{}, near_images<NS, G>(a.xmod, i0, j0, NS, sh0, cell, lane));
-            else site_pairs(std::false_type{}, NearImages{{0u, 0u, 0u}});
+            }
             const float v[7] = {eq, et[0], et[1], fq, ft[0], ft[1], fw};
 #pragma unroll
             for (int n = 0; n < 7; n++)
@@ -1840,8 +2021,9 @@ struct MixBox {
 };
 
 // Resident blocks per SM of the batched MIXED kernel: the argument table
-// is indexed at run time, which costs registers (4 x 128 threads leave 128,
-// no spills; at 5 it spills 100-200 bytes).
+// is indexed at run time, which costs registers (4 x 128 threads leave 128 and
+// up to 32 bytes of spills, around the pairs near half a box; at 5 it spills
+// 100-200 bytes).
 #ifndef PINYB200_MIX_BATCH_BLOCKS
 #define PINYB200_MIX_BATCH_BLOCKS 4
 #endif

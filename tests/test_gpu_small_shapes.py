@@ -242,3 +242,57 @@ def test_gradient_of_tables_without_a_term(oracle, model, nmol, beads):
         escale = abs(e0["vreal"]) + abs(e0["vself"]) + abs(dE)
         assert abs(out["fp64"][0][k] - dE) <= 1e-12 * escale
         assert abs(out["fp64"][1][k] - dF) <= 1e-12 * np.abs(f1 * fbar).sum()
+
+
+def _pairs_only(S):
+    """Without bonds, bends and exclusion correction, which see no images."""
+    return dict(S, nbond=0, nbend=0, necor=0, nghost=0)
+
+
+@pytest.mark.parametrize("model, nmol, cutoff", [(water.SPC_FW, 64, 5.5), (water.TIP4P_F, 65, 5.5),
+                                                 (water.SPC_FW, 130, 9.0)])
+@pytest.mark.parametrize("beads", [1, 2, 8, 32, 64])
+def test_sites_in_different_cells(oracle, model, nmol, cutoff, beads):
+    """Every site moved by lattice vectors of its own, as a program does that
+    wraps atoms one by one: a site pair's shift then differs from its molecules'
+    first sites' by up to four cells, and its image is what it was."""
+    spec, S, pos, xmod = _box(model, nmol, beads, 20, 6, cutoff=cutoff)
+    S = _pairs_only(S)
+    h = float(S["hmat"][0])
+    n = np.random.default_rng(5).integers(-1, 2, size=(pos.shape[1], 3))
+    moved = pos + h * n[None]
+    xm = None if xmod is None else xmod + h * n
+    f0, e0 = _oracle(oracle, S, pos, xmod)
+    fref, eref = _oracle(oracle, S, moved, xm)
+    assert np.linalg.norm(fref - f0) <= 1e-9 * np.linalg.norm(f0)
+    for precision in ("fp64", "mixed"):
+        for variant in (0, 2, 1):
+            f, e = _device(S, moved, xm, precision, tuning={1: variant})
+            _check(precision, f, e, fref, eref)
+            if precision == "fp64":
+                break
+
+
+def test_gradient_with_sites_in_different_cells():
+    """As above for the pair adjoint: each molecule's sites stay together for
+    bonds and exclusions, so one molecule of every three is moved as a whole and
+    the rest by sites would break them; whole cells' moves of whole molecules
+    leave every derivative as it was."""
+    import torch
+
+    from piny_b200.lib import DeviceBox
+    spec, S, pos, xmod = _box(water.TIP4P_F, 65, 8, 20, 6)
+    h = float(S["hmat"][0])
+    n = np.repeat(np.random.default_rng(5).integers(-2, 3, size=(65, 3)), 4, axis=0)
+    tan = params.tangents(spec, params.theta_of(spec.model), S)
+    fbar = torch.from_numpy(np.random.default_rng(3).normal(size=pos.shape)).cuda()
+    out = []
+    for p, x in ((pos, xmod), (pos + h * n[None], xmod + h * n)):
+        box = DeviceBox(S, 8, "mixed")
+        box.build_list(p[0], x, S["hmat"], S["cutskin2"])
+        box.grad_prepare(tan)
+        d, dx = torch.from_numpy(p).cuda(), torch.from_numpy(x).cuda()
+        out.append(box.grad(d.data_ptr(), dx.data_ptr(), S["hmat"], fbar.data_ptr()))
+        box.close()
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= 1e-6 * np.abs(a).max()
