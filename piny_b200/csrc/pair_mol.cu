@@ -1343,9 +1343,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
 //     every charged pair reads the same Coulomb table, so the tables that
 //     32 beads' knots scatter over stay few enough for L1;
 //   * the knot nint((r - rmin) dri) (force_npol.c:345-352) is taken with the
-//     1.5 * 2^23 rounding constant instead of float <-> int conversions, t
-//     clamped to the table's intervals (what clamping the knot does for
-//     every r inside the cutoff);
+//     1.5 * 2^23 rounding constant instead of float <-> int conversions; below
+//     rmin the first interval's cubic is continued, as PINY's clamped knot does;
 //   * molecules are uniform runs of sites: the j site index is mj * stride,
 //     not a load.
 // Pairs whose site-0 separation is within twice the molecular extent of half
@@ -1447,8 +1446,8 @@ __device__ __forceinline__ void mixed_near(const MixArgs &a, const MixSite &m, c
             }
             const float r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
             if (!(r2 < m.rc2)) continue;
-            const float t = fminf(fmaxf(fmaf(r2 * rsqrtf(r2), m.dri_f, -m.rmd), 0.0f), m.tmax);
-            const int kn = __float2int_rn(t);
+            const float t = fminf(fmaf(r2 * rsqrtf(r2), m.dri_f, -m.rmd), m.tmax);
+            const int kn = __float2int_rn(fmaxf(t, 0.0f));
             const float del = t - (float)kn;
             const float4 *row = a.tab + (m.toff[sp] + kn), *rfe = a.tabfe + 2 * (m.toff[sp] + kn);
             float dv = 0.0f;
@@ -1648,8 +1647,8 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                         const float r2 = rx * rx + ry * ry + rz * rz;
                         if (r2 < rc2) {
                             const float r = r2 * rsqrtf(r2);
-                            const float t = fminf(fmaxf(fmaf(r, dri, -rmd), 0.0f), tmax);
-                            const float tr = __fadd_rn(t, kRound);
+                            const float t = fminf(fmaf(r, dri, -rmd), tmax);
+                            const float tr = __fadd_rn(fmaxf(t, 0.0f), kRound);
                             const int kn = __float_as_int(tr) - __float_as_int(kRound);
                             const float del = t - __fsub_rn(tr, kRound);
                             // with energies: the force and energy rows of an interval
@@ -1822,8 +1821,8 @@ __device__ __forceinline__ void grad_near(const MixArgs &a, const MixSite &m, co
         const float r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
         if (!(r2 < m.rc2)) continue;
         const float ri = rsqrtf(r2);
-        const float t = fminf(fmaxf(fmaf(r2 * ri, m.dri_f, -m.rmd), 0.0f), m.tmax);
-        const int kn = __float2int_rn(t);
+        const float t = fminf(fmaf(r2 * ri, m.dri_f, -m.rmd), m.tmax);
+        const int kn = __float2int_rn(fmaxf(t, 0.0f));
         const float del = t - (float)kn;
         const float ur = u[0] * r[0] + u[1] * r[1] + u[2] * r[2];
         const float4 *row = a.tab + (m.toff[sp] + kn);
@@ -1950,8 +1949,8 @@ __global__ void __launch_bounds__(128, 4)
                     const float r2 = rx * rx + ry * ry + rz * rz;
                     if (!(r2 < m.rc2)) continue;
                     const float ri = rsqrtf(r2);
-                    const float t = fminf(fmaxf(fmaf(r2 * ri, m.dri_f, -m.rmd), 0.0f), m.tmax);
-                    const float tr = __fadd_rn(t, kRound);
+                    const float t = fminf(fmaf(r2 * ri, m.dri_f, -m.rmd), m.tmax);
+                    const float tr = __fadd_rn(fmaxf(t, 0.0f), kRound);
                     const int kn = __float_as_int(tr) - __float_as_int(kRound);
                     const float del = t - __fsub_rn(tr, kRound);
                     const float ux = ui[si][0] - uj[sj][0], uy = ui[si][1] - uj[sj][1], uz = ui[si][2] - uj[sj][2];

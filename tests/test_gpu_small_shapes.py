@@ -296,3 +296,43 @@ def test_gradient_with_sites_in_different_cells():
         box.close()
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= 1e-6 * np.abs(a).max()
+
+
+@pytest.mark.parametrize("model, nmol, beads, cutoff", [(water.SPC_FW, 65, 1, None), (water.SPC_FW, 216, 8, 5.0),
+                                                        (water.TIP4P_F, 216, 1, 5.0), (water.TIP4P_F, 300, 32, None),
+                                                        (water.TIP4P_F, 64, 4, 9.0)])
+def test_pairs_closer_than_the_tables(oracle, model, nmol, beads, cutoff):
+    """Two hydrogens nearer than the tables' first point: PINY continues the first
+    interval's cubic there."""
+    import torch
+
+    from piny_b200.lib import DeviceBox
+    spec, S, pos, xmod = _box(model, nmol, beads, 24, 6, cutoff=cutoff)
+    ns, last = spec.model.nsite, spec.nmol - 1
+    r = float(S["rmin_spl"][0])
+    # the last molecule: the first one's mirror image in a point 0.3 rmin beyond its first hydrogen
+    out = pos[:, 1] - pos[:, 0]
+    c = pos[:, 1] + 0.3 * r * out / np.linalg.norm(out, axis=1, keepdims=True)
+    pos[:, last * ns:] = 2.0 * c[:, None, :] - pos[:, :ns]
+    xmod = None if xmod is None else pos.mean(axis=0)
+    fref, eref = _oracle(oracle, S, pos, xmod, distribute=True)
+    force, grads = {}, {}
+    tan = None if ns == 3 else params.tangents(spec, params.theta_of(spec.model), S)
+    for precision in ("fp64", "mixed"):
+        force[precision], e = _device(S, pos, xmod, precision, distribute=True)
+        if ns == 3:
+            continue
+        box = DeviceBox(S, beads, precision)
+        box.build_list(pos[0], xmod, S["hmat"], S["cutskin2"])
+        box.grad_prepare(tan)
+        d, x = torch.from_numpy(pos).cuda(), None if xmod is None else torch.from_numpy(xmod).cuda()
+        fbar = torch.from_numpy(np.random.default_rng(3).normal(size=pos.shape)).cuda()
+        grads[precision] = box.grad(d.data_ptr(), None if x is None else x.data_ptr(), S["hmat"], fbar.data_ptr())
+        box.close()
+    norm = np.linalg.norm(fref)
+    assert np.linalg.norm(force["fp64"] - fref) <= 1e-12 * norm
+    # FP32 separations are sums of three values up to the box edge L, each
+    # rounded to 2^-24: 3 L 2^-24 of the pair's r = 0.11 Bohr, up to 1e-4
+    assert np.linalg.norm(force["mixed"] - fref) <= 1e-4 * norm
+    for a, b in zip(grads.get("mixed", ()), grads.get("fp64", ())):
+        assert np.abs(a - b).max() <= 1e-4 * np.abs(b).max()
