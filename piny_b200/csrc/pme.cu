@@ -1376,12 +1376,17 @@ TileArgs tile_args_of(pinyb200_ctx *c, int NI, int TT)
     t.T = TT;
     // fixed-point scale of the FP32 spread tile: every contribution q M_a M_b
     // M_c (bounded by max |q| times the B-spline's peak cubed) below 2^22
-    // after scaling, the range the rounding trick is exact in; at most 2^24
-    // (a resolution of 6e-8 against contributions of up to ~0.15)
+    // after scaling, the range the rounding trick is exact in; at most 2^24 (a
+    // resolution of 6e-8 against contributions of up to ~0.15), or 2^25 where
+    // even a full bin's charges on one grid point stay below 2^31 (order 8 of
+    // q-TIP4P/F: the force gradient of 1024 x 16 on 32^3 is 1.3e-7 off FP64 at
+    // 2^24, 5e-8 at 2^25 and with FP32 sums).  At 2^24 that takes 128 charges
+    // of one sign on a point.
     {
-        const double qmax = c->q_max, bmax = bspline_peak(NI);
-        int S = 24;
-        while (S > 8 && std::ldexp(qmax * bmax * bmax * bmax, S) >= 0.99 * std::ldexp(1.0, 22)) S--;
+        const double peak = bspline_peak(NI), most = c->q_max * peak * peak * peak;
+        int S = 25;
+        while (S > 8 && std::ldexp(most, S) >= 0.99 * std::ldexp(1.0, 22)) S--;
+        if (S == 25 && c->pme_cap * std::ldexp(most, S) >= std::ldexp(1.0, 31)) S = 24;
         t.qfix = (float)std::ldexp(1.0, S);
         t.qfix_inv = (float)std::ldexp(1.0, -S);
     }

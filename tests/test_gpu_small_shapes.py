@@ -336,3 +336,14 @@ def test_pairs_closer_than_the_tables(oracle, model, nmol, beads, cutoff):
     assert np.linalg.norm(force["mixed"] - fref) <= 1e-4 * norm
     for a, b in zip(grads.get("mixed", ()), grads.get("fp64", ())):
         assert np.abs(a - b).max() <= 1e-4 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("nmol, beads, grid, bound", [(216, 8, 32, 3e-6), (4096, 2, 64, 4e-6)])
+def test_mesh_forces_resolve_small_weights(nmol, beads, grid, bound):
+    """Mesh forces alone (no pair tables): MIXED within the rounding of a spread at
+    2^-25 (2.1e-6 and 2.8e-6 of the mesh force; 4.0e-6 and 5.4e-6 at 2^-24)."""
+    spec, S, pos, xmod = _box(water.TIP4P_F, nmol, beads, grid, 8, seed=3)
+    S = dict(S, nbond=0, nbend=0, necor=0, **{k: 0.0 * np.asarray(S[k]) for k in ("cv0", "cdv0", "cv0_c", "cdv0_c")})
+    f64, _ = _device(S, pos, xmod, "fp64")
+    f32, _ = _device(S, pos, xmod, "mixed")
+    assert np.linalg.norm(f32 - f64) <= bound * np.linalg.norm(f64)
