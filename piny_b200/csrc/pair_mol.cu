@@ -1799,11 +1799,11 @@ __global__ void __launch_bounds__(128, PINYB200_MIX_BLOCKS)
 // seven sums.
 template <int P, int NS>
 __device__ __forceinline__ void grad_near(const MixArgs &a, const MixSite &m, const Cell &cell, const GradPairSel &c,
-                                          const float4 &qs, const double *__restrict__ uT, int i0, int j0,
+                                          const double4 &qs, const double *__restrict__ uT, int i0, int j0,
                                           unsigned mask, int b, int lane, bool far, const double *sh0, double (&sum)[7])
 {
     constexpr int G = P >= 32 ? 32 : P;
-    const float *q = &qs.x;
+    const double *q = &qs.x;
     NearImages nim = {{0u, 0u, 0u}};
     if (!far) nim = near_images<NS, G>(a.xmod, i0, j0, NS, sh0, cell, lane);
 #pragma unroll 1
@@ -1831,7 +1831,7 @@ __device__ __forceinline__ void grad_near(const MixArgs &a, const MixSite &m, co
             const float4 cf = __ldg(row + T_CDV0C * m.tstride);
             const float sc = spline_eval<float4, float>(cf, del);
             if (c.dq) {
-                const float tq = (float)__ldg(c.dq + i) * q[sj] + q[si] * (float)__ldg(c.dq + j);
+                const float tq = (float)(__ldg(c.dq + i) * q[sj] + q[si] * __ldg(c.dq + j));
                 sum[0] += (double)(tq * spline_eval<float4, float>(__ldg(row + T_CV0C * m.tstride), del));
                 sum[3] += (double)(ur * (tq * sc));
             }
@@ -1863,13 +1863,15 @@ __device__ __forceinline__ void grad_near(const MixArgs &a, const MixSite &m, co
 //   tables   dE += S(tangent cv0), dF += (u . r) S(tangent cdv0)
 //   ghosts   dF += (u . w) dv + (u . r)(r . w) dv' / r,  w = w_i - w_j; only the
 //            M site (the last of four) moves
-// A molecule pair's terms are summed in FP32, molecule pairs in FP64.  No
-// forces, so no atomics but a block's seven sums.
+// u is formed as r is, from the first sites' FP64 values (a large common part of
+// the upstream gradient cancels); w and tq are FP64 differences and products,
+// rounded once.  The terms of one j site are summed in FP32, everything beyond
+// them in FP64.  No forces, so no atomics but a block's seven sums.
 template <int P, int NS, unsigned CM, unsigned VM>
 __global__ void __launch_bounds__(128, 4)
     mol_pair_grad_kernel(const __grid_constant__ MixArgs a, const __grid_constant__ MixSite m,
                          const __grid_constant__ Cell cell, const __grid_constant__ GradPairSel c,
-                         const __grid_constant__ float4 qs, const double *__restrict__ uT, double *__restrict__ gacc)
+                         const __grid_constant__ double4 qs, const double *__restrict__ uT, double *__restrict__ gacc)
 {
     constexpr int G = P >= 32 ? 32 : P, JPI = 32 / G;
     constexpr int SM = NS == 4 ? 3 : -1;  // the M site
@@ -1879,7 +1881,7 @@ __global__ void __launch_bounds__(128, 4)
     const int warp = ((int)blockIdx.x * 128 + (int)threadIdx.x) >> 5, nwarps = (int)gridDim.x * 4;
     const int b = (lane % G) + 32 * blockIdx.y;
     const double *__restrict__ posT = a.posT;
-    const float q[4] = {qs.x, qs.y, qs.z, qs.w};
+    const double q[4] = {qs.x, qs.y, qs.z, qs.w};
     const bool gw = SM >= 0 && c.w;
     double sum[7] = {0, 0, 0, 0, 0, 0, 0};  // eq, et0, et1, fq, ft0, ft1, fw
     const double ext2 = ext2_of(a.ext);
@@ -1887,18 +1889,20 @@ __global__ void __launch_bounds__(128, 4)
     for (int ch = warp; ch < nch; ch += nwarps) {
         const int mi = a.chunk[3 * ch], beg = a.chunk[3 * ch + 1], end = a.chunk[3 * ch + 2];
         const int i0 = mi * m.stride;
-        float ei[NS][3], ui[NS][3], wi[3] = {0, 0, 0};
+        float ei[NS][3], ui[NS][3];
+        double ui0[3], wi[3] = {0, 0, 0};
 #pragma unroll
         for (int s = 0; s < NS; s++)
 #pragma unroll
             for (int d = 0; d < 3; d++) {
                 const size_t o = (3 * (size_t)(i0 + s) + d) * P + b;
                 ei[s][d] = s == 0 ? 0.0f : a.offT[o];
-                ui[s][d] = (float)uT[o];
+                if (s == 0) ui0[d] = uT[o];
+                ui[s][d] = s == 0 ? 0.0f : (float)(uT[o] - ui0[d]);
             }
         if (gw)
 #pragma unroll
-            for (int d = 0; d < 3; d++) wi[d] = (float)c.w[(3 * (size_t)(i0 + NS - 1) + d) * P + b];
+            for (int d = 0; d < 3; d++) wi[d] = c.w[(3 * (size_t)(i0 + NS - 1) + d) * P + b];
         for (int k = beg + sub; k < end; k += JPI) {
             const int mj = __ldcg(a.mj + k);
             const unsigned mask = __ldcg(a.mask + k);
@@ -1916,29 +1920,34 @@ __global__ void __launch_bounds__(128, 4)
                 grad_near<P, NS>(a, m, cell, c, qs, uT, i0, j0, mask, b, lane, far_images(ext2, cell), sh0, sum);
                 continue;
             }
-            float dj[NS][3], uj[NS][3], wj[3] = {0, 0, 0};
+            float dj[NS][3], uj[NS][3];
+            double wj[3] = {0, 0, 0};
             {
-                double xj0[3];
+                // u_i - u_j as r: the first sites' in FP64, the others by their
+                // differences from the first
+                double xj0[3], uj0[3];
 #pragma unroll
                 for (int d = 0; d < 3; d++) {
                     xj0[d] = __ldcg(posT + (3 * (size_t)j0 + d) * P + b);
                     dj[0][d] = (float)(__dsub_rn(posT[(3 * (size_t)i0 + d) * P + b], xj0[d]) + sh0[d] * cell.h[4 * d]);
+                    uj0[d] = __ldcg(uT + (3 * (size_t)j0 + d) * P + b);
+                    uj[0][d] = (float)(ui0[d] - uj0[d]);
                 }
 #pragma unroll
-                for (int s = 0; s < NS; s++)
+                for (int s = 1; s < NS; s++)
 #pragma unroll
                     for (int d = 0; d < 3; d++) {
                         const size_t o = (3 * (size_t)(j0 + s) + d) * P + b;
-                        if (s > 0) dj[s][d] = dj[0][d] - __ldcg(a.offT + o);
-                        uj[s][d] = (float)__ldcg(uT + o);
+                        dj[s][d] = dj[0][d] - __ldcg(a.offT + o);
+                        uj[s][d] = uj[0][d] - (float)(__ldcg(uT + o) - uj0[d]);
                     }
                 if (gw)
 #pragma unroll
-                    for (int d = 0; d < 3; d++) wj[d] = (float)__ldcg(c.w + (3 * (size_t)(j0 + NS - 1) + d) * P + b);
+                    for (int d = 0; d < 3; d++) wj[d] = __ldcg(c.w + (3 * (size_t)(j0 + NS - 1) + d) * P + b);
             }
-            float eq = 0, et[2] = {0, 0}, fq = 0, ft[2] = {0, 0}, fw = 0;
 #pragma unroll
             for (int sj = 0; sj < NS; sj++) {
+                float eq = 0, et[2] = {0, 0}, fq = 0, ft[2] = {0, 0}, fw = 0;
 #pragma unroll
                 for (int si = 0; si < NS; si++) {
                     const int sp = si * NS + sj;
@@ -1953,7 +1962,7 @@ __global__ void __launch_bounds__(128, 4)
                     const float tr = __fadd_rn(fmaxf(t, 0.0f), kRound);
                     const int kn = __float_as_int(tr) - __float_as_int(kRound);
                     const float del = t - __fsub_rn(tr, kRound);
-                    const float ux = ui[si][0] - uj[sj][0], uy = ui[si][1] - uj[sj][1], uz = ui[si][2] - uj[sj][2];
+                    const float ux = ui[si][0] + uj[sj][0], uy = ui[si][1] + uj[sj][1], uz = ui[si][2] + uj[sj][2];
                     const float ur = ux * rx + uy * ry + uz * rz;
                     const bool mv = gw && (si == SM || sj == SM);
                     float dv = 0.0f, dvp = 0.0f;
@@ -1962,7 +1971,7 @@ __global__ void __launch_bounds__(128, 4)
                         ldg_keep_pair(a.tabfe + 2 * (m.toff[sp] + kn) + 2 * m.tstride, cf, ef);
                         const float sc = spline_eval<float4, float>(cf, del);
                         if (c.dq) {
-                            const float tq = (float)__ldg(c.dq + i0 + si) * q[sj] + q[si] * (float)__ldg(c.dq + j0 + sj);
+                            const float tq = (float)(__ldg(c.dq + i0 + si) * q[sj] + q[si] * __ldg(c.dq + j0 + sj));
                             eq += tq * spline_eval<float4, float>(ef, del);
                             fq += ur * (tq * sc);
                         }
@@ -1986,17 +1995,17 @@ __global__ void __launch_bounds__(128, 4)
                         }
                     }
                     if (mv) {
-                        const float wx = (si == SM ? wi[0] : 0.0f) - (sj == SM ? wj[0] : 0.0f),
-                                    wy = (si == SM ? wi[1] : 0.0f) - (sj == SM ? wj[1] : 0.0f),
-                                    wz = (si == SM ? wi[2] : 0.0f) - (sj == SM ? wj[2] : 0.0f);
+                        const float wx = (float)((si == SM ? wi[0] : 0.0) - (sj == SM ? wj[0] : 0.0)),
+                                    wy = (float)((si == SM ? wi[1] : 0.0) - (sj == SM ? wj[1] : 0.0)),
+                                    wz = (float)((si == SM ? wi[2] : 0.0) - (sj == SM ? wj[2] : 0.0));
                         fw += (ux * wx + uy * wy + uz * wz) * dv + ur * (rx * wx + ry * wy + rz * wz) * (dvp * ri);
                     }
                 }
-            }
-            const float v[7] = {eq, et[0], et[1], fq, ft[0], ft[1], fw};
+                const float v[7] = {eq, et[0], et[1], fq, ft[0], ft[1], fw};
 #pragma unroll
-            for (int n = 0; n < 7; n++)
-                if (v[n] != 0.0f) sum[n] += (double)v[n];
+                for (int n = 0; n < 7; n++)
+                    if (v[n] != 0.0f) sum[n] += (double)v[n];
+            }
         }
     }
 #pragma unroll
@@ -2476,8 +2485,7 @@ template <int P, int NS, unsigned CM, unsigned VM>
 static cudaError_t launch_grad_t(pinyb200_ctx *c, const Cell &cell, const GradPairSel &sel, const double *uT,
                                  double *gacc)
 {
-    const float4 q = make_float4((float)c->h_charge[0], (float)c->h_charge[1], (float)c->h_charge[2],
-                                 NS == 4 ? (float)c->h_charge[3] : 0.0f);
+    const double4 q = make_double4(c->h_charge[0], c->h_charge[1], c->h_charge[2], NS == 4 ? c->h_charge[3] : 0.0);
     const long long blocks = std::max<long long>(1, std::min<long long>((c->chunk_cap + 3) / 4, c->sm_count * 4LL));
     const dim3 grid((unsigned)blocks, P > 32 ? P / 32 : 1);
     mol_pair_grad_kernel<P, NS, CM, VM><<<grid, 128, 0, c->stream>>>(mix_args(c), mix_site(c), cell, sel, q, uT, gacc);

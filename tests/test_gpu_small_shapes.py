@@ -347,3 +347,28 @@ def test_mesh_forces_resolve_small_weights(nmol, beads, grid, bound):
     f64, _ = _device(S, pos, xmod, "fp64")
     f32, _ = _device(S, pos, xmod, "mixed")
     assert np.linalg.norm(f32 - f64) <= bound * np.linalg.norm(f64)
+
+
+@pytest.mark.parametrize("nmol, beads", [(216, 1), (216, 8), (130, 32)])
+def test_gradient_under_a_common_force(nmol, beads):
+    """An upstream gradient with a large common part, which no force sum sees:
+    it cancels in the FP64 differences of the pair adjoint (without the mesh,
+    whose FP32 spread holds the common part)."""
+    import torch
+
+    from piny_b200.lib import DeviceBox
+    spec, S, pos, xmod = _box(water.TIP4P_F, nmol, beads, 20, 6, seed=5)
+    S = dict(S, nktot=0)
+    tan = params.tangents(spec, params.theta_of(spec.model), S)
+    d, x = torch.from_numpy(pos).cuda(), None if xmod is None else torch.from_numpy(xmod).cuda()
+    fbar = torch.from_numpy(1e4 + np.random.default_rng(3).normal(size=pos.shape)).cuda()
+    out = []
+    for precision in ("fp64", "mixed"):
+        box = DeviceBox(S, beads, precision)
+        box.build_list(pos[0], xmod, S["hmat"], S["cutskin2"])
+        box.grad_prepare(tan)
+        out.append(box.grad(d.data_ptr(), None if x is None else x.data_ptr(), S["hmat"], fbar.data_ptr())[1])
+        box.close()
+    # FP32 pair terms: 1e-6 of a component, up to 1e-5 of one that is small by
+    # cancellation; differences of u rounded to FP32 were 5e-5 to 9e-3 off
+    assert np.all(np.abs(out[1] - out[0]) <= 3e-5 * np.abs(out[0]))
