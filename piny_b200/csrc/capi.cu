@@ -836,12 +836,16 @@ int pinyb200_build_list(pinyb200_ctx *c, const double *pos1, const double *xmod,
                     chunks.push_back(std::min(k + ch, mrow[m + 1]));
                 }
             c->nchunk = (int)(chunks.size() / 3);
-            if (!c->d_chunk || c->nchunk > c->chunk_cap) {
+            if (c->chunk_cap == 0 || c->nchunk > c->chunk_cap) c->chunk_cap = c->nchunk + c->nchunk / 4 + 256;
+            // a device rebuild that fits the molecule list has to find room for
+            // its chunks too: at most one in part per row beside the full ones
+            const long long room = c->mlist_cap / ch + c->nmol;
+            if (!c->d_chunk || room > c->chunk_room) {
                 if (c->d_chunk) cudaFree(c->d_chunk);
                 c->d_chunk = nullptr;
-                const long long cap = c->nchunk + c->nchunk / 4 + 256;
-                CK(cudaMalloc(&c->d_chunk, (size_t)cap * 3 * sizeof(int)));
-                c->chunk_cap = cap;
+                c->chunk_room = 0;
+                CK(cudaMalloc(&c->d_chunk, (size_t)room * 3 * sizeof(int)));
+                c->chunk_room = room;
             }
             CK(cudaMemcpy(c->d_chunk, chunks.data(), chunks.size() * sizeof(int), cudaMemcpyHostToDevice));
             if (!c->d_nchunk) CK(cudaMalloc(&c->d_nchunk, sizeof(int)));

@@ -246,8 +246,9 @@ struct pinyb200_ctx {
     long long mlist_cap = 0, nmp = 0;
     int nchunk = 0;
     int mol_iters = PINYB200_MOL_CHUNK;  // molecule pairs per chunk and lane group, set by the host build
-    int *d_chunk = nullptr;    // [chunk_cap][3]
-    long long chunk_cap = 0;
+    int *d_chunk = nullptr;    // [chunk_room][3]
+    long long chunk_cap = 0;   // chunks the launch shapes are made for (a quarter over the host build's)
+    long long chunk_room = 0;  // chunks of any list that fits mlist_cap
     int *d_nchunk = nullptr;   // device copy of the chunk count (the pair kernel reads it)
     // device list update (pinyb200_update_list_device)
     pinyb200::ListState *d_ls = nullptr;

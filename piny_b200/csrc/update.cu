@@ -90,7 +90,7 @@ __global__ void ls_chunk_fill_kernel(const int *gate, int nmol, const int *__res
 
 __global__ void ls_finish_kernel(const int *gate, ListState *ls, const long long *__restrict__ tot,
                                  const long long *__restrict__ chunk_tot, long long list_cap, long long mlist_cap,
-                                 long long chunk_cap, int use_mol, int *__restrict__ nchunk)
+                                 long long chunk_room, int use_mol, int *__restrict__ nchunk)
 {
     if (*gate == 0) return;
     ls->site_tot[0] = tot[0];
@@ -99,9 +99,9 @@ __global__ void ls_finish_kernel(const int *gate, ListState *ls, const long long
     if (use_mol) {
         ls->mol_tot[0] = tot[2];
         ls->mol_tot[1] = tot[3];
-        over |= tot[2] > mlist_cap || *chunk_tot > chunk_cap;
+        over |= tot[2] > mlist_cap || *chunk_tot > chunk_room;
         if (tot[3] != tot[1]) ls->mismatch = 1;
-        *nchunk = (int)(*chunk_tot < chunk_cap ? *chunk_tot : chunk_cap);
+        *nchunk = (int)(*chunk_tot < chunk_room ? *chunk_tot : chunk_room);
     }
     if (over) ls->overflow = 1;
     ls->rebuilds += 1;
@@ -173,12 +173,12 @@ int list_update_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_xm
             cudaSuccess)
             return record_error(c, PINYB200_ERR_CUDA, cudaGetErrorString(e));
         ls_chunk_fill_kernel<<<blocks, 256, 0, st>>>(gate, c->nmol, c->d_mrow, ch, c->d_mchunk,
-                                                     c->d_mchunk + c->nmol, c->d_chunk, c->chunk_cap);
+                                                     c->d_mchunk + c->nmol, c->d_chunk, c->chunk_room);
     } else if ((e = launch_build_list(c, cell, d_pos, xm, c->d_cs, 0, gate, st)) != cudaSuccess ||
                (e = launch_build_list(c, cell, d_pos, xm, c->d_cs, 1, gate, st)) != cudaSuccess) {
         return record_error(c, PINYB200_ERR_CUDA, cudaGetErrorString(e));
     }
-    ls_finish_kernel<<<1, 1, 0, st>>>(gate, ls, c->d_tot, chunk_tot, c->list_cap, c->mlist_cap, c->chunk_cap,
+    ls_finish_kernel<<<1, 1, 0, st>>>(gate, ls, c->d_tot, chunk_tot, c->list_cap, c->mlist_cap, c->chunk_room,
                                       mol ? 1 : 0, c->d_nchunk);
     ls_clear_rows_kernel<<<(natm + 256) / 256, 256, 0, st>>>(gate, ls, natm, c->d_row, c->d_rowA, c->nmol,
                                                               mol ? c->d_mrow : nullptr);

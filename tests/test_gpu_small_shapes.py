@@ -372,3 +372,45 @@ def test_gradient_under_a_common_force(nmol, beads):
     # FP32 pair terms: 1e-6 of a component, up to 1e-5 of one that is small by
     # cancellation; differences of u rounded to FP32 were 5e-5 to 9e-3 off
     assert np.all(np.abs(out[1] - out[0]) <= 3e-5 * np.abs(out[0]))
+
+
+def _atoms(n, edge, cutoff, beads, seed):
+    """A fluid of one-site molecules with the O-O term of q-SPC/Fw and no charges (Bohr)."""
+    spec = water.BoxSpec(water.SPC_FW, n, edge, beads, 298.0, seed, cutoff=cutoff, grid=16, order=6)
+    W = system.build_system(spec, water.build_positions(spec) / water.BOHR)
+    S = dict(W, natm=n, atm_typ=np.zeros(n, np.int32), charge=np.zeros(n), excl_off=np.zeros(n + 1, np.int32),
+             excl_j=np.zeros(1, np.int32), nktot=0, necor=0, nbond=0, nbend=0, nghost=0)
+    rng = np.random.default_rng(seed)
+    g = int(np.ceil(n ** (1 / 3)))
+    cell = np.stack(np.meshgrid(*[np.arange(g)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n] * (edge / g)
+    pos = cell[None] + rng.normal(scale=0.05, size=(beads, n, 3))
+    return S, pos / water.BOHR
+
+
+@pytest.mark.parametrize("beads", [1, 8, 32])
+def test_device_rebuild_keeps_its_room(beads):
+    """A denser configuration whose pairs still fit the reserved lists (a quarter
+    and 1024 more than at the host build): the chunks cut from it fit theirs."""
+    import torch
+
+    from piny_b200.lib import DeviceBox
+    S, pos = _atoms(216, 30.0, 5.0, beads, 3)
+    closer = pos * 0.8 + 1.0
+    xmod, xm2 = (pos.mean(axis=0), closer.mean(axis=0)) if beads > 1 else (None, None)
+    box = DeviceBox(S, beads, "fp64")
+    n0 = box.build_list(pos[0], xmod, S["hmat"], S["cutskin2"])
+    box.list_set_spread(0.0)
+    d = torch.from_numpy(closer).cuda()
+    dx = None if xm2 is None else torch.from_numpy(xm2).cuda()
+    f = torch.zeros_like(d)
+    e = box.energy_force_device(d.data_ptr(), None if dx is None else dx.data_ptr(), S["hmat"], f.data_ptr(),
+                                update_list=True)
+    st = box.list_status()
+    assert st["rebuilt_last"] == 1 and n0 * 1.25 + 300 < st["npairs"] < n0 * 1.25 + 1024
+    fresh = DeviceBox(S, beads, "fp64")
+    fresh.build_list(closer[0], xm2, S["hmat"], S["cutskin2"])
+    fref, eref = fresh.energy_force(closer, xm2, S["hmat"])
+    assert np.linalg.norm(f.cpu().numpy() - fref) <= 1e-12 * np.linalg.norm(fref)
+    assert abs(e["vintert"] - eref["vintert"]) <= 1e-11 * abs(eref["vintert"])
+    box.close()
+    fresh.close()
