@@ -434,19 +434,20 @@ int pinyb200_set_tuning(pinyb200_ctx *ctx, const int *choice);
  * launch, captured on the first call and again whenever a device pointer, a
  * cell or the flags change, after one plain run of every box.  When every
  * box is MIXED with the molecule-pair kernel (q-TIP4P/F or q-SPC/Fw site
- * pattern), an orthorhombic cell and the compact PME path, and flags hold
- * neither PINYB200_UPDATE_LIST, PINYB200_SITE_PAIRS nor
+ * pattern), holds identical water molecules (sites O H H or O H H M, one O-H
+ * bond type, one bend, M placed from O H H), has an orthorhombic cell, and
+ * flags hold neither PINYB200_UPDATE_LIST, PINYB200_SITE_PAIRS nor
  * PINYB200_BATCH_BRANCHES, the graph holds multi-box kernels: each phase
- * (staging, PME bin / spread / three FFT passes / gather, pair forces,
- * intramolecular terms, finishing) is one persistent launch per group of
- * boxes sharing its compile-time shape, walking every (box, bead, tile or
- * chunk) block of the group; the groups' PME chains, pair launches and the
- * intramolecular launch are parallel branches of the graph.  Otherwise
- * every box is a parallel branch of its own kernels.  Where the multi-box
- * kernels cover the boxes, the capture times both forms on the call's
- * inputs and keeps the faster, unless flags ask for one form
- * (PINYB200_BATCH_KERNELS or PINYB200_BATCH_BRANCHES).  The call returns when the work is done.  PINY's Python
- * driver reaches several replicas through one energy_control call per CLASS
+ * (staging with records and bins, spread / three FFT passes / gather, pair
+ * forces, finishing) is one persistent launch per group of boxes sharing its
+ * compile-time shape, walking every (box, bead, tile or chunk) block of the
+ * group; the groups' PME chains and pair launches are parallel branches of the
+ * graph.  Otherwise every box is a parallel branch of its own kernels.  Where
+ * the multi-box kernels cover the boxes, the capture times both forms on the
+ * call's inputs and keeps the faster, unless flags ask for one form
+ * (PINYB200_BATCH_KERNELS, which changes nothing where they do not cover the
+ * boxes, or PINYB200_BATCH_BRANCHES).  The call returns when the work is done.
+ * PINY's Python driver reaches several replicas through one energy_control call per CLASS
  * (python/piny/piny.pyx:426-436); this entry point has no counterpart there.
  */
 typedef struct pinyb200_batch pinyb200_batch;
@@ -505,11 +506,17 @@ int pinyb200_grad(pinyb200_ctx *ctx, const double *d_pos, const double *d_xmod,
                   const double *hmat, const double *d_fbar, double *dE,
                   double *dF, void *stream);
 
-/* Milliseconds of the last evaluation, from the kernels' time stamps (boxes of
- * water molecules) or CUDA events (other systems): 0 device work,
- * 1 pair forces, 2 PME, 3 intramolecular, 4 the whole host-buffer call of
- * pinyb200_energy_force (copies included).  PME runs on a second stream of
- * the context, concurrently with 1 and 3, so 1 + 2 + 3 may exceed 0. */
+/* Milliseconds of the last evaluation: 0 device work, 1 pair forces, 2 PME,
+ * 3 intramolecular, 4 the whole host-buffer call of pinyb200_energy_force
+ * (copies included).  PME runs on a second stream of the context, concurrently
+ * with 1 and 3, so 1 + 2 + 3 may exceed 0.
+ * Boxes of identical water molecules take them from time stamps of the
+ * kernels: 0 from the first kernel's start to the last one's end, 2 from the
+ * spread to the gather (grid clear, records and bins belong to the staging
+ * before it), 3 the finishing kernel, which also adds the PME forces,
+ * distributes the ghosts' and writes the forces out.  Other systems take them
+ * from CUDA events: 2 with grid clear and binning, 3 the intramolecular
+ * kernels alone.  The two are not comparable phase by phase. */
 int pinyb200_last_timing(pinyb200_ctx *ctx, float *ms, int n);
 
 /* Per-kernel timing, for measurement.  With on != 0 every later evaluation

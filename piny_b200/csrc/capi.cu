@@ -1110,11 +1110,17 @@ static int water_enqueue(pinyb200_ctx *c, const double *d_pos, const double *d_x
         return e;
     };
     CK(cudaEventRecord(c->ev_fork, c->stream));
-    if (overlap) CK(cudaStreamWaitEvent(pme, c->ev_fork, 0));
-    CK(on(pme, launch_pme_clear));
-    CK(kt_mark(c, "pme_grid_clear (memset)"));
+    if (overlap) {
+        CK(cudaStreamWaitEvent(pme, c->ev_fork, 0));
+        CK(on(pme, launch_pme_clear));
+    }
     CK(launch_water_stage(c, cell, d_pos, d_xmod));
     CK(kt_mark(c, "stage"));
+    if (!overlap) {
+        // on the one stream behind the first kernel's time stamp
+        CK(launch_pme_clear(c));
+        CK(kt_mark(c, "pme_grid_clear (memset)"));
+    }
     CK(cudaEventRecord(c->ev_stage, c->stream));
     if (overlap) CK(cudaStreamWaitEvent(pme, c->ev_stage, 0));
     {
