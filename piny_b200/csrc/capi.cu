@@ -670,7 +670,6 @@ int pinyb200_create(const pinyb200_system *s, int nbeads, int precision, pinyb20
     }
     const size_t nb = (size_t)natm * 3 * nbeads;
     CK(cudaMalloc(&c->d_posT, nb * sizeof(double)));
-    if (precision == PINYB200_MIXED) CK(cudaMalloc(&c->d_offT, nb * sizeof(float)));
     CK(cudaMalloc(&c->d_forceT, nb * sizeof(double)));
     CK(cudaMalloc(&c->d_pos_aos, nb * sizeof(double)));
     CK(cudaMalloc(&c->d_force_aos, nb * sizeof(double)));
@@ -738,6 +737,7 @@ int pinyb200_create(const pinyb200_system *s, int nbeads, int precision, pinyb20
             for (size_t m = 0; m < mstart.size(); m++) strided &= mstart[m] == (int)m * n0;
             c->mol_stride = strided ? n0 : 0;
             if (strided && precision == PINYB200_MIXED) mixed_setup(c, s, n0);
+            if (c->mix_ok) CK(cudaMalloc(&c->d_offT, nb * sizeof(float)));
             if (strided) water_setup(c, s, n0);
         }
     }

@@ -576,6 +576,8 @@ __global__ void __launch_bounds__(FftGeom<N>::CONV_T, fft_blocks<R, N>(FftGeom<N
 
 // The mesh edges built: PINY's 2^a 3^b 5^c sizes that are multiples of 4, from
 // 16 to 128 (set_pme_grid chooses among these).  X(N) for each.
+// FP64 up to 108: a context refuses FP64 meshes above 117 points (pme_plane_smem).
+#define PINYB200_FFT_MAX_FP64 108
 #define PINYB200_FFT_EDGES(X)                                                                                    \
     X(16) X(20) X(24) X(32) X(36) X(40) X(48) X(60) X(64) X(72) X(80) X(96) X(100) X(108) X(120) X(128)
 

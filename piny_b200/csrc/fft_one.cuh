@@ -40,7 +40,11 @@ cudaError_t launch_fft_fixed(pinyb200_ctx *c, int N, int P, const FftArgs &f)
 {
     switch (N) {
 #define PINYB200_FFT_CASE(n) \
-    case n: return launch_fft_n<R, n>(c, P, f);
+    case n:                                                          \
+        if constexpr (sizeof(R) == 4 || n <= PINYB200_FFT_MAX_FP64)  \
+            return launch_fft_n<R, n>(c, P, f);                      \
+        else                                                         \
+            return cudaErrorInvalidValue;
         PINYB200_FFT_EDGES(PINYB200_FFT_CASE)
 #undef PINYB200_FFT_CASE
     default: return cudaErrorInvalidValue;

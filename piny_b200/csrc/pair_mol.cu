@@ -1386,7 +1386,7 @@ struct MixArgs {
 // every box of one model, so a multi-box launch takes them once, outside
 // its per-box table.
 struct MixSite {
-    int ntyp, nuniq, nsplin, stride;
+    int nsplin, stride;
     int toff[16];        // per site pair si * NS + sj: u * nsplin + 2, its rows at nint(t) = 0
     float q2[16];        // charge product of the site pair
     int eflag[16];       // tables the site pair uses: 1 vdW, 2 Coulomb
@@ -2413,8 +2413,6 @@ static MixSite mix_site(const pinyb200_ctx *c)
     const DeviceSystem &s = c->sys;
     MixSite m;
     memset(&m, 0, sizeof(m));
-    m.ntyp = s.ntyp;
-    m.nuniq = s.nuniq;
     m.nsplin = s.nsplin;
     m.stride = c->mol_stride;
     for (int k = 0; k < 16; k++) {

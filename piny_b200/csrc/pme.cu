@@ -41,14 +41,6 @@
 
 namespace pinyb200 {
 
-// Stencil of one charge and bead from the position array.
-__device__ __forceinline__ void stencil_origin(const PmeArgs &a, const Cell &cell, int at, int b, int ni, int &la,
-                                               int &lb, int &lc, double &fa, double &fb, double &fc)
-{
-    stencil_of(a, cell, a.posT[(3 * (size_t)at + 0) * a.P + b], a.posT[(3 * (size_t)at + 1) * a.P + b],
-               a.posT[(3 * (size_t)at + 2) * a.P + b], ni, la, lb, lc, fa, fb, fc);
-}
-
 // Largest value of the order-n cardinal B-spline (PINY's m[] over the
 // fractional offset, ewald3d_pme.c:301-338), sampled finely: a bound for the
 // fixed-point spread.
@@ -394,7 +386,7 @@ __device__ __forceinline__ typename Vec4<R>::T load_frac(const void *rw, int idx
 // Bin kernel of the compact path: one thread per (charge, bead), stencil
 // origin in FP64 with PINY's operation order, record
 // (atom, la, lb, lc) + (fa, fb, fc, q), record number filed under its tile.
-template <typename R, int NI>
+template <typename R>
 __device__ __forceinline__ void pme_bin_compact_body(const PmeArgs &a, const Cell &cell, const TileArgs &t,
                                                      const VBlk vb)
 {
@@ -407,12 +399,12 @@ __device__ __forceinline__ void pme_bin_compact_body(const PmeArgs &a, const Cel
                        a.posT[(3 * (size_t)at + 1) * a.P + b], a.posT[(3 * (size_t)at + 2) * a.P + b]);
 }
 
-template <typename R, int NI>
+template <typename R>
 __global__ void __launch_bounds__(256) pme_bin_compact_kernel(const __grid_constant__ PmeArgs a,
                                                               const __grid_constant__ Cell cell,
                                                               const __grid_constant__ TileArgs t)
 {
-    pme_bin_compact_body<R, NI>(a, cell, t, hw_blk());
+    pme_bin_compact_body<R>(a, cell, t, hw_blk());
 }
 
 // Weights one spread lane needs (lanes = 8 a points x 4 b rows): its a
@@ -487,9 +479,10 @@ __device__ __forceinline__ void spread_warp_global(const PmeArgs &a, R *g, int l
 // bead), one warp per record into a shared copy of the tile, the copy added
 // to the grid once), with the weights evaluated in the block and the next
 // record read ahead.
-template <typename R, int NI, int TT>
+template <int NI, int TT>
 __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileArgs &t, const VBlk vb)
 {
+    typedef float R;
     typedef TileGeom<NI, TT> TG;
     typedef typename Vec4<R>::T R4;
     constexpr int NTB = SpreadW<R, NI>::NTB;
@@ -541,14 +534,12 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
                     for (int i = 0; i < NTB; i++) {
                         if (lb4 + 4 * i >= NI) continue;
                         const int o = off0 + (tc * TG::E + 4 * i) * TG::PA + 8 * s;
-                        {
-                            // fixed point: v 2^S + 1.5 2^23 is exact to the nearest
-                            // integer for |v 2^S| < 2^22, whose bits less those of
-                            // 1.5 2^23 are that integer; integer shared atomics run
-                            // at twice the rate of FP32 ones
-                            const float y = fmaf(cq * w.mb[i], t.qfix, 12582912.0f);
-                            atomicAdd((int *)tl + o, __float_as_int(y) - 0x4B400000);
-                        }
+                        // fixed point: v 2^S + 1.5 2^23 is exact to the nearest
+                        // integer for |v 2^S| < 2^22, whose bits less those of
+                        // 1.5 2^23 are that integer; integer shared atomics run
+                        // at five times the rate of FP32 ones
+                        const float y = fmaf(cq * w.mb[i], t.qfix, 12582912.0f);
+                        atomicAdd((int *)tl + o, __float_as_int(y) - 0x4B400000);
                     }
                 }
             }
@@ -570,7 +561,7 @@ __device__ __forceinline__ void spread_tile_c_body(const PmeArgs &a, const TileA
     }
     __syncthreads();
     constexpr int NROW = TG::E * TG::E;
-    if (sizeof(R) == 4 && (a.Na & 3) == 0) {
+    if ((a.Na & 3) == 0) {
         constexpr int NQ = TG::PA / 4;
         constexpr int RPI = 32 / NQ;
         for (int r0 = warp * RPI; r0 < NROW; r0 += nwarp * RPI) {
@@ -714,12 +705,12 @@ __global__ void __launch_bounds__(256, 2) spread_own_kernel(const __grid_constan
     }
 }
 
-template <typename R, int NI, int TT>
+template <int NI, int TT>
 __global__ void __launch_bounds__(256) spread_tile_c_kernel(const __grid_constant__ PmeArgs a,
                                                             const __grid_constant__ TileArgs t)
 {
     stamp_start(a.stamp, T_PME0);
-    spread_tile_c_body<R, NI, TT>(a, t, hw_blk());
+    spread_tile_c_body<NI, TT>(a, t, hw_blk());
 }
 
 // Gather weights of one record for lane l8 of an 8-lane group: its a
@@ -1422,12 +1413,12 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy, 
         if (err != cudaSuccess) return err;
         const long long nt = (long long)a.nchrg * a.P;
         const int threads = 256;
-        pme_bin_compact_kernel<R, NI><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
+        pme_bin_compact_kernel<R><<<(unsigned)((nt + threads - 1) / threads), threads, 0, c->stream>>>(a, cell, t);
         if ((err = kt_mark(c, "pme_bin")) != cudaSuccess) return err;
     }
     const size_t st = (size_t)TileGeom<NI, TT>::NPT * sizeof(R), ss_spread = spread_smem<R, NI, TT>();
     if (ss_spread > 48 * 1024 - sizeof(PolyTab<R, NI>)) {
-        if constexpr (!f64) err = smem_optin((const void *)spread_tile_c_kernel<R, NI, TT>, (int)ss_spread);
+        if constexpr (!f64) err = smem_optin((const void *)spread_tile_c_kernel<NI, TT>, (int)ss_spread);
         if (err != cudaSuccess) return err;
     }
     if constexpr (f64) {
@@ -1440,7 +1431,7 @@ static cudaError_t launch_pme_t(pinyb200_ctx *c, const Cell &cell, bool energy, 
     }
     const dim3 tgrid((unsigned)t.ntile, (unsigned)(a.P * t.nshare));
     if constexpr (f64) spread_own_kernel<NI, TT><<<tgrid, 256, spread_own_smem<NI, TT>(), c->stream>>>(a, t);
-    else spread_tile_c_kernel<R, NI, TT><<<tgrid, 256, ss_spread, c->stream>>>(a, t);
+    else spread_tile_c_kernel<NI, TT><<<tgrid, 256, ss_spread, c->stream>>>(a, t);
     if ((err = kt_mark(c, "pme_spread")) != cudaSuccess) return err;
     const R *twbase = (const R *)(f64 ? (const void *)c->d_twiddle64 : (const void *)c->d_twiddle32);
     const R *tw[3] = {twbase, twbase + 2 * 256, twbase + 4 * 256};
@@ -1560,10 +1551,10 @@ struct FftBox {
     int energy;
 };
 
-template <typename R, int NI, int TT>
+template <int NI, int TT>
 __global__ void __launch_bounds__(256) spread_batch_kernel(const __grid_constant__ BoxTab<PmeBox> t)
 {
-    PINYB200_BOX_LOOP(t, i, vb, (spread_tile_c_body<R, NI, TT>(t.arg[i].a, t.arg[i].t, vb)));
+    PINYB200_BOX_LOOP(t, i, vb, (spread_tile_c_body<NI, TT>(t.arg[i].a, t.arg[i].t, vb)));
 }
 
 template <typename R, int NI, int TT>
@@ -1614,8 +1605,8 @@ static cudaError_t pme_batch_tiles(const std::vector<PmeBox> &bx, const std::vec
     }
     if (stage == 0) {
         const size_t ss = spread_smem<R, NI, TT>();
-        return launch_tables(tb, (const void *)spread_batch_kernel<R, NI, TT>, 256, ss, sm_count,
-                             [&](const BoxTab<PmeBox> &t, int g) { spread_batch_kernel<R, NI, TT><<<g, 256, ss, st>>>(t); });
+        return launch_tables(tb, (const void *)spread_batch_kernel<NI, TT>, 256, ss, sm_count,
+                             [&](const BoxTab<PmeBox> &t, int g) { spread_batch_kernel<NI, TT><<<g, 256, ss, st>>>(t); });
     }
     const size_t sg = (size_t)TileGeom<NI, TT>::NPT * sizeof(R);
     return launch_tables(tb, (const void *)gather_batch_kernel<R, NI, TT>, 256, sg, sm_count,

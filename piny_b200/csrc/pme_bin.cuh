@@ -35,8 +35,8 @@ __device__ __forceinline__ void scaled(double s, int N, int &i0, double &frac)
 // First grid index per axis of one charge's stencil and the fractional
 // offsets.  PINY's points ia-(j-2), j = 1..n, are the n consecutive indices
 // ia-n+1 .. ia (wrapped), and point j carries weight m[j]; so grid index
-// lo + t (t = 0..n-1) carries m[n - t].  The binning and both tile kernels
-// call this same FP64 code, so they agree on every charge's tile.
+// lo + t (t = 0..n-1) carries m[n - t].  Evaluated once per charge and bead, when
+// its record is written; the tile kernels read the record.
 __device__ __forceinline__ void stencil_of(const PmeArgs &a, const Cell &cell, double x, double y, double z, int ni,
                                            int &la, int &lb, int &lc, double &fa, double &fb, double &fc)
 {

@@ -58,7 +58,8 @@ def test_mesh_edges(oracle, grid):
     spec, S, pos, xmod = _box(water.SPC_FW, 27, 1, grid, 6, edge=12.4, cutoff=5.5)
     assert S["ngrid_a"] == grid
     fref, eref = _oracle(oracle, S, pos, xmod)
-    # FP64 planes above 117 x 117 points do not fit a block's shared memory
+    # a context refuses FP64 meshes above 117 points a side, as before these
+    # transforms: a plane of the run-time-length ones does not fit a block
     for precision in ("fp64", "mixed") if grid <= 108 else ("mixed",):
         f, e = _device(S, pos, xmod, precision)
         _check(precision, f, e, fref, eref)
