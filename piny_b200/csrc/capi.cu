@@ -399,7 +399,8 @@ static void water_setup(pinyb200_ctx *c, const pinyb200_system *s, int n0)
 // with pair type p and table u = inter_map[p], its row offset u * nsplin + 2,
 // charge product and which of the tables (Coulomb, vdW) it reads
 // (force_npol.c:339-375).  Set only when every site pair shares the cutoff
-// and the spline grid; otherwise mix_ok stays false and mol_pair_kernel runs.
+// and the spline grid, and the tables reach the cutoff; otherwise mix_ok stays
+// false and mol_pair_kernel runs.
 static void mixed_setup(pinyb200_ctx *c, const pinyb200_system *s, int n0)
 {
     const int NS = c->mol_ns;
@@ -417,6 +418,8 @@ static void mixed_setup(pinyb200_ctx *c, const pinyb200_system *s, int n0)
             if (s->cutoff[p] != s->cutoff[p0] || s->rmin_spl[u] != s->rmin_spl[u0] ||
                 s->dri_spl[u] != s->dri_spl[u0] || s->dr_spl[u] != s->dr_spl[u0])
                 return;  // not uniform: mol_pair_kernel
+            if (!((s->cutoff[p] - s->rmin_spl[u]) * s->dri_spl[u] < s->nsplin - 5 + 0.49))
+                return;  // past the last knot, which mol_pair_kernel clamps
             bool vdw = false;
             for (size_t k = 0; k < per; k++)
                 vdw |= s->cv0[(size_t)u * per + k] != 0.0 || s->cdv0[(size_t)u * per + k] != 0.0;
@@ -441,7 +444,6 @@ static void mixed_setup(pinyb200_ctx *c, const pinyb200_system *s, int n0)
     c->mix_rc2 = (float)(s->cutoff[p0] * s->cutoff[p0]);
     c->mix_dri = (float)s->dri_spl[u0];
     c->mix_rmd = (float)(s->rmin_spl[u0] * s->dri_spl[u0]);
-    c->mix_tmax = (float)(s->nsplin - 5);
     // force and energy rows of each interval side by side, for the
     // evaluations with energies: [vdW, Coulomb][u][k][force, energy]
     {

@@ -212,7 +212,7 @@ struct pinyb200_ctx {
     int mix_coul_u = -1;  // table whose Coulomb rows every charged pair reads, or -1
     float mix_q2[16] = {0};
     float4 *d_tabfe = nullptr;  // [2][nuniq][nsplin][2] vdW / Coulomb force and energy rows side by side
-    float mix_rc2 = 0, mix_dri = 0, mix_rmd = 0, mix_tmax = 0;
+    float mix_rc2 = 0, mix_dri = 0, mix_rmd = 0;
     bool mol_ok = false;       // the current molecule list matches the site list
     // identical molecules of sites O H H (M) whose bonds, bend, exclusion
     // corrections and M site are water's: the fused staging and finishing serve them

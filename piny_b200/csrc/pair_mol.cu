@@ -1344,7 +1344,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? PINYB200_MOL_BLOCKS32 : 
 //     32 beads' knots scatter over stay few enough for L1;
 //   * the knot nint((r - rmin) dri) (force_npol.c:345-352) is taken with the
 //     1.5 * 2^23 rounding constant instead of float <-> int conversions; below
-//     rmin the first interval's cubic is continued, as PINY's clamped knot does;
+//     rmin the first interval's cubic is continued, as PINY's clamped knot does
+//     (down to r = 0, where the reciprocal square root leaves a NaN that the
+//     maximum with r's or t's least value drops); the cutoff lies within the
+//     tables;
 //   * molecules are uniform runs of sites: the j site index is mj * stride,
 //     not a load.
 // Pairs whose site-0 separation is within twice the molecular extent of half
@@ -1392,7 +1395,7 @@ struct MixSite {
     int eflag[16];       // tables the site pair uses: 1 vdW, 2 Coulomb
     int tstride;         // nuniq * nsplin, the distance between table kinds
     int coul;            // first row of the one Coulomb table
-    float rc2, dri_f, rmd, tmax;  // cutoff^2, 1/dr, rmin/dr, last interval
+    float rc2, dri_f, rmd;  // cutoff^2, 1/dr, rmin/dr
 };
 
 // Resident blocks per SM of the MIXED molecule-pair kernel: 5 x 128
@@ -1416,7 +1419,7 @@ constexpr unsigned kSpcCoul = 0x1FFu, kSpcVdw = 0x1u;       // O H H: all charge
 // each of them), far images site pair by site pair.  The j sites are a loop, so
 // that the main loop keeps its registers.  Pair phase against a second unrolled
 // copy of the main loop with FP32 cell edges: 75 -> 62 us (256 SPC/Fw x 32),
-// 57 -> 44 (216 TIP4P/F x 32), 366 -> 369 (4096 TIP4P/F x 32, no such pairs).
+// 57 -> 44 (216 TIP4P/F x 32), 366 -> 371 (4096 TIP4P/F x 32, no such pairs).
 template <int P, int NS, bool ENERGY>
 __device__ __forceinline__ void mixed_near(const MixArgs &a, const MixSite &m, const Cell &cell, int i0, int j0,
                                            unsigned mask, int b, int lane, bool far, const double *sh0,
@@ -1446,7 +1449,7 @@ __device__ __forceinline__ void mixed_near(const MixArgs &a, const MixSite &m, c
             }
             const float r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
             if (!(r2 < m.rc2)) continue;
-            const float t = fminf(fmaf(r2 * rsqrtf(r2), m.dri_f, -m.rmd), m.tmax);
+            const float t = fmaxf(fmaf(r2 * rsqrtf(r2), m.dri_f, -m.rmd), -m.rmd);
             const int kn = __float2int_rn(fmaxf(t, 0.0f));
             const float del = t - (float)kn;
             const float4 *row = a.tab + (m.toff[sp] + kn), *rfe = a.tabfe + 2 * (m.toff[sp] + kn);
@@ -1536,7 +1539,7 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
     const int sub = lane / G;
     const int b = (lane % G) + 32 * vb.y;  // bead
     const double *__restrict__ posT = a.posT;
-    const float rc2 = m.rc2, dri = m.dri_f, rmd = m.rmd, tmax = m.tmax;
+    const float rc2 = m.rc2, dri = m.dri_f, rmd = m.rmd;
     constexpr float kRound = 12582912.0f;  // 1.5 * 2^23: x + kRound - kRound = nearest integer of x
 
     const double ext2 = ext2_of(a.ext);  // image test margin of this evaluation
@@ -1646,9 +1649,9 @@ __device__ __forceinline__ void mol_pair_mixed_body(const MixArgs &a, const MixS
                         const float rz = dj[sj][2] + ei[si][2];
                         const float r2 = rx * rx + ry * ry + rz * rz;
                         if (r2 < rc2) {
-                            const float r = r2 * rsqrtf(r2);
-                            const float t = fminf(fmaf(r, dri, -rmd), tmax);
-                            const float tr = __fadd_rn(fmaxf(t, 0.0f), kRound);
+                            const float r = fmaxf(r2 * rsqrtf(r2), 0.0f);
+                            const float t = fmaf(r, dri, -rmd);
+                            const float tr = fmaxf(__fadd_rn(t, kRound), kRound);
                             const int kn = __float_as_int(tr) - __float_as_int(kRound);
                             const float del = t - __fsub_rn(tr, kRound);
                             // with energies: the force and energy rows of an interval
@@ -1821,7 +1824,7 @@ __device__ __forceinline__ void grad_near(const MixArgs &a, const MixSite &m, co
         const float r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
         if (!(r2 < m.rc2)) continue;
         const float ri = rsqrtf(r2);
-        const float t = fminf(fmaf(r2 * ri, m.dri_f, -m.rmd), m.tmax);
+        const float t = fmaxf(fmaf(r2 * ri, m.dri_f, -m.rmd), -m.rmd);
         const int kn = __float2int_rn(fmaxf(t, 0.0f));
         const float del = t - (float)kn;
         const float ur = u[0] * r[0] + u[1] * r[1] + u[2] * r[2];
@@ -1958,7 +1961,7 @@ __global__ void __launch_bounds__(128, 4)
                     const float r2 = rx * rx + ry * ry + rz * rz;
                     if (!(r2 < m.rc2)) continue;
                     const float ri = rsqrtf(r2);
-                    const float t = fminf(fmaf(r2 * ri, m.dri_f, -m.rmd), m.tmax);
+                    const float t = fmaxf(fmaf(r2 * ri, m.dri_f, -m.rmd), -m.rmd);
                     const float tr = __fadd_rn(fmaxf(t, 0.0f), kRound);
                     const int kn = __float_as_int(tr) - __float_as_int(kRound);
                     const float del = t - __fsub_rn(tr, kRound);
@@ -2425,7 +2428,6 @@ static MixSite mix_site(const pinyb200_ctx *c)
     m.rc2 = c->mix_rc2;
     m.dri_f = c->mix_dri;
     m.rmd = c->mix_rmd;
-    m.tmax = c->mix_tmax;
     return m;
 }
 
