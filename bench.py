@@ -1287,6 +1287,8 @@ def main():
     # roofline of the dominant kernel by serialised time; its duration is
     # the one measured inside the timed steps (pair phase / PME phase)
     hbm, peak_kind = peaks()
+    # phases as pinyb200_last_timing gives them: for water boxes "intra" is the
+    # finishing kernel (intramolecular terms, force sum, output), "pme" spread to gather
     names = ["total", "pair", "pme", "intra"]
     dom_k = max(kernels, key=lambda k: k["ms"])
     pme_ms = sum(k["ms"] for k in kernels if k["kernel"].startswith("pme_"))

@@ -145,7 +145,8 @@ struct GradPairArgs {
 // sums stay in registers.  Bound: FP64 separations and conversions, and the
 // L2 reads of positions and u.  1024 TIP4P/F x 16 beads, FP32: 405 us (2164
 // as one thread per (row, bead) with a loop over all channels per pair).
-// Serves FP64 and systems without the MIXED molecule-pair kernel.
+// Serves FP64, systems without the MIXED molecule-pair kernel and passes whose
+// table tangents reach beyond the site pairs with a vdW term.
 template <typename R>
 __global__ void __launch_bounds__(128) grad_pair_kernel(const __grid_constant__ GradPairArgs a,
                                                         const __grid_constant__ GradPairSel c,

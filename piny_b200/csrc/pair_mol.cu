@@ -1869,7 +1869,8 @@ __device__ __forceinline__ void grad_near(const MixArgs &a, const MixSite &m, co
 // u is formed as r is, from the first sites' FP64 values (a large common part of
 // the upstream gradient cancels); w and tq are FP64 differences and products,
 // rounded once.  The terms of one j site are summed in FP32, everything beyond
-// them in FP64.  No forces, so no atomics but a block's seven sums.
+// them in FP64.  No forces, so no atomics but a block's seven sums.  101 us at
+// 1024 TIP4P/F x 16 beads (405 as a warp per site row, grad_pair_kernel).
 template <int P, int NS, unsigned CM, unsigned VM>
 __global__ void __launch_bounds__(128, 4)
     mol_pair_grad_kernel(const __grid_constant__ MixArgs a, const __grid_constant__ MixSite m,

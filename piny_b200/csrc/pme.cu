@@ -1980,7 +1980,7 @@ __device__ __forceinline__ void adjoint_hessian(PHI phi, const Piece<R, NI <= 8 
 // memory (phi, then chi in its place), 8 lanes a record.  The contraction is
 // linear, so each potential's terms are added on their own.  Bound:
 // shared-memory reads, 128 a record and lane.  1024 TIP4P/F x 16 beads, 32^3,
-// FP32: 277 us as one thread per record reading global memory.
+// FP32: 277 us as one thread per record reading global memory, 127 here.
 template <typename R, int NI, int TT>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 && NI <= 8 ? 2 : 1) pme_adjoint_gather_kernel(const __grid_constant__ PmeArgs a,
                                                                  const __grid_constant__ Cell cell,
