@@ -1420,6 +1420,9 @@ constexpr unsigned kSpcCoul = 0x1FFu, kSpcVdw = 0x1u;       // O H H: all charge
 // that the main loop keeps its registers.  Pair phase against a second unrolled
 // copy of the main loop with FP32 cell edges: 75 -> 62 us (256 SPC/Fw x 32),
 // 57 -> 44 (216 TIP4P/F x 32), 366 -> 371 (4096 TIP4P/F x 32, no such pairs).
+// Whole calls of small boxes, same two forms: 206 -> 181 us (230 SPC/Fw x 64),
+// 83 -> 92 (260 SPC/Fw x 8: too few warps to hide the loop's chain of loads; all
+// separations of a j site first, or its rows prefetched to L1, were no faster).
 template <int P, int NS, bool ENERGY>
 __device__ __forceinline__ void mixed_near(const MixArgs &a, const MixSite &m, const Cell &cell, int i0, int j0,
                                            unsigned mask, int b, int lane, bool far, const double *sh0,
